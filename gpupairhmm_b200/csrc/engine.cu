@@ -2,16 +2,16 @@
 // per-batch launch sequence and its CUDA-graph replay.
 //
 // Launch sequence of one batch (all on one stream, replayed as one graph):
-//   pack_reads / pack_haps      caller SoA -> packed HBM layout
+//   pack                        caller SoA -> packed HBM layout; the batch's fills
 //   bin_count, hist_scan,
-//   schedule, bin_scatter       sorted work list + per-bucket task ranges
+//   bin_scatter                 sorted work list
 //   fp32_bucket_kernel<G,R,MT>  one launch per non-empty length bucket
 //   fp64_rescue_kernel<scaled>  pairs flagged by the FP32 pass, in doubles
 //   fp64_rescue_kernel<ext>     the few beyond the scaled doubles' range
 // Compared with the reference executor (gpuworker.cuh:559-973) there is no
 // device-to-host synchronisation inside a batch: the host derives bucket sizes
-// from the record structure it already holds, and the kernels read their task
-// ranges from device memory.
+// and every bucket's range of work items from the record structure it already
+// holds.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -109,11 +109,11 @@ Engine::Engine(const pairhmm_options_t& opts) : opts_(opts) {
 }
 
 std::vector<DevBuf*> Engine::all_buffers() {
-    return {&ph2pr_, &rules_maxlen_, &rules_rank_, &per_task_, &config_, &in_read_bases_, &in_bq_,
+    return {&ph2pr_, &rules_rank_, &in_read_bases_, &in_bq_,
             &in_iq_, &in_dq_, &in_read_off_, &in_read_len_, &in_hap_bases_, &in_hap_off_, &in_hap_len_,
             &read_record_, &read_local_, &rec_haps_, &rec_hap_base_, &rec_pair_base_, &read_start_,
             &hap_start_, &read_pack_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
-            &sched_, &scores_, &scratch_, &lens_tmp_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
+            &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
             &rescue_ext_, &rsort_,
             &in_gq_, &read_gcp_};
 }
@@ -222,7 +222,6 @@ pairhmm_status_t Engine::init() {
     PHMM_CUDA(counters_.ensure(sizeof(unsigned long long) * kCtrTotal));
     // FP64 list sort: per-class histogram (uint32) then cursors (uint64)
     PHMM_CUDA(rsort_.ensure((sizeof(unsigned int) + sizeof(unsigned long long)) * kFp64Classes * kRescueHBins));
-    PHMM_CUDA(sched_.ensure(sizeof(Schedule)));
     ready_ = true;
     return upload_rules();
 }
@@ -255,26 +254,15 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
 pairhmm_status_t Engine::upload_rules() {
     const int nb = (int)rules_.size();
     rule_cfg_.assign(nb, nullptr);
-    std::vector<int32_t> maxlen(nb), rank(nb), per(nb), cfg(nb);
+    std::vector<int32_t> rank(nb);
     for (int b = 0; b < nb; ++b) {
         rule_cfg_[b] =
             find_fp32_config(rules_[b].G, rules_[b].R, rules_[b].multi_tile, rules_[b].packed, opts_.gcp != 0);
         if (!rule_cfg_[b]) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile rule without compiled kernel");
-        maxlen[b] = rules_[b].max_len;
         rank[b] = opts_.mode == PAIRHMM_MODE_PLAIN ? b : nb - 1 - b;
     }
-    for (int b = 0; b < nb; ++b) {
-        per[rank[b]] = rule_cfg_[b]->per_warp();
-        cfg[rank[b]] = b;
-    }
-    PHMM_CUDA(rules_maxlen_.ensure(sizeof(int32_t) * nb));
     PHMM_CUDA(rules_rank_.ensure(sizeof(int32_t) * nb));
-    PHMM_CUDA(per_task_.ensure(sizeof(int32_t) * nb));
-    PHMM_CUDA(config_.ensure(sizeof(int32_t) * nb));
-    PHMM_CUDA(cudaMemcpy(rules_maxlen_.ptr, maxlen.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice));
     PHMM_CUDA(cudaMemcpy(rules_rank_.ptr, rank.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice));
-    PHMM_CUDA(cudaMemcpy(per_task_.ptr, per.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice));
-    PHMM_CUDA(cudaMemcpy(config_.ptr, cfg.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice));
     return PAIRHMM_OK;
 }
 
@@ -537,7 +525,7 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(hap_start_.ensure(8 * nh));
     PHMM_CUDA(read_pack_.ensure(4 * (x.pack_positions + kReadSlackPos)));
     PHMM_CUDA(hap_code_.ensure(x.code_bytes + kHapSlack));
-    const int64_t nbins = (int64_t)rules_.size() * (opts_.mode == PAIRHMM_MODE_PLAIN ? 1 : kHBins);
+    const int64_t nbins = (int64_t)rules_.size() * hbins_of(x);
     PHMM_CUDA(hist_.ensure(4 * nbins));
     PHMM_CUDA(cursor_.ensure(8 * nbins));
     PHMM_CUDA(items_.ensure(sizeof(Item) * np));
@@ -563,6 +551,11 @@ pairhmm_status_t Engine::upload_index(const BatchIndex& x, cudaStream_t s) {
     };
     PHMM_CUDA(uploader_.run(opts_.device, copies, s));
     return PAIRHMM_OK;
+}
+
+// haplotype-length classes of a batch's work list (prep_kernels.cuh)
+int64_t Engine::hbins_of(const BatchIndex& x) const {
+    return opts_.mode == PAIRHMM_MODE_PLAIN ? 4 : round_up((int64_t)std::min(kHBins - 1, x.max_hap_len) + 1, 4);
 }
 
 int64_t Engine::index_bytes(const BatchIndex& x) {
@@ -611,20 +604,20 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     if (stage == 0) {
     launches_ = 0;
     fp32_launches_ = 0;
-    // zero the histogram and the work/rescue counters, pad the haplotype codes
-    // (a kernel, not memset nodes: see launch_fill)
-    {
-        uint8_t* const ptr[4] = {hap_code_.as<uint8_t>() + x.code_bytes, hist_.as<uint8_t>(),
-                                 counters_.as<uint8_t>(), rsort_.as<uint8_t>()};
-        const long long bytes[4] = {kHapSlack, (long long)sizeof(unsigned int) * nb * (plain ? 1 : kHBins),
-                                    (long long)sizeof(unsigned long long) * kCtrTotal,
-                                    (long long)sizeof(unsigned int) * kFp64Classes * kRescueHBins};
-        const int value[4] = {4, 0, 0, 0};
-        PHMM_CUDA(launch_fill(ptr, bytes, value, 4, s));
-        launches_ += 1;
-    }
-    PHMM_CUDA(launch_pack(pa, prep_grid, s));
-    launches_ += 2;
+    // zero the histogram and the work/rescue counters, pad the haplotype codes, and
+    // pack the inputs, in one launch
+    FillArgs fa{};
+    fa.ptr[0] = reinterpret_cast<uint32_t*>(hap_code_.as<uint8_t>() + x.code_bytes);  // 16-byte aligned
+    fa.words[0] = kHapSlack / 4;
+    fa.value[0] = 0x04040404u;
+    fa.ptr[1] = hist_.as<uint32_t>();
+    fa.words[1] = (long long)nb * hbins_of(x);
+    fa.ptr[2] = counters_.as<uint32_t>();
+    fa.words[2] = 2 * kCtrTotal;
+    fa.ptr[3] = rsort_.as<uint32_t>();
+    fa.words[3] = kFp64Classes * kRescueHBins;
+    PHMM_CUDA(launch_pack(pa, fa, prep_grid, s));
+    launches_ += 1;
     }
 
     BinArgs ba{};
@@ -639,14 +632,17 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     ba.unit_bucket = unit_bucket_.as<int32_t>();
     ba.num_units = (int64_t)x.unit_read0.size();
     ba.nbuckets = nb;
-    ba.hbins = plain ? 1 : kHBins;
+    ba.hcap = plain ? 0 : std::min(kHBins - 1, x.max_hap_len);
+    ba.hbins = (int)hbins_of(x);
+    for (int rank = 0; rank < nb; ++rank)
+        ba.ranks.begin[rank + 1] = ba.ranks.begin[rank] + x.bucket_items[plain ? rank : nb - 1 - rank];
     ba.bucket_rank = rules_rank_.as<int32_t>();
     ba.hist = hist_.as<unsigned int>();
     ba.cursor = cursor_.as<unsigned long long>();
     ba.items = items_.as<Item>();
     if (stage == 0) {
-    PHMM_CUDA(launch_binning(ba, prep_grid, s, per_task_.as<int>(), config_.as<int>(), sched_.as<Schedule>(), nb));
-    launches_ += 4;
+    PHMM_CUDA(launch_binning(ba, prep_grid, s));
+    launches_ += 3;
     return PAIRHMM_OK;
     }
 
@@ -702,9 +698,8 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
             const ConfigInfo* c = rule_cfg_[b];
             Fp32LaunchArgs la{};
             la.view = v;
-            la.items = items_.as<Item>();
-            la.sched = sched_.as<Schedule>();
-            la.rank = rank;
+            la.items = items_.as<Item>() + ba.ranks.begin[rank];
+            la.num_items = x.bucket_items[b];
             la.persistent = plan.persistent[b];
             la.counter = counters + rank;
             la.scratch = static_cast<char*>(scratch_.ptr) + plan.scratch_off[b];

@@ -121,6 +121,7 @@ private:
     pairhmm_status_t upload_index(const BatchIndex& idx, cudaStream_t s);
     int persistent_grid(const void* kernel, size_t smem) const;
     static int64_t index_bytes(const BatchIndex& x);
+    int64_t hbins_of(const BatchIndex& x) const;
 
     pairhmm_options_t opts_;
     std::vector<TileRule> rules_;
@@ -141,14 +142,14 @@ private:
     std::string last_error_;
 
     // device buffers
-    DevBuf ph2pr_, rules_maxlen_, rules_rank_, per_task_, config_;
+    DevBuf ph2pr_, rules_rank_;
     DevBuf in_read_bases_, in_bq_, in_iq_, in_dq_, in_read_off_, in_read_len_;
     DevBuf in_gq_, read_gcp_;  // gcp mode: uploaded gcp qualities, per-read gcp
     DevBuf in_hap_bases_, in_hap_off_, in_hap_len_;
     DevBuf read_record_, read_local_, rec_haps_, rec_hap_base_, rec_pair_base_, read_start_, hap_start_;
     DevBuf unit_read0_, unit_read1_, unit_bucket_;
-    DevBuf read_pack_, hap_code_, hist_, cursor_, items_, rescue_, counters_, sched_, scores_, scratch_;
-    DevBuf lens_tmp_, rescue_off_, rescue_ext_, rsort_;
+    DevBuf read_pack_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
+    DevBuf rescue_off_, rescue_ext_, rsort_;
     // host-to-device uploads (caller inputs, index) and the reused index
     HostUploader uploader_;
     BatchIndex idx_;

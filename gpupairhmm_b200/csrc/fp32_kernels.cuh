@@ -26,8 +26,8 @@ constexpr int fp32_min_ctas(int R, bool MT, bool PK) {
 
 template <int G, int R, bool MT, bool PK, bool GCP = false>
 __global__ void __launch_bounds__(kBlockThreads, fp32_min_ctas(R, MT, PK))
-fp32_bucket_kernel(DevView v, const Item* __restrict__ items, const Schedule* __restrict__ s, int rank,
-                   int persistent, unsigned long long* counter, float4* scratch, int64_t rows) {
+fp32_bucket_kernel(DevView v, const Item* __restrict__ items, long long num_items, int persistent,
+                   unsigned long long* counter, float4* scratch, int64_t rows) {
     static_assert(!(MT && PK), "the packed kernel is single tile");
     static_assert(!(GCP && PK), "gcp mode runs the scalar kernel");
     using W = WavefrontOf<G, R, MT, PK, GCP>;
@@ -39,10 +39,8 @@ fp32_bucket_kernel(DevView v, const Item* __restrict__ items, const Schedule* __
     for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = v.ph2pr[i];
     __syncthreads();
 
-    const long long ib = s->item_begin[rank];
-    const long long ie = s->item_begin[rank + 1];
     const int per = W::NG;
-    const long long ntasks = (ie - ib + per - 1) / per;
+    const long long ntasks = (num_items + per - 1) / per;
     const long long gwarp = (long long)blockIdx.x * kWarpsPerBlock + warp;
     float4* wscratch = MT ? scratch + gwarp * (long long)per * 2 * rows : nullptr;
 
@@ -54,8 +52,8 @@ fp32_bucket_kernel(DevView v, const Item* __restrict__ items, const Schedule* __
             tsk = (long long)__shfl_sync(kFullMask, x, 0);
         }
         if (tsk >= ntasks) break;
-        const long long first = ib + tsk * per;
-        const int n = (int)((ie - first) < per ? (ie - first) : per);
+        const long long first = tsk * per;
+        const int n = (int)((num_items - first) < per ? (num_items - first) : per);
         if constexpr (PK) W::run(v, items + first, n, wtab, ph);
         else W::run(v, items + first, n, wtab, ph, wscratch, rows);
         if (!persistent) break;
@@ -67,7 +65,7 @@ cudaError_t launch_fp32_bucket(const Fp32LaunchArgs& a) {
     using W = WavefrontOf<G, R, MT, PK, GCP>;
     const size_t smem = (32 + (size_t)kWarpsPerBlock * W::kTableFloat4) * sizeof(float4);
     fp32_bucket_kernel<G, R, MT, PK, GCP><<<a.grid, kBlockThreads, smem, a.stream>>>(
-        a.view, a.items, a.sched, a.rank, a.persistent, a.counter, static_cast<float4*>(a.scratch), a.rows);
+        a.view, a.items, a.num_items, a.persistent, a.counter, static_cast<float4*>(a.scratch), a.rows);
     return cudaGetLastError();
 }
 

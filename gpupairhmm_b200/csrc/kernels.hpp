@@ -17,9 +17,8 @@ constexpr int kWarpsPerBlock = kBlockThreads / 32;
 
 struct Fp32LaunchArgs {
     DevView view;
-    const Item* items;
-    const Schedule* sched;
-    int rank;                       // bucket rank this launch serves
+    const Item* items;              // the bucket's first work item
+    long long num_items;
     int persistent;                 // 1: warps loop on an atomic task counter
     unsigned long long* counter;    // per-rank task counter (persistent)
     void* scratch;                  // multi-tile border storage
@@ -72,14 +71,11 @@ size_t fp64_scratch_bytes_per_row(int cls, bool ext);  // per warp, per border r
 const void* fp64_kernel(int cls, bool gcp, bool ext, bool fuse = false);
 int fp64_per_warp(int cls);
 
-// Preparation kernels.
-cudaError_t launch_pack(const PrepArgs& a, int grid, cudaStream_t s);
-// byte fills of n <= kFillRanges device ranges in one kernel launch
-cudaError_t launch_fill(uint8_t* const* ptr, const long long* bytes, const int* value, int n, cudaStream_t s);
+// Preparation kernels.  The pack launch also runs the batch's fills.
+cudaError_t launch_pack(const PrepArgs& a, const FillArgs& f, int grid, cudaStream_t s);
 // FP64 class lists sorted by haplotype length (count, scan, scatter)
 cudaError_t launch_rescue_sort(const RescueSortArgs& a, int grid, cudaStream_t s);
-cudaError_t launch_binning(BinArgs a, int grid, cudaStream_t s, const int* per_task_dev,
-                           const int* config_dev, Schedule* sched, int nranks);
+cudaError_t launch_binning(const BinArgs& a, int grid, cudaStream_t s);
 
 // FP32 FFMA throughput probe used to measure the roofline denominator:
 // `iters` dependent-chain-free FMAs per thread over grid x 256 threads.

@@ -195,30 +195,18 @@ cudaError_t launch_fp64_rescue(const Fp64LaunchArgs& a) {
 }
 
 // ---------------------------------------------------------------- preparation
-cudaError_t launch_pack(const PrepArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_pack(const PrepArgs& a, const FillArgs& f, int grid, cudaStream_t s) {
     // a warp per read / haplotype with every warp resident at once where the batch
     // allows: each warp's work is short, so latency is hidden by warps in flight
     auto warps_grid = [&](int64_t n) {
         const int64_t g = (n + 7) / 8;  // 8 warps per 256-thread block
-        return (int)std::max<int64_t>(grid, std::min<int64_t>(g, int64_t(1) << 20));
+        return (int)std::max<int64_t>(1, std::min<int64_t>(g, int64_t(1) << 20));
     };
-    pack_reads_kernel<<<warps_grid(a.num_reads), 256, 0, s>>>(a);
-    pack_haps_kernel<<<warps_grid(a.num_haps), 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fill(uint8_t* const* ptr, const long long* bytes, const int* value, int n, cudaStream_t s) {
-    FillArgs a{};
     long long most = 0;
-    for (int k = 0; k < kFillRanges; ++k) {
-        a.ptr[k] = k < n ? ptr[k] : nullptr;
-        a.bytes[k] = k < n ? bytes[k] : 0;
-        a.value[k] = k < n ? value[k] : 0;
-        most = a.bytes[k] > most ? a.bytes[k] : most;
-    }
-    if (most == 0) return cudaSuccess;
-    const long long blocks = (most + 255) / 256;
-    fill_kernel<<<(int)(blocks < 1024 ? blocks : 1024), 256, 0, s>>>(a);
+    for (long long w : f.words) most = std::max(most, w);
+    const int fill_blocks = (int)std::max<long long>(1, std::min<long long>((most + 1023) / 1024, grid));
+    const int read_blocks = warps_grid(a.num_reads), hap_blocks = warps_grid(a.num_haps);
+    pack_kernel<<<fill_blocks + read_blocks + hap_blocks, 256, 0, s>>>(a, f, fill_blocks, read_blocks);
     return cudaGetLastError();
 }
 
@@ -229,13 +217,11 @@ cudaError_t launch_rescue_sort(const RescueSortArgs& a, int grid, cudaStream_t s
     return cudaGetLastError();
 }
 
-cudaError_t launch_binning(BinArgs a, int grid, cudaStream_t s, const int* per_task_dev,
-                           const int* config_dev, Schedule* sched, int nranks) {
-    const int nbins = a.nbuckets * a.hbins;
-    bin_count_kernel<<<grid, 256, 0, s>>>(a);
-    hist_scan_kernel<<<1, kHistScanThreads, 0, s>>>(a.hist, a.cursor, nbins);
-    schedule_kernel<<<1, 32, 0, s>>>(a.cursor, a.hist, nranks, a.hbins, per_task_dev, config_dev, sched);
-    bin_scatter_kernel<<<grid, 256, 0, s>>>(a);
+cudaError_t launch_binning(const BinArgs& a, int grid, cudaStream_t s) {
+    const int units_grid = (int)std::max<int64_t>(1, std::min<int64_t>((a.num_units + 255) / 256, grid));
+    bin_count_kernel<<<units_grid, 256, 0, s>>>(a);
+    hist_scan_kernel<<<a.nbuckets, kHistScanThreads, 0, s>>>(a.hist, a.cursor, a.hbins, a.ranks);
+    bin_scatter_kernel<<<units_grid, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -3,11 +3,12 @@
 //
 // Work list: every item (a unit of one or two reads of a record, placed in a
 // length bucket by the host, against one haplotype) gets a bin
-// (bucket rank, 4095 - min(H, 4095)) so that an exclusive scan over bins
-// followed by an atomic scatter sorts the items by tile bucket (largest tiles
-// first) and, inside a bucket, by haplotype length descending.  Warps of the persistent kernel then take consecutive items, so
-// the groups of a warp have nearly equal haplotype lengths (little idle work)
-// and the longest pairs start first (short tail).  The order of pairs with the
+// (bucket rank, cap - min(H, cap)), cap the batch's longest haplotype or 4095, so
+// that an exclusive scan over each rank's bins followed by an atomic scatter
+// sorts the items by tile bucket (largest tiles first) and, inside a bucket, by
+// haplotype length descending.  Warps of the persistent kernel then take
+// consecutive items, so the groups of a warp have nearly equal haplotype lengths
+// (little idle work) and the longest pairs start first (short tail).  The order of pairs with the
 // same bin is not deterministic; each pair still writes its own output slot,
 // so results are.
 #pragma once
@@ -16,7 +17,7 @@
 
 namespace phmm {
 
-constexpr int kHBins = 4096;     // haplotype-length classes per bucket
+constexpr int kHBins = 4096;     // most haplotype-length classes per bucket
 constexpr int kMaxBuckets = 48;
 
 struct PrepArgs {
@@ -47,6 +48,16 @@ struct PrepArgs {
     uint8_t* read_gcp;              // [num_reads], gcp mode only (else null)
 };
 
+// Byte fills of up to kFillRanges device ranges (4-byte aligned, whole words) by
+// the pack kernel's first blocks.  Not memset nodes: a copy engine may run those,
+// where they queue behind other streams' pending copies.
+constexpr int kFillRanges = 4;
+struct FillArgs {
+    uint32_t* ptr[kFillRanges];
+    long long words[kFillRanges];
+    uint32_t value[kFillRanges];
+};
+
 #ifdef PHMM_PREP_KERNELS_IMPL
 __device__ __forceinline__ uint32_t pack_position(uint32_t base, uint32_t bq, uint32_t iq, uint32_t dq) {
     bq = bq > 127u ? 127u : bq;
@@ -55,13 +66,17 @@ __device__ __forceinline__ uint32_t pack_position(uint32_t base, uint32_t bq, ui
     return code_of((uint8_t)base) | (bq << 8) | (iq << 16) | (dq << 24);
 }
 
+// One launch prepares a batch's arrays: the first fill_blocks blocks fill, the
+// next read_blocks pack reads, the rest pack haplotypes.  As three launches the
+// stage's chain was two launch gaps longer, which is most of the time of a call
+// of one small region (see hist_scan_kernel for the stage's figures).
 // Warp per read; a lane packs 4 consecutive positions and stores them as one
 // 16-byte word group.  Where the four source arrays are 4-byte aligned at the
 // read's offset, whole groups inside the read are read with one 4-byte load
 // per array; the read's ragged end (and unaligned sources) go byte by byte.
-__global__ void pack_reads_kernel(PrepArgs a) {
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int64_t nblocks) {
+    const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = (nblocks * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     for (int64_t i = warp; i < a.num_reads; i += nwarps) {
         const int L = a.read_lengths[i];
@@ -103,9 +118,9 @@ __global__ void pack_reads_kernel(PrepArgs a) {
 // where the source is 4-byte aligned and the 16 positions are inside the
 // haplotype) and stores them as one 16-byte word; the padding to 16 bytes is
 // code 4.
-__global__ void pack_haps_kernel(PrepArgs a) {
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void pack_haps(const PrepArgs& a, int64_t block, int64_t nblocks) {
+    const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = (nblocks * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
     for (int64_t i = warp; i < a.num_haps; i += nwarps) {
         const int H = a.hap_lengths[i];
@@ -139,7 +154,27 @@ __global__ void pack_haps_kernel(PrepArgs a) {
     }
 }
 
+__global__ void __launch_bounds__(256)
+pack_kernel(PrepArgs a, FillArgs f, int fill_blocks, int read_blocks) {
+    const int b = blockIdx.x;
+    if (b < fill_blocks) {
+        for (int k = 0; k < kFillRanges; ++k)
+            for (long long i = (long long)b * blockDim.x + threadIdx.x; i < f.words[k];
+                 i += (long long)fill_blocks * blockDim.x)
+                f.ptr[k][i] = f.value[k];
+    } else if (b < fill_blocks + read_blocks) {
+        pack_reads(a, b - fill_blocks, read_blocks);
+    } else {
+        pack_haps(a, b - fill_blocks - read_blocks, gridDim.x - fill_blocks - read_blocks);
+    }
+}
+
 #endif  // PHMM_PREP_KERNELS_IMPL
+
+// First work item of every bucket rank (and the end of the last), known to the host.
+struct RankItems {
+    long long begin[kMaxBuckets + 1];
+};
 
 struct BinArgs {
     const int32_t* hap_lengths;
@@ -153,16 +188,17 @@ struct BinArgs {
     const int32_t* unit_bucket;     // [num_units]
     int64_t num_units;
     int nbuckets;
-    int hbins;                      // kHBins (engine) or 1 (plain)
+    int hcap;                       // longest haplotype class (0: all in one class, the plain form)
+    int hbins;                      // haplotype-length classes per bucket: hcap + 1, up to a multiple of 4
     const int32_t* bucket_rank;     // [nbuckets] bin-major position of each bucket
     unsigned int* hist;             // [nbuckets * hbins]
     unsigned long long* cursor;     // [nbuckets * hbins] scatter positions
+    RankItems ranks;
     Item* items;
 };
 
 __device__ __forceinline__ int bin_of(const BinArgs& a, int bucket, int H) {
-    const int hc = a.hbins > 1 ? (a.hbins - 1 - (H < a.hbins - 1 ? H : a.hbins - 1)) : 0;
-    return a.bucket_rank[bucket] * a.hbins + hc;
+    return a.bucket_rank[bucket] * a.hbins + a.hcap - (H < a.hcap ? H : a.hcap);
 }
 
 #ifdef PHMM_PREP_KERNELS_IMPL
@@ -213,80 +249,52 @@ __global__ void bin_scatter_kernel(BinArgs a) {
     }
 }
 
-// Byte fills of up to kFillRanges device ranges in one launch.  Used instead of
-// cudaMemsetAsync inside the captured stages: a memset node may be run by a
-// copy engine, where it queues behind other streams' pending copies.
-constexpr int kFillRanges = 4;
-struct FillArgs {
-    uint8_t* ptr[kFillRanges];
-    long long bytes[kFillRanges];
-    int value[kFillRanges];
-};
-__global__ void fill_kernel(FillArgs a) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (int k = 0; k < kFillRanges; ++k)
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.bytes[k]; i += stride)
-            a.ptr[k][i] = (uint8_t)a.value[k];
-}
-
-// single-block exclusive scan of the histogram into cursor (n up to a few 1e5).
-// The block is kept small (kHistScanThreads) so that it finds room on an SM
-// next to the long-running blocks of another engine's kernels.
+// Exclusive scan of the histogram into cursor: block r scans the hbins bins of
+// rank r from the rank's first item, which the host knows (it counts every
+// bucket's items).  kHistScanThreads threads take 4 bins each per round, so loads
+// and stores are whole 16- and 32-byte words; the block is small enough to find
+// room on an SM next to the long-running blocks of another engine's kernels.
+// One block over all ranks' 4,096 bins, 432 bins a thread, was most of the stage:
+// 0.21 ms a call whatever the batch, now 0.03 ms (one region of 32 x 4 pairs).
 constexpr int kHistScanThreads = 256;
 __global__ void __launch_bounds__(kHistScanThreads)
-hist_scan_kernel(const unsigned int* hist, unsigned long long* cursor, int n) {
-    __shared__ unsigned long long part[kHistScanThreads];
-    const int tid = threadIdx.x;
-    const int per = (n + blockDim.x - 1) / blockDim.x;
-    const int b = tid * per;
-    const int e = b + per < n ? b + per : n;
-    unsigned long long s = 0;
-    for (int i = b; i < e; ++i) s += hist[i];
-    part[tid] = s;
-    __syncthreads();
-    if (tid == 0) {
-        unsigned long long run = 0;
-        for (int i = 0; i < (int)blockDim.x; ++i) { const unsigned long long x = part[i]; part[i] = run; run += x; }
+hist_scan_kernel(const unsigned int* hist, unsigned long long* cursor, int hbins, RankItems items) {
+    __shared__ unsigned int wsum[kHistScanThreads / 32];
+    const int rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (items.begin[rank] == items.begin[rank + 1]) return;
+    const unsigned int* h = hist + (long long)rank * hbins;
+    unsigned long long* cur = cursor + (long long)rank * hbins;
+    unsigned long long base = (unsigned long long)items.begin[rank];
+    for (int b0 = 0; b0 < hbins; b0 += 4 * kHistScanThreads) {  // hbins is a multiple of 4
+        const int b = b0 + 4 * tid;
+        uint4 n = make_uint4(0u, 0u, 0u, 0u);
+        if (b < hbins) n = *reinterpret_cast<const uint4*>(h + b);
+        const unsigned int mine = n.x + n.y + n.z + n.w;
+        unsigned int incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned int y = __shfl_up_sync(kFullMask, incl, d);
+            if (lane >= d) incl += y;
+        }
+        __syncthreads();  // the previous round's sums are read
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        unsigned int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kHistScanThreads / 32; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (b < hbins) {
+            const unsigned long long c0 = base + before + incl - mine;
+            ulonglong2* out = reinterpret_cast<ulonglong2*>(cur + b);
+            out[0] = make_ulonglong2(c0, c0 + n.x);
+            out[1] = make_ulonglong2(c0 + n.x + n.y, c0 + n.x + n.y + n.z);
+        }
+        base += all;
     }
-    __syncthreads();
-    unsigned long long run = part[tid];
-    for (int i = b; i < e; ++i) { cursor[i] = run; run += hist[i]; }
 }
 
-#endif  // PHMM_PREP_KERNELS_IMPL
-
-// Per-rank item ranges and warp-task ranges for the persistent kernel.
-struct Schedule {
-    int nranks;
-    int total_tasks_hi;                       // unused padding
-    long long total_tasks;
-    long long item_begin[kMaxBuckets + 1];    // by rank
-    long long task_begin[kMaxBuckets + 1];    // by rank
-    int per_task[kMaxBuckets];                // items per warp task, by rank
-    int config[kMaxBuckets];                  // kernel config id, by rank
-};
-
-#ifdef PHMM_PREP_KERNELS_IMPL
-// one thread: cursor holds bin starts (before scatter); derive the schedule
-__global__ void schedule_kernel(const unsigned long long* bin_start, const unsigned int* hist, int nranks,
-                                int hbins, const int* per_task, const int* config, Schedule* s) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    long long tasks = 0;
-    s->nranks = nranks;
-    for (int r = 0; r < nranks; ++r) {
-        const long long b0 = (long long)bin_start[r * hbins];
-        const long long last = (long long)bin_start[(r + 1) * hbins - 1] + hist[(r + 1) * hbins - 1];
-        s->item_begin[r] = b0;
-        s->task_begin[r] = tasks;
-        s->per_task[r] = per_task[r];
-        s->config[r] = config[r];
-        const long long n = last - b0;
-        tasks += (n + per_task[r] - 1) / per_task[r];
-        if (r == nranks - 1) s->item_begin[nranks] = last;
-    }
-    s->task_begin[nranks] = tasks;
-    s->total_tasks = tasks;
-}
 #endif  // PHMM_PREP_KERNELS_IMPL
 
 // ---------------------------------------------------------------- FP64 list order
