@@ -408,7 +408,7 @@ def run_serving(args, local_rank):
 
     eng = g.Engine(device=local_rank)
     # regions with a read beyond the longest single tile run on the multi-tile slots
-    single_max = max(m for m, _, _, kind in eng.tile_table() if kind != 1)
+    single_max = max(m for m, _, _, kind in eng.tile_table() if kind not in (1, 4))
     heavy = [int(np.max(r.read_lengths)) > single_max for r in pool.regions]
     warm = eng.submit_many(pool, range(300))  # warm the queue's engines (a burst of both kinds)
     for i, tk in enumerate(warm):

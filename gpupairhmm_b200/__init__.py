@@ -412,7 +412,8 @@ class Engine:
     # ------------------------------------------------------------ tuning
     def tile_table(self) -> list[tuple[int, int, int, int]]:
         """(max read length, G, R, kind) with kind 0 = one tile, 1 = multi-tile,
-        2 = one tile, two reads per group in packed FP32."""
+        2 = one tile, two reads per group in packed FP32, 3 = the same with exact
+        tiles, 4 = exact tiles over a block of G/32 warps."""
         n = ctypes.c_int32()
         _check(lib().pairhmm_get_tile_table(self._h, None, None, None, None, 0, ctypes.byref(n)), self._h)
         arrs = [np.zeros(n.value, dtype=np.int32) for _ in range(4)]

@@ -1,4 +1,4 @@
-"""Autotuner for the engine's tile table on the local GPU.
+"""Autotuner for tables of padded tiles on the local GPU.
 
 For each read-length class (16 positions wide up to 1024, wider beyond) it
 times every compiled single-tile configuration (G lanes x R positions, with
@@ -6,11 +6,12 @@ G*R >= the class's longest read) on synthetic pairs of that class -- read
 length uniform in the class, haplotype length = read length + U{50..400},
 base quality U{10..40}, ins/del 40 -- and keeps the fastest.  Classes beyond
 the largest single tile are timed with the multi-tile configurations.
-Adjacent classes with the same winner merge into one rule.
+Adjacent classes with the same winner merge into one rule.  The engine's own
+table takes padded tiles only outside 33-640 positions, where it has exact tiles
+(engine.cu); ``Engine.set_tile_table`` takes any table.
 
-Outputs:
+Output:
   gpupairhmm_b200/tuning_sm100a.json   every measurement and the table
-  gpupairhmm_b200/csrc/tuned_table.inc the table compiled into the engine
 
   python -m gpupairhmm_b200.autotune [--pairs-per-class N] [--repeats K] [--only LO-HI]
 
@@ -129,12 +130,6 @@ def write_outputs(results, rules):
                       for a, b, c, d in rules],
             "classes": results}
     (HERE / "tuning_sm100a.json").write_text(json.dumps(meta, indent=1))
-    lines = ["// Generated by gpupairhmm_b200/autotune.py on a B200; see tuning_sm100a.json.",
-             "// {max read length, G, R, multi-tile, packed}"]
-    for a, b, c, d in rules:
-        lines.append(f"{{{a if a < (1 << 30) else '1 << 30'}, {b}, {c}, {'true' if d == 1 else 'false'}, "
-                     f"{'true' if d == 2 else 'false'}}},")
-    (HERE / "csrc" / "tuned_table.inc").write_text("\n".join(lines) + "\n")
 
 
 def main():
@@ -159,7 +154,6 @@ def main():
         out = Path(a.outdir)
         out.mkdir(parents=True, exist_ok=True)
         (out / "tuning_sm100a.json").write_text((HERE / "tuning_sm100a.json").read_text())
-        (out / "tuned_table.inc").write_text((HERE / "csrc" / "tuned_table.inc").read_text())
 
 
 if __name__ == "__main__":

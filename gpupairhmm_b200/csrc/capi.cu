@@ -351,8 +351,9 @@ pairhmm_status_t pairhmm_set_tile_table(pairhmm_engine_t* h, const int32_t* max_
     return guarded(h, [&] {
         std::vector<phmm::TileRule> rules(n);
         for (int i = 0; i < n; ++i) {
-            if (multi_tile[i] < 0 || multi_tile[i] > 2) return PAIRHMM_ERR_INVALID_ARGUMENT;
-            rules[i] = {max_len[i], group[i], regs[i], multi_tile[i] == 1, multi_tile[i] == 2};
+            const int k = multi_tile[i];
+            if (k < 0 || k > 4) return PAIRHMM_ERR_INVALID_ARGUMENT;
+            rules[i] = {max_len[i], group[i], regs[i], k == 1 || k == 4, k == 2 || k == 3, k >= 3};
         }
         return finish(h, h->engine->set_tile_table(rules));
     });
@@ -368,7 +369,7 @@ pairhmm_status_t pairhmm_get_tile_table(pairhmm_engine_t* h, int32_t* max_len, i
         max_len[i] = r[i].max_len;
         group[i] = r[i].G;
         regs[i] = r[i].R;
-        multi_tile[i] = r[i].multi_tile ? 1 : (r[i].packed ? 2 : 0);
+        multi_tile[i] = r[i].exact ? (r[i].multi_tile ? 4 : 3) : r[i].multi_tile ? 1 : r[i].packed ? 2 : 0;
     }
     return PAIRHMM_OK;
 }

@@ -73,8 +73,12 @@ struct ExtList {
 struct DevView;
 __device__ __forceinline__ void append_rescue(const DevView& v, int cls, const Task& t);
 
+struct ReadMeta;
+
 struct DevView {
     const uint32_t* read_pack;
+    const float4* read_coef;    // wavefront_tile.cuh's coefficients, by packed position
+    const ReadMeta* read_meta;
     const int64_t* read_start;  // in positions, multiple of 4
     const int32_t* read_len;
     const uint8_t* hap_code;

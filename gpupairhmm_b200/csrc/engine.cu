@@ -39,13 +39,29 @@ constexpr int kCtrTotal = kMaxBuckets + 4 * kFp64Classes;
 // resident warps of that class's kernel on 148 SMs)
 constexpr int64_t kFuseMaxPairs = 2048;
 
+// Exact tiles for reads of lo+1 .. hi positions on groups of G lanes, one rule per
+// R (a lane's positions).
+void add_exact_rules(std::vector<TileRule>& rules, int G, int lo, int hi) {
+    for (int R = lo / G + 1; R * G <= hi; ++R) rules.push_back({R * G, G, R, G > 32, G <= 32, true});
+}
+
 std::vector<TileRule> engine_default_rules() {
-    // Tile per read-length bucket for the persistent engine, measured on a B200
-    // by gpupairhmm_b200/autotune.py (every compiled configuration timed on each
-    // 16-position length class; adjacent classes with one winner merged).
-    return {
-#include "tuned_table.inc"
-    };
+    // The two shortest classes keep the padded tiles autotune.py picked for them;
+    // from 33 positions on exact tiles with as many positions per lane as fit (the
+    // per-step work of a lane is amortised over them) and at least 11 once a group
+    // of 16 or 32 lanes is needed.
+    std::vector<TileRule> rules = {{16, 4, 4, false, false}, {32, 4, 8, false, true}};
+    add_exact_rules(rules, 8, 32, 160);
+    add_exact_rules(rules, 16, 160, 320);
+    add_exact_rules(rules, 32, 320, 640);
+    rules.push_back({768, 32, 24, false});
+    rules.push_back({896, 32, 28, false});
+    rules.push_back({1024, 32, 32, false});
+    rules.push_back({1280, 32, 20, true});
+    rules.push_back({1536, 32, 24, true});
+    rules.push_back({1792, 32, 28, true});
+    rules.push_back({1 << 30, 32, 32, true});
+    return rules;
 }
 
 std::vector<TileRule> plain_rules() {
@@ -62,12 +78,32 @@ std::vector<TileRule> plain_rules() {
 }
 
 std::vector<TileRule> gcp_rules() {
-    // gcp mode (eps and beta per read): the scalar kernels compiled with that
-    // option (fp32_gcp.cu), one per length class.
-    return {
-        {64, 4, 16, false},   {128, 8, 16, false},  {160, 8, 20, false},    {256, 16, 16, false},
-        {512, 32, 16, false}, {1024, 32, 32, false}, {1 << 30, 32, 32, true},
-    };
+    // gcp mode (eps and beta per read): the exact tiles, and around them the padded
+    // scalar kernels compiled with that option (fp32_gcp.cu).
+    std::vector<TileRule> rules = {{32, 4, 16, false}};
+    add_exact_rules(rules, 8, 32, 160);
+    add_exact_rules(rules, 16, 160, 320);
+    add_exact_rules(rules, 32, 320, 640);
+    rules.push_back({1024, 32, 32, false});
+    rules.push_back({1 << 30, 32, 32, true});
+    return rules;
+}
+
+// The table of a batch of few pairs: the same, with 32 lanes a group wherever an
+// exact tile has fewer.  Results do not change: the exact tiles' do not depend on the
+// shape, and the other classes stay.
+std::vector<TileRule> small_rules(const std::vector<TileRule>& rules) {
+    std::vector<TileRule> small;
+    for (size_t i = 0; i < rules.size(); ++i) {
+        if (!rules[i].exact || rules[i].G > 32) {
+            small.push_back(rules[i]);
+            continue;
+        }
+        const int lo = i ? rules[i - 1].max_len : 0;
+        while (i + 1 < rules.size() && rules[i + 1].exact && rules[i + 1].G <= 32) ++i;
+        add_exact_rules(small, 32, lo, rules[i].max_len);
+    }
+    return small;
 }
 
 inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -104,15 +140,19 @@ void DevBuf::release() {
     cap = 0;
 }
 
-Engine::Engine(const pairhmm_options_t& opts) : opts_(opts) {
-    rules_ = opts_.mode == PAIRHMM_MODE_PLAIN ? plain_rules() : opts_.gcp ? gcp_rules() : engine_default_rules();
+namespace {
+std::vector<TileRule> default_rules(const pairhmm_options_t& o) {
+    return o.mode == PAIRHMM_MODE_PLAIN ? plain_rules() : o.gcp ? gcp_rules() : engine_default_rules();
 }
+}  // namespace
+
+Engine::Engine(const pairhmm_options_t& opts) : opts_(opts) { tables_[0].rules = default_rules(opts_); }
 
 std::vector<DevBuf*> Engine::all_buffers() {
-    return {&ph2pr_, &rules_rank_, &in_read_bases_, &in_bq_,
+    return {&ph2pr_, &in_read_bases_, &in_bq_,
             &in_iq_, &in_dq_, &in_read_off_, &in_read_len_, &in_hap_bases_, &in_hap_off_, &in_hap_len_,
             &read_record_, &read_local_, &rec_haps_, &rec_hap_base_, &rec_pair_base_, &read_start_,
-            &hap_start_, &read_pack_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
+            &hap_start_, &read_pack_, &read_coef_, &read_meta_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
             &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
             &rescue_ext_, &rsort_,
             &in_gq_, &read_gcp_};
@@ -203,17 +243,6 @@ pairhmm_status_t Engine::init() {
     PHMM_CUDA(cudaEventCreate(&ev_prep_));
     PHMM_CUDA(cudaEventCreate(&ev_fp32_));
 
-    // dynamic shared memory opt-in for every kernel on this device
-    for (const ConfigInfo& c : fp32_configs())
-        PHMM_CUDA(cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem_bytes));
-    for (int c = 0; c < kFp64Classes; ++c)
-        for (const bool gcp : {false, true})
-            for (const bool ext : {false, true})
-                for (const bool fuse : {false, true})
-                    PHMM_CUDA(cudaFuncSetAttribute(fp64_kernel(c, gcp, ext, fuse),
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)fp64_smem_bytes(c, ext)));
-
     // probability table p(q) = float(10^(-q/10)) (gpuworker.cuh:473-486)
     float table[128];
     for (int i = 0; i < 128; ++i) table[i] = (float)std::pow(10.0, (-i) / 10.0);
@@ -223,7 +252,7 @@ pairhmm_status_t Engine::init() {
     // FP64 list sort: per-class histogram (uint32) then cursors (uint64)
     PHMM_CUDA(rsort_.ensure((sizeof(unsigned int) + sizeof(unsigned long long)) * kFp64Classes * kRescueHBins));
     ready_ = true;
-    return upload_rules();
+    return build_tables(default_rules(opts_));
 }
 
 pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
@@ -235,35 +264,58 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
     for (size_t i = 0; i < rules.size(); ++i) {
         if (rules[i].packed && rules[i].multi_tile)
             return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "packed rules are single tile");
-        if (!find_fp32_config(rules[i].G, rules[i].R, rules[i].multi_tile, rules[i].packed, opts_.gcp != 0))
+        if (!find_fp32_config(rules[i].G, rules[i].R, rules[i].multi_tile, rules[i].packed, rules[i].exact,
+                              opts_.gcp != 0))
             return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table names a configuration that is not compiled");
         if (i > 0 && rules[i].max_len <= rules[i - 1].max_len)
             return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table bounds must increase");
-        if (!rules[i].multi_tile && rules[i].max_len > rules[i].G * rules[i].R)
+        if ((!rules[i].multi_tile || rules[i].exact) && rules[i].max_len > rules[i].G * rules[i].R)
             return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "single-tile rule shorter than its bucket");
+        if (rules[i].exact && (i ? rules[i - 1].max_len : 0) < rules[i].G * (rules[i].R - 1))
+            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "exact tile for reads of fewer positions than it takes");
     }
-    if (!rules.back().multi_tile) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "last rule must be multi-tile");
-    rules_ = rules;
+    if (!rules.back().multi_tile || rules.back().exact) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "last rule must be multi-tile");
     for (cudaGraphExec_t& g : graph_exec_) {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
     }
-    return ready_ ? upload_rules() : PAIRHMM_OK;
+    if (ready_) return build_tables(rules);
+    tables_[0].rules = rules;
+    return PAIRHMM_OK;
 }
 
-pairhmm_status_t Engine::upload_rules() {
-    const int nb = (int)rules_.size();
-    rule_cfg_.assign(nb, nullptr);
-    std::vector<int32_t> rank(nb);
-    for (int b = 0; b < nb; ++b) {
-        rule_cfg_[b] =
-            find_fp32_config(rules_[b].G, rules_[b].R, rules_[b].multi_tile, rules_[b].packed, opts_.gcp != 0);
-        if (!rule_cfg_[b]) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile rule without compiled kernel");
-        rank[b] = opts_.mode == PAIRHMM_MODE_PLAIN ? b : nb - 1 - b;
-    }
-    PHMM_CUDA(rules_rank_.ensure(sizeof(int32_t) * nb));
-    PHMM_CUDA(cudaMemcpy(rules_rank_.ptr, rank.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice));
+pairhmm_status_t Engine::build_tables(const std::vector<TileRule>& rules) {
+    TileTable built[2];
+    built[0].rules = rules;
+    if (rules == default_rules(opts_) && opts_.mode != PAIRHMM_MODE_PLAIN) built[1].rules = small_rules(rules);
+    for (TileTable& t : built)
+        for (const TileRule& r : t.rules) {
+            t.cfg.push_back(find_fp32_config(r.G, r.R, r.multi_tile, r.packed, r.exact, opts_.gcp != 0));
+            if (!t.cfg.back()) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile rule without compiled kernel");
+            t.exact = t.exact || r.exact;
+        }
+    if (built[0].rules.size() > kMaxBuckets || built[1].rules.size() > kMaxBuckets)
+        return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table size");
+    for (int i = 0; i < 2; ++i) tables_[i] = std::move(built[i]);
+    table_ = &tables_[0];
     return PAIRHMM_OK;
+}
+
+// A batch of few pairs leaves most of the chip idle and takes as long as its longest
+// pair, one step per haplotype position; on 32 lanes instead of 8 or 16 a step works
+// on a quarter or half of the positions.  What counts is the pairs per length class:
+// the classes are launches of their own, each with its own last wave.  FP32 stage,
+// table for few / for many pairs: reads of one length (100) 128 pairs 0.018 / 0.029 ms,
+// 2,048 pairs 0.027 / 0.029, 4,096 pairs 0.045 / 0.031; (250) 1,024 pairs 0.043 / 0.062,
+// 2,048 pairs 0.072 / 0.066; uneven regions (13 classes) 395 pairs 0.057 / 0.088,
+// 6,500 pairs 0.19 / 0.24, 13,000 pairs 0.31 / 0.29, 27,000 pairs 0.48 / 0.40.
+void Engine::choose_table(int64_t pairs, const int32_t* read_lengths, int64_t num_reads) {
+    table_ = &tables_[0];
+    if (tables_[1].rules.empty() || pairs > kSmallPairs * (int64_t)tables_[0].rules.size()) return;
+    uint64_t seen = 0;
+    static_assert(kMaxBuckets <= 64, "one bit per class");
+    for (int64_t i = 0; i < num_reads; ++i) seen |= uint64_t(1) << bucket_of_host(read_lengths[i], tables_[0].rules);
+    if (pairs <= kSmallPairs * __builtin_popcountll(seen)) table_ = &tables_[1];
 }
 
 pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector<TileRule>& rules, BatchIndex& x,
@@ -524,8 +576,12 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(unit_bucket_.ensure(4 * nr));
     PHMM_CUDA(hap_start_.ensure(8 * nh));
     PHMM_CUDA(read_pack_.ensure(4 * (x.pack_positions + kReadSlackPos)));
+    if (table_->exact) {
+        PHMM_CUDA(read_coef_.ensure(sizeof(float4) * std::max<int64_t>(x.pack_positions, 1)));
+        PHMM_CUDA(read_meta_.ensure(sizeof(ReadMeta) * nr));
+    }
     PHMM_CUDA(hap_code_.ensure(x.code_bytes + kHapSlack));
-    const int64_t nbins = (int64_t)rules_.size() * hbins_of(x);
+    const int64_t nbins = (int64_t)table_->rules.size() * hbins_of(x);
     PHMM_CUDA(hist_.ensure(4 * nbins));
     PHMM_CUDA(cursor_.ensure(8 * nbins));
     PHMM_CUDA(items_.ensure(sizeof(Item) * np));
@@ -564,17 +620,23 @@ int64_t Engine::index_bytes(const BatchIndex& x) {
            8 * (int64_t)(x.rec_hap_base.size() + x.rec_pair_base.size() + x.read_start.size() + x.hap_start.size());
 }
 
-int Engine::persistent_grid(const void* kernel, size_t smem) const {
+// The grid of a persistent launch: every block that fits at once.  A kernel's shared
+// memory opt-in and occupancy are asked for on its first use (each loads the kernel's
+// code, so an engine pays for the few tiles its batches need, not for all).
+int Engine::persistent_grid(const void* kernel, int threads, size_t smem) {
+    const auto it = blocks_per_sm_.find(kernel);
+    if (it != blocks_per_sm_.end()) return it->second * num_sms_;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlockThreads, smem) != cudaSuccess ||
-        per_sm < 1)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
+    blocks_per_sm_.emplace(kernel, per_sm);
     return per_sm * num_sms_;
 }
 
 pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const BatchIndex& x, const Plan& plan,
                                           float* d_scores, cudaStream_t s, int stage) {
-    const int nb = (int)rules_.size();
+    const int nb = (int)table_->rules.size();
     const bool plain = opts_.mode == PAIRHMM_MODE_PLAIN;
     const int prep_grid = 4 * num_sms_;
 
@@ -601,6 +663,9 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     pa.num_haps = x.num_haps;
     pa.read_pack = read_pack_.as<uint32_t>();
     pa.hap_code = hap_code_.as<uint8_t>();
+    pa.read_coef = table_->exact ? read_coef_.as<float4>() : nullptr;
+    pa.read_meta = table_->exact ? read_meta_.as<ReadMeta>() : nullptr;
+    pa.ph2pr = ph2pr_.as<float>();
     if (stage == 0) {
     launches_ = 0;
     fp32_launches_ = 0;
@@ -636,7 +701,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     ba.hbins = (int)hbins_of(x);
     for (int rank = 0; rank < nb; ++rank)
         ba.ranks.begin[rank + 1] = ba.ranks.begin[rank] + x.bucket_items[plain ? rank : nb - 1 - rank];
-    ba.bucket_rank = rules_rank_.as<int32_t>();
+    ba.reversed = !plain;
     ba.hist = hist_.as<unsigned int>();
     ba.cursor = cursor_.as<unsigned long long>();
     ba.items = items_.as<Item>();
@@ -649,6 +714,8 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     unsigned long long* counters = counters_.as<unsigned long long>();
     DevView v{};
     v.read_pack = pa.read_pack;
+    v.read_coef = pa.read_coef;
+    v.read_meta = pa.read_meta;
     v.read_start = pa.read_start;
     v.read_len = in.read_lengths;
     v.hap_code = pa.hap_code;
@@ -695,7 +762,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
         for (int rank = 0; rank < nb; ++rank) {
             const int b = plain ? rank : nb - 1 - rank;
             if (x.bucket_items[b] == 0) continue;
-            const ConfigInfo* c = rule_cfg_[b];
+            const ConfigInfo* c = table_->cfg[b];
             Fp32LaunchArgs la{};
             la.view = v;
             la.items = items_.as<Item>() + ba.ranks.begin[rank];
@@ -755,8 +822,8 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     return PAIRHMM_OK;
 }
 
-Engine::Plan Engine::make_plan(const BatchIndex& x) const {
-    const int nb = (int)rules_.size();
+Engine::Plan Engine::make_plan(const BatchIndex& x) {
+    const int nb = (int)table_->rules.size();
     const bool plain = opts_.mode == PAIRHMM_MODE_PLAIN;
     Plan p;
     p.rows = round_up((int64_t)x.max_hap_len + 2 * 32 + 8, 64);
@@ -767,16 +834,17 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) const {
     // the border scratch, out of an equal share of the budget
     int n_mt = 0;
     for (int b = 0; b < nb; ++b)
-        if (x.bucket_items[b] != 0 && rule_cfg_[b]->multi_tile) ++n_mt;
+        if (x.bucket_items[b] != 0 && table_->cfg[b]->scratch_bytes_per_row) ++n_mt;
     const int64_t mt_budget = kScratchBudget / std::max(1, n_mt);
     int64_t scratch = 0, fp32_scratch = 0;
     for (int b = 0; b < nb; ++b) {
         if (x.bucket_items[b] == 0) continue;
-        const ConfigInfo* c = rule_cfg_[b];
-        const int64_t tasks = (x.bucket_items[b] + c->per_warp() - 1) / c->per_warp();
-        const int64_t need_blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-        int64_t grid = plain ? need_blocks : std::min<int64_t>(persistent_grid(c->kernel, c->smem_bytes), need_blocks);
-        if (c->multi_tile) {
+        const ConfigInfo* c = table_->cfg[b];
+        const int64_t tasks = (x.bucket_items[b] + c->per_task - 1) / c->per_task;
+        const int64_t need_blocks = (tasks + c->tasks_per_block - 1) / c->tasks_per_block;
+        const int64_t resident = persistent_grid(c->kernel, c->block_threads, c->smem_bytes);
+        int64_t grid = plain ? need_blocks : std::min(resident, need_blocks);
+        if (c->scratch_bytes_per_row) {
             const int64_t per_warp = (int64_t)c->scratch_bytes_per_row * p.rows;
             const int64_t cap_blocks = std::max<int64_t>(1, mt_budget / (per_warp * kWarpsPerBlock));
             grid = std::min(grid, cap_blocks);
@@ -789,8 +857,12 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) const {
         p.persistent[b] = (!plain || grid < need_blocks) ? 1 : 0;
     }
     for (int c = 0; c < kFp64Classes; ++c) {
+        if (x.class_pairs[c] == 0) continue;
+        if (c == kFp64Classes - 1)   // the fused form's opt-in; its grid is the scaled tier's
+            persistent_grid(fp64_kernel(c, opts_.gcp != 0, false, true), kBlockThreads, fp64_smem_bytes(c, false));
         for (const bool tier_ext : {false, true}) {
-            int64_t grid = persistent_grid(fp64_kernel(c, opts_.gcp != 0, tier_ext), fp64_smem_bytes(c, tier_ext));
+            int64_t grid = persistent_grid(fp64_kernel(c, opts_.gcp != 0, tier_ext), kBlockThreads,
+                                            fp64_smem_bytes(c, tier_ext));
             const int64_t per_warp = (int64_t)fp64_scratch_bytes_per_row(c, tier_ext) * p.rows;
             if (per_warp > 0) {
                 grid = std::min<int64_t>(grid, std::max<int64_t>(1, kScratchBudget / (per_warp * kWarpsPerBlock)));
@@ -886,7 +958,8 @@ pairhmm_status_t Engine::host_begin(const pairhmm_batch_t& b, float* scores, cud
     };
     if (opts_.gcp) inputs.push_back({in_gq_.ptr, b.gcp_quals + rlo, (size_t)rn});
     cudaError_t up = uploader_.start(opts_.device, inputs, s);
-    st = build_index(b, rules_, idx_, err);
+    choose_table(rg.num_pairs, b.read_lengths, rg.num_reads);
+    st = build_index(b, table_->rules, idx_, err);
     const cudaError_t upf = uploader_.finish();
     if (up == cudaSuccess) up = upf;
     if (up != cudaSuccess) return cuda_fail(up, "input upload");
@@ -987,7 +1060,7 @@ pairhmm_status_t Engine::compute_host(const pairhmm_batch_t& b, float* scores) {
         o.pipeline_chunks = 1;
         twin_ = std::make_unique<Engine>(o);
         pairhmm_status_t st = twin_->init();
-        if (st == PAIRHMM_OK) st = twin_->set_tile_table(rules_);
+        if (st == PAIRHMM_OK) st = twin_->set_tile_table(tables_[0].rules);
         if (st != PAIRHMM_OK) {
             last_error_ = "twin engine: " + twin_->last_error();
             twin_.reset();
@@ -1105,7 +1178,10 @@ pairhmm_status_t Engine::compute_device(const pairhmm_batch_t& b, int32_t, int32
     hb.read_offsets = nullptr;
     hb.hap_offsets = nullptr;
     std::string err;
-    pairhmm_status_t st = build_index(hb, rules_, idx_, err);
+    int64_t pairs = 0;
+    for (int64_t g = 0; g < b.num_records; ++g) pairs += (int64_t)std::max(rpr[g], 0) * std::max(hpr[g], 0);
+    choose_table(pairs, rl.data(), nr);
+    pairhmm_status_t st = build_index(hb, table_->rules, idx_, err);
     const BatchIndex& x = idx_;
     if (st != PAIRHMM_OK) return fail(st, err);
     stats_ = pairhmm_stats_t{};

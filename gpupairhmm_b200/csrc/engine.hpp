@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/pairhmm_b200.h"
@@ -21,7 +22,20 @@ struct TileRule {
     int G;
     int R;
     bool multi_tile;
-    bool packed = false;  // two reads of a record per group, packed FP32 (single tile)
+    bool packed = false;  // two reads of a record per group, packed FP32
+    bool exact = false;   // lanes hold R or R-1 positions (wavefront_tile.cuh)
+};
+
+inline bool operator==(const TileRule& a, const TileRule& b) {
+    return a.max_len == b.max_len && a.G == b.G && a.R == b.R && a.multi_tile == b.multi_tile &&
+           a.packed == b.packed && a.exact == b.exact;
+}
+
+// A tile table with its compiled kernels.
+struct TileTable {
+    std::vector<TileRule> rules;
+    std::vector<const ConfigInfo*> cfg;
+    bool exact = false;   // some rule is exact: the preparation forms coefficients
 };
 
 // Per-batch index derived on the host from the record structure.
@@ -84,7 +98,7 @@ public:
 
     // Replace the tile table of the current mode (autotuner).
     pairhmm_status_t set_tile_table(const std::vector<TileRule>& rules);
-    const std::vector<TileRule>& tile_table() const { return rules_; }
+    const std::vector<TileRule>& tile_table() const { return tables_[0].rules; }
     int device() const { return opts_.device; }
     bool gcp() const { return opts_.gcp != 0; }
     int64_t budget_bytes() const { return opts_.device_budget_bytes; }
@@ -100,7 +114,9 @@ private:
     pairhmm_status_t host_begin(const pairhmm_batch_t& b, float* scores, cudaEvent_t mark_start,
                                 cudaEvent_t mark_end);
     pairhmm_status_t host_end();
-    pairhmm_status_t upload_rules();
+    pairhmm_status_t build_tables(const std::vector<TileRule>& rules);
+    // the table for a batch of these reads and this many pairs becomes the current one
+    void choose_table(int64_t pairs, const int32_t* read_lengths, int64_t num_reads);
     pairhmm_status_t run_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, float* d_scores,
                                   cudaStream_t s);
     struct Plan {
@@ -112,27 +128,30 @@ private:
         std::vector<int64_t> scratch_off;   // by bucket: multi-tile kernels run side by side
         size_t scratch_bytes = 0;
     };
-    Plan make_plan(const BatchIndex& idx) const;
+    Plan make_plan(const BatchIndex& idx);
     // stage 0: packing + work list, 1: FP32 launches, 2: FP64 pass
     pairhmm_status_t enqueue_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, const Plan& plan,
                                       float* d_scores, cudaStream_t s, int stage);
     pairhmm_status_t ensure_buffers(const BatchIndex& idx, bool host_inputs);
     pairhmm_status_t ensure_inputs(const InputRanges& r);
     pairhmm_status_t upload_index(const BatchIndex& idx, cudaStream_t s);
-    int persistent_grid(const void* kernel, size_t smem) const;
+    int persistent_grid(const void* kernel, int threads, size_t smem);
     static int64_t index_bytes(const BatchIndex& x);
     int64_t hbins_of(const BatchIndex& x) const;
 
     pairhmm_options_t opts_;
-    std::vector<TileRule> rules_;
-    std::vector<const ConfigInfo*> rule_cfg_;
+    // tables_[0] is the engine's table, tables_[1] (default tables only) the one for
+    // batches of few pairs, with groups as wide as possible (choose_table)
+    TileTable tables_[2];
+    const TileTable* table_ = &tables_[0];
     int num_sms_ = 0;
+    std::unordered_map<const void*, int> blocks_per_sm_;  // kernels used so far
     bool ready_ = false;
     cudaStream_t stream_ = nullptr;
     // the launches of one stage (bucket kernels, FP64 classes) fork onto side
     // streams so that their tails overlap and a small batch's buckets run side
     // by side; they join back into stream_ before the stage ends
-    static constexpr int kSideStreams = 4;
+    static constexpr int kSideStreams = 8;
     cudaStream_t side_[kSideStreams] = {};
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
@@ -142,13 +161,13 @@ private:
     std::string last_error_;
 
     // device buffers
-    DevBuf ph2pr_, rules_rank_;
+    DevBuf ph2pr_;
     DevBuf in_read_bases_, in_bq_, in_iq_, in_dq_, in_read_off_, in_read_len_;
     DevBuf in_gq_, read_gcp_;  // gcp mode: uploaded gcp qualities, per-read gcp
     DevBuf in_hap_bases_, in_hap_off_, in_hap_len_;
     DevBuf read_record_, read_local_, rec_haps_, rec_hap_base_, rec_pair_base_, read_start_, hap_start_;
     DevBuf unit_read0_, unit_read1_, unit_bucket_;
-    DevBuf read_pack_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
+    DevBuf read_pack_, read_coef_, read_meta_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
     DevBuf rescue_off_, rescue_ext_, rsort_;
     // host-to-device uploads (caller inputs, index) and the reused index
     HostUploader uploader_;
@@ -157,6 +176,8 @@ private:
     // kMaxChunks) alternate between this engine and its twin; only the first
     // chunk's upload is exposed (uneven workload, 10.9 M pairs: 8 chunks 185.1 ms,
     // 4 chunks 186.8 ms end to end)
+    // pairs per occupied length class up to which a batch counts as small
+    static constexpr int64_t kSmallPairs = 1024;
     static constexpr int64_t kChunkPairs = int64_t(1) << 20;
     static constexpr int64_t kMaxChunks = 8;
     std::unique_ptr<Engine> twin_;

@@ -78,6 +78,9 @@ ConfigInfo make_fp32_config() {
     c.multi_tile = MT;
     c.packed = PK;
     c.gcp = GCP;
+    c.per_task = W::NG;
+    c.block_threads = kBlockThreads;
+    c.tasks_per_block = kWarpsPerBlock;
     c.smem_bytes = (32 + (size_t)kWarpsPerBlock * W::kTableFloat4) * sizeof(float4);
     c.scratch_bytes_per_row = MT ? (size_t)W::NG * 2 * sizeof(float4) : 0;
     c.kernel = reinterpret_cast<const void*>(&fp32_bucket_kernel<G, R, MT, PK, GCP>);

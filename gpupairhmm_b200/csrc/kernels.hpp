@@ -44,13 +44,15 @@ struct Fp64LaunchArgs {
 };
 
 struct ConfigInfo {
-    int G;
+    int G;                           // lanes per group (above 32: the warps of a block)
     int R;
-    bool multi_tile;
-    bool packed;                     // two reads per group with packed FP32 (single tile)
+    bool multi_tile;                 // reads beyond one warp's tile
+    bool packed;                     // two reads per group with packed FP32
+    bool exact;                      // wavefront_tile.cuh: read lengths (G*(R-1), G*R] only
     bool gcp;                        // eps/beta per read (gcp mode)
-    int tile() const { return G * R; }
-    int per_warp() const { return 32 / G; }   // items per warp task
+    int per_task;                    // items per task (of a warp, or of a block)
+    int block_threads;
+    int tasks_per_block;             // tasks a block works on at a time
     size_t smem_bytes;               // dynamic shared memory per CTA
     size_t scratch_bytes_per_row;    // per warp, per border row (both buffers)
     const void* kernel;
@@ -59,7 +61,7 @@ struct ConfigInfo {
 
 // All compiled FP32 configurations.
 const std::vector<ConfigInfo>& fp32_configs();
-const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed = false, bool gcp = false);
+const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed, bool exact, bool gcp);
 
 // FP64 pass, one kernel per length class and tier (misc_kernels.cu): the
 // scaled tier (ext = false) recomputes every flagged pair, the extended tier

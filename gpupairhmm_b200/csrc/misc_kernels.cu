@@ -16,6 +16,12 @@ void register_fp32_g16(std::vector<ConfigInfo>& out);
 void register_fp32_g32(std::vector<ConfigInfo>& out);
 void register_fp32_gcp(std::vector<ConfigInfo>& out);
 void register_fp32_geven(std::vector<ConfigInfo>& out);
+void register_tile_g8(std::vector<ConfigInfo>& out);
+void register_tile_g16(std::vector<ConfigInfo>& out);
+void register_tile_g32(std::vector<ConfigInfo>& out);
+void register_tile_gcp_g8(std::vector<ConfigInfo>& out);
+void register_tile_gcp_g16(std::vector<ConfigInfo>& out);
+void register_tile_gcp_g32(std::vector<ConfigInfo>& out);
 
 const std::vector<ConfigInfo>& fp32_configs() {
     static std::vector<ConfigInfo> all;
@@ -27,13 +33,21 @@ const std::vector<ConfigInfo>& fp32_configs() {
         register_fp32_g32(all);
         register_fp32_geven(all);
         register_fp32_gcp(all);
+        register_tile_g8(all);
+        register_tile_g16(all);
+        register_tile_g32(all);
+        register_tile_gcp_g8(all);
+        register_tile_gcp_g16(all);
+        register_tile_gcp_g32(all);
     });
     return all;
 }
 
-const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed, bool gcp) {
+const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed, bool exact, bool gcp) {
     for (const auto& c : fp32_configs())
-        if (c.G == G && c.R == R && c.multi_tile == multi_tile && c.packed == packed && c.gcp == gcp) return &c;
+        if (c.G == G && c.R == R && c.multi_tile == multi_tile && c.packed == packed && c.exact == exact &&
+            c.gcp == gcp)
+            return &c;
     return nullptr;
 }
 

@@ -14,11 +14,12 @@
 #pragma once
 
 #include "device_common.cuh"
+#include "wavefront_tile.cuh"
 
 namespace phmm {
 
 constexpr int kHBins = 4096;     // most haplotype-length classes per bucket
-constexpr int kMaxBuckets = 48;
+constexpr int kMaxBuckets = 64;
 
 struct PrepArgs {
     // caller arrays (device)
@@ -46,6 +47,9 @@ struct PrepArgs {
     uint32_t* read_pack;
     uint8_t* hap_code;
     uint8_t* read_gcp;              // [num_reads], gcp mode only (else null)
+    float4* read_coef;              // wavefront_tile.cuh's coefficients by packed position, and
+    ReadMeta* read_meta;            // what it needs per read (null: no exact tile in the table)
+    const float* ph2pr;             // 128 probabilities
 };
 
 // Byte fills of up to kFillRanges device ranges (4-byte aligned, whole words) by
@@ -74,6 +78,9 @@ __device__ __forceinline__ uint32_t pack_position(uint32_t base, uint32_t bq, ui
 // 16-byte word group.  Where the four source arrays are 4-byte aligned at the
 // read's offset, whole groups inside the read are read with one 4-byte load
 // per array; the read's ragged end (and unaligned sources) go byte by byte.
+// The exact-tile kernel's coefficients are formed here, once per read instead of
+// once per pair (8.5 haplotypes a read in the uneven workload, three divisions a
+// position): 16 bytes a position that stay in L2 between a read's haplotypes.
 __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int64_t nblocks) {
     const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (nblocks * blockDim.x) >> 5;
@@ -93,6 +100,18 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
             const uint32_t g = L > 0 ? a.gcp_quals[src] : 10u;
             a.read_gcp[i] = (uint8_t)(g > 127u ? 127u : g);
         }
+        float beta = kBeta, range = 0.0f;
+        uint32_t key = kNoKey, flags = 0;
+        bool same = true;   // gap qualities of the lane's positions equal the first position's
+        if (a.read_coef && L > 0) {
+            key = min((uint32_t)iq[0], 127u);
+            if (a.gcp_quals) {
+                const uint32_t g = min((uint32_t)a.gcp_quals[src], 127u);
+                key |= g << 8;
+                beta = (float)(1.0 - (double)a.ph2pr[g]);  // gpuworker.cuh:1049
+                if (!(beta >= kMinAlpha)) flags = 1u;      // gcp quality 0: nothing to rescale by
+            }
+        }
         for (int c = lane * 4; c < Lp; c += 128) {
             uint32_t w[4];
             if (aligned && c + 3 < L) {
@@ -110,6 +129,45 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                     w[j] = c + j < L ? pack_position(rb[c + j], bq[c + j], iq[c + j], dq[c + j]) : 4u;
             }
             dst[c >> 2] = make_uint4(w[0], w[1], w[2], w[3]);
+            if (a.read_coef) {
+                float4* coef = a.read_coef + a.read_start[i] + c;
+                float d = a.ph2pr[(w[0] >> 16) & 0x7fu], sg = a.ph2pr[(w[0] >> 24) & 0x7fu];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (c + j >= L) break;
+                    same = same && (w[j] >> 16) == (key & 0xffu) * 0x101u;
+                    const bool end = c + j + 1 >= L;
+                    float dn = d, sn = sg, an = beta;
+                    if (!end) {
+                        if (j < 3) {
+                            dn = a.ph2pr[(w[j < 3 ? j + 1 : 3] >> 16) & 0x7fu];
+                            sn = a.ph2pr[(w[j < 3 ? j + 1 : 3] >> 24) & 0x7fu];
+                        } else {
+                            dn = a.ph2pr[min((uint32_t)iq[c + 4], 127u)];
+                            sn = a.ph2pr[min((uint32_t)dq[c + 4], 127u)];
+                        }
+                        an = 1.0f - (dn + sn);
+                    }
+                    const float4 cf = tile_coefficients(a.ph2pr[(w[j] >> 8) & 0x7fu], d, sg, an, dn, beta);
+                    coef[j] = cf;
+                    range = fmaxf(range, 1.0f / dn + 2.0f * (1.0f + cf.y));
+                    if (!(fabsf(1.0f - (d + sg)) >= kMinAlpha)) flags |= 1u;
+                    if (end) a.read_meta[i].w_end = tile_weight(beta, dn, beta);
+                    d = dn;
+                    sg = sn;
+                }
+            }
+        }
+        if (a.read_coef) {
+            same = __all_sync(kFullMask, same);
+            flags = __any_sync(kFullMask, flags != 0u) ? 1u : 0u;
+            // positive floats order as their bits; an infinite or NaN bound stays the largest
+            range = __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(range)));
+            if (lane == 0) {
+                a.read_meta[i].range = range;
+                a.read_meta[i].key = same ? key : kNoKey;
+                a.read_meta[i].flags = flags;
+            }
         }
     }
 }
@@ -190,7 +248,7 @@ struct BinArgs {
     int nbuckets;
     int hcap;                       // longest haplotype class (0: all in one class, the plain form)
     int hbins;                      // haplotype-length classes per bucket: hcap + 1, up to a multiple of 4
-    const int32_t* bucket_rank;     // [nbuckets] bin-major position of each bucket
+    bool reversed;                  // bucket b's rank is nbuckets - 1 - b (largest tiles first), else b
     unsigned int* hist;             // [nbuckets * hbins]
     unsigned long long* cursor;     // [nbuckets * hbins] scatter positions
     RankItems ranks;
@@ -198,7 +256,7 @@ struct BinArgs {
 };
 
 __device__ __forceinline__ int bin_of(const BinArgs& a, int bucket, int H) {
-    return a.bucket_rank[bucket] * a.hbins + a.hcap - (H < a.hcap ? H : a.hcap);
+    return (a.reversed ? a.nbuckets - 1 - bucket : bucket) * a.hbins + a.hcap - (H < a.hcap ? H : a.hcap);
 }
 
 #ifdef PHMM_PREP_KERNELS_IMPL

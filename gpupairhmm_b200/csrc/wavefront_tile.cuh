@@ -1,0 +1,382 @@
+// Exact-tile wavefront: the PairHMM forward recurrence for reads whose length
+// lies in (NL*(R-1), NL*R], NL the lanes of a group, so that every lane holds R
+// or R-1 read positions and no position is padding.
+//
+// What bounds the cell.  A scheduler reads two 32-bit register operands per lane
+// and cycle: an FFMA with three distinct register operands runs at 0.64 of the
+// FMA peak, one with two (the third an immediate, a constant or a uniform
+// register) at 0.95; FFMA2 and DFMA alike (measured with dependent-chain loops of
+// each form).  The five-instruction cell of wavefront_fp32.cuh reads 13 operands,
+// 6.5 cycles, and ran at 0.60-0.63 of the pipe, scalar or packed.  So the
+// recurrence is scaled here for few register operands, not few instructions:
+//   I unscaled (true I times the pair's scale), eps an immediate
+//   N = n_c*M with n_c = beta*delta_{c+1}/beta, so that what N feeds into the next
+//       column's I has weight 1
+//   D^ = D/d_c with d_c = sigma_c/n_c, so that what N feeds into D has weight 1
+//     P(j,c)  = w_c*N(j-1,c-1) + X(j,c-1)      w_c = alpha_c/(beta*delta_c)
+//     N(j,c)  = l_c(h_j)*P(j,c)                l_c = beta*n_c*lambda
+//     I^(j,c) = eps*I^(j,c-1) + N(j-1,c-1)     (I one row behind, as in the reference)
+//     X(j,c)  = x_c*D^(j-1,c) + I^(j,c)        x_c = d_c
+//     D^(j,c) = eps*D^(j-1,c) + N(j-1,c)
+// 12 operands a cell, and 10 for reads whose gap-open qualities have one value at
+// every position, for insertions and deletions alike (the usual case): w comes from
+// a uniform register and x is 1.  A warp decides per task; both paths do the same
+// arithmetic, so a pair's result does not depend on which one ran, nor on the
+// group's shape: every cell, and the order of the result's sum, is the same for
+// all G, R and W.
+//
+// Exact lanes.  The eps of I being a constant, I cannot be carried unchanged
+// through padding behind the read's end.  Lanes t < m = L - NL*(R-1) hold R
+// positions, the others R-1; a lane hands on the values of its last position (one
+// select per value).  The last lane of the group always holds the read's end, so
+//     T(j) = w_L*N(j,L-1) + I^(j+1,L-1) = M(j,L-1) + I(j,L-1),   w_L = 1/n_{L-1}
+// is added up there and nowhere else.  4 % less of the uneven workload's cells are
+// padding than with tiles of a multiple of 16 positions.
+//
+// Range (FP32).  N lies 1/delta below M (2^13 at gap quality 40), which costs the
+// low end of the range; the boundary D enters as FLT_MAX/8 instead of
+// (FLT_MAX/16)/H, which gives most of it back.  See tile_threshold.
+//
+// W > 1: the group is the W warps of a block, for reads beyond one warp's tile.
+// Warp v runs kLag blocks of kBlock steps behind warp v-1 and takes that warp's
+// last column, row by row, from a ring in shared memory; a block barrier after
+// every kBlock steps is the only synchronisation.
+#pragma once
+
+#include "device_common.cuh"
+
+namespace phmm {
+
+// Arithmetic of a lane's value: one pair in FP32 or FP64, or two pairs that share
+// a haplotype in packed FP32 (x = read A, y = read B).
+template <class V>
+struct LaneOps;
+
+template <>
+struct LaneOps<float> {
+    using S = float;
+    static constexpr int kSides = 1;
+    __device__ __forceinline__ static float make(float a, float) { return a; }
+    __device__ __forceinline__ static float fma(float a, float b, float c) { return fmaf(a, b, c); }
+    __device__ __forceinline__ static float mul(float a, float b) { return a * b; }
+    __device__ __forceinline__ static float add(float a, float b) { return a + b; }
+    __device__ __forceinline__ static float up(float v, int G) { return __shfl_up_sync(kFullMask, v, 1, G); }
+    __device__ __forceinline__ static float sel(const bool (&p)[1], float a, float b) { return p[0] ? a : b; }
+    // the value all lanes (and sides) hold, in a uniform register
+    __device__ __forceinline__ static float uniform(float v) {
+        return __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(v)));
+    }
+    __device__ __forceinline__ static float side(float v, int) { return v; }
+    __device__ __forceinline__ static void reload(const void* p, float (&v)[4]) {
+        asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                     : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    }
+};
+
+template <>
+struct LaneOps<float2> {
+    using S = float;
+    static constexpr int kSides = 2;
+    __device__ __forceinline__ static float2 make(float a, float b) { return make_float2(a, b); }
+    __device__ __forceinline__ static float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+    __device__ __forceinline__ static float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+    __device__ __forceinline__ static float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+    __device__ __forceinline__ static float2 up(float2 v, int G) {
+        return make_float2(__shfl_up_sync(kFullMask, v.x, 1, G), __shfl_up_sync(kFullMask, v.y, 1, G));
+    }
+    __device__ __forceinline__ static float2 sel(const bool (&p)[2], float2 a, float2 b) {
+        return make_float2(p[0] ? a.x : b.x, p[1] ? a.y : b.y);
+    }
+    __device__ __forceinline__ static float2 uniform(float2 v) {
+        const float u = LaneOps<float>::uniform(v.x);
+        return make_float2(u, u);
+    }
+    __device__ __forceinline__ static float side(float2 v, int s) { return s ? v.y : v.x; }
+    __device__ __forceinline__ static void reload(const void* p, float2 (&v)[2]) {
+        asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y)
+                     : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    }
+};
+
+// Boundary value of D (times beta it is what the first column receives); the
+// pair's scale is kTileD0 * H, D being 1/H there.
+constexpr float kTileD0 = FLT_MAX / 8.0f;
+
+// Smallest sum of T the FP32 pass keeps.  N, I and D^ each round by at most 2^-150
+// in the denormal range; as terms of T they weigh at most 1/n, 1 and d, range being
+// the read's largest 1/n + 2*(1 + d), and every path reaches the last position at
+// most once, so S >= L*H*2^-127*range keeps the error below 2^-23 of S.  The second
+// term is rescue_threshold in this scale (the sum there is beta*T over
+// (FLT_MAX/16)/H): no pair that wavefront_fp32.cuh would pass on is kept here.
+__device__ __forceinline__ float tile_threshold(int L, int H, float range) {
+    const float cells = (float)L * (float)H * 0x1p-127f;
+    return fmaxf(cells * range, 3.0f * cells * (float)H * (2.0f / kBeta));
+}
+
+// One read position's coefficients for this kernel (w, x, l of a match, l of a
+// mismatch) from its own and the next position's gap probabilities; past the read's
+// end a_next = beta and d_next = d.  l takes n from the rounded w of the next
+// column, so that w and l multiply to alpha*lambda up to l's own rounding: where
+// every position has the same gap quality a rounding of both would add up along
+// the read.
+__device__ __forceinline__ float tile_weight(float a, float d, float beta) { return a / (beta * d); }
+__device__ __forceinline__ float4 tile_coefficients(float p, float d, float s, float a_next, float d_next, float beta) {
+    const float w = tile_weight(1.0f - (d + s), d, beta);
+    const float wn = tile_weight(a_next, d_next, beta);
+    float g = beta * d_next, e = 0.0f;  // beta*n
+    if (wn != 0.0f) {
+        g = a_next / wn;
+        e = fmaf(-g, wn, a_next) / wn;
+    }
+    const float lm = 1.0f - p;   // pairhmm_kernels.cuh:1244
+    const float lx = p / 3.0f;   // pairhmm_kernels.cuh:1250
+    return make_float4(w, s == d_next ? 1.0f : beta * s / g, fmaf(lm, g, lm * e), fmaf(lx, g, lx * e));
+}
+
+// What the preparation notes per read.
+struct ReadMeta {
+    float w_end;     // 1/n of the last position
+    float range;     // see tile_threshold
+    uint32_t key;    // gap quality | gcp << 8 where insertions and deletions have the one quality at
+                     // every position, else kNoKey
+    uint32_t flags;  // bit 0: some |alpha| < kMinAlpha, the FP64 pass computes the read's pairs
+};
+static_assert(sizeof(ReadMeta) == 16, "ReadMeta is one 16-byte word");
+constexpr uint32_t kNoKey = 0xffffffffu;
+
+template <class V, int G, int R, int W, bool GCP>
+struct TileWavefront {
+    using O = LaneOps<V>;
+    using S = typename O::S;
+    static_assert(W == 1 || G == 32, "a group of several warps fills them");
+    static_assert(R >= 2, "a lane holds R or R-1 positions, at least one");
+    static constexpr int NS = O::kSides;
+    static constexpr int NG = 32 / G;    // groups per warp
+    static constexpr int NL = G * W;     // lanes per group
+    static constexpr int VN = 16 / (int)sizeof(V);     // values per 16-byte table word
+    static constexpr int Q = (R + VN - 1) / VN;        // table words per lane and code
+    static constexpr int kTableWords = 5 * Q * 32;     // per warp
+    static constexpr int kBlock = 16;    // steps between block barriers (W > 1)
+    // blocks a warp runs behind the one before it: row j leaves that warp's last lane
+    // at step j + 31, and the step before row j takes it, so block b needs the other's
+    // block b + 2 finished
+    static constexpr int kLag = 3;
+    static constexpr int kRing = 64;     // rows per ring; reader and writer are within 32 rows
+    struct alignas(16) Word { V v[VN]; };
+    struct alignas(16) RingRow { V n, i, x; };
+    static constexpr size_t kSmemBytes = (size_t)kTableWords * sizeof(Word);  // per warp, the table
+    static constexpr size_t kRingBytes = W > 1 ? (size_t)(W - 1) * kRing * sizeof(RingRow) : 0;  // per block
+
+    struct Reads {
+        const float4* coef[NS];     // the read's coefficients, position 0 first
+        const uint32_t* pack[NS];   // packed words (the base code in the low byte)
+        int L[NS];
+        S w_end[NS];
+        S eps[NS];                  // GCP only
+    };
+
+    template <bool UNI>
+    __device__ __forceinline__ static void loop(const Reads& rd, const uint32_t* hw, int H, int K, Word* tab,
+                                                RingRow* ring, int t, int warp, int lane, double (&acc)[NS]) {
+        const int u = warp * 32 + t;   // lane of the group
+        bool full[NS];
+        V wv[UNI ? 1 : R], xv[UNI ? 1 : R], N[R], D[R];
+        {
+            float w[NS][UNI ? 1 : R], x[NS][UNI ? 1 : R];
+            int p0[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const int m = rd.L[s] - NL * (R - 1);
+                full[s] = u < m;
+                p0[s] = u * (R - 1) + min_i(u, m);
+                if constexpr (UNI) w[s][0] = __ldg(&rd.coef[s]->x);
+            }
+            if constexpr (!UNI) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float2 wx = p0[s] + r < rd.L[s]
+                                              ? __ldg(reinterpret_cast<const float2*>(rd.coef[s] + p0[s] + r))
+                                              : make_float2(0.f, 0.f);
+                        w[s][r] = wx.x;
+                        x[s][r] = wx.y;
+                    }
+                // w and x go through the lane's table slots once: kept as loaded, in 16-byte
+                // coefficient words, ptxas put their pairs together again at every step
+                // (three moves a position, a quarter of the step)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    Word ww, xw;
+#pragma unroll
+                    for (int k = 0; k < VN; ++k) {
+                        const int r = q * VN + k < R ? q * VN + k : R - 1;
+                        ww.v[k] = O::make(w[0][r], w[NS - 1][r]);
+                        xw.v[k] = O::make(x[0][r], x[NS - 1][r]);
+                    }
+                    tab[q * 32 + lane] = ww;
+                    tab[(Q + q) * 32 + lane] = xw;
+                }
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    V ww[VN], xw[VN];
+                    O::reload(tab + q * 32 + lane, ww);
+                    O::reload(tab + (Q + q) * 32 + lane, xw);
+#pragma unroll
+                    for (int k = 0; k < VN; ++k)
+                        if (q * VN + k < R) {
+                            wv[q * VN + k] = ww[k];
+                            xv[q * VN + k] = xw[k];
+                        }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                Word words[5];
+#pragma unroll
+                for (int k = 0; k < VN; ++k) {
+                    const int r = q * VN + k;
+                    float l[NS][5];
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        float2 cf = make_float2(0.f, 0.f);
+                        uint32_t code = 0;
+                        const int c = p0[s] + r;
+                        if (r < R && c < rd.L[s]) {
+                            cf = __ldg(reinterpret_cast<const float2*>(rd.coef[s] + c) + 1);
+                            code = __ldg(rd.pack[s] + c) & 0xffu;
+                        }
+#pragma unroll
+                        for (int h = 0; h < 5; ++h)
+                            l[s][h] = (code == 4u || h == 4 || code == (uint32_t)h) ? cf.x : cf.y;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 5; ++h) words[h].v[k] = O::make(l[0][h], l[NS - 1][h]);
+                    if (r < R) {
+                        N[r] = O::make(0.f, 0.f);
+                        D[r] = O::make(0.f, 0.f);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 5; ++h) tab[(h * Q + q) * 32 + lane] = words[h];
+            }
+            if constexpr (UNI) {
+                wv[0] = O::uniform(O::make(w[0][0], w[NS - 1][0]));
+            }
+        }
+        V eps = O::make(kEps, kEps);
+        if constexpr (GCP) {
+            eps = O::make(rd.eps[0], rd.eps[NS - 1]);
+            if constexpr (UNI) eps = O::uniform(eps);
+        }
+        const V wend = O::make(rd.w_end[0], rd.w_end[NS - 1]);
+        const V zero = O::make(0.f, 0.f), d0 = O::make(kTileD0, kTileD0);
+        const bool first = u == 0;
+        // the result lane adds the rows up to its pair's last step
+        const int kres = u == NL - 1 ? H + G - 1 : -1;
+
+        V Nl = zero;   // this lane's last N of the step before (the row T needs)
+        V Ml = zero, Mul = zero, Iul = zero, Xul = first ? d0 : zero;
+        int h = 4;
+        // code words of this group's haplotype; behind its end the last word is re-read
+        // (those rows are past the result's last one)
+        const int wlast = ((H + 15) & ~15) / 4 - 1;
+        uint32_t wcur = __ldg(hw);
+        uint32_t wnext = __ldg(hw + 1);
+        auto four_steps = [&](int k0) {
+            const uint32_t wpref = __ldg(hw + min_i((k0 >> 2) + 2, wlast));
+            V a4 = zero;
+#pragma unroll
+            for (int s4 = 0; s4 < 4; ++s4) {
+                const int k = k0 + s4;
+                int hn = __shfl_up_sync(kFullMask, h, 1, G);
+                if (t == 0) hn = (int)((wcur >> (8 * s4)) & 0xffu);
+                h = hn;
+                const Word* row = tab + h * (Q * 32) + lane;
+                // a position first forms what the next one takes from its old N, so that N is
+                // replaced in place (with the old N carried along instead, the compiler moves
+                // the lane's N by one register a step, on the FMA pipe)
+                V P = O::fma(Mul, wv[0], Xul), I = O::fma(Iul, eps, Mul), X = zero, Ip = zero, Xp = zero, Ilast = zero;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const Word lw = row[q * 32];
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) {
+                        const int r = q * VN + i;
+                        if (r < R) {
+                            if (r == R - 1) {
+                                Ip = Ilast;
+                                Xp = X;
+                            }
+                            if constexpr (UNI) X = O::add(D[r], I);
+                            else X = O::fma(D[r], xv[r], I);
+                            D[r] = O::fma(D[r], eps, N[r]);
+                            const V Nnew = O::mul(lw.v[i], P);
+                            Ilast = I;
+                            if (r + 1 < R) {
+                                P = O::fma(N[r], wv[UNI ? 0 : (r + 1 < R ? r + 1 : r)], X);
+                                I = O::fma(I, eps, N[r]);
+                            }
+                            N[r] = Nnew;
+                        }
+                    }
+                }
+                V Id = Ilast, Xd = X;
+                Id = O::sel(full, Id, Ip);
+                Xd = O::sel(full, Xd, Xp);
+                const V T = O::fma(Nl, wend, Id);
+                if (k <= kres) a4 = O::add(a4, T);
+                Nl = O::sel(full, N[R - 1], N[R - 2]);
+                if (W > 1 && warp + 1 < W && t == 31 && k >= 31)
+                    ring[warp * kRing + ((k - 31) & (kRing - 1))] = RingRow{Nl, Id, Xd};
+                Mul = Ml;
+                Ml = O::up(Nl, G);
+                Iul = O::up(Id, G);
+                Xul = O::up(Xd, G);
+                if (W > 1 && warp > 0) {
+                    const RingRow b = ring[(warp - 1) * kRing + ((k + 1) & (kRing - 1))];  // broadcast
+                    if (t == 0) {
+                        Ml = b.n;
+                        Iul = b.i;
+                        Xul = b.x;
+                    }
+                } else if (first || (W == 1 && t == 0)) {
+                    Ml = zero;
+                    Iul = zero;
+                    Xul = d0;
+                }
+            }
+            if (kres >= 0) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) acc[s] += (double)O::side(a4, s);
+            }
+            wcur = wnext;
+            wnext = wpref;
+        };
+        if constexpr (W == 1) {
+            for (int k0 = 0; k0 < K; k0 += 4) four_steps(k0);
+        } else {
+            const int nblk = (H + 32 + kBlock - 1) / kBlock;
+            const int nsuper = nblk + kLag * (W - 1);
+            for (int ss = 0; ss < nsuper; ++ss) {
+                const int b = ss - kLag * warp;
+                if (b >= 0 && b < nblk) {  // warp-uniform
+                    if (b == 0 && warp > 0) {  // row 0, before the first step
+                        const RingRow r0 = ring[(warp - 1) * kRing];
+                        if (t == 0) {
+                            Ml = r0.n;
+                            Iul = r0.i;
+                            Xul = r0.x;
+                        }
+                    }
+                    for (int k0 = b * kBlock; k0 < (b + 1) * kBlock; k0 += 4) four_steps(k0);
+                }
+                __syncthreads();
+            }
+        }
+    }
+};
+
+}  // namespace phmm

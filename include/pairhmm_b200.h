@@ -199,11 +199,14 @@ pairhmm_status_t pairhmm_serving_stats(pairhmm_engine_t* engine, pairhmm_serving
  * group[i] lanes holding regs[i] read positions each (tile = group*regs).
  * kind[i] (the `multi_tile` argument): 0 = one tile, 1 = several tiles
  * (reads longer than the tile), 2 = one tile with two reads of a record per
- * group in packed FP32 arithmetic.  This is the run-time form of the
+ * group in packed FP32 arithmetic, 3 = the same with exact tiles (the class must
+ * lie within (group*(regs-1), group*regs]), 4 = exact tiles over a block of
+ * group/32 warps, one read per group.  This is the run-time form of the
  * reference's compile-time tuning tables (tuningconfigs.hpp:33-269) and of its
  * partition rule "first tile size >= read length" (utility_kernels.cuh:45-57).
  * Only compiled (group, regs, kind) triples are accepted; the last entry must
- * be multi-tile.
+ * be of kind 1.  The default table has a twin for batches of few pairs, which
+ * pairhmm_get_tile_table does not list; results are the same with either.
  */
 pairhmm_status_t pairhmm_set_tile_table(pairhmm_engine_t* engine, const int32_t* max_len, const int32_t* group,
                                         const int32_t* regs, const int32_t* multi_tile, int32_t n);

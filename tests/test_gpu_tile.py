@@ -1,0 +1,104 @@
+"""Exact-tile kernels (wavefront_tile.cuh): every tile's shortest and longest read and
+one in between, against the FP64 oracle (parity tolerance, conftest); and the
+property the tables rely on, that a pair's score does not depend on the group's
+shape, on the reads that share its group, or on which path (one gap quality or
+per-position coefficients) its warp took: bitwise."""
+import numpy as np
+import pytest
+
+import gpupairhmm_b200 as g
+import oracle
+from conftest import assert_log10_close
+from gpupairhmm_b200.synth import ACGT, _Builder
+
+pytestmark = pytest.mark.gpu
+
+
+def _records(lengths, gaps, seed, extra=(1, 60), reads=3):
+    """One record per read length: reads cut from the first haplotype (1% errors),
+    the last read unrelated; gap qualities one value per batch ("one"), one per read
+    ("read") or one per position ("each"); gcp qualities per read."""
+    rng = np.random.default_rng(seed)
+    b = _Builder()
+    gcp = []
+    for L in lengths:
+        H = L + rng.integers(*extra, size=2)
+        H[1] = max(1, int(H[1]) - L // 2)
+        base = ACGT[rng.integers(0, 4, size=int(H.max()))]
+        rs = []
+        for i in range(reads):
+            r = base[:L].copy() if i + 1 < reads else ACGT[rng.integers(0, 4, size=L)]
+            m = rng.random(L) < 0.01
+            r[m] = ACGT[rng.integers(0, 4, size=int(m.sum()))]
+            rs.append(r)
+        n = reads * L
+        if gaps == "one":
+            iq = dq = np.full(n, 40)
+        elif gaps == "read":
+            iq = dq = np.repeat(rng.integers(20, 46, size=reads), L)
+        else:
+            iq, dq = rng.integers(10, 46, size=n), rng.integers(10, 46, size=n)
+        b.add_concat(np.full(reads, L), np.concatenate(rs), rng.integers(2, 41, size=n).astype(np.uint8),
+                     iq.astype(np.uint8), dq.astype(np.uint8), H, np.concatenate([base[:h] for h in H]))
+        gcp += [np.repeat(rng.integers(1, 45, size=reads), L)]
+    batch = b.build()
+    q = np.concatenate(gcp)
+    off = np.asarray(batch.read_offsets)
+    at = 0
+    for o, L in zip(off, batch.read_lengths):
+        batch.gcp_quals[o:o + L] = q[at:at + L]
+        at += L
+    return batch
+
+
+def _edges(rules):
+    out, lo = [], 0
+    for max_len, G, R, kind in rules:
+        if kind >= 3:
+            out += [lo + 1, (lo + 1 + max_len) // 2, max_len]
+        lo = max_len
+    return sorted(set(out))
+
+
+@pytest.mark.parametrize("gcp", [False, True])
+@pytest.mark.parametrize("gaps", ["one", "read", "each"])
+@pytest.mark.parametrize("small", [False, True])
+def test_exact_tiles_match_oracle(small, gaps, gcp):
+    """small: the default engine's table for few pairs (32 lanes); else the same
+    batch on an engine that always takes the table for many."""
+    with g.Engine(gcp=gcp) as e:
+        rules = e.tile_table()
+        if not small:
+            # any other table than the default one has no second table
+            e.set_tile_table([(rules[0][0] - 1,) + rules[0][1:]] + rules[1:] if rules[0][3] != 0 else
+                             [(8, 4, 16 if gcp else 4, 0)] + rules)
+        b = _records(_edges(rules), gaps, seed=7 + len(gaps))
+        got = e.compute(b)
+    assert_log10_close(got, oracle.batch_log10(b, gcp=gcp), what=f"{gaps} gcp={gcp} small={small}")
+
+
+@pytest.mark.parametrize("gcp", [False, True])
+@pytest.mark.parametrize("gaps", ["one", "read", "each"])
+def test_score_does_not_depend_on_group_shape(gaps, gcp):
+    """Reads of 129-160 (8 x 17..20 or 32 x 5) and 161-320 positions (16 x 11..20 or
+    32 x 6..10), many per record so that units pair different reads."""
+    b = _records([129, 136, 137, 150, 160, 161, 176, 200, 320], gaps, seed=3, reads=5)
+    with g.Engine(gcp=gcp) as e:
+        rules = e.tile_table()
+        few = e.compute(b)
+        e.set_tile_table([(8, 4, 16 if gcp else 4, 0)] + rules)   # the table for many pairs
+        many = e.compute(b)
+        one = e.compute(b.select_records(3, 4))
+    np.testing.assert_array_equal(few, many)
+    np.testing.assert_array_equal(one, many[3 * 10:4 * 10])
+
+
+def test_exact_rules_are_checked():
+    with g.Engine() as e:
+        e.set_tile_table([(152, 32, 24, 0), (160, 8, 20, 3), (1 << 30, 32, 32, 1)])
+        assert e.tile_table()[1] == (160, 8, 20, 3)
+        for bad in ([(151, 32, 24, 0), (160, 8, 20, 3), (1 << 30, 32, 32, 1)],   # 152 is one lane's worth short
+                    [(152, 32, 24, 0), (161, 8, 20, 3), (1 << 30, 32, 32, 1)],   # longer than the tile
+                    [(152, 32, 24, 0), (156, 4, 39, 3), (1 << 30, 32, 32, 1)]):  # not compiled
+            with pytest.raises(g.PairHMMError):
+                e.set_tile_table(bad)
