@@ -221,7 +221,7 @@ pairhmm_status_t pairhmm_batch_counts(const pairhmm_batch_t* batch, int64_t* pai
     std::string err;
     pairhmm_status_t s;
     try {
-        s = phmm::Engine::build_index(*batch, {{1 << 30, 32, 32, true, false}}, x, err);
+        s = phmm::Engine::build_index(*batch, {{1 << 30, 32, 32, true, false}}, phmm::Fp64Table{}, x, err);
     } catch (...) {
         return PAIRHMM_ERR_OUT_OF_MEMORY;
     }
@@ -353,7 +353,7 @@ pairhmm_status_t pairhmm_set_tile_table(pairhmm_engine_t* h, const int32_t* max_
         for (int i = 0; i < n; ++i) {
             const int k = multi_tile[i];
             if (k < 0 || k > 4) return PAIRHMM_ERR_INVALID_ARGUMENT;
-            rules[i] = {max_len[i], group[i], regs[i], k == 1 || k == 4, k == 2 || k == 3, k >= 3};
+            rules[i] = {max_len[i], group[i], regs[i], k == 1 || (k >= 3 && max_len[i] > 1024), k == 2 || k == 3, k >= 3};
         }
         return finish(h, h->engine->set_tile_table(rules));
     });
@@ -369,7 +369,7 @@ pairhmm_status_t pairhmm_get_tile_table(pairhmm_engine_t* h, int32_t* max_len, i
         max_len[i] = r[i].max_len;
         group[i] = r[i].G;
         regs[i] = r[i].R;
-        multi_tile[i] = r[i].exact ? (r[i].multi_tile ? 4 : 3) : r[i].multi_tile ? 1 : r[i].packed ? 2 : 0;
+        multi_tile[i] = r[i].exact ? (r[i].packed ? 3 : 4) : r[i].multi_tile ? 1 : r[i].packed ? 2 : 0;
     }
     return PAIRHMM_OK;
 }

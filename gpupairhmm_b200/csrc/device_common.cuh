@@ -61,17 +61,25 @@ struct Item {
 };
 static_assert(sizeof(Item) == 32, "Item must be 32 bytes");
 
-// Where the FP64 pass's scaled tier sends the pairs beyond its range: the
-// extended tier's class lists (same class offsets as the rescue lists) and
-// their counts.
+// Length classes of the FP64 pass (one list and one launch each); at most as many
+// extended-tier classes.
+constexpr int kMaxFp64Classes = 64;
+// read length -> class, lengths above kFp64LutMax in the last entry
+constexpr int kFp64LutMax = 4096;
+constexpr int kFp64LutSize = kFp64LutMax + 2;
+
+// Where a launch of the FP64 pass's scaled tier sends the pairs beyond its range:
+// list `cls` of the extended tier.
 struct ExtList {
     Task* base;
-    const long long* off;        // [kFp64Classes]
-    unsigned long long* count;   // [kFp64Classes]
+    const long long* off;        // [kMaxFp64Classes]
+    unsigned long long* count;   // [kMaxFp64Classes]
+    int cls;
+    __device__ __forceinline__ void append(const Task& t) const {
+        const unsigned long long slot = atomicAdd(count + cls, 1ull);
+        base[off[cls] + (long long)slot] = t;
+    }
 };
-
-struct DevView;
-__device__ __forceinline__ void append_rescue(const DevView& v, int cls, const Task& t);
 
 struct ReadMeta;
 
@@ -85,9 +93,10 @@ struct DevView {
     const int64_t* hap_start;  // in bytes, multiple of 16
     const int32_t* hap_len;
     float* scores;
-    Task* rescue_base;          // flagged pairs, one list per read-length class (fp64_class)
-    const long long* rescue_off;  // [kFp64Classes] start of each class list in rescue_base
-    unsigned long long* rescue_count;  // [kFp64Classes]
+    Task* rescue_base;          // flagged pairs, one list per read-length class
+    const uint8_t* rescue_class;  // [kFp64LutSize] class of a read length
+    const long long* rescue_off;  // [kMaxFp64Classes] start of each class list in rescue_base
+    unsigned long long* rescue_count;  // [kMaxFp64Classes]
     int rescue_enabled;
     const float* ph2pr;         // 128 floats in global memory
     // gcp mode only (else null): the gcp quality of each read's first position,
@@ -103,17 +112,9 @@ __device__ __forceinline__ uint32_t code_of(uint8_t c) {
 
 __device__ __forceinline__ int min_i(int a, int b) { return a < b ? a : b; }
 
-// FP64 pass length classes (tile = G x R): 64 = 4x16, 96 = 8x12, 128 = 8x16,
-// 160 = 16x10, 192 = 16x12, 256 = 16x16, then 32x16 multi-tile for longer reads.
-constexpr int kFp64Classes = 7;
-constexpr int kFp64ClassMax[kFp64Classes - 1] = {64, 96, 128, 160, 192, 256};
-__host__ __device__ __forceinline__ int fp64_class(int L) {
-    return L <= 64 ? 0 : L <= 96 ? 1 : L <= 128 ? 2 : L <= 160 ? 3 : L <= 192 ? 4 : L <= 256 ? 5 : 6;
-}
-
-// Appends a flagged pair to its FP64 class list (rare: one global load for the
-// list start).
-__device__ __forceinline__ void append_rescue(const DevView& v, int cls, const Task& t) {
+// Appends a flagged pair to the FP64 list of its read's length.
+__device__ __forceinline__ void append_rescue(const DevView& v, int L, const Task& t) {
+    const int cls = v.rescue_class[min_i(L, kFp64LutMax + 1)];
     const unsigned long long slot = atomicAdd(v.rescue_count + cls, 1ull);
     v.rescue_base[v.rescue_off[cls] + (long long)slot] = t;
 }

@@ -13,6 +13,7 @@
 // and every bucket's range of work items from the record structure it already
 // holds.
 #include <algorithm>
+#include <bitset>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -31,35 +32,42 @@ constexpr int64_t kScratchBudget = int64_t(4) << 30;  // border scratch cap per 
 // task counters, then per FP64 length class the scaled tier's list counts, the
 // extended tier's list counts, and the two tiers' task counters.
 constexpr int kCtrScaled = kMaxBuckets;
-constexpr int kCtrExt = kMaxBuckets + kFp64Classes;
-constexpr int kCtrTaskScaled = kMaxBuckets + 2 * kFp64Classes;
-constexpr int kCtrTaskExt = kMaxBuckets + 3 * kFp64Classes;
-constexpr int kCtrTotal = kMaxBuckets + 4 * kFp64Classes;
+constexpr int kCtrExt = kMaxBuckets + kMaxFp64Classes;
+constexpr int kCtrTaskScaled = kMaxBuckets + 2 * kMaxFp64Classes;
+constexpr int kCtrTaskExt = kMaxBuckets + 3 * kMaxFp64Classes;
+constexpr int kCtrTotal = kMaxBuckets + 4 * kMaxFp64Classes;
+// pairs up to which the FP64 lists are not sorted by haplotype length: at most two
+// rounds of resident warps, so the order decides little and the three launches of the
+// sort are a third of the stage of a small batch
+constexpr int64_t kNoSortPairs = 4096;
 // multi-tile FP64 pairs up to which the two tiers run fused (about one round of
 // resident warps of that class's kernel on 148 SMs)
 constexpr int64_t kFuseMaxPairs = 2048;
 
+// Reads beyond this count as multi-tile (the stats' multi_tile_pairs, the serving
+// queue's slots), on whatever kernel they run.
+constexpr int kLongRead = 1024;
+
 // Exact tiles for reads of lo+1 .. hi positions on groups of G lanes, one rule per
 // R (a lane's positions).
 void add_exact_rules(std::vector<TileRule>& rules, int G, int lo, int hi) {
-    for (int R = lo / G + 1; R * G <= hi; ++R) rules.push_back({R * G, G, R, G > 32, G <= 32, true});
+    for (int R = lo / G + 1; R * G <= hi; ++R)
+        rules.push_back({R * G, G, R, R * G > kLongRead, G <= 32, true});
 }
 
 std::vector<TileRule> engine_default_rules() {
     // The two shortest classes keep the padded tiles autotune.py picked for them;
     // from 33 positions on exact tiles with as many positions per lane as fit (the
     // per-step work of a lane is amortised over them) and at least 11 once a group
-    // of 16 or 32 lanes is needed.
+    // of 16 or 32 lanes is needed.  Reads of 641-2,048 positions: one warp with two or
+    // three parts in turn; beyond, blocks of 8 warps.
     std::vector<TileRule> rules = {{16, 4, 4, false, false}, {32, 4, 8, false, true}};
     add_exact_rules(rules, 8, 32, 160);
     add_exact_rules(rules, 16, 160, 320);
     add_exact_rules(rules, 32, 320, 640);
-    rules.push_back({768, 32, 24, false});
-    rules.push_back({896, 32, 28, false});
-    rules.push_back({1024, 32, 32, false});
-    rules.push_back({1280, 32, 20, true});
-    rules.push_back({1536, 32, 24, true});
-    rules.push_back({1792, 32, 28, true});
+    add_exact_rules(rules, 64, 640, 1536);
+    add_exact_rules(rules, 96, 1536, 2016);
+    add_exact_rules(rules, 256, 1792, 4096);
     rules.push_back({1 << 30, 32, 32, true});
     return rules;
 }
@@ -84,19 +92,26 @@ std::vector<TileRule> gcp_rules() {
     add_exact_rules(rules, 8, 32, 160);
     add_exact_rules(rules, 16, 160, 320);
     add_exact_rules(rules, 32, 320, 640);
-    rules.push_back({1024, 32, 32, false});
+    add_exact_rules(rules, 64, 640, 1536);
+    add_exact_rules(rules, 96, 1536, 2016);
+    add_exact_rules(rules, 256, 1792, 4096);
     rules.push_back({1 << 30, 32, 32, true});
     return rules;
 }
 
 // The table of a batch of few pairs: the same, with 32 lanes a group wherever an
-// exact tile has fewer.  Results do not change: the exact tiles' do not depend on the
+// exact tile has fewer, and blocks of 8 warps (256 lanes) from 641 positions on.  Results do not change: the exact tiles' do not depend on the
 // shape, and the other classes stay.
 std::vector<TileRule> small_rules(const std::vector<TileRule>& rules) {
     std::vector<TileRule> small;
     for (size_t i = 0; i < rules.size(); ++i) {
-        if (!rules[i].exact || rules[i].G > 32) {
+        if (!rules[i].exact || rules[i].G == 256) {
             small.push_back(rules[i]);
+            continue;
+        }
+        if (rules[i].G > 32) {   // 641-2,016 positions; the blocks start at 1,793
+            while (i + 1 < rules.size() && rules[i + 1].exact && rules[i + 1].G < 256) ++i;
+            add_exact_rules(small, 256, 512, 1792);
             continue;
         }
         const int lo = i ? rules[i - 1].max_len : 0;
@@ -104,6 +119,63 @@ std::vector<TileRule> small_rules(const std::vector<TileRule>& rules) {
         add_exact_rules(small, 32, lo, rules[i].max_len);
     }
     return small;
+}
+
+// FP64 classes: exact tiles on groups of 8-32 lanes (wide: 32); from 641 positions on
+// blocks of 4 warps (wide, and from 2,049 on: 8); padded kernels for the shortest and
+// the longest reads.  One warp with the parts in turn was no faster where the pairs
+// fill the chip (400 long-read regions 74.5 against 75.1 ms, 64 regions 13.8 against
+// 13.3), although it can stop at a part's end, and needs border rows in memory.  The
+// extended tier, which few pairs reach, has the padded kernels up to 640 positions.
+pairhmm_status_t make_fp64_table(bool wide, bool gcp, Fp64Table& t) {
+    struct Span { int G, lo, hi; };
+    const std::vector<Span> narrow = {{8, 32, 160}, {16, 160, 320}, {32, 320, 640}};
+    std::vector<Span> spans = wide ? std::vector<Span>{{32, 32, 640}} : narrow;
+    if (wide) spans.push_back({256, 512, 2048});   // from 641 on: the classes before it end there
+    else spans.push_back({128, 640, 2048});
+    spans.push_back({256, 2048, 4096});
+    struct Padded { int max_len, G, R; };
+    static constexpr Padded kExt[] = {{64, 4, 16},   {96, 8, 12},    {128, 8, 16}, {160, 16, 10},
+                                      {192, 16, 12}, {256, 16, 16}, {640, 32, 16}};
+    auto ext_of = [&](int hi, int G, int R) {
+        // padded extended kernels are shared by the classes within their bound
+        if (G <= 32 && hi <= 640) {
+            const Padded* e = kExt;
+            while (hi > e->max_len) ++e;
+            const Fp64Config* cfg = find_fp64_config(e->G, e->R, false, true, gcp);
+            if (!t.exts.empty() && t.exts.back().cfg == cfg) return (int)t.exts.size() - 1;
+            t.exts.push_back({cfg, 0, 0, false});
+        } else {
+            // blocks of 8 warps whatever the scaled tier has: few pairs come this far, and one
+            // warp alone would still be on its first pair when the other classes are done
+            t.exts.push_back({G > 32 ? find_fp64_config(256, (hi + 255) / 256, true, true, gcp)
+                                     : find_fp64_config(G, R, false, true, gcp), 0, 0, true});
+        }
+        return (int)t.exts.size() - 1;
+    };
+    auto add = [&](int hi, int G, int R, bool exact) {
+        t.classes.push_back({hi, find_fp64_config(G, R, exact, false, gcp), ext_of(hi, G, R)});
+    };
+    add(32, 4, 16, false);
+    for (const Span& sp : spans)
+        for (int R = sp.lo / sp.G + 1; R * sp.G <= sp.hi; ++R) add(R * sp.G, sp.G, R, true);
+    add(INT32_MAX, 32, 16, false);
+    t.fused = find_fp64_config(32, 16, false, false, gcp, true);
+    if (!t.fused || t.classes.size() > kMaxFp64Classes) return PAIRHMM_ERR_UNSUPPORTED;
+    for (size_t c = 0; c < t.classes.size(); ++c) {
+        Fp64Table::Ext& e = t.exts[t.classes[c].ext];
+        if (!t.classes[c].scaled || !e.cfg) return PAIRHMM_ERR_UNSUPPORTED;
+        const Fp64Config& k = *t.classes[c].scaled;   // exact: more than G*(R-1) positions
+        if (k.exact && (c ? t.classes[c - 1].max_len : 0) < k.G * (k.R - 1)) return PAIRHMM_ERR_UNSUPPORTED;
+        if (c == 0 || t.classes[c - 1].ext != t.classes[c].ext) e.first = (int)c;
+        e.last = (int)c;
+    }
+    t.lut.resize(kFp64LutSize);
+    for (int L = 0, c = 0; L < kFp64LutSize; ++L) {
+        while (L > t.classes[c].max_len) ++c;
+        t.lut[L] = (uint8_t)c;
+    }
+    return PAIRHMM_OK;
 }
 
 inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -141,6 +213,26 @@ void DevBuf::release() {
 }
 
 namespace {
+// what is wrong with a tile table (null: nothing)
+const char* check_rules(const std::vector<TileRule>& rules, bool gcp) {
+    if (rules.empty() || (int)rules.size() > kMaxBuckets) return "tile table size";
+    for (size_t i = 0; i < rules.size(); ++i) {
+        if (rules[i].packed && rules[i].multi_tile)
+            return "packed rules are single tile";
+        if (!find_fp32_config(rules[i].G, rules[i].R, rules[i].multi_tile, rules[i].packed, rules[i].exact,
+                              gcp))
+            return "tile table names a configuration that is not compiled";
+        if (i > 0 && rules[i].max_len <= rules[i - 1].max_len)
+            return "tile table bounds must increase";
+        if ((!rules[i].multi_tile || rules[i].exact) && rules[i].max_len > rules[i].G * rules[i].R)
+            return "single-tile rule shorter than its bucket";
+        if (rules[i].exact && (i ? rules[i - 1].max_len : 0) < rules[i].G * (rules[i].R - 1))
+            return "exact tile for reads of fewer positions than it takes";
+    }
+    if (!rules.back().multi_tile || rules.back().exact) return "last rule must be multi-tile";
+    return nullptr;
+}
+
 std::vector<TileRule> default_rules(const pairhmm_options_t& o) {
     return o.mode == PAIRHMM_MODE_PLAIN ? plain_rules() : o.gcp ? gcp_rules() : engine_default_rules();
 }
@@ -154,7 +246,7 @@ std::vector<DevBuf*> Engine::all_buffers() {
             &read_record_, &read_local_, &rec_haps_, &rec_hap_base_, &rec_pair_base_, &read_start_,
             &hap_start_, &read_pack_, &read_coef_, &read_meta_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
             &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
-            &rescue_ext_, &rsort_,
+            &rescue_ext_, &rsort_, &fp64_lut_[0], &fp64_lut_[1],
             &in_gq_, &read_gcp_};
 }
 
@@ -237,7 +329,7 @@ pairhmm_status_t Engine::init() {
             b->stream = stream_;
         }
     }
-    PHMM_CUDA(cudaMallocHost(&host_hdr_, 256));
+    PHMM_CUDA(cudaMallocHost(&host_hdr_, sizeof(unsigned long long) * 2 * kMaxFp64Classes));
     PHMM_CUDA(cudaEventCreate(&ev0_));
     PHMM_CUDA(cudaEventCreate(&ev1_));
     PHMM_CUDA(cudaEventCreate(&ev_prep_));
@@ -250,7 +342,13 @@ pairhmm_status_t Engine::init() {
     PHMM_CUDA(cudaMemcpy(ph2pr_.ptr, table, sizeof(table), cudaMemcpyHostToDevice));
     PHMM_CUDA(counters_.ensure(sizeof(unsigned long long) * kCtrTotal));
     // FP64 list sort: per-class histogram (uint32) then cursors (uint64)
-    PHMM_CUDA(rsort_.ensure((sizeof(unsigned int) + sizeof(unsigned long long)) * kFp64Classes * kRescueHBins));
+    PHMM_CUDA(rsort_.ensure((sizeof(unsigned int) + sizeof(unsigned long long)) * kMaxFp64Classes * kRescueHBins));
+    for (int w = 0; w < 2; ++w) {
+        if (make_fp64_table(w == 1, opts_.gcp != 0, fp64_tables_[w]) != PAIRHMM_OK)
+            return fail(PAIRHMM_ERR_UNSUPPORTED, "FP64 class without compiled kernel");
+        PHMM_CUDA(fp64_lut_[w].ensure(kFp64LutSize));
+        PHMM_CUDA(cudaMemcpy(fp64_lut_[w].ptr, fp64_tables_[w].lut.data(), kFp64LutSize, cudaMemcpyHostToDevice));
+    }
     ready_ = true;
     return build_tables(default_rules(opts_));
 }
@@ -260,21 +358,8 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
         const pairhmm_status_t t = twin_->set_tile_table(rules);
         if (t != PAIRHMM_OK) return fail(t, twin_->last_error());
     }
-    if (rules.empty() || (int)rules.size() > kMaxBuckets) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table size");
-    for (size_t i = 0; i < rules.size(); ++i) {
-        if (rules[i].packed && rules[i].multi_tile)
-            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "packed rules are single tile");
-        if (!find_fp32_config(rules[i].G, rules[i].R, rules[i].multi_tile, rules[i].packed, rules[i].exact,
-                              opts_.gcp != 0))
-            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table names a configuration that is not compiled");
-        if (i > 0 && rules[i].max_len <= rules[i - 1].max_len)
-            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table bounds must increase");
-        if ((!rules[i].multi_tile || rules[i].exact) && rules[i].max_len > rules[i].G * rules[i].R)
-            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "single-tile rule shorter than its bucket");
-        if (rules[i].exact && (i ? rules[i - 1].max_len : 0) < rules[i].G * (rules[i].R - 1))
-            return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "exact tile for reads of fewer positions than it takes");
-    }
-    if (!rules.back().multi_tile || rules.back().exact) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "last rule must be multi-tile");
+    const char* wrong = check_rules(rules, opts_.gcp != 0);
+    if (wrong) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, wrong);
     for (cudaGraphExec_t& g : graph_exec_) {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
@@ -288,14 +373,15 @@ pairhmm_status_t Engine::build_tables(const std::vector<TileRule>& rules) {
     TileTable built[2];
     built[0].rules = rules;
     if (rules == default_rules(opts_) && opts_.mode != PAIRHMM_MODE_PLAIN) built[1].rules = small_rules(rules);
-    for (TileTable& t : built)
+    for (TileTable& t : built) {
+        const char* wrong = t.rules.empty() ? nullptr : check_rules(t.rules, opts_.gcp != 0);
+        if (wrong) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, wrong);
         for (const TileRule& r : t.rules) {
             t.cfg.push_back(find_fp32_config(r.G, r.R, r.multi_tile, r.packed, r.exact, opts_.gcp != 0));
             if (!t.cfg.back()) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile rule without compiled kernel");
             t.exact = t.exact || r.exact;
         }
-    if (built[0].rules.size() > kMaxBuckets || built[1].rules.size() > kMaxBuckets)
-        return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile table size");
+    }
     for (int i = 0; i < 2; ++i) tables_[i] = std::move(built[i]);
     table_ = &tables_[0];
     return PAIRHMM_OK;
@@ -309,17 +395,26 @@ pairhmm_status_t Engine::build_tables(const std::vector<TileRule>& rules) {
 // 2,048 pairs 0.027 / 0.029, 4,096 pairs 0.045 / 0.031; (250) 1,024 pairs 0.043 / 0.062,
 // 2,048 pairs 0.072 / 0.066; uneven regions (13 classes) 395 pairs 0.057 / 0.088,
 // 6,500 pairs 0.19 / 0.24, 13,000 pairs 0.31 / 0.29, 27,000 pairs 0.48 / 0.40.
-void Engine::choose_table(int64_t pairs, const int32_t* read_lengths, int64_t num_reads) {
+// A long read's pair counts as the 8 warps it takes in the small table.
+void Engine::choose_table(int64_t num_records, const int32_t* reads_per_record, const int32_t* haps_per_record,
+                          const int32_t* read_lengths, int64_t pairs) {
     table_ = &tables_[0];
+    fp64_ = &fp64_tables_[0];
     if (tables_[1].rules.empty() || pairs > kSmallPairs * (int64_t)tables_[0].rules.size()) return;
-    uint64_t seen = 0;
-    static_assert(kMaxBuckets <= 64, "one bit per class");
-    for (int64_t i = 0; i < num_reads; ++i) seen |= uint64_t(1) << bucket_of_host(read_lengths[i], tables_[0].rules);
-    if (pairs <= kSmallPairs * __builtin_popcountll(seen)) table_ = &tables_[1];
+    std::bitset<kMaxBuckets> seen;
+    int64_t weight = 0, i = 0;
+    for (int64_t g = 0; g < num_records; ++g)
+        for (int32_t r = 0; r < reads_per_record[g]; ++r, ++i) {
+            seen.set(bucket_of_host(read_lengths[i], tables_[0].rules));
+            weight += (read_lengths[i] > 640 ? 8 : 1) * (int64_t)std::max(haps_per_record[g], 0);
+        }
+    if (weight > kSmallPairs * (int64_t)seen.count()) return;
+    table_ = &tables_[1];
+    fp64_ = &fp64_tables_[1];
 }
 
-pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector<TileRule>& rules, BatchIndex& x,
-                                     std::string& err) {
+pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector<TileRule>& rules,
+                                     const Fp64Table& fp64, BatchIndex& x, std::string& err) {
     // Scalars reset; vectors keep their storage between calls (an engine
     // reuses one index, so a batch of the same size touches no fresh pages).
     x.num_records = x.num_reads = x.num_haps = x.num_pairs = x.cells = 0;
@@ -328,7 +423,7 @@ pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector
     x.pack_positions = x.code_bytes = 0;
     x.multi_tile_pairs = 0;
     for (int64_t& c : x.class_pairs) c = 0;
-    for (int64_t& c : x.class_start) c = 0;
+    for (int64_t& c : x.list_start) c = 0;
     x.unit_read0.clear();
     x.unit_read1.clear();
     x.unit_bucket.clear();
@@ -438,7 +533,7 @@ pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector
             sl += L;
             const int bk = L <= lut_max ? lut[L] : bucket_of_host(L, rules);
             x.bucket_pairs[bk] += H;
-            x.class_pairs[fp64_class(L)] += H;
+            x.class_pairs[fp64.class_of(L)] += H;
             if (multi[bk]) x.multi_tile_pairs += H;
             if (packed[bk]) {
                 if (pending[bk] < 0) {
@@ -468,8 +563,9 @@ pairhmm_status_t Engine::build_index(const pairhmm_batch_t& b, const std::vector
     }
     {
         int64_t off = 0;
-        for (int c = 0; c < kFp64Classes; ++c) {
-            x.class_start[c] = off;
+        for (size_t c = 0; c < fp64.classes.size(); ++c) {
+            if ((int)c == fp64.exts[fp64.classes[c].ext].first) x.list_start[kMaxFp64Classes + fp64.classes[c].ext] = off;
+            x.list_start[c] = off;
             off += x.class_pairs[c];
         }
     }
@@ -576,10 +672,8 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(unit_bucket_.ensure(4 * nr));
     PHMM_CUDA(hap_start_.ensure(8 * nh));
     PHMM_CUDA(read_pack_.ensure(4 * (x.pack_positions + kReadSlackPos)));
-    if (table_->exact) {
-        PHMM_CUDA(read_coef_.ensure(sizeof(float4) * std::max<int64_t>(x.pack_positions, 1)));
-        PHMM_CUDA(read_meta_.ensure(sizeof(ReadMeta) * nr));
-    }
+    if (table_->exact) PHMM_CUDA(read_coef_.ensure(sizeof(float4) * std::max<int64_t>(x.pack_positions, 1)));
+    PHMM_CUDA(read_meta_.ensure(sizeof(ReadMeta) * nr));
     PHMM_CUDA(hap_code_.ensure(x.code_bytes + kHapSlack));
     const int64_t nbins = (int64_t)table_->rules.size() * hbins_of(x);
     PHMM_CUDA(hist_.ensure(4 * nbins));
@@ -587,7 +681,7 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(items_.ensure(sizeof(Item) * np));
     PHMM_CUDA(rescue_.ensure(sizeof(Task) * np));  // class lists laid out back to back
     PHMM_CUDA(rescue_ext_.ensure(sizeof(Task) * np));  // the extended tier's, same offsets
-    PHMM_CUDA(rescue_off_.ensure(sizeof(int64_t) * kFp64Classes));
+    PHMM_CUDA(rescue_off_.ensure(sizeof(x.list_start)));
     return PAIRHMM_OK;
 }
 
@@ -603,7 +697,7 @@ pairhmm_status_t Engine::upload_index(const BatchIndex& x, cudaStream_t s) {
         {unit_read0_.ptr, x.unit_read0.data(), 4 * x.unit_read0.size()},
         {unit_read1_.ptr, x.unit_read1.data(), 4 * x.unit_read1.size()},
         {unit_bucket_.ptr, x.unit_bucket.data(), 4 * x.unit_bucket.size()},
-        {rescue_off_.ptr, x.class_start, sizeof(x.class_start)},
+        {rescue_off_.ptr, x.list_start, sizeof(x.list_start)},
     };
     PHMM_CUDA(uploader_.run(opts_.device, copies, s));
     return PAIRHMM_OK;
@@ -664,7 +758,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     pa.read_pack = read_pack_.as<uint32_t>();
     pa.hap_code = hap_code_.as<uint8_t>();
     pa.read_coef = table_->exact ? read_coef_.as<float4>() : nullptr;
-    pa.read_meta = table_->exact ? read_meta_.as<ReadMeta>() : nullptr;
+    pa.read_meta = read_meta_.as<ReadMeta>();
     pa.ph2pr = ph2pr_.as<float>();
     if (stage == 0) {
     launches_ = 0;
@@ -680,7 +774,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     fa.ptr[2] = counters_.as<uint32_t>();
     fa.words[2] = 2 * kCtrTotal;
     fa.ptr[3] = rsort_.as<uint32_t>();
-    fa.words[3] = kFp64Classes * kRescueHBins;
+    fa.words[3] = (long long)fp64_->classes.size() * kRescueHBins;
     PHMM_CUDA(launch_pack(pa, fa, prep_grid, s));
     launches_ += 1;
     }
@@ -723,6 +817,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     v.hap_len = in.hap_lengths;
     v.scores = d_scores;
     v.rescue_base = rescue_.as<Task>();
+    v.rescue_class = fp64_lut_[fp64_ == &fp64_tables_[1]].as<uint8_t>();
     v.rescue_off = rescue_off_.as<long long>();
     v.rescue_count = counters + kCtrScaled;
     v.rescue_enabled = (!plain && opts_.fp64_rescue) ? 1 : 0;
@@ -731,19 +826,19 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
 
     // FP64 pass: first sort each class's list by haplotype length into the
     // work-item buffer (free once the FP32 stage is done), same class offsets
-    Task* const fp64_lists = items_.as<Task>();
-    int64_t fp64_upper = 0;  // pairs the FP64 lists could hold
-    for (int c = 0; c < kFp64Classes; ++c) fp64_upper += x.class_pairs[c];
-    if (stage == 2 && fp64_upper > 0) {
-        const int64_t upper = fp64_upper;
+    const int64_t upper = x.num_pairs;  // pairs the FP64 lists could hold
+    const bool sorted = upper > kNoSortPairs;
+    Task* const fp64_lists = sorted ? items_.as<Task>() : rescue_.as<Task>();
+    if (stage == 2 && sorted) {
         RescueSortArgs ra{};
         ra.in = rescue_.as<Task>();
         ra.out = fp64_lists;
+        ra.classes = (int)fp64_->classes.size();
         ra.off = rescue_off_.as<long long>();
         ra.count = counters + kCtrScaled;
         ra.hap_len = in.hap_lengths;
         ra.hist = rsort_.as<unsigned int>();
-        ra.cursor = reinterpret_cast<unsigned long long*>(rsort_.as<unsigned int>() + kFp64Classes * kRescueHBins);
+        ra.cursor = reinterpret_cast<unsigned long long*>(rsort_.as<unsigned int>() + kMaxFp64Classes * kRescueHBins);
         const int sort_grid = (int)std::max<int64_t>(1, std::min<int64_t>((upper + 255) / 256, 8 * (int64_t)num_sms_));
         PHMM_CUDA(launch_rescue_sort(ra, sort_grid, s));
         launches_ += 3;
@@ -779,38 +874,58 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
         }
     } else {
         // stage 2: FP64 pass over flagged pairs (FP32 underflow, or degenerate alpha):
-        // per length class the scaled tier, then on the same stream the extended
-        // tier over the pairs the scaled tier handed on (for the multi-tile class of
-        // a small batch, inside the scaled tier's launch); only the last class uses
-        // the border scratch (the two tiers of a class run in turn, so they share it)
-        const ExtList ext{rescue_ext_.as<Task>(), rescue_off_.as<long long>(), counters + kCtrExt};
-        // a few long pairs (at most a round of resident warps): the multi-tile scaled tier
-        // runs a pair's extended form right after it in the same warp, so the batch waits
-        // for one pass instead of two
-        const bool fuse_mt = x.class_pairs[kFp64Classes - 1] <= kFuseMaxPairs;
-        for (int c = 0; c < kFp64Classes; ++c) {
+        // per length class the scaled tier, then the extended tier over the pairs the
+        // scaled tier handed on.  An extended class that serves one scaled class runs
+        // right behind it on the same stream (for the padded multi-tile class of a small
+        // batch, inside the scaled tier's launch); the others once all scaled launches
+        // are done.
+        auto launch = [&](const Fp64Config* cfg, bool tier_ext, int list, int grid, int64_t scratch, int ext_cls,
+                          cudaStream_t on) {
+            Fp64LaunchArgs fa{};
+            fa.view = v;
+            fa.ext_list = {rescue_ext_.as<Task>(), rescue_off_.as<long long>() + kMaxFp64Classes, counters + kCtrExt,
+                           ext_cls};
+            fa.items = (tier_ext ? rescue_ext_.as<Task>() : fp64_lists) +
+                       x.list_start[tier_ext ? kMaxFp64Classes + list : list];
+            fa.count = counters + (tier_ext ? kCtrExt : kCtrScaled) + list;
+            fa.counter = counters + (tier_ext ? kCtrTaskExt : kCtrTaskScaled) + list;
+            fa.scratch = static_cast<char*>(scratch_.ptr) + scratch;
+            fa.rows = plan.rows;
+            fa.grid = grid;
+            fa.stream = on;
+            ++launches_;
+            return cfg->launch(fa);
+        };
+        const int last = (int)fp64_->classes.size() - 1;
+        bool shared_ext[kMaxFp64Classes] = {};
+        for (int c = last; c >= 0; --c) {
             if (x.class_pairs[c] == 0) continue;
-            const cudaStream_t sc = next_stream();
-            const bool fuse = fuse_mt && c == kFp64Classes - 1;
-            for (const bool tier_ext : {false, true}) {
-                if (tier_ext && fuse) continue;
-                Fp64LaunchArgs fa{};
-                fa.fuse = fuse && !tier_ext;
-                fa.view = v;
-                fa.cls = c;
-                fa.gcp = opts_.gcp != 0;
-                fa.ext = tier_ext;
-                fa.ext_list = ext;
-                fa.items = (tier_ext ? rescue_ext_.as<Task>() : fp64_lists) + x.class_start[c];
-                fa.count = counters + (tier_ext ? kCtrExt : kCtrScaled) + c;
-                fa.counter = counters + (tier_ext ? kCtrTaskExt : kCtrTaskScaled) + c;
-                fa.scratch = scratch_.ptr;
-                fa.rows = plan.rows;
-                fa.grid = tier_ext ? plan.fp64_ext_grid[c] : plan.fp64_grid[c];
-                fa.stream = sc;
-                PHMM_CUDA(launch_fp64_rescue(fa));
-                ++launches_;
+            const Fp64Table::Class& k = fp64_->classes[c];
+            const Fp64Table::Ext& e = fp64_->exts[k.ext];
+            const cudaStream_t on = next_stream();
+            // a few long pairs (at most a round of resident warps): one pass instead of two
+            const bool fuse = c == last && x.class_pairs[c] <= kFuseMaxPairs;
+            PHMM_CUDA(launch(fuse ? fp64_->fused : k.scaled, false, c, plan.fp64_grid[c], plan.fp64_scratch[c], k.ext,
+                             on));
+            if (!e.own_stream) shared_ext[k.ext] = true;
+            else if (!fuse)
+                PHMM_CUDA(launch(e.cfg, true, k.ext, plan.fp64_ext_grid[k.ext], plan.fp64_ext_scratch[k.ext], 0, on));
+        }
+        bool any = false;
+        for (bool b : shared_ext) any = any || b;
+        if (any) {
+            if (fork) {
+                for (int i = 0; i < kSideStreams; ++i) {
+                    PHMM_CUDA(cudaEventRecord(join_[i], side_[i]));
+                    PHMM_CUDA(cudaStreamWaitEvent(s, join_[i], 0));
+                }
+                PHMM_CUDA(cudaEventRecord(fork_, s));
+                for (int i = 0; i < kSideStreams; ++i) PHMM_CUDA(cudaStreamWaitEvent(side_[i], fork_, 0));
             }
+            for (int e = 0; e < (int)fp64_->exts.size(); ++e)
+                if (shared_ext[e])
+                    PHMM_CUDA(launch(fp64_->exts[e].cfg, true, e, plan.fp64_ext_grid[e], plan.fp64_ext_scratch[e], 0,
+                                     next_stream()));
         }
     }
     if (fork) {
@@ -856,23 +971,45 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
         // the plain form runs one task per warp; a grid capped by scratch loops on the counter
         p.persistent[b] = (!plain || grid < need_blocks) ? 1 : 0;
     }
-    for (int c = 0; c < kFp64Classes; ++c) {
-        if (x.class_pairs[c] == 0) continue;
-        if (c == kFp64Classes - 1)   // the fused form's opt-in; its grid is the scaled tier's
-            persistent_grid(fp64_kernel(c, opts_.gcp != 0, false, true), kBlockThreads, fp64_smem_bytes(c, false));
-        for (const bool tier_ext : {false, true}) {
-            int64_t grid = persistent_grid(fp64_kernel(c, opts_.gcp != 0, tier_ext), kBlockThreads,
-                                            fp64_smem_bytes(c, tier_ext));
-            const int64_t per_warp = (int64_t)fp64_scratch_bytes_per_row(c, tier_ext) * p.rows;
-            if (per_warp > 0) {
-                grid = std::min<int64_t>(grid, std::max<int64_t>(1, kScratchBudget / (per_warp * kWarpsPerBlock)));
-                scratch = std::max(scratch, grid * kWarpsPerBlock * per_warp);
-            }
-            // no more warps than flagged pairs could need
-            const int64_t need = (x.class_pairs[c] + fp64_per_warp(c) - 1) / fp64_per_warp(c);
-            grid = std::min<int64_t>(grid, std::max<int64_t>(1, (need + kWarpsPerBlock - 1) / kWarpsPerBlock));
-            (tier_ext ? p.fp64_ext_grid : p.fp64_grid)[c] = (int)grid;
+    // FP64 launches: no more blocks than the class's pairs could need.  Kernels with
+    // border scratch may run at the same time, so each has its own slice, out of an
+    // equal share of the budget; an extended class of one scaled class runs behind it
+    // and shares its slice.
+    int n_scratch = 0;
+    for (size_t c = 0; c < fp64_->classes.size(); ++c)
+        if (x.class_pairs[c] > 0) n_scratch += fp64_->classes[c].scaled->scratch_bytes_per_row > 0;
+    for (const Fp64Table::Ext& e : fp64_->exts) n_scratch += e.cfg->scratch_bytes_per_row > 0 && !e.own_stream;
+    auto fp64_grid = [&](const Fp64Config* c, int64_t pairs, int64_t& bytes) {
+        const int64_t tasks = (pairs + c->per_task - 1) / c->per_task;
+        int64_t grid = std::min<int64_t>(persistent_grid(c->kernel, c->block_threads, c->smem_bytes),
+                                         (tasks + c->tasks_per_block - 1) / c->tasks_per_block);
+        grid = std::max<int64_t>(grid, 1);
+        bytes = 0;
+        if (c->scratch_bytes_per_row) {
+            const int64_t per_block = (int64_t)c->scratch_bytes_per_row * p.rows * c->tasks_per_block;
+            grid = std::min(grid, std::max<int64_t>(1, kScratchBudget / std::max(1, n_scratch) / per_block));
+            bytes = round_up(grid * per_block, 256);
         }
+        return (int)grid;
+    };
+    for (size_t i = 0; i < fp64_->exts.size(); ++i) {
+        const Fp64Table::Ext& e = fp64_->exts[i];
+        int64_t pairs = 0, slice = 0, bytes = 0;
+        for (int c = e.first; c <= e.last; ++c) {
+            if (x.class_pairs[c] == 0) continue;
+            pairs += x.class_pairs[c];
+            const Fp64Config* scaled = fp64_->classes[c].scaled;
+            p.fp64_scratch[c] = scratch;
+            p.fp64_grid[c] = fp64_grid(scaled, x.class_pairs[c], bytes);
+            if (e.own_stream) slice = bytes;
+            else scratch += bytes;
+            if (c + 1 == (int)fp64_->classes.size())   // the fused form has the scaled form's grid
+                persistent_grid(fp64_->fused->kernel, fp64_->fused->block_threads, fp64_->fused->smem_bytes);
+        }
+        if (pairs == 0) continue;
+        p.fp64_ext_scratch[i] = scratch;
+        p.fp64_ext_grid[i] = fp64_grid(e.cfg, pairs, bytes);
+        scratch += std::max(slice, bytes);
     }
     p.scratch_bytes = (size_t)std::max<int64_t>(std::max(scratch, fp32_scratch), 256);
     return p;
@@ -958,8 +1095,8 @@ pairhmm_status_t Engine::host_begin(const pairhmm_batch_t& b, float* scores, cud
     };
     if (opts_.gcp) inputs.push_back({in_gq_.ptr, b.gcp_quals + rlo, (size_t)rn});
     cudaError_t up = uploader_.start(opts_.device, inputs, s);
-    choose_table(rg.num_pairs, b.read_lengths, rg.num_reads);
-    st = build_index(b, table_->rules, idx_, err);
+    choose_table(b.num_records, b.reads_per_record, b.haps_per_record, b.read_lengths, rg.num_pairs);
+    st = build_index(b, table_->rules, *fp64_, idx_, err);
     const cudaError_t upf = uploader_.finish();
     if (up == cudaSuccess) up = upf;
     if (up != cudaSuccess) return cuda_fail(up, "input upload");
@@ -993,14 +1130,14 @@ pairhmm_status_t Engine::host_begin(const pairhmm_batch_t& b, float* scores, cud
     // rescue counts and (into page-locked memory) scores come down now; scores
     // for pageable memory go through the uploader's slots in host_end
     PHMM_CUDA(cudaMemcpyAsync(host_hdr_, counters_.as<unsigned long long>() + kCtrScaled,
-                              sizeof(unsigned long long) * 2 * kFp64Classes, cudaMemcpyDeviceToHost, s));
+                              sizeof(unsigned long long) * 2 * kMaxFp64Classes, cudaMemcpyDeviceToHost, s));
     pend_direct_ = HostUploader::is_page_locked(scores);
     if (pend_direct_)
         PHMM_CUDA(cudaMemcpyAsync(scores, scores_.ptr, 4 * (size_t)x.num_pairs, cudaMemcpyDeviceToHost, s));
     pend_scores_ = scores;
     pend_pairs_ = x.num_pairs;
     stats_.h2d_bytes = 4 * rn + hn + 12 * x.num_reads + 12 * x.num_haps + index_bytes(x);
-    stats_.d2h_bytes = 4 * x.num_pairs + (int64_t)sizeof(unsigned long long) * 2 * kFp64Classes;
+    stats_.d2h_bytes = 4 * x.num_pairs + (int64_t)sizeof(unsigned long long) * 2 * kMaxFp64Classes;
     stats_.launches = launches_;
     stats_.fp32_launches = fp32_launches_;
     pending_ = true;
@@ -1016,8 +1153,7 @@ pairhmm_status_t Engine::host_end() {
         PHMM_CUDA(uploader_.download(opts_.device, pend_scores_, scores_.ptr, 4 * (size_t)pend_pairs_, s));
     PHMM_CUDA(cudaStreamSynchronize(s));
     // per class: the scaled tier's counts, then the extended tier's
-    unsigned long long rescued_by_class[2 * kFp64Classes] = {};
-    static_assert(sizeof(rescued_by_class) <= 256, "rescue counts fit the landing spot");
+    unsigned long long rescued_by_class[2 * kMaxFp64Classes] = {};
     std::memcpy(rescued_by_class, host_hdr_, sizeof(rescued_by_class));
     float ms = 0.f, a = 0.f, b2 = 0.f, c = 0.f;
     PHMM_CUDA(cudaEventElapsedTime(&ms, ev0_, ev1_));
@@ -1030,9 +1166,9 @@ pairhmm_status_t Engine::host_end() {
     stats_.fp64_ms = c;
     stats_.rescued = 0;
     stats_.rescued_ext = 0;
-    for (int c = 0; c < kFp64Classes; ++c) {
+    for (int c = 0; c < kMaxFp64Classes; ++c) {
         stats_.rescued += (int64_t)rescued_by_class[c];
-        stats_.rescued_ext += (int64_t)rescued_by_class[kFp64Classes + c];
+        stats_.rescued_ext += (int64_t)rescued_by_class[kMaxFp64Classes + c];
     }
     return PAIRHMM_OK;
 }
@@ -1180,8 +1316,8 @@ pairhmm_status_t Engine::compute_device(const pairhmm_batch_t& b, int32_t, int32
     std::string err;
     int64_t pairs = 0;
     for (int64_t g = 0; g < b.num_records; ++g) pairs += (int64_t)std::max(rpr[g], 0) * std::max(hpr[g], 0);
-    choose_table(pairs, rl.data(), nr);
-    pairhmm_status_t st = build_index(hb, table_->rules, idx_, err);
+    choose_table(b.num_records, rpr.data(), hpr.data(), rl.data(), pairs);
+    pairhmm_status_t st = build_index(hb, table_->rules, *fp64_, idx_, err);
     const BatchIndex& x = idx_;
     if (st != PAIRHMM_OK) return fail(st, err);
     stats_ = pairhmm_stats_t{};

@@ -35,7 +35,26 @@ inline bool operator==(const TileRule& a, const TileRule& b) {
 struct TileTable {
     std::vector<TileRule> rules;
     std::vector<const ConfigInfo*> cfg;
-    bool exact = false;   // some rule is exact: the preparation forms coefficients
+    bool exact = false;   // some rule is exact: the preparation forms FP32 coefficients
+};
+
+// Length classes of the FP64 pass and their kernels.
+struct Fp64Table {
+    struct Class {
+        int max_len;
+        const Fp64Config* scaled;
+        int ext;                      // extended-tier class of its pairs
+    };
+    struct Ext {
+        const Fp64Config* cfg;
+        int first, last;              // its scaled classes
+        bool own_stream;              // one scaled class: runs right behind it
+    };
+    std::vector<Class> classes;
+    std::vector<Ext> exts;
+    const Fp64Config* fused = nullptr;  // fused form of the last class
+    std::vector<uint8_t> lut;           // class of a read length (kFp64LutSize)
+    int class_of(int L) const { return lut.empty() ? 0 : lut[L <= kFp64LutMax ? L : kFp64LutMax + 1]; }
 };
 
 // Per-batch index derived on the host from the record structure.
@@ -50,8 +69,10 @@ struct BatchIndex {
     std::vector<int64_t> bucket_pairs;              // by bucket index
     std::vector<int64_t> bucket_items;              // work items (unit x haplotype) by bucket
     std::vector<int32_t> unit_read0, unit_read1, unit_bucket;  // units: 1 or 2 reads of a record
-    int64_t class_pairs[kFp64Classes] = {};         // by FP64 length class (fp64_class)
-    int64_t class_start[kFp64Classes] = {};         // start of each class's FP64 list
+    int64_t class_pairs[kMaxFp64Classes] = {};      // by FP64 length class
+    // starts of the FP64 lists: the scaled tier's by class, then the extended tier's by
+    // its classes (each holds the pairs of consecutive scaled classes)
+    int64_t list_start[2 * kMaxFp64Classes] = {};
     int64_t multi_tile_pairs = 0;
 };
 
@@ -105,7 +126,7 @@ public:
     int num_sms() const { return num_sms_; }
 
     static pairhmm_status_t build_index(const pairhmm_batch_t& b, const std::vector<TileRule>& rules,
-                                        BatchIndex& idx, std::string& err);
+                                        const Fp64Table& fp64, BatchIndex& idx, std::string& err);
     // gcp: the batch must carry gcp qualities, none 0 at a read's first position
     static pairhmm_status_t scan_inputs(const pairhmm_batch_t& b, InputRanges& r, std::string& err, bool gcp);
 
@@ -115,16 +136,19 @@ private:
                                 cudaEvent_t mark_end);
     pairhmm_status_t host_end();
     pairhmm_status_t build_tables(const std::vector<TileRule>& rules);
-    // the table for a batch of these reads and this many pairs becomes the current one
-    void choose_table(int64_t pairs, const int32_t* read_lengths, int64_t num_reads);
+    // the table for a batch of these records becomes the current one
+    void choose_table(int64_t num_records, const int32_t* reads_per_record, const int32_t* haps_per_record,
+                      const int32_t* read_lengths, int64_t pairs);
     pairhmm_status_t run_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, float* d_scores,
                                   cudaStream_t s);
     struct Plan {
         int64_t rows = 0;                 // border rows per buffer
         std::vector<int> grid;            // by bucket
         std::vector<int> persistent;      // by bucket
-        int fp64_grid[kFp64Classes] = {};   // by FP64 length class: scaled tier
-        int fp64_ext_grid[kFp64Classes] = {};  // extended tier
+        int fp64_grid[kMaxFp64Classes] = {};      // by FP64 length class: scaled tier
+        int fp64_ext_grid[kMaxFp64Classes] = {};  // by extended-tier class
+        int64_t fp64_scratch[kMaxFp64Classes] = {};      // border scratch offsets of the
+        int64_t fp64_ext_scratch[kMaxFp64Classes] = {};  // kernels that need it
         std::vector<int64_t> scratch_off;   // by bucket: multi-tile kernels run side by side
         size_t scratch_bytes = 0;
     };
@@ -144,6 +168,9 @@ private:
     // batches of few pairs, with groups as wide as possible (choose_table)
     TileTable tables_[2];
     const TileTable* table_ = &tables_[0];
+    Fp64Table fp64_tables_[2];          // FP64 classes: on 8-32 lanes, and as wide as possible
+    const Fp64Table* fp64_ = &fp64_tables_[0];
+    DevBuf fp64_lut_[2];
     int num_sms_ = 0;
     std::unordered_map<const void*, int> blocks_per_sm_;  // kernels used so far
     bool ready_ = false;
@@ -151,7 +178,7 @@ private:
     // the launches of one stage (bucket kernels, FP64 classes) fork onto side
     // streams so that their tails overlap and a small batch's buckets run side
     // by side; they join back into stream_ before the stage ends
-    static constexpr int kSideStreams = 8;
+    static constexpr int kSideStreams = 16;
     cudaStream_t side_[kSideStreams] = {};
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;

@@ -11,26 +11,34 @@ namespace phmm {
 // 64-thread blocks: the paths with per-position w and x hold 8R + ~50 registers a
 // lane (packed), so up to R = 10 six blocks fit 168 registers and beyond that four
 // blocks; the shared tables (2.5 KB a warp and position pair) allow as many.
-template <class V, int R, int W>
+// Scalar groups hold 4R + ~60: serial parts take eight blocks up to R = 14 and six up
+// to R = 24 (168 registers), block groups 16 warps.
+template <class V, int R, int W, bool SERIAL>
 constexpr int tile_min_ctas() {
-    return W > 1 ? 16 / W : (R <= 10 ? 6 : 4);
+    return SERIAL ? (R <= 14 ? 8 : 6) : W > 1 ? 16 / W : (R <= 10 ? 6 : 4);
 }
 
-template <class V, int G, int R, int W, bool GCP>
-__global__ void __launch_bounds__(W == 1 ? kBlockThreads : 32 * W, tile_min_ctas<V, R, W>())
-fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items, unsigned long long* counter) {
-    using T = TileWavefront<V, G, R, W, GCP>;
+template <class V, int G, int R, int W, bool GCP, bool SERIAL>
+__global__ void __launch_bounds__(W == 1 || SERIAL ? kBlockThreads : 32 * W, tile_min_ctas<V, R, W, SERIAL>())
+fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items, unsigned long long* counter,
+                 void* scratch, int64_t rows) {
+    using T = TileWavefront<V, G, R, W, GCP, false, SERIAL>;
     extern __shared__ float4 smem[];
-    constexpr int kWarps = W == 1 ? kWarpsPerBlock : W;
+    constexpr int kWarps = T::kWarps;
+    static_assert(T::kBlockGroup || kWarps == kWarpsPerBlock, "independent warps");
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     auto* tab = reinterpret_cast<typename T::Word*>(smem) + warp * T::kTableWords;
-    auto* ring = reinterpret_cast<typename T::RingRow*>(reinterpret_cast<char*>(smem) + kWarps * T::kSmemBytes);
+    auto* ring = reinterpret_cast<typename T::RingRow*>(reinterpret_cast<char*>(smem) + kWarps * T::kSmemBytes) +
+                 (SERIAL ? warp * T::kRing : 0);
+    auto* border = SERIAL ? static_cast<typename T::RingRow*>(scratch) +
+                                ((int64_t)blockIdx.x * kWarps + warp) * rows
+                          : nullptr;
     __shared__ unsigned next;
     const unsigned ntasks = (unsigned)((num_items + T::NG - 1) / T::NG);
     while (true) {
         unsigned x = 0;
-        if constexpr (W == 1) {
+        if constexpr (!T::kBlockGroup) {
             if (lane == 0) x = (unsigned)atomicAdd(counter, 1ull);
         } else {
             if (threadIdx.x == 0) next = (unsigned)atomicAdd(counter, 1ull);
@@ -49,9 +57,9 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
         const int t = lane - grp * G;
         const bool active = grp < ntask;
         const Item* item = items + first + (active ? grp : 0);
-        double acc[T::NS];
+        typename T::Sum sum;
 #pragma unroll
-        for (int s = 0; s < T::NS; ++s) acc[s] = 0.0;
+        for (int s = 0; s < T::NS; ++s) sum.s[s] = 0.0;
         {
             const Item it = *item;
             const int H = v.hap_len[it.hap];
@@ -74,12 +82,16 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
             // every read of the task has the one gap quality
             const bool uni = __reduce_min_sync(kFullMask, kmin) == __reduce_max_sync(kFullMask, kmax) &&
                              kmax != kNoKey;
-            const int K = W == 1 ? (int)((__reduce_max_sync(kFullMask, (unsigned)(H + G)) + 3u) & ~3u) : 0;
-            if (uni) T::template loop<true>(rd, hw, H, K, tab, ring, t, W == 1 ? 0 : warp, lane, acc);
-            else T::template loop<false>(rd, hw, H, K, tab, ring, t, W == 1 ? 0 : warp, lane, acc);
+            const int K = T::kBlockGroup ? 0 : (int)((__reduce_max_sync(kFullMask, (unsigned)(H + G)) + 3u) & ~3u);
+            double stop = 0.0;
+            if (SERIAL && v.rescue_enabled)
+                stop = (double)tile_threshold(rd.L[0], H, v.read_meta[item->read0].range);
+            rd.ph = v.ph2pr;
+            T::run(rd, hw, H, K, uni, tab, ring, border, rows, t, T::kBlockGroup ? warp : 0, lane, stop, sum);
         }
 
-        if (active && t == G - 1 && (W == 1 || warp == W - 1)) {
+        // a serial pair that stopped has no sum: below any threshold
+        if (active && t == G - 1 && (!T::kBlockGroup || warp == W - 1)) {
             // the item is read again rather than kept in registers over the steps
             const volatile Item* vi = item;
             const int hap = vi->hap;
@@ -91,30 +103,28 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
                 const int64_t out = s ? vi->out1 : vi->out0;
                 const int L = v.read_len[read];
                 const ReadMeta meta = v.read_meta[read];
-                v.scores[out] = (float)(log10(acc[s] / (double)H) - log10((double)kTileD0));
+                v.scores[out] = (float)(log10(sum.s[s] / (double)H) - log10((double)kTileD0));
                 if ((meta.flags & 1u) ||
-                    (v.rescue_enabled && !(acc[s] >= (double)tile_threshold(L, H, meta.range) &&
-                                           acc[s] <= (double)FLT_MAX)))
-                    append_rescue(v, fp64_class(L), Task{read, hap, out});
+                    (v.rescue_enabled && !(sum.s[s] >= (double)tile_threshold(L, H, meta.range) &&
+                                           sum.s[s] <= (double)FLT_MAX)))
+                    append_rescue(v, L, Task{read, hap, out});
             }
         }
         __syncwarp();
     }
 }
 
-template <class V, int G, int R, int W, bool GCP>
+template <class V, int G, int R, int W, bool GCP, bool SERIAL = false>
 cudaError_t launch_fp32_tile(const Fp32LaunchArgs& a) {
-    using T = TileWavefront<V, G, R, W, GCP>;
-    constexpr int kWarps = W == 1 ? kWarpsPerBlock : W;
-    fp32_tile_kernel<V, G, R, W, GCP><<<a.grid, 32 * kWarps, kWarps * T::kSmemBytes + T::kRingBytes, a.stream>>>(
-        a.view, a.items, a.num_items, a.counter);
+    using T = TileWavefront<V, G, R, W, GCP, false, SERIAL>;
+    fp32_tile_kernel<V, G, R, W, GCP, SERIAL><<<a.grid, 32 * T::kWarps, T::kBlockSmem, a.stream>>>(
+        a.view, a.items, a.num_items, a.counter, a.scratch, a.rows);
     return cudaGetLastError();
 }
 
-template <class V, int G, int R, int W, bool GCP>
+template <class V, int G, int R, int W, bool GCP, bool SERIAL = false>
 ConfigInfo make_tile_config() {
-    using T = TileWavefront<V, G, R, W, GCP>;
-    constexpr int kWarps = W == 1 ? kWarpsPerBlock : W;
+    using T = TileWavefront<V, G, R, W, GCP, false, SERIAL>;
     ConfigInfo c{};
     c.G = T::NL;
     c.R = R;
@@ -123,11 +133,12 @@ ConfigInfo make_tile_config() {
     c.exact = true;
     c.gcp = GCP;
     c.per_task = T::NG;
-    c.block_threads = 32 * kWarps;
-    c.tasks_per_block = W == 1 ? kWarpsPerBlock : 1;
-    c.smem_bytes = kWarps * T::kSmemBytes + T::kRingBytes;
-    c.kernel = reinterpret_cast<const void*>(&fp32_tile_kernel<V, G, R, W, GCP>);
-    c.launch = &launch_fp32_tile<V, G, R, W, GCP>;
+    c.block_threads = 32 * T::kWarps;
+    c.tasks_per_block = T::kBlockGroup ? 1 : T::kWarps;
+    c.smem_bytes = T::kBlockSmem;
+    c.scratch_bytes_per_row = SERIAL ? sizeof(typename T::RingRow) : 0;
+    c.kernel = reinterpret_cast<const void*>(&fp32_tile_kernel<V, G, R, W, GCP, SERIAL>);
+    c.launch = &launch_fp32_tile<V, G, R, W, GCP, SERIAL>;
     return c;
 }
 
@@ -137,6 +148,16 @@ void register_tiles(std::vector<ConfigInfo>& out) {
     if constexpr (R0 <= R1) {
         out.push_back(make_tile_config<float2, G, R0, 1, GCP>());
         register_tiles<G, R0 + 1, R1, GCP>(out);
+    }
+}
+
+// configurations of 32*W lanes x R, one read per group: blocks of W warps, or one warp
+// with W parts in turn
+template <int W, int R0, int R1, bool GCP, bool SERIAL>
+void register_long(std::vector<ConfigInfo>& out) {
+    if constexpr (R0 <= R1) {
+        out.push_back(make_tile_config<float, 32, R0, W, GCP, SERIAL>());
+        register_long<W, R0 + 1, R1, GCP, SERIAL>(out);
     }
 }
 

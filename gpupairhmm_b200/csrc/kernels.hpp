@@ -29,18 +29,34 @@ struct Fp32LaunchArgs {
 
 struct Fp64LaunchArgs {
     DevView view;
-    int cls;                         // length class (fp64_class)
-    bool gcp;                        // gcp mode kernel
-    bool ext;                        // extended-range tier (per-lane exponents)
     ExtList ext_list;                // scaled tier: where pairs beyond its range go
-    bool fuse = false;               // multi-tile scaled tier: run the extended form in the same warp
-    const Task* items;               // that class's rescue list
+    const Task* items;               // the class's rescue list
     const unsigned long long* count; // number of items (device)
     unsigned long long* counter;     // task counter
-    void* scratch;                   // border storage (class 2 only)
+    void* scratch;                   // border storage (padded multi-tile kernels only)
     int64_t rows;
     int grid;
     cudaStream_t stream;
+};
+
+// A compiled kernel of the FP64 pass.  Exact tiles take reads of (G*(R-1), G*R]
+// positions; the padded kernels (wavefront_fp64.cuh) up to G*R, or any length
+// (multi_tile).
+struct Fp64Config {
+    int G;
+    int R;
+    bool ext;                        // extended tier (per-lane exponents)
+    bool gcp;
+    bool exact;
+    bool multi_tile;                 // padded kernel, tile after tile
+    bool fused;                      // scaled tier that runs a pair's extended form in the same warp
+    int per_task;
+    int block_threads;
+    int tasks_per_block;
+    size_t smem_bytes;
+    size_t scratch_bytes_per_row;    // per warp, per border row
+    const void* kernel;
+    cudaError_t (*launch)(const Fp64LaunchArgs&);
 };
 
 struct ConfigInfo {
@@ -63,15 +79,10 @@ struct ConfigInfo {
 const std::vector<ConfigInfo>& fp32_configs();
 const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed, bool exact, bool gcp);
 
-// FP64 pass, one kernel per length class and tier (misc_kernels.cu): the
-// scaled tier (ext = false) recomputes every flagged pair, the extended tier
-// (ext = true) the pairs beyond the scaled tier's range.  gcp selects the
-// gcp-mode kernels (eps/beta per read).
-cudaError_t launch_fp64_rescue(const Fp64LaunchArgs& a);
-size_t fp64_smem_bytes(int cls, bool ext);
-size_t fp64_scratch_bytes_per_row(int cls, bool ext);  // per warp, per border row
-const void* fp64_kernel(int cls, bool gcp, bool ext, bool fuse = false);
-int fp64_per_warp(int cls);
+// All compiled kernels of the FP64 pass.  The scaled tier (ext = false) recomputes
+// every flagged pair, the extended tier (ext = true) the pairs beyond its range.
+const std::vector<Fp64Config>& fp64_configs();
+const Fp64Config* find_fp64_config(int G, int R, bool exact, bool ext, bool gcp, bool fused = false);
 
 // Preparation kernels.  The pack launch also runs the batch's fills.
 cudaError_t launch_pack(const PrepArgs& a, const FillArgs& f, int grid, cudaStream_t s);

@@ -22,6 +22,8 @@ void register_tile_g32(std::vector<ConfigInfo>& out);
 void register_tile_gcp_g8(std::vector<ConfigInfo>& out);
 void register_tile_gcp_g16(std::vector<ConfigInfo>& out);
 void register_tile_gcp_g32(std::vector<ConfigInfo>& out);
+void register_long(std::vector<ConfigInfo>& out);
+void register_long_gcp(std::vector<ConfigInfo>& out);
 
 const std::vector<ConfigInfo>& fp32_configs() {
     static std::vector<ConfigInfo> all;
@@ -39,29 +41,26 @@ const std::vector<ConfigInfo>& fp32_configs() {
         register_tile_gcp_g8(all);
         register_tile_gcp_g16(all);
         register_tile_gcp_g32(all);
+        register_long(all);
+        register_long_gcp(all);
     });
     return all;
 }
 
 const ConfigInfo* find_fp32_config(int G, int R, bool multi_tile, bool packed, bool exact, bool gcp) {
     for (const auto& c : fp32_configs())
-        if (c.G == G && c.R == R && c.multi_tile == multi_tile && c.packed == packed && c.exact == exact &&
+        if (c.G == G && c.R == R && c.exact == exact && (exact || c.multi_tile == multi_tile) && c.packed == packed &&
             c.gcp == gcp)
             return &c;
     return nullptr;
 }
 
 // ---------------------------------------------------------------- FP64 pass
-// Tiles per length class.  A step's cost is mostly per lane (hand-off, scale
-// conversion, renormalisation), so the single-tile classes take 12-16
-// positions per lane where the registers allow (2 warps per scheduler at
-// 216-255 registers beat 4 warps at 8 positions: FP64 pass of the uneven
-// workload -6%, of 250-bp reads -9%); 160 keeps 16 x 10 at 168 registers.
-// Multi-tile: 512-row tiles (32 x 16) halve the tiles of a long pair against
-// 32 x 8 (long-read workload's FP64 pass 38.3 -> 26.9 ms; one long-read
-// region's 11.5 -> 7.3 ms).  Both tiers use the same tiles: the scaled tier
-// (EXT = false) takes every flagged pair, the extended tier (EXT = true) the
-// few the scaled tier hands on.
+// Padded kernels of the FP64 pass (wavefront_fp64.cuh), where fp64_tile.cuh has no
+// exact tile: both tiers of reads up to 32 positions and beyond 4,096, and the
+// extended tier of reads up to 640, which few pairs reach.  A step's cost is mostly
+// per lane (hand-off, scale conversion, renormalisation), so the tiles take 12-16
+// positions per lane where the registers allow; 160 keeps 16 x 10 at 168 registers.
 template <bool EXT> using W64c0 = Fp64Wavefront<4, 16, false, false, EXT>;
 template <bool EXT> using W64c1 = Fp64Wavefront<8, 12, false, false, EXT>;
 template <bool EXT> using W64c2 = Fp64Wavefront<8, 16, false, false, EXT>;
@@ -69,13 +68,9 @@ template <bool EXT> using W64c3 = Fp64Wavefront<16, 10, false, false, EXT>;
 template <bool EXT> using W64c4 = Fp64Wavefront<16, 12, false, false, EXT>;
 template <bool EXT> using W64c5 = Fp64Wavefront<16, 16, false, false, EXT>;
 template <bool EXT> using W64c6 = Fp64Wavefront<32, 16, true, false, EXT>;
-static_assert(W64c0<true>::T == kFp64ClassMax[0] && W64c1<true>::T == kFp64ClassMax[1] &&
-                  W64c2<true>::T == kFp64ClassMax[2] && W64c3<true>::T == kFp64ClassMax[3] &&
-                  W64c4<true>::T == kFp64ClassMax[4] && W64c5<true>::T == kFp64ClassMax[5],
-              "class bounds follow the tiles");
 
-// The multi-tile class's scaled tier runs the extended form of a pair right
-// after it in the same warp when the pair needs it, so the border ring and the
+// The multi-tile kernel's scaled tier runs the extended form of a pair right after
+// it in the same warp when the pair needs it (FUSE), so the border ring and the
 // scratch rows are sized for the extended form's 32-byte rows.
 template <class W>
 using Fp64ExtOf = Fp64Wavefront<W::G_, W::R_, W::kMT, W::kGCP, true>;
@@ -119,7 +114,7 @@ fp64_rescue_kernel(DevView v, const Task* __restrict__ items, const unsigned lon
                 __syncwarp();
                 WE::run(v, items + first, ntask, ph, wtab, reinterpret_cast<typename WE::Border*>(ring_bytes),
                         reinterpret_cast<typename WE::Border*>(wscratch), rows, ext, false);
-                if (lane == 0) atomicAdd(ext.count + (kFp64Classes - 1), 1ull);  // counted with the extended tier
+                if (lane == 0) atomicAdd(ext.count + ext.cls, 1ull);  // counted with the extended tier
             }
         }
     }
@@ -131,7 +126,7 @@ size_t fp64_smem_for() {
            (size_t)kWarpsPerBlock * W::kRing * fp64_ring_entry<W>();
 }
 
-// gcp-mode twins of the class kernels (same tiles, eps/beta per read)
+// gcp-mode twins (same tiles, eps/beta per read)
 template <class W>
 struct WithGcp;
 template <int G, int R, bool MT, bool EXT>
@@ -139,73 +134,73 @@ struct WithGcp<Fp64Wavefront<G, R, MT, false, EXT>> {
     using type = Fp64Wavefront<G, R, MT, true, EXT>;
 };
 
-#define PHMM_FP64_DISPATCH_T(cls, X, EXPR)    \
-    switch (cls) {                             \
-        case 0: { using W = W64c0<X>; EXPR; }  \
-        case 1: { using W = W64c1<X>; EXPR; }  \
-        case 2: { using W = W64c2<X>; EXPR; }  \
-        case 3: { using W = W64c3<X>; EXPR; }  \
-        case 4: { using W = W64c4<X>; EXPR; }  \
-        case 5: { using W = W64c5<X>; EXPR; }  \
-        default: { using W = W64c6<X>; EXPR; } \
-    }
-#define PHMM_FP64_DISPATCH(cls, ext, EXPR)                               \
-    do {                                                                 \
-        if (ext) { PHMM_FP64_DISPATCH_T(cls, true, EXPR) }               \
-        else { PHMM_FP64_DISPATCH_T(cls, false, EXPR) }                  \
-    } while (0)
-
-// the gcp twin has the same tables and ring, so the same shared memory
-size_t fp64_smem_bytes(int cls, bool ext) { PHMM_FP64_DISPATCH(cls, ext, return fp64_smem_for<W>()); }
-// one border buffer per warp, shared by all tile boundaries of its pair
-size_t fp64_scratch_bytes_per_row(int cls, bool) {
-    return cls == kFp64Classes - 1 ? sizeof(Border64) : 0;  // both forms of the multi-tile class
-}
-// the kernel of a class and tier; fuse picks the multi-tile scaled tier's fused form
-template <class W>
-const void* fp64_kernel_of(bool gcp, bool fuse) {
-    using WG = typename WithGcp<W>::type;
-    if constexpr (W::kMT && !W::kEXT) {
-        if (fuse)
-            return gcp ? reinterpret_cast<const void*>(&fp64_rescue_kernel<WG, true>)
-                       : reinterpret_cast<const void*>(&fp64_rescue_kernel<W, true>);
-    }
-    return gcp ? reinterpret_cast<const void*>(&fp64_rescue_kernel<WG, false>)
-               : reinterpret_cast<const void*>(&fp64_rescue_kernel<W, false>);
-}
-const void* fp64_kernel(int cls, bool gcp, bool ext, bool fuse) {
-    PHMM_FP64_DISPATCH(cls, ext, return fp64_kernel_of<W>(gcp, fuse));
-}
-int fp64_per_warp(int cls) { PHMM_FP64_DISPATCH(cls, true, return W::NG); }
-
-template <class K>
-cudaError_t fp64_launch_as(const Fp64LaunchArgs& a, void* scr, size_t smem) {
-    K::launch(a, scr, smem);
+template <class W, bool FUSE>
+cudaError_t launch_fp64_padded(const Fp64LaunchArgs& a) {
+    fp64_rescue_kernel<W, FUSE><<<a.grid, kBlockThreads, fp64_smem_for<W>(), a.stream>>>(
+        a.view, a.items, a.count, a.counter, W::kMT ? a.scratch : nullptr, a.rows, a.ext_list);
     return cudaGetLastError();
 }
-template <class W, bool FUSE>
-struct Fp64Launch {
-    static void launch(const Fp64LaunchArgs& a, void* scr, size_t smem) {
-        fp64_rescue_kernel<W, FUSE><<<a.grid, kBlockThreads, smem, a.stream>>>(a.view, a.items, a.count, a.counter,
-                                                                              scr, a.rows, a.ext_list);
-    }
-};
-template <class W>
-cudaError_t fp64_launch_of(const Fp64LaunchArgs& a, void* scr, size_t smem) {
-    using WG = typename WithGcp<W>::type;
-    if constexpr (W::kMT && !W::kEXT) {
-        if (a.fuse)
-            return a.gcp ? fp64_launch_as<Fp64Launch<WG, true>>(a, scr, smem)
-                         : fp64_launch_as<Fp64Launch<W, true>>(a, scr, smem);
-    }
-    return a.gcp ? fp64_launch_as<Fp64Launch<WG, false>>(a, scr, smem)
-                 : fp64_launch_as<Fp64Launch<W, false>>(a, scr, smem);
+
+template <class W, bool FUSE = false>
+Fp64Config make_padded64_config() {
+    Fp64Config c{};
+    c.G = W::G_;
+    c.R = W::R_;
+    c.ext = W::kEXT;
+    c.gcp = W::kGCP;
+    c.multi_tile = W::kMT;
+    c.fused = FUSE;
+    c.per_task = W::NG;
+    c.block_threads = kBlockThreads;
+    c.tasks_per_block = kWarpsPerBlock;
+    c.smem_bytes = fp64_smem_for<W>();
+    // one border buffer per warp, shared by all tile boundaries of its pair
+    c.scratch_bytes_per_row = W::kMT ? sizeof(Border64) : 0;
+    c.kernel = reinterpret_cast<const void*>(&fp64_rescue_kernel<W, FUSE>);
+    c.launch = &launch_fp64_padded<W, FUSE>;
+    return c;
 }
 
-cudaError_t launch_fp64_rescue(const Fp64LaunchArgs& a) {
-    void* scr = a.cls == kFp64Classes - 1 ? a.scratch : nullptr;
-    const size_t smem = fp64_smem_bytes(a.cls, a.ext);
-    PHMM_FP64_DISPATCH(a.cls, a.ext, return fp64_launch_of<W>(a, scr, smem));
+template <class W>
+void register_padded64(std::vector<Fp64Config>& out) {
+    out.push_back(make_padded64_config<W>());
+    out.push_back(make_padded64_config<typename WithGcp<W>::type>());
+}
+
+void register_tile64_g8(std::vector<Fp64Config>& out);
+void register_tile64_g16(std::vector<Fp64Config>& out);
+void register_tile64_g32(std::vector<Fp64Config>& out);
+void register_long64(std::vector<Fp64Config>& out);
+void register_long64_gcp(std::vector<Fp64Config>& out);
+
+const std::vector<Fp64Config>& fp64_configs() {
+    static std::vector<Fp64Config> all;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        register_padded64<W64c0<false>>(all);
+        register_padded64<W64c6<false>>(all);
+        all.push_back(make_padded64_config<W64c6<false>, true>());
+        all.push_back(make_padded64_config<WithGcp<W64c6<false>>::type, true>());
+        register_padded64<W64c0<true>>(all);
+        register_padded64<W64c1<true>>(all);
+        register_padded64<W64c2<true>>(all);
+        register_padded64<W64c3<true>>(all);
+        register_padded64<W64c4<true>>(all);
+        register_padded64<W64c5<true>>(all);
+        register_padded64<W64c6<true>>(all);
+        register_tile64_g8(all);
+        register_tile64_g16(all);
+        register_tile64_g32(all);
+        register_long64(all);
+        register_long64_gcp(all);
+    });
+    return all;
+}
+
+const Fp64Config* find_fp64_config(int G, int R, bool exact, bool ext, bool gcp, bool fused) {
+    for (const auto& c : fp64_configs())
+        if (c.G == G && c.R == R && c.exact == exact && c.ext == ext && c.gcp == gcp && c.fused == fused) return &c;
+    return nullptr;
 }
 
 // ---------------------------------------------------------------- preparation
@@ -226,7 +221,7 @@ cudaError_t launch_pack(const PrepArgs& a, const FillArgs& f, int grid, cudaStre
 
 cudaError_t launch_rescue_sort(const RescueSortArgs& a, int grid, cudaStream_t s) {
     rescue_count_kernel<<<grid, 256, 0, s>>>(a);
-    rescue_scan_kernel<<<1, 32 * kFp64Classes, 0, s>>>(a);
+    rescue_scan_kernel<<<a.classes, 32, 0, s>>>(a);
     rescue_scatter_kernel<<<grid, 256, 0, s>>>(a);
     return cudaGetLastError();
 }

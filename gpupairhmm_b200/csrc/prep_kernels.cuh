@@ -19,7 +19,7 @@
 namespace phmm {
 
 constexpr int kHBins = 4096;     // most haplotype-length classes per bucket
-constexpr int kMaxBuckets = 64;
+constexpr int kMaxBuckets = 96;
 
 struct PrepArgs {
     // caller arrays (device)
@@ -47,8 +47,9 @@ struct PrepArgs {
     uint32_t* read_pack;
     uint8_t* hap_code;
     uint8_t* read_gcp;              // [num_reads], gcp mode only (else null)
-    float4* read_coef;              // wavefront_tile.cuh's coefficients by packed position, and
-    ReadMeta* read_meta;            // what it needs per read (null: no exact tile in the table)
+    float4* read_coef;              // wavefront_tile.cuh's FP32 coefficients by packed position
+                                    // (null: no exact FP32 tile in the table), and
+    ReadMeta* read_meta;            // what its kernels need per read
     const float* ph2pr;             // 128 probabilities
 };
 
@@ -103,7 +104,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
         float beta = kBeta, range = 0.0f;
         uint32_t key = kNoKey, flags = 0;
         bool same = true;   // gap qualities of the lane's positions equal the first position's
-        if (a.read_coef && L > 0) {
+        if (L > 0) {
             key = min((uint32_t)iq[0], 127u);
             if (a.gcp_quals) {
                 const uint32_t g = min((uint32_t)a.gcp_quals[src], 127u);
@@ -129,8 +130,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                     w[j] = c + j < L ? pack_position(rb[c + j], bq[c + j], iq[c + j], dq[c + j]) : 4u;
             }
             dst[c >> 2] = make_uint4(w[0], w[1], w[2], w[3]);
-            if (a.read_coef) {
-                float4* coef = a.read_coef + a.read_start[i] + c;
+            {
                 float d = a.ph2pr[(w[0] >> 16) & 0x7fu], sg = a.ph2pr[(w[0] >> 24) & 0x7fu];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -149,7 +149,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                         an = 1.0f - (dn + sn);
                     }
                     const float4 cf = tile_coefficients(a.ph2pr[(w[j] >> 8) & 0x7fu], d, sg, an, dn, beta);
-                    coef[j] = cf;
+                    if (a.read_coef) a.read_coef[a.read_start[i] + c + j] = cf;
                     range = fmaxf(range, 1.0f / dn + 2.0f * (1.0f + cf.y));
                     if (!(fabsf(1.0f - (d + sg)) >= kMinAlpha)) flags |= 1u;
                     if (end) a.read_meta[i].w_end = tile_weight(beta, dn, beta);
@@ -158,7 +158,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                 }
             }
         }
-        if (a.read_coef) {
+        {
             same = __all_sync(kFullMask, same);
             flags = __any_sync(kFullMask, flags != 0u) ? 1u : 0u;
             // positive floats order as their bits; an infinite or NaN bound stays the largest
@@ -367,11 +367,12 @@ constexpr int kRescueHBins = 512;
 struct RescueSortArgs {
     const Task* in;                   // class lists in append order
     Task* out;                        // the same lists, sorted
-    const long long* off;             // [kFp64Classes] list starts
-    const unsigned long long* count;  // [kFp64Classes] list lengths
+    int classes;
+    const long long* off;             // [classes] list starts
+    const unsigned long long* count;  // [classes] list lengths
     const int32_t* hap_len;
-    unsigned int* hist;               // [kFp64Classes * kRescueHBins], zeroed before the batch
-    unsigned long long* cursor;       // [kFp64Classes * kRescueHBins]
+    unsigned int* hist;               // [classes * kRescueHBins], zeroed before the batch
+    unsigned long long* cursor;       // [classes * kRescueHBins]
 };
 
 __device__ __forceinline__ int rescue_hbin(int H) {
@@ -382,7 +383,7 @@ __device__ __forceinline__ int rescue_hbin(int H) {
 #ifdef PHMM_PREP_KERNELS_IMPL
 __global__ void rescue_count_kernel(RescueSortArgs a) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (int c = 0; c < kFp64Classes; ++c) {
+    for (int c = 0; c < a.classes; ++c) {
         const long long n = (long long)a.count[c];
         const Task* in = a.in + a.off[c];
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -393,9 +394,9 @@ __global__ void rescue_count_kernel(RescueSortArgs a) {
 }
 
 // one warp per class: exclusive scan of its bins (16 per lane) from the list start
-__global__ void __launch_bounds__(32 * kFp64Classes) rescue_scan_kernel(RescueSortArgs a) {
+__global__ void __launch_bounds__(32) rescue_scan_kernel(RescueSortArgs a) {
     constexpr int kPer = kRescueHBins / 32;
-    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x, lane = threadIdx.x;
     const unsigned int* h = a.hist + c * kRescueHBins + lane * kPer;
     unsigned long long sum = 0;
 #pragma unroll
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(32 * kFp64Classes) rescue_scan_kernel(RescueSo
 
 __global__ void rescue_scatter_kernel(RescueSortArgs a) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (int c = 0; c < kFp64Classes; ++c) {
+    for (int c = 0; c < a.classes; ++c) {
         const long long n = (long long)a.count[c];
         const Task* in = a.in + a.off[c];
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {

@@ -406,14 +406,14 @@ struct Fp32Wavefront {
         degenerate = (dmask & gmask) != 0u;
         if (valid && handed_off && t == 0) {
             v.scores[task.out] = -INFINITY;  // the FP64 pass writes the result
-            append_rescue(v, fp64_class(L), task);
+            append_rescue(v, L, task);
         }
         if (valid && !handed_off && t == rlane) {
             const float res = (float)(log10(accd) - (log10((double)kScale) + log10((double)beta)));
             v.scores[task.out] = res;
             if (degenerate ||
                 (v.rescue_enabled && !(accd >= (double)rescue_threshold(L, H) && accd <= (double)FLT_MAX))) {
-                append_rescue(v, fp64_class(L), task);
+                append_rescue(v, L, task);
             }
         }
     }

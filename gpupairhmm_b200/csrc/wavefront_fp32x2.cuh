@@ -244,13 +244,13 @@ struct Fp32x2Wavefront {
         if (resA) {
             v.scores[it.out0] = (float)(log10(accdA) - off);
             if (degA || (v.rescue_enabled && !(accdA >= (double)rescue_threshold(LA, H) && accdA <= (double)FLT_MAX))) {
-                append_rescue(v, fp64_class(LA), Task{ra, it.hap, it.out0});
+                append_rescue(v, LA, Task{ra, it.hap, it.out0});
             }
         }
         if (resB) {
             v.scores[it.out1] = (float)(log10(accdB) - off);
             if (degB || (v.rescue_enabled && !(accdB >= (double)rescue_threshold(LB, H) && accdB <= (double)FLT_MAX))) {
-                append_rescue(v, fp64_class(LB), Task{rb, it.hap, it.out1});
+                append_rescue(v, LB, Task{rb, it.hap, it.out1});
             }
         }
     }

@@ -56,6 +56,7 @@
 #include <type_traits>
 
 #include "device_common.cuh"
+#include "wavefront_tile.cuh"
 
 namespace phmm {
 
@@ -85,16 +86,9 @@ __device__ __forceinline__ int border_e(const Border64S&) { return 0; }
 __device__ __forceinline__ int border_ei(const Border64& b) { return b.ei; }
 __device__ __forceinline__ int border_ei(const Border64S&) { return 0; }
 
-// 2^k as a double for k clamped to the normal range (exact power of two)
-__device__ __forceinline__ double pow2i(int k) {
-    k = k < -1022 ? -1022 : (k > 1023 ? 1023 : k);
-    return __longlong_as_double((long long)(k + 1023) << 52);
-}
-
 // Scaled tier: the D boundary's power-of-two factor over the reference's scale,
 // and the smallest sum it keeps (relative error of the subnormal roundings
 // below 5*2^-45 above it).
-constexpr int kScaledExp = 836;
 __host__ __device__ __forceinline__ double scaled_tier_threshold(int L, int H) {
     return (double)L * (double)H * 0x1p-1030;
 }
@@ -382,11 +376,7 @@ struct Fp64Wavefront {
                     for (int d = 16; d >= 1; d >>= 1) mass += __shfl_xor_sync(kFullMask, mass, d);
                     if (mass < 0.5 * scaled_tier_threshold(L, H)) {  // warp-uniform: one pair per warp
                         if (fuse) return valid;
-                        if (valid && t == 0) {
-                            const int cls = fp64_class(L);
-                            const unsigned long long slot = atomicAdd(ext.count + cls, 1ull);
-                            ext.base[ext.off[cls] + (long long)slot] = task;
-                        }
+                        if (valid && t == 0) ext.append(task);
                         return false;  // no score: the extended tier writes it
                     }
                 }
@@ -402,11 +392,7 @@ struct Fp64Wavefront {
                 res = log10(acc) - (double)eacc * 0.30102999566398119521 - log10((double)kScale) - log10(beta);
             if (GCP && !(beta > 0.0)) res = NAN;
             v.scores[task.out] = (float)res;
-            if (to_ext && !fuse) {
-                const int cls = fp64_class(L);
-                const unsigned long long slot = atomicAdd(ext.count + cls, 1ull);
-                ext.base[ext.off[cls] + (long long)slot] = task;
-            }
+            if (to_ext && !fuse) ext.append(task);
         }
         if (MT && !EXT && fuse) return __any_sync(kFullMask, to_ext);
         return false;

@@ -37,11 +37,23 @@
 // low end of the range; the boundary D enters as FLT_MAX/8 instead of
 // (FLT_MAX/16)/H, which gives most of it back.  See tile_threshold.
 //
-// W > 1: the group is the W warps of a block, for reads beyond one warp's tile.
-// Warp v runs kLag blocks of kBlock steps behind warp v-1 and takes that warp's
-// last column, row by row, from a ring in shared memory; a block barrier after
-// every kBlock steps is the only synchronisation.
+// W > 1: reads beyond one warp's tile, the group's lanes being those of W warps.
+//   Block groups: the W warps of a block.  Warp v runs kLag blocks of kBlock steps
+//   behind warp v-1 and takes that warp's last column, row by row, from a ring in
+//   shared memory; a block barrier after every kBlock steps is the only
+//   synchronisation.  For batches of few pairs: a pair takes 1/W of the time.
+//   SERIAL: one warp runs the W parts in turn, the last column of each going to the
+//   next through global memory (L2), fetched 32 rows at a time into a shared ring.
+//   For batches that fill the chip: no barriers, no pipeline to fill, and a pair that
+//   will not reach the pass's threshold stops at the first part's end: every path to
+//   the result leaves a column once and nothing on it exceeds 1, so the sum is at
+//   most the mass sum_j (M + I + D)(j) on the column; below half the threshold the
+//   sum would fail it too.
+// Both do the same arithmetic as one group of 32*W lanes.
 #pragma once
+
+#include <climits>
+#include <type_traits>
 
 #include "device_common.cuh"
 
@@ -100,9 +112,36 @@ struct LaneOps<float2> {
     }
 };
 
+template <>
+struct LaneOps<double> {
+    using S = double;
+    static constexpr int kSides = 1;
+    __device__ __forceinline__ static double make(double a, double) { return a; }
+    __device__ __forceinline__ static double fma(double a, double b, double c) { return ::fma(a, b, c); }
+    __device__ __forceinline__ static double mul(double a, double b) { return a * b; }
+    __device__ __forceinline__ static double add(double a, double b) { return a + b; }
+    __device__ __forceinline__ static double up(double v, int G) { return __shfl_up_sync(kFullMask, v, 1, G); }
+    __device__ __forceinline__ static double sel(const bool (&p)[1], double a, double b) { return p[0] ? a : b; }
+    __device__ __forceinline__ static double uniform(double v) {
+        const unsigned lo = __reduce_max_sync(kFullMask, (unsigned)__double2loint(v));
+        const unsigned hi = __reduce_max_sync(kFullMask, (unsigned)__double2hiint(v));
+        return __hiloint2double((int)hi, (int)lo);
+    }
+    __device__ __forceinline__ static double side(double v, int) { return v; }
+};
+
+// 2^k as a double for k clamped to the normal range (exact power of two)
+__device__ __forceinline__ double pow2i(int k) {
+    k = k < -1022 ? -1022 : (k > 1023 ? 1023 : k);
+    return __longlong_as_double((long long)(k + 1023) << 52);
+}
+
 // Boundary value of D (times beta it is what the first column receives); the
 // pair's scale is kTileD0 * H, D being 1/H there.
 constexpr float kTileD0 = FLT_MAX / 8.0f;
+// FP64, scaled tier: D enters 2^836 higher (near 2^961, which leaves 2^62 of headroom).
+constexpr int kScaledExp = 836;
+constexpr double kScaled = 0x1p836;
 
 // Smallest sum of T the FP32 pass keeps.  N, I and D^ each round by at most 2^-150
 // in the denormal range; as terms of T they weigh at most 1/n, 1 and d, range being
@@ -113,6 +152,12 @@ constexpr float kTileD0 = FLT_MAX / 8.0f;
 __device__ __forceinline__ float tile_threshold(int L, int H, float range) {
     const float cells = (float)L * (float)H * 0x1p-127f;
     return fmaxf(cells * range, 3.0f * cells * (float)H * (2.0f / kBeta));
+}
+
+// Smallest sum the FP64 pass's scaled tier keeps: the same terms each round by at most
+// 2^-1075 in the subnormal range, so above this the sum is exact to about 2^-44.
+__device__ __forceinline__ double scaled_tile_threshold(int L, int H, float range) {
+    return (double)L * (double)H * (double)range * 0x1p-1030;
 }
 
 // One read position's coefficients for this kernel (w, x, l of a match, l of a
@@ -146,15 +191,22 @@ struct ReadMeta {
 static_assert(sizeof(ReadMeta) == 16, "ReadMeta is one 16-byte word");
 constexpr uint32_t kNoKey = 0xffffffffu;
 
-template <class V, int G, int R, int W, bool GCP>
+// EXT (FP64): a lane keeps its values as true * 2^e with its own exponent e, for
+// pairs whose values span more than a double's range; see wavefront_fp64.cuh, whose
+// extended tier works the same way.
+template <class V, int G, int R, int W, bool GCP, bool EXT = false, bool SERIAL = false>
 struct TileWavefront {
     using O = LaneOps<V>;
     using S = typename O::S;
+    static constexpr bool kDouble = std::is_same<S, double>::value;
     static_assert(W == 1 || G == 32, "a group of several warps fills them");
     static_assert(R >= 2, "a lane holds R or R-1 positions, at least one");
+    static_assert(!EXT || kDouble, "lane exponents go with doubles");
     static constexpr int NS = O::kSides;
     static constexpr int NG = 32 / G;    // groups per warp
     static constexpr int NL = G * W;     // lanes per group
+    static constexpr bool kBlockGroup = W > 1 && !SERIAL;
+    static_assert(!SERIAL || (W > 1 && NS == 1 && !kDouble), "serial parts: one FP32 read per warp");
     static constexpr int VN = 16 / (int)sizeof(V);     // values per 16-byte table word
     static constexpr int Q = (R + VN - 1) / VN;        // table words per lane and code
     static constexpr int kTableWords = 5 * Q * 32;     // per warp
@@ -165,35 +217,89 @@ struct TileWavefront {
     static constexpr int kLag = 3;
     static constexpr int kRing = 64;     // rows per ring; reader and writer are within 32 rows
     struct alignas(16) Word { V v[VN]; };
-    struct alignas(16) RingRow { V n, i, x; };
+    struct alignas(16) RingRow {
+        V n, i, x;
+        int e;   // EXT: exponent of all three
+    };
+    // steps unrolled.  A batch of long reads has some 14 classes of few pairs, whose kernels
+    // run side by side: at 4 steps (11 KB of code each) they thrashed the instruction cache,
+    // 64 long-read regions' FP32 stage 14.6 ms against 7.0 at 2 steps and 7.9 at 1
+    static constexpr int kUnroll = SERIAL ? 2 : 4;
+    static constexpr int kMaxShift = 640;   // EXT: largest scale difference a hand-off converts
     static constexpr size_t kSmemBytes = (size_t)kTableWords * sizeof(Word);  // per warp, the table
-    static constexpr size_t kRingBytes = W > 1 ? (size_t)(W - 1) * kRing * sizeof(RingRow) : 0;  // per block
+    static constexpr int kWarps = kBlockGroup ? W : 2;   // per block
+    // rings per block; a group's first part reads its (constant) boundary from one too,
+    // so that no step branches on which part it runs
+    static constexpr int kRings = W > 1 ? kWarps : 0;
+    static constexpr int kBorderPad = 32;   // serial: row j sits at entry j + 32 of a buffer
+    static constexpr size_t kBlockSmem = kWarps * kSmemBytes + kRings * kRing * sizeof(RingRow);
 
     struct Reads {
-        const float4* coef[NS];     // the read's coefficients, position 0 first
+        const float4* coef[NS];     // FP32: the read's coefficients, position 0 first
+        const float* ph;            // FP64: the probabilities, coefficients are formed in double
         const uint32_t* pack[NS];   // packed words (the base code in the low byte)
         int L[NS];
         S w_end[NS];
         S eps[NS];                  // GCP only
+        S beta;                     // FP64
+    };
+    struct Sum {
+        double s[NS];               // sum of T over the haplotype's rows, in the result lane
+        int e;                      // EXT: its exponent
     };
 
+    // FP64 coefficients.  Probabilities are the 32-bit model parameters, alpha and
+    // 1 - p formed in FP32 as the reference forms them, everything else in double.
+    struct Gap {
+        double i;   // 1/(beta*delta)
+        float d, s;
+    };
+    __device__ __forceinline__ static Gap gap(const Reads& rd, int c) {
+        const uint32_t w = __ldg(rd.pack[0] + c);
+        const float d = __ldg(rd.ph + ((w >> 16) & 0x7fu));
+        return Gap{1.0 / (rd.beta * (double)d), d, __ldg(rd.ph + ((w >> 24) & 0x7fu))};
+    }
+
+    // One warp's part of a group.  warp: its number in the group (0 where a warp holds
+    // whole groups).  ring: the block's rings (block groups) or the warp's own (serial).
+    // border: serial, the warp's column buffer of `rows` rows.
+    // UNI: one gap quality at all positions of all the warp's reads
     template <bool UNI>
     __device__ __forceinline__ static void loop(const Reads& rd, const uint32_t* hw, int H, int K, Word* tab,
-                                                RingRow* ring, int t, int warp, int lane, double (&acc)[NS]) {
+                                                RingRow* ring, RingRow* border, int64_t rows, int t, int warp,
+                                                int lane, Sum& sum) {
         const int u = warp * 32 + t;   // lane of the group
         bool full[NS];
         V wv[UNI ? 1 : R], xv[UNI ? 1 : R], N[R], D[R];
         {
-            float w[NS][UNI ? 1 : R], x[NS][UNI ? 1 : R];
+            S w[NS][UNI ? 1 : R], x[NS][UNI ? 1 : R];
             int p0[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 const int m = rd.L[s] - NL * (R - 1);
                 full[s] = u < m;
                 p0[s] = u * (R - 1) + min_i(u, m);
-                if constexpr (UNI) w[s][0] = __ldg(&rd.coef[s]->x);
+                if constexpr (UNI) {
+                    if constexpr (kDouble) {
+                        const Gap g = gap(rd, 0);
+                        w[s][0] = (double)(1.0f - (g.d + g.s)) * g.i;
+                    } else {
+                        w[s][0] = __ldg(&rd.coef[s]->x);
+                    }
+                }
             }
-            if constexpr (!UNI) {
+            if constexpr (!UNI && kDouble) {
+                Gap g = gap(rd, min_i(p0[0], rd.L[0] - 1));
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int c = p0[0] + r;
+                    const Gap n = gap(rd, min_i(c + 1, rd.L[0] - 1));   // past the end the last position's again
+                    wv[r] = c < rd.L[0] ? (double)(1.0f - (g.d + g.s)) * g.i : 0.0;
+                    xv[r] = c >= rd.L[0] ? 0.0 : g.s == n.d ? 1.0 : rd.beta * (double)g.s * n.i;
+                    g = n;
+                }
+            }
+            if constexpr (!UNI && !kDouble) {
 #pragma unroll
                 for (int s = 0; s < NS; ++s)
 #pragma unroll
@@ -238,19 +344,29 @@ struct TileWavefront {
 #pragma unroll
                 for (int k = 0; k < VN; ++k) {
                     const int r = q * VN + k;
-                    float l[NS][5];
+                    S l[NS][5];
 #pragma unroll
                     for (int s = 0; s < NS; ++s) {
-                        float2 cf = make_float2(0.f, 0.f);
+                        S lm = 0, lx = 0;
                         uint32_t code = 0;
                         const int c = p0[s] + r;
                         if (r < R && c < rd.L[s]) {
-                            cf = __ldg(reinterpret_cast<const float2*>(rd.coef[s] + c) + 1);
-                            code = __ldg(rd.pack[s] + c) & 0xffu;
+                            const uint32_t word = __ldg(rd.pack[s] + c);
+                            code = word & 0xffu;
+                            if constexpr (kDouble) {
+                                const uint32_t next = __ldg(rd.pack[s] + min_i(c + 1, rd.L[s] - 1));
+                                const float p = __ldg(rd.ph + ((word >> 8) & 0x7fu));
+                                const double n = rd.beta * (double)__ldg(rd.ph + ((next >> 16) & 0x7fu));
+                                lm = (double)(1.0f - p) * n;
+                                lx = (double)(p / 3.0f) * n;
+                            } else {
+                                const float2 cf = __ldg(reinterpret_cast<const float2*>(rd.coef[s] + c) + 1);
+                                lm = cf.x;
+                                lx = cf.y;
+                            }
                         }
 #pragma unroll
-                        for (int h = 0; h < 5; ++h)
-                            l[s][h] = (code == 4u || h == 4 || code == (uint32_t)h) ? cf.x : cf.y;
+                        for (int h = 0; h < 5; ++h) l[s][h] = (code == 4u || h == 4 || code == (uint32_t)h) ? lm : lx;
                     }
 #pragma unroll
                     for (int h = 0; h < 5; ++h) words[h].v[k] = O::make(l[0][h], l[NS - 1][h]);
@@ -272,29 +388,92 @@ struct TileWavefront {
             if constexpr (UNI) eps = O::uniform(eps);
         }
         const V wend = O::make(rd.w_end[0], rd.w_end[NS - 1]);
-        const V zero = O::make(0.f, 0.f), d0 = O::make(kTileD0, kTileD0);
+        constexpr S kD0 = kDouble && !EXT ? (S)kTileD0 * (S)kScaled : (S)kTileD0;
+        const V zero = O::make(0.f, 0.f), d0 = O::make(kD0, kD0);
         const bool first = u == 0;
         // the result lane adds the rows up to its pair's last step
         const int kres = u == NL - 1 ? H + G - 1 : -1;
 
         V Nl = zero;   // this lane's last N of the step before (the row T needs)
         V Ml = zero, Mul = zero, Iul = zero, Xul = first ? d0 : zero;
+        // EXT: exponents of this lane, and of Ml, Mul, and Iul and Xul
+        int e = 0, eMl = 0, eMul = 0, eIul = 0;
+        bool empty = !first;
+        sum.e = 0;
         int h = 4;
         // code words of this group's haplotype; behind its end the last word is re-read
         // (those rows are past the result's last one)
         const int wlast = ((H + 15) & ~15) / 4 - 1;
         uint32_t wcur = __ldg(hw);
         uint32_t wnext = __ldg(hw + 1);
+        RingRow fetched{};   // serial: row 32*b + t of the block of 32 rows after the next
+        const RingRow* left = ring;      // rows of the column before this part
+        RingRow* right = border;         // rows of its last column, one per step
+        const bool writer = W > 1 && warp + 1 < W && t == 31;
+        if constexpr (SERIAL) {
+            __syncwarp();
+            if (warp > 0) {
+                ring[t] = border[kBorderPad + t];   // a buffer has more than 96 rows
+                fetched = border[kBorderPad + 32 + t];
+            } else {
+                ring[t] = ring[32 + t] = RingRow{zero, zero, d0, 0};
+            }
+            __syncwarp();
+        }
+        if constexpr (kBlockGroup) {
+            // warp v writes ring v + 1 and reads ring v; ring 0 holds the boundary
+            left = ring + warp * kRing;
+            right = ring + (warp + 1) * kRing;
+            if (warp == 0) ring[t] = ring[32 + t] = RingRow{zero, zero, d0, 0};
+            __syncwarp();
+        }
         auto four_steps = [&](int k0) {
             const uint32_t wpref = __ldg(hw + min_i((k0 >> 2) + 2, wlast));
+            if constexpr (SERIAL) {
+                if (warp > 0 && (k0 & 31) == 0) {
+                    __syncwarp();
+                    ring[(k0 + 32 + t) & (kRing - 1)] = fetched;
+                    __syncwarp();
+                    if (kBorderPad + 64 + (int64_t)k0 + t < rows) fetched = border[kBorderPad + 64 + k0 + t];
+                }
+            }
             V a4 = zero;
-#pragma unroll
+#pragma unroll kUnroll
             for (int s4 = 0; s4 < 4; ++s4) {
                 const int k = k0 + s4;
                 int hn = __shfl_up_sync(kFullMask, h, 1, G);
                 if (t == 0) hn = (int)((wcur >> (8 * s4)) & 0xffu);
                 h = hn;
                 const Word* row = tab + h * (Q * 32) + lane;
+                if constexpr (EXT) {
+                    // lanes fill in the wavefront's first pass: centre the lane's scale on the
+                    // first values it receives
+                    if (k0 < G + 8 && empty && (Mul != 0.0 || Xul != 0.0 || Iul != 0.0)) {
+                        const double xi = fmax(fabs(Xul), fabs(Iul));
+                        e = Mul != 0.0 ? eMul - ilogb(fabs(Mul)) : eIul - ilogb(xi);
+                        empty = false;
+                    }
+                    if (e - (eMul < eIul ? eMul : eIul) > kMaxShift) {
+                        // a neighbour's values far above this lane's scale: coarsen the scale by
+                        // an exact power of two first, so that the conversion cannot overflow;
+                        // what falls out of range is negligible next to the incoming values
+                        const int dM = Mul != 0.0 ? e - eMul : INT_MIN;
+                        const int dI = (Xul != 0.0 || Iul != 0.0) ? e - eIul : INT_MIN;
+                        const int over = (dM > dI ? dM : dI) - kMaxShift;
+                        if (over > 0) {
+                            const double f = over > 1022 ? 0.0 : pow2i(-over);
+#pragma unroll
+                            for (int r = 0; r < R; ++r) { N[r] *= f; D[r] *= f; }
+                            Nl *= f;
+                            if (k <= kres) sum.s[0] *= f;
+                            e -= over;
+                        }
+                    }
+                    const double fM = pow2i(e - eMul), fI = pow2i(e - eIul);
+                    Mul *= fM;
+                    Iul *= fI;
+                    Xul *= fI;
+                }
                 // a position first forms what the next one takes from its old N, so that N is
                 // replaced in place (with the old N carried along instead, the compiler moves
                 // the lane's N by one register a step, on the FMA pipe)
@@ -327,35 +506,85 @@ struct TileWavefront {
                 Id = O::sel(full, Id, Ip);
                 Xd = O::sel(full, Xd, Xp);
                 const V T = O::fma(Nl, wend, Id);
-                if (k <= kres) a4 = O::add(a4, T);
+                if constexpr (kDouble) {
+                    if (k <= kres) sum.s[0] += T;
+                } else {
+                    if (k <= kres) a4 = O::add(a4, T);
+                }
                 Nl = O::sel(full, N[R - 1], N[R - 2]);
-                if (W > 1 && warp + 1 < W && t == 31 && k >= 31)
-                    ring[warp * kRing + ((k - 31) & (kRing - 1))] = RingRow{Nl, Id, Xd};
+                if constexpr (W > 1) {
+                    // the last lane is at row k - 31; rows before the first land in the padding
+                    // (serial) or in slots the next part has not reached yet.  serial: the row
+                    // was fetched by this warp 64 steps ago or more
+                    if (writer) right[SERIAL ? k + 1 : (k + 33) & (kRing - 1)] = RingRow{Nl, Id, Xd, e};
+                }
                 Mul = Ml;
                 Ml = O::up(Nl, G);
                 Iul = O::up(Id, G);
                 Xul = O::up(Xd, G);
-                if (W > 1 && warp > 0) {
-                    const RingRow b = ring[(warp - 1) * kRing + ((k + 1) & (kRing - 1))];  // broadcast
+                if constexpr (EXT) {   // values travel with the sender's exponent
+                    eMul = eMl;
+                    eMl = __shfl_up_sync(kFullMask, e, 1, G);
+                    eIul = eMl;
+                }
+                if constexpr (W > 1) {
+                    const RingRow b = left[(k + 1) & (kRing - 1)];  // broadcast
                     if (t == 0) {
                         Ml = b.n;
                         Iul = b.i;
                         Xul = b.x;
+                        eMl = eIul = b.e;
                     }
-                } else if (first || (W == 1 && t == 0)) {
+                } else if (t == 0) {
                     Ml = zero;
                     Iul = zero;
                     Xul = d0;
+                    eMl = eIul = 0;
+                }
+                if constexpr (EXT) {
+                    // renormalise every 16 steps (exact powers of two); a value moves by at most
+                    // 2^13 per row, so lanes stay within 2^300 of their scale meanwhile
+                    if ((k & 15) == 15) {
+                        double mx = fmax(k <= kres ? fabs(sum.s[0]) : 0.0, fmax(fabs(Id), fabs(Xd)));
+#pragma unroll
+                        for (int r = 0; r < R; ++r) mx = fmax(mx, fmax(fabs(N[r]), fabs(D[r])));
+                        if (mx > 0.0) {
+                            const int fe = ilogb(mx);
+                            if (fe > 64 || fe < -64) {
+                                const int kk = -fe < -1022 ? -1022 : (-fe > 1023 ? 1023 : -fe);
+                                const double f = pow2i(kk);
+#pragma unroll
+                                for (int r = 0; r < R; ++r) { N[r] *= f; D[r] *= f; }
+                                Nl *= f;
+                                if (k <= kres) sum.s[0] *= f;
+                                e += kk;
+                            }
+                        }
+                    }
+                    // past its last row a group's values are not the pair's and must not
+                    // rescale the finished sum
+                    if (k <= kres) sum.e = e;
                 }
             }
-            if (kres >= 0) {
+            if constexpr (!kDouble) {
+                if (kres >= 0) {
 #pragma unroll
-                for (int s = 0; s < NS; ++s) acc[s] += (double)O::side(a4, s);
+                    for (int s = 0; s < NS; ++s) sum.s[s] += (double)O::side(a4, s);
+                }
             }
             wcur = wnext;
             wnext = wpref;
         };
-        if constexpr (W == 1) {
+        if constexpr (!kBlockGroup) {
+            if (SERIAL && warp > 0) {  // row 0, before the first step
+                const RingRow r0 = left[0];
+                if (t == 0) {
+                    Ml = r0.n;
+                    Iul = r0.i;
+                    Xul = r0.x;
+                    eMl = eIul = r0.e;
+                }
+            }
             for (int k0 = 0; k0 < K; k0 += 4) four_steps(k0);
         } else {
             const int nblk = (H + 32 + kBlock - 1) / kBlock;
@@ -364,11 +593,12 @@ struct TileWavefront {
                 const int b = ss - kLag * warp;
                 if (b >= 0 && b < nblk) {  // warp-uniform
                     if (b == 0 && warp > 0) {  // row 0, before the first step
-                        const RingRow r0 = ring[(warp - 1) * kRing];
+                        const RingRow r0 = left[0];
                         if (t == 0) {
                             Ml = r0.n;
                             Iul = r0.i;
                             Xul = r0.x;
+                            eMl = eIul = r0.e;
                         }
                     }
                     for (int k0 = b * kBlock; k0 < (b + 1) * kBlock; k0 += 4) four_steps(k0);
@@ -376,6 +606,34 @@ struct TileWavefront {
                 __syncthreads();
             }
         }
+    }
+
+    // All parts of a warp's task.  threshold: below half of it on a part's last column
+    // a serial pair stops (0: never).  Returns false if it stopped.
+    __device__ __forceinline__ static bool run(const Reads& rd, const uint32_t* hw, int H, int K, bool uni, Word* tab,
+                                               RingRow* ring, RingRow* border, int64_t rows, int t, int warp, int lane,
+                                               double threshold, Sum& sum) {
+        if constexpr (!SERIAL) {
+            if (uni) loop<true>(rd, hw, H, K, tab, ring, border, rows, t, warp, lane, sum);
+            else loop<false>(rd, hw, H, K, tab, ring, border, rows, t, warp, lane, sum);
+        } else {
+            for (int part = 0; part < W; ++part) {
+                if (uni) loop<true>(rd, hw, H, K, tab, ring, border, rows, t, part, lane, sum);
+                else loop<false>(rd, hw, H, K, tab, ring, border, rows, t, part, lane, sum);
+                __syncwarp();   // the part's rows are written
+                if (threshold > 0.0 && part + 1 < W) {
+                    // M = N/n, I + D one row up = X on the part's last column
+                    const int c = (part + 1) * 32 * (R - 1) + min_i((part + 1) * 32, rd.L[0] - NL * (R - 1));
+                    const double inv_n = 1.0 / (double)__ldg(rd.ph + ((__ldg(rd.pack[0] + c) >> 16) & 0x7fu));
+                    double mass = 0.0;
+                    for (int j = t; j <= H; j += 32) mass += (double)border[kBorderPad + j].n * inv_n + (double)border[kBorderPad + j].x;
+#pragma unroll
+                    for (int d = 16; d >= 1; d >>= 1) mass += __shfl_xor_sync(kFullMask, mass, d);
+                    if (mass < 0.5 * threshold) return false;   // warp-uniform
+                }
+            }
+        }
+        return true;
     }
 };
 

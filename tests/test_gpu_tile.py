@@ -102,3 +102,33 @@ def test_exact_rules_are_checked():
                     [(152, 32, 24, 0), (156, 4, 39, 3), (1 << 30, 32, 32, 1)]):  # not compiled
             with pytest.raises(g.PairHMMError):
                 e.set_tile_table(bad)
+
+
+@pytest.mark.parametrize("gcp", [False, True])
+@pytest.mark.parametrize("gaps", ["one", "each"])
+def test_fp64_tiles_match_oracle(gaps, gcp):
+    """Unrelated high-quality reads at the edges of the FP64 classes (8, 16 and 32 lanes,
+    blocks of 4 and 8 warps, and past them), on haplotypes shorter and longer than the
+    read: every pair is recomputed in double, some beyond the scaled tier's range.  On
+    the tables for few and for many pairs, bitwise the same."""
+    rng = np.random.default_rng(5)
+    b = _Builder()
+    for L in (32, 33, 40, 41, 160, 161, 176, 320, 321, 352, 640, 641, 768, 769, 1024, 1025, 1152, 1793, 2016, 2017,
+              2048, 2049, 2304, 2305, 4096, 4097):
+        H = np.array([rng.integers(1, 60), max(2, L // 3), L + rng.integers(0, 200)])
+        n = 2 * L
+        q = rng.integers(35, 46, size=n) if gaps == "each" else np.full(n, 45)
+        b.add_concat(np.full(2, L), ACGT[rng.integers(0, 4, size=n)], rng.integers(38, 42, size=n).astype(np.uint8),
+                     q.astype(np.uint8), q.astype(np.uint8), H, ACGT[rng.integers(0, 4, size=int(H.sum()))])
+    batch = b.build()
+    batch.gcp_quals[:] = 10 if not gcp else 20
+    want = oracle.batch_log10(batch, gcp=gcp)
+    with g.Engine(gcp=gcp) as e:
+        few = e.compute(batch)
+        st = e.stats()
+        rules = e.tile_table()
+        e.set_tile_table([(8, 4, 16 if gcp else 4, 0)] + rules)
+        many = e.compute(batch)
+    assert want.min() < -650 and st.rescued > 0.9 * (want < -70).sum() and st.rescued_ext > 0
+    assert_log10_close(few, want, what="FP64 tiles")
+    np.testing.assert_array_equal(few, many)
