@@ -85,8 +85,7 @@ struct ReadMeta;
 
 struct DevView {
     const uint32_t* read_pack;
-    const float4* read_coef;    // wavefront_tile.cuh's coefficients, by packed position
-    const ReadMeta* read_meta;
+    const ReadMeta* read_meta;  // wavefront_tile.cuh
     const int64_t* read_start;  // in positions, multiple of 4
     const int32_t* read_len;
     const uint8_t* hap_code;

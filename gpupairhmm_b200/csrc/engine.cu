@@ -244,7 +244,7 @@ std::vector<DevBuf*> Engine::all_buffers() {
     return {&ph2pr_, &in_read_bases_, &in_bq_,
             &in_iq_, &in_dq_, &in_read_off_, &in_read_len_, &in_hap_bases_, &in_hap_off_, &in_hap_len_,
             &read_record_, &read_local_, &rec_haps_, &rec_hap_base_, &rec_pair_base_, &read_start_,
-            &hap_start_, &read_pack_, &read_coef_, &read_meta_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
+            &hap_start_, &read_pack_, &read_meta_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
             &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
             &rescue_ext_, &rsort_, &fp64_lut_[0], &fp64_lut_[1],
             &in_gq_, &read_gcp_};
@@ -298,6 +298,14 @@ pairhmm_status_t Engine::reserve_pool(size_t bytes) {
     return PAIRHMM_OK;
 }
 
+pairhmm_status_t Engine::ensure_side_streams(int n) {
+    for (int i = 0; i < n; ++i) {
+        if (!side_[i]) PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
+        if (!join_[i]) PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
+    }
+    return PAIRHMM_OK;
+}
+
 pairhmm_status_t Engine::init() {
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
@@ -311,10 +319,6 @@ pairhmm_status_t Engine::init() {
     if (prop.major < 10) return fail(PAIRHMM_ERR_UNSUPPORTED, "the kernels are built for sm_100a");
     num_sms_ = prop.multiProcessorCount;
     PHMM_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    for (int i = 0; i < kSideStreams; ++i) {
-        PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
-        PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
-    }
     PHMM_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
     {
         cudaMemPoolProps props{};
@@ -379,7 +383,6 @@ pairhmm_status_t Engine::build_tables(const std::vector<TileRule>& rules) {
         for (const TileRule& r : t.rules) {
             t.cfg.push_back(find_fp32_config(r.G, r.R, r.multi_tile, r.packed, r.exact, opts_.gcp != 0));
             if (!t.cfg.back()) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "tile rule without compiled kernel");
-            t.exact = t.exact || r.exact;
         }
     }
     for (int i = 0; i < 2; ++i) tables_[i] = std::move(built[i]);
@@ -672,7 +675,6 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(unit_bucket_.ensure(4 * nr));
     PHMM_CUDA(hap_start_.ensure(8 * nh));
     PHMM_CUDA(read_pack_.ensure(4 * (x.pack_positions + kReadSlackPos)));
-    if (table_->exact) PHMM_CUDA(read_coef_.ensure(sizeof(float4) * std::max<int64_t>(x.pack_positions, 1)));
     PHMM_CUDA(read_meta_.ensure(sizeof(ReadMeta) * nr));
     PHMM_CUDA(hap_code_.ensure(x.code_bytes + kHapSlack));
     const int64_t nbins = (int64_t)table_->rules.size() * hbins_of(x);
@@ -757,7 +759,6 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     pa.num_haps = x.num_haps;
     pa.read_pack = read_pack_.as<uint32_t>();
     pa.hap_code = hap_code_.as<uint8_t>();
-    pa.read_coef = table_->exact ? read_coef_.as<float4>() : nullptr;
     pa.read_meta = read_meta_.as<ReadMeta>();
     pa.ph2pr = ph2pr_.as<float>();
     if (stage == 0) {
@@ -808,7 +809,6 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     unsigned long long* counters = counters_.as<unsigned long long>();
     DevView v{};
     v.read_pack = pa.read_pack;
-    v.read_coef = pa.read_coef;
     v.read_meta = pa.read_meta;
     v.read_start = pa.read_start;
     v.read_len = in.read_lengths;
@@ -845,14 +845,24 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     }
 
     // engine form: the stage's launches go round-robin onto the side streams
-    // (forked from s, joined back below); the plain form keeps one stream
-    const bool fork = !plain;
+    // (forked from s, joined back below); the plain form, and a single launch, keep s
+    const int nside = plan.side[stage];
     int nlaunch = 0;
-    auto next_stream = [&]() { return fork ? side_[nlaunch++ % kSideStreams] : s; };
-    if (fork) {
-        PHMM_CUDA(cudaEventRecord(fork_, s));
-        for (int i = 0; i < kSideStreams; ++i) PHMM_CUDA(cudaStreamWaitEvent(side_[i], fork_, 0));
-    }
+    auto next_stream = [&]() { return nside ? side_[nlaunch++ % nside] : s; };
+    auto fork = [&]() {
+        if (nside) PHMM_CUDA(cudaEventRecord(fork_, s));
+        for (int i = 0; i < nside; ++i) PHMM_CUDA(cudaStreamWaitEvent(side_[i], fork_, 0));
+        return PAIRHMM_OK;
+    };
+    auto join = [&]() {
+        for (int i = 0; i < nside; ++i) {
+            PHMM_CUDA(cudaEventRecord(join_[i], side_[i]));
+            PHMM_CUDA(cudaStreamWaitEvent(s, join_[i], 0));
+        }
+        return PAIRHMM_OK;
+    };
+    pairhmm_status_t fs = fork();
+    if (fs != PAIRHMM_OK) return fs;
     if (stage == 1) {
         for (int rank = 0; rank < nb; ++rank) {
             const int b = plain ? rank : nb - 1 - rank;
@@ -914,27 +924,14 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
         bool any = false;
         for (bool b : shared_ext) any = any || b;
         if (any) {
-            if (fork) {
-                for (int i = 0; i < kSideStreams; ++i) {
-                    PHMM_CUDA(cudaEventRecord(join_[i], side_[i]));
-                    PHMM_CUDA(cudaStreamWaitEvent(s, join_[i], 0));
-                }
-                PHMM_CUDA(cudaEventRecord(fork_, s));
-                for (int i = 0; i < kSideStreams; ++i) PHMM_CUDA(cudaStreamWaitEvent(side_[i], fork_, 0));
-            }
+            if ((fs = join()) != PAIRHMM_OK || (fs = fork()) != PAIRHMM_OK) return fs;
             for (int e = 0; e < (int)fp64_->exts.size(); ++e)
                 if (shared_ext[e])
                     PHMM_CUDA(launch(fp64_->exts[e].cfg, true, e, plan.fp64_ext_grid[e], plan.fp64_ext_scratch[e], 0,
                                      next_stream()));
         }
     }
-    if (fork) {
-        for (int i = 0; i < kSideStreams; ++i) {
-            PHMM_CUDA(cudaEventRecord(join_[i], side_[i]));
-            PHMM_CUDA(cudaStreamWaitEvent(s, join_[i], 0));
-        }
-    }
-    return PAIRHMM_OK;
+    return join();
 }
 
 Engine::Plan Engine::make_plan(const BatchIndex& x) {
@@ -1012,6 +1009,10 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
         scratch += std::max(slice, bytes);
     }
     p.scratch_bytes = (size_t)std::max<int64_t>(std::max(scratch, fp32_scratch), 256);
+    int launches[3] = {};
+    for (int b = 0; b < nb; ++b) launches[1] += x.bucket_items[b] != 0;
+    for (int64_t n : x.class_pairs) launches[2] += n != 0;
+    for (int st = 1; st < 3; ++st) p.side[st] = plain || launches[st] < 2 ? 0 : std::min(launches[st], kSideStreams);
     return p;
 }
 
@@ -1021,6 +1022,8 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     // every buffer the launches reference exists before capture starts
     const Plan plan = make_plan(x);
     PHMM_CUDA(scratch_.ensure(plan.scratch_bytes));
+    const pairhmm_status_t side = ensure_side_streams(std::max(plan.side[1], plan.side[2]));
+    if (side != PAIRHMM_OK) return side;
     cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
     for (int stage = 0; stage < 3; ++stage) {
         if (!opts_.use_graphs) {

@@ -35,7 +35,6 @@ inline bool operator==(const TileRule& a, const TileRule& b) {
 struct TileTable {
     std::vector<TileRule> rules;
     std::vector<const ConfigInfo*> cfg;
-    bool exact = false;   // some rule is exact: the preparation forms FP32 coefficients
 };
 
 // Length classes of the FP64 pass and their kernels.
@@ -149,6 +148,7 @@ private:
         int fp64_ext_grid[kMaxFp64Classes] = {};  // by extended-tier class
         int64_t fp64_scratch[kMaxFp64Classes] = {};      // border scratch offsets of the
         int64_t fp64_ext_scratch[kMaxFp64Classes] = {};  // kernels that need it
+        int side[3] = {};                 // side streams of a stage: one per launch, up to kSideStreams
         std::vector<int64_t> scratch_off;   // by bucket: multi-tile kernels run side by side
         size_t scratch_bytes = 0;
     };
@@ -179,8 +179,9 @@ private:
     // streams so that their tails overlap and a small batch's buckets run side
     // by side; they join back into stream_ before the stage ends
     static constexpr int kSideStreams = 16;
-    cudaStream_t side_[kSideStreams] = {};
+    cudaStream_t side_[kSideStreams] = {};   // created as batches need them
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
+    pairhmm_status_t ensure_side_streams(int n);
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
     int64_t launches_ = 0, fp32_launches_ = 0;
     cudaGraphExec_t graph_exec_[3] = {nullptr, nullptr, nullptr};  // prep, FP32, FP64
@@ -194,7 +195,7 @@ private:
     DevBuf in_hap_bases_, in_hap_off_, in_hap_len_;
     DevBuf read_record_, read_local_, rec_haps_, rec_hap_base_, rec_pair_base_, read_start_, hap_start_;
     DevBuf unit_read0_, unit_read1_, unit_bucket_;
-    DevBuf read_pack_, read_coef_, read_meta_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
+    DevBuf read_pack_, read_meta_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
     DevBuf rescue_off_, rescue_ext_, rsort_;
     // host-to-device uploads (caller inputs, index) and the reused index
     HostUploader uploader_;

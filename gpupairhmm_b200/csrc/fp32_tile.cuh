@@ -23,7 +23,11 @@ __global__ void __launch_bounds__(W == 1 || SERIAL ? kBlockThreads : 32 * W, til
 fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items, unsigned long long* counter,
                  void* scratch, int64_t rows) {
     using T = TileWavefront<V, G, R, W, GCP, false, SERIAL>;
-    extern __shared__ float4 smem[];
+    extern __shared__ float4 smem_all[];
+    float* ph = reinterpret_cast<float*>(smem_all);  // 128 probabilities
+    float4* smem = smem_all + 32;
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = v.ph2pr[i];
+    __syncthreads();
     constexpr int kWarps = T::kWarps;
     static_assert(T::kBlockGroup || kWarps == kWarpsPerBlock, "independent warps");
     const int warp = threadIdx.x >> 5;
@@ -70,11 +74,14 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
             for (int s = 0; s < T::NS; ++s) {
                 const int read = s && it.read1 >= 0 ? it.read1 : it.read0;
                 rd.L[s] = v.read_len[read];
-                const int64_t start = v.read_start[read];
-                rd.coef[s] = v.read_coef + start;
-                rd.pack[s] = v.read_pack + start;
-                rd.w_end[s] = v.read_meta[read].w_end;
-                if constexpr (GCP) rd.eps[s] = v.ph2pr[v.read_gcp[read]];
+                rd.pack[s] = v.read_pack + v.read_start[read];
+                rd.beta[s] = kBeta;
+                rd.inv_beta[s] = 1.0f / kBeta;
+                if constexpr (GCP) {
+                    rd.eps[s] = ph[v.read_gcp[read]];
+                    rd.beta[s] = (float)(1.0 - (double)rd.eps[s]);  // gpuworker.cuh:1049
+                    rd.inv_beta[s] = 1.0f / rd.beta[s];
+                }
                 const unsigned key = v.read_meta[read].key;
                 kmin = min(kmin, key);
                 kmax = max(kmax, key);
@@ -86,7 +93,7 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
             double stop = 0.0;
             if (SERIAL && v.rescue_enabled)
                 stop = (double)tile_threshold(rd.L[0], H, v.read_meta[item->read0].range);
-            rd.ph = v.ph2pr;
+            rd.ph = ph;
             T::run(rd, hw, H, K, uni, tab, ring, border, rows, t, T::kBlockGroup ? warp : 0, lane, stop, sum);
         }
 
@@ -103,7 +110,7 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
                 const int64_t out = s ? vi->out1 : vi->out0;
                 const int L = v.read_len[read];
                 const ReadMeta meta = v.read_meta[read];
-                v.scores[out] = (float)(log10(sum.s[s] / (double)H) - log10((double)kTileD0));
+                v.scores[out] = (float)(log10(sum.s[s] / (double)H) - log10((double)kTileD0) - (double)meta.bias);
                 if ((meta.flags & 1u) ||
                     (v.rescue_enabled && !(sum.s[s] >= (double)tile_threshold(L, H, meta.range) &&
                                            sum.s[s] <= (double)FLT_MAX)))

@@ -20,7 +20,11 @@ __global__ void __launch_bounds__(W == 1 ? kBlockThreads : 32 * W, tile64_min_ct
 fp64_tile_kernel(DevView v, const Task* __restrict__ items, const unsigned long long* count,
                  unsigned long long* counter, ExtList ext) {
     using T = TileWavefront<double, G, R, W, GCP, EXT>;
-    extern __shared__ double2 smem64[];
+    extern __shared__ double2 smem64_all[];
+    float* ph = reinterpret_cast<float*>(smem64_all);  // 128 probabilities
+    double2* smem64 = smem64_all + 32;
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = v.ph2pr[i];
+    __syncthreads();
     constexpr int kWarps = T::kWarps;
     static_assert(T::kBlockGroup || kWarps == kWarpsPerBlock, "independent warps");
     const int warp = threadIdx.x >> 5;
@@ -57,11 +61,10 @@ fp64_tile_kernel(DevView v, const Task* __restrict__ items, const unsigned long 
             typename T::Reads rd;
             rd.L[0] = v.read_len[it.read];
             rd.pack[0] = v.read_pack + v.read_start[it.read];
-            rd.ph = v.ph2pr;
-            const float eps = GCP ? v.ph2pr[v.read_gcp[it.read]] : kEps;
+            rd.ph = ph;
+            const float eps = GCP ? ph[v.read_gcp[it.read]] : kEps;
             rd.eps[0] = (double)eps;
-            rd.beta = GCP ? (double)(float)(1.0 - (double)eps) : (double)kBeta;  // gpuworker.cuh:1049
-            rd.w_end[0] = 1.0 / (double)v.ph2pr[(__ldg(rd.pack[0] + rd.L[0] - 1) >> 16) & 0x7fu];
+            rd.beta[0] = GCP ? (double)(float)(1.0 - (double)eps) : (double)kBeta;  // gpuworker.cuh:1049
             const unsigned key = v.read_meta[it.read].key;
             const unsigned kmax = __reduce_max_sync(kFullMask, key);
             const bool uni = __reduce_min_sync(kFullMask, key) == kmax && kmax != kNoKey;
@@ -78,7 +81,7 @@ fp64_tile_kernel(DevView v, const Task* __restrict__ items, const unsigned long 
             if (sum.s[0] > 0.0)
                 res = log10(sum.s[0] / (double)H) - (double)e * 0.30102999566398119521 - log10((double)kTileD0);
             // gcp quality 0: beta = 0, nothing to rescale by
-            const bool none = GCP && !((float)(1.0 - (double)v.ph2pr[v.read_gcp[read]]) > 0.0f);
+            const bool none = GCP && !((float)(1.0 - (double)ph[v.read_gcp[read]]) > 0.0f);
             v.scores[out] = none ? NAN : (float)res;
             if (!EXT && !none &&
                 !(sum.s[0] >= scaled_tile_threshold(L, H, v.read_meta[read].range) && sum.s[0] <= DBL_MAX))

@@ -47,9 +47,7 @@ struct PrepArgs {
     uint32_t* read_pack;
     uint8_t* hap_code;
     uint8_t* read_gcp;              // [num_reads], gcp mode only (else null)
-    float4* read_coef;              // wavefront_tile.cuh's FP32 coefficients by packed position
-                                    // (null: no exact FP32 tile in the table), and
-    ReadMeta* read_meta;            // what its kernels need per read
+    ReadMeta* read_meta;            // what the exact-tile kernels need per read
     const float* ph2pr;             // 128 probabilities
 };
 
@@ -79,9 +77,9 @@ __device__ __forceinline__ uint32_t pack_position(uint32_t base, uint32_t bq, ui
 // 16-byte word group.  Where the four source arrays are 4-byte aligned at the
 // read's offset, whole groups inside the read are read with one 4-byte load
 // per array; the read's ragged end (and unaligned sources) go byte by byte.
-// The exact-tile kernel's coefficients are formed here, once per read instead of
-// once per pair (8.5 haplotypes a read in the uneven workload, three divisions a
-// position): 16 bytes a position that stay in L2 between a read's haplotypes.
+// Also notes per read what the exact-tile kernels ask of all its positions.  Forming
+// their coefficients here too, 16 bytes a position, was measured: 2.3 times the
+// stage's time (0.11 -> 0.25 ms for 2,000 uneven regions) for 1% of the FP32 stage's.
 __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int64_t nblocks) {
     const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (nblocks * blockDim.x) >> 5;
@@ -101,7 +99,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
             const uint32_t g = L > 0 ? a.gcp_quals[src] : 10u;
             a.read_gcp[i] = (uint8_t)(g > 127u ? 127u : g);
         }
-        float beta = kBeta, range = 0.0f;
+        float range = 0.0f, bias = 0.0f, beta = kBeta;
         uint32_t key = kNoKey, flags = 0;
         bool same = true;   // gap qualities of the lane's positions equal the first position's
         if (L > 0) {
@@ -113,6 +111,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                 if (!(beta >= kMinAlpha)) flags = 1u;      // gcp quality 0: nothing to rescale by
             }
         }
+        const float inv_beta = 1.0f / beta;
         for (int c = lane * 4; c < Lp; c += 128) {
             uint32_t w[4];
             if (aligned && c + 3 < L) {
@@ -136,23 +135,17 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                 for (int j = 0; j < 4; ++j) {
                     if (c + j >= L) break;
                     same = same && (w[j] >> 16) == (key & 0xffu) * 0x101u;
-                    const bool end = c + j + 1 >= L;
-                    float dn = d, sn = sg, an = beta;
-                    if (!end) {
-                        if (j < 3) {
-                            dn = a.ph2pr[(w[j < 3 ? j + 1 : 3] >> 16) & 0x7fu];
-                            sn = a.ph2pr[(w[j < 3 ? j + 1 : 3] >> 24) & 0x7fu];
-                        } else {
-                            dn = a.ph2pr[min((uint32_t)iq[c + 4], 127u)];
-                            sn = a.ph2pr[min((uint32_t)dq[c + 4], 127u)];
-                        }
-                        an = 1.0f - (dn + sn);
+                    float dn = d, sn = sg;   // past the end the last position's
+                    if (c + j + 1 < L) {
+                        const uint32_t in = j < 3 ? (w[j < 3 ? j + 1 : 3] >> 16) & 0x7fu : min((uint32_t)iq[c + 4], 127u);
+                        const uint32_t sd = j < 3 ? (w[j < 3 ? j + 1 : 3] >> 24) & 0x7fu : min((uint32_t)dq[c + 4], 127u);
+                        dn = a.ph2pr[in];
+                        sn = a.ph2pr[sd];
                     }
-                    const float4 cf = tile_coefficients(a.ph2pr[(w[j] >> 8) & 0x7fu], d, sg, an, dn, beta);
-                    if (a.read_coef) a.read_coef[a.read_start[i] + c + j] = cf;
-                    range = fmaxf(range, 1.0f / dn + 2.0f * (1.0f + cf.y));
+                    const TileLink k = tile_link(c + j + 1 < L ? 1.0f - (dn + sn) : beta, dn, beta, inv_beta);
+                    range = fmaxf(range, k.id + 2.0f * (1.0f + sg * k.id));
+                    bias += tile_emission_error(1.0f - a.ph2pr[(w[j] >> 8) & 0x7fu], k);
                     if (!(fabsf(1.0f - (d + sg)) >= kMinAlpha)) flags |= 1u;
-                    if (end) a.read_meta[i].w_end = tile_weight(beta, dn, beta);
                     d = dn;
                     sg = sn;
                 }
@@ -163,7 +156,10 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
             flags = __any_sync(kFullMask, flags != 0u) ? 1u : 0u;
             // positive floats order as their bits; an infinite or NaN bound stays the largest
             range = __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(range)));
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) bias += __shfl_xor_sync(kFullMask, bias, d);
             if (lane == 0) {
+                a.read_meta[i].bias = bias * 0.43429448f;
                 a.read_meta[i].range = range;
                 a.read_meta[i].key = same ? key : kNoKey;
                 a.read_meta[i].flags = flags;

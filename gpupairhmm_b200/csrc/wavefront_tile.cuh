@@ -160,33 +160,47 @@ __device__ __forceinline__ double scaled_tile_threshold(int L, int H, float rang
     return (double)L * (double)H * (double)range * 0x1p-1030;
 }
 
-// One read position's coefficients for this kernel (w, x, l of a match, l of a
-// mismatch) from its own and the next position's gap probabilities; past the read's
-// end a_next = beta and d_next = d.  l takes n from the rounded w of the next
-// column, so that w and l multiply to alpha*lambda up to l's own rounding: where
-// every position has the same gap quality a rounding of both would add up along
-// the read.
-__device__ __forceinline__ float tile_weight(float a, float d, float beta) { return a / (beta * d); }
-__device__ __forceinline__ float4 tile_coefficients(float p, float d, float s, float a_next, float d_next, float beta) {
-    const float w = tile_weight(1.0f - (d + s), d, beta);
-    const float wn = tile_weight(a_next, d_next, beta);
-    float g = beta * d_next, e = 0.0f;  // beta*n
-    if (wn != 0.0f) {
-        g = a_next / wn;
-        e = fmaf(-g, wn, a_next) / wn;
+// FP32 coefficients of a column boundary: w of a position from its alpha and gap-open
+// probability d, and g = beta*n of the position before it (with e, what g lacks of
+// alpha/w in single precision).  l takes n from the rounded w of the next column, so
+// that w and l multiply to alpha*lambda up to l's own rounding: where every position
+// has the same gap quality a rounding of both would add up along the read.  For the
+// same reason w may come from approximate reciprocals (two instead of four divisions a
+// position: gcp mode with per-read gcp qualities 8.28 -> 7.7 ms of FP32 stage).  Past
+// the read's end alpha is beta and d the last position's.
+struct TileLink {
+    float w, g, e, id;   // id = 1/d
+};
+__device__ __forceinline__ TileLink tile_link(float a, float d, float beta, float inv_beta) {
+    const float id = __fdividef(1.0f, d);
+    TileLink k{a * (id * inv_beta), beta * d, 0.0f, id};
+    if (k.w != 0.0f) {
+        const float rw = __fdividef(1.0f, k.w);
+        k.g = a * rw;
+        k.e = fmaf(-k.g, k.w, a) * rw;
     }
-    const float lm = 1.0f - p;   // pairhmm_kernels.cuh:1244
-    const float lx = p / 3.0f;   // pairhmm_kernels.cuh:1250
-    return make_float4(w, s == d_next ? 1.0f : beta * s / g, fmaf(lm, g, lm * e), fmaf(lx, g, lx * e));
+    return k;
+}
+
+// l of a match (pm = 1 - p) or mismatch (pm = p/3), rounded once.
+__device__ __forceinline__ float tile_emission(float pm, const TileLink& next) {
+    return fmaf(pm, next.g, pm * next.e);
+}
+// Relative error of that rounding.  A read of few distinct qualities has few distinct
+// errors, which add up along the path of matches (250 bases of quality 35-41: 9e-7 of
+// log10 on average); their sum is taken off the score.
+__device__ __forceinline__ float tile_emission_error(float pm, const TileLink& next) {
+    const float l = tile_emission(pm, next);
+    return l != 0.0f ? -(fmaf(pm, next.g, -l) + pm * next.e) / l : 0.0f;
 }
 
 // What the preparation notes per read.
 struct ReadMeta {
-    float w_end;     // 1/n of the last position
     float range;     // see tile_threshold
     uint32_t key;    // gap quality | gcp << 8 where insertions and deletions have the one quality at
                      // every position, else kNoKey
     uint32_t flags;  // bit 0: some |alpha| < kMinAlpha, the FP64 pass computes the read's pairs
+    float bias;      // log10 of what rounding the match l of every position did to their product
 };
 static_assert(sizeof(ReadMeta) == 16, "ReadMeta is one 16-byte word");
 constexpr uint32_t kNoKey = 0xffffffffu;
@@ -232,32 +246,34 @@ struct TileWavefront {
     // so that no step branches on which part it runs
     static constexpr int kRings = W > 1 ? kWarps : 0;
     static constexpr int kBorderPad = 32;   // serial: row j sits at entry j + 32 of a buffer
-    static constexpr size_t kBlockSmem = kWarps * kSmemBytes + kRings * kRing * sizeof(RingRow);
+    static constexpr size_t kBlockSmem = 128 * sizeof(float) + kWarps * kSmemBytes + kRings * kRing * sizeof(RingRow);
 
     struct Reads {
-        const float4* coef[NS];     // FP32: the read's coefficients, position 0 first
-        const float* ph;            // FP64: the probabilities, coefficients are formed in double
-        const uint32_t* pack[NS];   // packed words (the base code in the low byte)
+        const float* ph;            // the probabilities (shared memory)
+        const uint32_t* pack[NS];   // packed words of the read's positions
         int L[NS];
-        S w_end[NS];
         S eps[NS];                  // GCP only
-        S beta;                     // FP64
+        S beta[NS];
+        float inv_beta[NS];         // FP32
     };
     struct Sum {
         double s[NS];               // sum of T over the haplotype's rows, in the result lane
         int e;                      // EXT: its exponent
     };
 
-    // FP64 coefficients.  Probabilities are the 32-bit model parameters, alpha and
-    // 1 - p formed in FP32 as the reference forms them, everything else in double.
+    // Probabilities are the 32-bit model parameters, alpha, 1 - p and p/3 formed in FP32
+    // as the reference forms them; FP64 forms the coefficients in double.
     struct Gap {
-        double i;   // 1/(beta*delta)
         float d, s;
     };
-    __device__ __forceinline__ static Gap gap(const Reads& rd, int c) {
-        const uint32_t w = __ldg(rd.pack[0] + c);
-        const float d = __ldg(rd.ph + ((w >> 16) & 0x7fu));
-        return Gap{1.0 / (rd.beta * (double)d), d, __ldg(rd.ph + ((w >> 24) & 0x7fu))};
+    __device__ __forceinline__ static Gap gap(const Reads& rd, int s, int c) {
+        const uint32_t w = __ldg(rd.pack[s] + c);
+        return Gap{rd.ph[(w >> 16) & 0x7fu], rd.ph[(w >> 24) & 0x7fu]};
+    }
+    // the boundary before position c, c = L being the read's end
+    __device__ __forceinline__ static TileLink link(const Reads& rd, int s, int c) {
+        const Gap g = gap(rd, s, min_i(c, rd.L[s] - 1));
+        return tile_link(c < rd.L[s] ? 1.0f - (g.d + g.s) : (float)rd.beta[s], g.d, (float)rd.beta[s], rd.inv_beta[s]);
     }
 
     // One warp's part of a group.  warp: its number in the group (0 where a warp holds
@@ -273,6 +289,8 @@ struct TileWavefront {
         V wv[UNI ? 1 : R], xv[UNI ? 1 : R], N[R], D[R];
         {
             S w[NS][UNI ? 1 : R], x[NS][UNI ? 1 : R];
+            float lg[NS][UNI || kDouble ? 1 : R], le[NS][UNI || kDouble ? 1 : R];
+            TileLink mid[NS], last[NS];   // UNI: towards every position but the one past the end, and towards that
             int p0[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
@@ -281,38 +299,49 @@ struct TileWavefront {
                 p0[s] = u * (R - 1) + min_i(u, m);
                 if constexpr (UNI) {
                     if constexpr (kDouble) {
-                        const Gap g = gap(rd, 0);
-                        w[s][0] = (double)(1.0f - (g.d + g.s)) * g.i;
+                        const Gap g = gap(rd, s, 0);
+                        w[s][0] = (double)(1.0f - (g.d + g.s)) * (1.0 / (rd.beta[s] * (double)g.d));
                     } else {
-                        w[s][0] = __ldg(&rd.coef[s]->x);
+                        mid[s] = link(rd, s, 0);
+                        last[s] = link(rd, s, rd.L[s]);
+                        w[s][0] = mid[s].w;
                     }
                 }
             }
             if constexpr (!UNI && kDouble) {
-                Gap g = gap(rd, min_i(p0[0], rd.L[0] - 1));
+                Gap g = gap(rd, 0, min_i(p0[0], rd.L[0] - 1));
+                double i = 1.0 / (rd.beta[0] * (double)g.d);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int c = p0[0] + r;
-                    const Gap n = gap(rd, min_i(c + 1, rd.L[0] - 1));   // past the end the last position's again
-                    wv[r] = c < rd.L[0] ? (double)(1.0f - (g.d + g.s)) * g.i : 0.0;
-                    xv[r] = c >= rd.L[0] ? 0.0 : g.s == n.d ? 1.0 : rd.beta * (double)g.s * n.i;
+                    const Gap n = gap(rd, 0, min_i(c + 1, rd.L[0] - 1));   // past the end the last position's again
+                    const double in = 1.0 / (rd.beta[0] * (double)n.d);
+                    wv[r] = c < rd.L[0] ? (double)(1.0f - (g.d + g.s)) * i : 0.0;
+                    xv[r] = c >= rd.L[0] ? 0.0 : g.s == n.d ? 1.0 : rd.beta[0] * (double)g.s * in;
                     g = n;
+                    i = in;
                 }
             }
             if constexpr (!UNI && !kDouble) {
 #pragma unroll
-                for (int s = 0; s < NS; ++s)
+                for (int s = 0; s < NS; ++s) {
+                    Gap g = gap(rd, s, min_i(p0[s], rd.L[s] - 1));
+                    w[s][0] = link(rd, s, min_i(p0[s], rd.L[s])).w;
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        const float2 wx = p0[s] + r < rd.L[s]
-                                              ? __ldg(reinterpret_cast<const float2*>(rd.coef[s] + p0[s] + r))
-                                              : make_float2(0.f, 0.f);
-                        w[s][r] = wx.x;
-                        x[s][r] = wx.y;
+                        const int c = p0[s] + r;
+                        const TileLink k = link(rd, s, min_i(c + 1, rd.L[s]));
+                        const Gap n = gap(rd, s, min_i(c + 1, rd.L[s] - 1));
+                        x[s][r] = c >= rd.L[s] ? 0.0f : g.s == n.d ? 1.0f : g.s * k.id;
+                        if (r + 1 < R) w[s][r + 1 < R ? r + 1 : r] = k.w;
+                        lg[s][r] = k.g;
+                        le[s][r] = k.e;
+                        g = n;
                     }
-                // w and x go through the lane's table slots once: kept as loaded, in 16-byte
-                // coefficient words, ptxas put their pairs together again at every step
-                // (three moves a position, a quarter of the step)
+                }
+                // w and x go through the lane's table slots once: otherwise ptxas put the pairs
+                // together from their halves again at every step (three moves a position, a
+                // quarter of the step)
 #pragma unroll
                 for (int q = 0; q < Q; ++q) {
                     Word ww, xw;
@@ -353,16 +382,22 @@ struct TileWavefront {
                         if (r < R && c < rd.L[s]) {
                             const uint32_t word = __ldg(rd.pack[s] + c);
                             code = word & 0xffu;
+                            const float p = rd.ph[(word >> 8) & 0x7fu];
+                            const float pm = 1.0f - p;    // pairhmm_kernels.cuh:1244
+                            const float px = p / 3.0f;    // pairhmm_kernels.cuh:1250
                             if constexpr (kDouble) {
-                                const uint32_t next = __ldg(rd.pack[s] + min_i(c + 1, rd.L[s] - 1));
-                                const float p = __ldg(rd.ph + ((word >> 8) & 0x7fu));
-                                const double n = rd.beta * (double)__ldg(rd.ph + ((next >> 16) & 0x7fu));
-                                lm = (double)(1.0f - p) * n;
-                                lx = (double)(p / 3.0f) * n;
+                                const double n = rd.beta[0] * (double)gap(rd, 0, min_i(c + 1, rd.L[0] - 1)).d;
+                                lm = (double)pm * n;
+                                lx = (double)px * n;
                             } else {
-                                const float2 cf = __ldg(reinterpret_cast<const float2*>(rd.coef[s] + c) + 1);
-                                lm = cf.x;
-                                lx = cf.y;
+                                const bool end = c + 1 >= rd.L[s];
+                                TileLink k = end ? last[s] : mid[s];
+                                if constexpr (!UNI) {
+                                    k.g = lg[s][r < R ? r : 0];
+                                    k.e = le[s][r < R ? r : 0];
+                                }
+                                lm = tile_emission(pm, k);
+                                lx = tile_emission(px, k);
                             }
                         }
 #pragma unroll
@@ -387,7 +422,9 @@ struct TileWavefront {
             eps = O::make(rd.eps[0], rd.eps[NS - 1]);
             if constexpr (UNI) eps = O::uniform(eps);
         }
-        const V wend = O::make(rd.w_end[0], rd.w_end[NS - 1]);
+        V wend;   // 1/n of the read's last position
+        if constexpr (kDouble) wend = 1.0 / (double)gap(rd, 0, rd.L[0] - 1).d;
+        else wend = O::make(link(rd, 0, rd.L[0]).w, link(rd, NS - 1, rd.L[NS - 1]).w);
         constexpr S kD0 = kDouble && !EXT ? (S)kTileD0 * (S)kScaled : (S)kTileD0;
         const V zero = O::make(0.f, 0.f), d0 = O::make(kD0, kD0);
         const bool first = u == 0;
@@ -624,7 +661,7 @@ struct TileWavefront {
                 if (threshold > 0.0 && part + 1 < W) {
                     // M = N/n, I + D one row up = X on the part's last column
                     const int c = (part + 1) * 32 * (R - 1) + min_i((part + 1) * 32, rd.L[0] - NL * (R - 1));
-                    const double inv_n = 1.0 / (double)__ldg(rd.ph + ((__ldg(rd.pack[0] + c) >> 16) & 0x7fu));
+                    const double inv_n = 1.0 / (double)gap(rd, 0, c).d;
                     double mass = 0.0;
                     for (int j = t; j <= H; j += 32) mass += (double)border[kBorderPad + j].n * inv_n + (double)border[kBorderPad + j].x;
 #pragma unroll
