@@ -245,15 +245,14 @@ std::vector<DevBuf*> Engine::all_buffers() {
             &in_iq_, &in_dq_, &in_read_off_, &in_read_len_, &in_hap_bases_, &in_hap_off_, &in_hap_len_,
             &read_record_, &read_local_, &rec_haps_, &rec_hap_base_, &rec_pair_base_, &read_start_,
             &hap_start_, &read_pack_, &read_meta_, &hap_code_, &hist_, &cursor_, &items_, &rescue_, &counters_,
-            &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &rescue_off_,
+            &scores_, &scratch_, &unit_read0_, &unit_read1_, &unit_bucket_, &arena_, &rescue_off_,
             &rescue_ext_, &rsort_, &fp64_lut_[0], &fp64_lut_[1],
             &in_gq_, &read_gcp_};
 }
 
 Engine::~Engine() {
     if (ready_) cudaSetDevice(opts_.device);
-    for (cudaGraphExec_t& g : graph_exec_)
-        if (g) cudaGraphExecDestroy(g);
+    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     for (DevBuf* b : all_buffers()) b->release();
     if (stream_) cudaStreamSynchronize(stream_);
     if (pool_) cudaMemPoolDestroy(pool_);
@@ -364,10 +363,8 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
     }
     const char* wrong = check_rules(rules, opts_.gcp != 0);
     if (wrong) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, wrong);
-    for (cudaGraphExec_t& g : graph_exec_) {
-        if (g) cudaGraphExecDestroy(g);
-        g = nullptr;
-    }
+    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
+    graph_exec_ = nullptr;
     if (ready_) return build_tables(rules);
     tables_[0].rules = rules;
     return PAIRHMM_OK;
@@ -645,35 +642,9 @@ pairhmm_status_t Engine::ensure_inputs(const InputRanges& r) {
     return PAIRHMM_OK;
 }
 
-pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
-    const int64_t nr = std::max<int64_t>(x.num_reads, 1), nh = std::max<int64_t>(x.num_haps, 1);
-    const int64_t ng = std::max<int64_t>(x.num_records, 1), np = std::max<int64_t>(x.num_pairs, 1);
-    if (host_inputs) {
-        const int64_t rb = std::max<int64_t>(x.read_bytes - x.read_min, 1);
-        const int64_t hb = std::max<int64_t>(x.hap_bytes - x.hap_min, 1);
-        PHMM_CUDA(in_read_bases_.ensure(rb));
-        PHMM_CUDA(in_bq_.ensure(rb));
-        PHMM_CUDA(in_iq_.ensure(rb));
-        PHMM_CUDA(in_dq_.ensure(rb));
-        if (opts_.gcp) PHMM_CUDA(in_gq_.ensure(rb));
-        PHMM_CUDA(in_read_off_.ensure(8 * nr));
-        PHMM_CUDA(in_read_len_.ensure(4 * nr));
-        PHMM_CUDA(in_hap_bases_.ensure(hb));
-        PHMM_CUDA(in_hap_off_.ensure(8 * nh));
-        PHMM_CUDA(in_hap_len_.ensure(4 * nh));
-        PHMM_CUDA(scores_.ensure(4 * np));
-    }
-    PHMM_CUDA(read_record_.ensure(4 * nr));
-    PHMM_CUDA(read_local_.ensure(4 * nr));
+pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x) {
+    const int64_t nr = std::max<int64_t>(x.num_reads, 1), np = std::max<int64_t>(x.num_pairs, 1);
     if (opts_.gcp) PHMM_CUDA(read_gcp_.ensure(nr));
-    PHMM_CUDA(rec_haps_.ensure(4 * ng));
-    PHMM_CUDA(rec_hap_base_.ensure(8 * ng));
-    PHMM_CUDA(rec_pair_base_.ensure(8 * ng));
-    PHMM_CUDA(read_start_.ensure(8 * nr));
-    PHMM_CUDA(unit_read0_.ensure(4 * nr));
-    PHMM_CUDA(unit_read1_.ensure(4 * nr));
-    PHMM_CUDA(unit_bucket_.ensure(4 * nr));
-    PHMM_CUDA(hap_start_.ensure(8 * nh));
     PHMM_CUDA(read_pack_.ensure(4 * (x.pack_positions + kReadSlackPos)));
     PHMM_CUDA(read_meta_.ensure(sizeof(ReadMeta) * nr));
     PHMM_CUDA(hap_code_.ensure(x.code_bytes + kHapSlack));
@@ -683,25 +654,97 @@ pairhmm_status_t Engine::ensure_buffers(const BatchIndex& x, bool host_inputs) {
     PHMM_CUDA(items_.ensure(sizeof(Item) * np));
     PHMM_CUDA(rescue_.ensure(sizeof(Task) * np));  // class lists laid out back to back
     PHMM_CUDA(rescue_ext_.ensure(sizeof(Task) * np));  // the extended tier's, same offsets
-    PHMM_CUDA(rescue_off_.ensure(sizeof(x.list_start)));
     return PAIRHMM_OK;
 }
 
+namespace {
+// The index's arrays: where each one's device pointer goes, its host data and bytes.
+struct IndexArray {
+    const void** ptr;
+    const void* src;
+    size_t bytes;
+};
+}  // namespace
+
+#define PHMM_INDEX_ARRAYS(x)                                                                        \
+    {                                                                                               \
+        {(const void**)&ix_.read_record, x.read_record.data(), 4 * x.read_record.size()},           \
+        {(const void**)&ix_.read_local, x.read_local.data(), 4 * x.read_local.size()},              \
+        {(const void**)&ix_.rec_haps, x.rec_haps.data(), 4 * x.rec_haps.size()},                    \
+        {(const void**)&ix_.rec_hap_base, x.rec_hap_base.data(), 8 * x.rec_hap_base.size()},        \
+        {(const void**)&ix_.rec_pair_base, x.rec_pair_base.data(), 8 * x.rec_pair_base.size()},     \
+        {(const void**)&ix_.read_start, x.read_start.data(), 8 * x.read_start.size()},              \
+        {(const void**)&ix_.hap_start, x.hap_start.data(), 8 * x.hap_start.size()},                 \
+        {(const void**)&ix_.unit_read0, x.unit_read0.data(), 4 * x.unit_read0.size()},              \
+        {(const void**)&ix_.unit_read1, x.unit_read1.data(), 4 * x.unit_read1.size()},              \
+        {(const void**)&ix_.unit_bucket, x.unit_bucket.data(), 4 * x.unit_bucket.size()},           \
+        {(const void**)&ix_.list_start, x.list_start, sizeof(x.list_start)},                        \
+    }
+
 pairhmm_status_t Engine::upload_index(const BatchIndex& x, cudaStream_t s) {
-    const std::vector<HostUploader::Copy> copies = {
-        {read_record_.ptr, x.read_record.data(), 4 * x.read_record.size()},
-        {read_local_.ptr, x.read_local.data(), 4 * x.read_local.size()},
-        {rec_haps_.ptr, x.rec_haps.data(), 4 * x.rec_haps.size()},
-        {rec_hap_base_.ptr, x.rec_hap_base.data(), 8 * x.rec_hap_base.size()},
-        {rec_pair_base_.ptr, x.rec_pair_base.data(), 8 * x.rec_pair_base.size()},
-        {read_start_.ptr, x.read_start.data(), 8 * x.read_start.size()},
-        {hap_start_.ptr, x.hap_start.data(), 8 * x.hap_start.size()},
-        {unit_read0_.ptr, x.unit_read0.data(), 4 * x.unit_read0.size()},
-        {unit_read1_.ptr, x.unit_read1.data(), 4 * x.unit_read1.size()},
-        {unit_bucket_.ptr, x.unit_bucket.data(), 4 * x.unit_bucket.size()},
-        {rescue_off_.ptr, x.list_start, sizeof(x.list_start)},
-    };
+    if ((size_t)index_bytes(x) + sizeof(x.list_start) <= HostUploader::kGatherBytes / 2)
+        return upload_gathered(x, nullptr, nullptr, s);
+    DevBuf* const bufs[] = {&read_record_,  &read_local_, &rec_haps_,   &rec_hap_base_, &rec_pair_base_, &read_start_,
+                            &hap_start_,    &unit_read0_, &unit_read1_, &unit_bucket_,  &rescue_off_};
+    const IndexArray arrays[] = PHMM_INDEX_ARRAYS(x);
+    static_assert(sizeof(bufs) / sizeof(bufs[0]) == sizeof(arrays) / sizeof(arrays[0]), "a buffer per array");
+    std::vector<HostUploader::Copy> copies;
+    for (size_t i = 0; i < sizeof(arrays) / sizeof(arrays[0]); ++i) {
+        PHMM_CUDA(bufs[i]->ensure(std::max<size_t>(arrays[i].bytes, 1)));
+        *arrays[i].ptr = bufs[i]->ptr;
+        copies.push_back({bufs[i]->ptr, arrays[i].src, arrays[i].bytes});
+    }
     PHMM_CUDA(uploader_.run(opts_.device, copies, s));
+    return PAIRHMM_OK;
+}
+
+size_t Engine::input_bytes(const InputRanges& r, bool gcp) {
+    return (size_t)((gcp ? 5 : 4) * (r.read_end - r.read_min) + (r.hap_end - r.hap_min) + 12 * r.num_reads +
+                    12 * r.num_haps);
+}
+
+pairhmm_status_t Engine::upload_gathered(const BatchIndex& x, const InputRanges* r, pairhmm_batch_t* in,
+                                         cudaStream_t s) {
+    const IndexArray index[] = PHMM_INDEX_ARRAYS(x);
+    std::vector<HostUploader::Part> parts;
+    parts.reserve(24);
+    std::vector<const void**> ptrs;
+    ptrs.reserve(24);
+    size_t total = 0;
+    auto add = [&](const void** ptr, const void* src, size_t bytes) {
+        parts.push_back({total, src, bytes});
+        ptrs.push_back(ptr);
+        total += (bytes + 15) & ~size_t(15);
+    };
+    if (r) {
+        const size_t rn = (size_t)(r->read_end - r->read_min), hn = (size_t)(r->hap_end - r->hap_min);
+        add((const void**)&in->read_bases, in->read_bases + r->read_min, rn);
+        add((const void**)&in->base_quals, in->base_quals + r->read_min, rn);
+        add((const void**)&in->ins_quals, in->ins_quals + r->read_min, rn);
+        add((const void**)&in->del_quals, in->del_quals + r->read_min, rn);
+        if (opts_.gcp) add((const void**)&in->gcp_quals, in->gcp_quals + r->read_min, rn);
+        add((const void**)&in->hap_bases, in->hap_bases + r->hap_min, hn);
+        add((const void**)&in->read_offsets, in->read_offsets, 8 * (size_t)r->num_reads);
+        add((const void**)&in->read_lengths, in->read_lengths, 4 * (size_t)r->num_reads);
+        add((const void**)&in->hap_offsets, in->hap_offsets, 8 * (size_t)r->num_haps);
+        add((const void**)&in->hap_lengths, in->hap_lengths, 4 * (size_t)r->num_haps);
+    }
+    for (const IndexArray& a : index) add(a.ptr, a.src, a.bytes);
+    PHMM_CUDA(arena_.ensure(total));
+    PHMM_CUDA(uploader_.gather(opts_.device, arena_.ptr, total, parts, s));
+    for (size_t i = 0; i < ptrs.size(); ++i) *ptrs[i] = arena_.as<uint8_t>() + parts[i].offset;
+    if (r) {
+        // the caller's absolute offsets stay valid: byte arrays are shifted to their start
+        auto shift = [](const uint8_t*& p, int64_t lo) {
+            p = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) - (uintptr_t)lo);
+        };
+        shift(in->read_bases, r->read_min);
+        shift(in->base_quals, r->read_min);
+        shift(in->ins_quals, r->read_min);
+        shift(in->del_quals, r->read_min);
+        if (opts_.gcp) shift(in->gcp_quals, r->read_min);
+        shift(in->hap_bases, r->hap_min);
+    }
     return PAIRHMM_OK;
 }
 
@@ -748,13 +791,13 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     pa.hap_lengths = in.hap_lengths;
     pa.gcp_quals = opts_.gcp ? in.gcp_quals : nullptr;
     pa.read_gcp = opts_.gcp ? read_gcp_.as<uint8_t>() : nullptr;
-    pa.read_record = read_record_.as<int32_t>();
-    pa.read_local = read_local_.as<int32_t>();
-    pa.rec_haps = rec_haps_.as<int32_t>();
-    pa.rec_hap_base = rec_hap_base_.as<int64_t>();
-    pa.rec_pair_base = rec_pair_base_.as<int64_t>();
-    pa.read_start = read_start_.as<int64_t>();
-    pa.hap_start = hap_start_.as<int64_t>();
+    pa.read_record = ix_.read_record;
+    pa.read_local = ix_.read_local;
+    pa.rec_haps = ix_.rec_haps;
+    pa.rec_hap_base = ix_.rec_hap_base;
+    pa.rec_pair_base = ix_.rec_pair_base;
+    pa.read_start = ix_.read_start;
+    pa.hap_start = ix_.hap_start;
     pa.num_reads = x.num_reads;
     pa.num_haps = x.num_haps;
     pa.read_pack = read_pack_.as<uint32_t>();
@@ -787,9 +830,9 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     ba.rec_haps = pa.rec_haps;
     ba.rec_hap_base = pa.rec_hap_base;
     ba.rec_pair_base = pa.rec_pair_base;
-    ba.unit_read0 = unit_read0_.as<int32_t>();
-    ba.unit_read1 = unit_read1_.as<int32_t>();
-    ba.unit_bucket = unit_bucket_.as<int32_t>();
+    ba.unit_read0 = ix_.unit_read0;
+    ba.unit_read1 = ix_.unit_read1;
+    ba.unit_bucket = ix_.unit_bucket;
     ba.num_units = (int64_t)x.unit_read0.size();
     ba.nbuckets = nb;
     ba.hcap = plain ? 0 : std::min(kHBins - 1, x.max_hap_len);
@@ -818,7 +861,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     v.scores = d_scores;
     v.rescue_base = rescue_.as<Task>();
     v.rescue_class = fp64_lut_[fp64_ == &fp64_tables_[1]].as<uint8_t>();
-    v.rescue_off = rescue_off_.as<long long>();
+    v.rescue_off = ix_.list_start;
     v.rescue_count = counters + kCtrScaled;
     v.rescue_enabled = (!plain && opts_.fp64_rescue) ? 1 : 0;
     v.ph2pr = ph2pr_.as<float>();
@@ -834,7 +877,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
         ra.in = rescue_.as<Task>();
         ra.out = fp64_lists;
         ra.classes = (int)fp64_->classes.size();
-        ra.off = rescue_off_.as<long long>();
+        ra.off = ix_.list_start;
         ra.count = counters + kCtrScaled;
         ra.hap_len = in.hap_lengths;
         ra.hist = rsort_.as<unsigned int>();
@@ -893,7 +936,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
                           cudaStream_t on) {
             Fp64LaunchArgs fa{};
             fa.view = v;
-            fa.ext_list = {rescue_ext_.as<Task>(), rescue_off_.as<long long>() + kMaxFp64Classes, counters + kCtrExt,
+            fa.ext_list = {rescue_ext_.as<Task>(), ix_.list_start + kMaxFp64Classes, counters + kCtrExt,
                            ext_cls};
             fa.items = (tier_ext ? rescue_ext_.as<Task>() : fp64_lists) +
                        x.list_start[tier_ext ? kMaxFp64Classes + list : list];
@@ -1024,45 +1067,46 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     PHMM_CUDA(scratch_.ensure(plan.scratch_bytes));
     const pairhmm_status_t side = ensure_side_streams(std::max(plan.side[1], plan.side[2]));
     if (side != PAIRHMM_OK) return side;
-    cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
-    for (int stage = 0; stage < 3; ++stage) {
-        if (!opts_.use_graphs) {
-            pairhmm_status_t st = enqueue_pipeline(in, x, plan, d_scores, s, stage);
+    const cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
+    if (!opts_.use_graphs) {
+        for (int stage = 0; stage < 3; ++stage) {
+            const pairhmm_status_t st = enqueue_pipeline(in, x, plan, d_scores, s, stage);
             if (st != PAIRHMM_OK) return st;
-        } else {
-            cudaGraph_t graph = nullptr;
-            PHMM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            pairhmm_status_t st = enqueue_pipeline(in, x, plan, d_scores, s, stage);
-            cudaError_t ce = cudaStreamEndCapture(s, &graph);
-            if (st != PAIRHMM_OK) {
-                if (graph) cudaGraphDestroy(graph);
-                return st;
-            }
-            if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
-            cudaGraphExec_t& exec = graph_exec_[stage];
-            bool updated = false;
-            if (exec) {
-                cudaGraphExecUpdateResultInfo info{};
-                if (cudaGraphExecUpdate(exec, graph, &info) == cudaSuccess) updated = true;
-                else {
-                    cudaGetLastError();
-                    cudaGraphExecDestroy(exec);
-                    exec = nullptr;
-                }
-            }
-            if (!updated) {
-                ce = cudaGraphInstantiate(&exec, graph, 0);
-                if (ce != cudaSuccess) {
-                    cudaGraphDestroy(graph);
-                    exec = nullptr;
-                    return cuda_fail(ce, "cudaGraphInstantiate");
-                }
-            }
-            cudaGraphDestroy(graph);
-            PHMM_CUDA(cudaGraphLaunch(exec, s));
+            PHMM_CUDA(cudaEventRecord(marks[stage], s));
         }
-        PHMM_CUDA(cudaEventRecord(marks[stage], s));
+        return PAIRHMM_OK;
     }
+    // one graph for the three stages, the marks between them recorded by its nodes
+    cudaGraph_t graph = nullptr;
+    PHMM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    pairhmm_status_t st = PAIRHMM_OK;
+    for (int stage = 0; stage < 3 && st == PAIRHMM_OK; ++stage) {
+        st = enqueue_pipeline(in, x, plan, d_scores, s, stage);
+        if (st != PAIRHMM_OK) break;
+        const cudaError_t me = cudaEventRecordWithFlags(marks[stage], s, cudaEventRecordExternal);
+        if (me != cudaSuccess) st = cuda_fail(me, "cudaEventRecordWithFlags");
+    }
+    cudaError_t ce = cudaStreamEndCapture(s, &graph);
+    if (st != PAIRHMM_OK) {
+        if (graph) cudaGraphDestroy(graph);
+        return st;
+    }
+    if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
+    if (graph_exec_) {
+        cudaGraphExecUpdateResultInfo info{};
+        if (cudaGraphExecUpdate(graph_exec_, graph, &info) != cudaSuccess) {
+            cudaGetLastError();
+            cudaGraphExecDestroy(graph_exec_);
+            graph_exec_ = nullptr;
+        }
+    }
+    if (!graph_exec_) {
+        ce = cudaGraphInstantiate(&graph_exec_, graph, 0);
+        if (ce != cudaSuccess) graph_exec_ = nullptr;
+    }
+    cudaGraphDestroy(graph);
+    if (ce != cudaSuccess) return cuda_fail(ce, "cudaGraphInstantiate");
+    PHMM_CUDA(cudaGraphLaunch(graph_exec_, s));
     return PAIRHMM_OK;
 }
 
@@ -1079,52 +1123,62 @@ pairhmm_status_t Engine::host_begin(const pairhmm_batch_t& b, float* scores, cud
     stats_ = pairhmm_stats_t{};
     pending_ = false;
     if (rg.num_pairs == 0) return PAIRHMM_OK;
-    if ((st = ensure_inputs(rg)) != PAIRHMM_OK) return st;
     cudaStream_t s = stream_;
-    // only the byte range the batch references is copied; device base pointers
-    // are shifted so the caller's absolute offsets stay valid
-    const int64_t rlo = rg.read_min, rn = rg.read_end - rg.read_min;
-    const int64_t hlo = rg.hap_min, hn = rg.hap_end - rg.hap_min;
-    std::vector<HostUploader::Copy> inputs = {
-        {in_read_bases_.ptr, b.read_bases + rlo, (size_t)rn},
-        {in_bq_.ptr, b.base_quals + rlo, (size_t)rn},
-        {in_iq_.ptr, b.ins_quals + rlo, (size_t)rn},
-        {in_dq_.ptr, b.del_quals + rlo, (size_t)rn},
-        {in_read_off_.ptr, b.read_offsets, (size_t)(8 * rg.num_reads)},
-        {in_read_len_.ptr, b.read_lengths, (size_t)(4 * rg.num_reads)},
-        {in_hap_bases_.ptr, b.hap_bases + hlo, (size_t)hn},
-        {in_hap_off_.ptr, b.hap_offsets, (size_t)(8 * rg.num_haps)},
-        {in_hap_len_.ptr, b.hap_lengths, (size_t)(4 * rg.num_haps)},
-    };
-    if (opts_.gcp) inputs.push_back({in_gq_.ptr, b.gcp_quals + rlo, (size_t)rn});
-    cudaError_t up = uploader_.start(opts_.device, inputs, s);
     choose_table(b.num_records, b.reads_per_record, b.haps_per_record, b.read_lengths, rg.num_pairs);
-    st = build_index(b, table_->rules, *fp64_, idx_, err);
-    const cudaError_t upf = uploader_.finish();
-    if (up == cudaSuccess) up = upf;
-    if (up != cudaSuccess) return cuda_fail(up, "input upload");
-    if (st != PAIRHMM_OK) return fail(st, err);
     const BatchIndex& x = idx_;
+    pairhmm_batch_t dev = b;
+    // upper bound of what a gathered upload takes, alignment included
+    const size_t gathered = input_bytes(rg, opts_.gcp != 0) + 28 * (size_t)rg.num_reads + 8 * (size_t)rg.num_haps +
+                            20 * (size_t)b.num_records + sizeof(x.list_start) + 512;
+    if (gathered <= HostUploader::kGatherBytes) {
+        PHMM_CUDA(scores_.ensure(4 * rg.num_pairs));
+        if ((st = build_index(b, table_->rules, *fp64_, idx_, err)) != PAIRHMM_OK) return fail(st, err);
+        if ((st = ensure_buffers(x)) != PAIRHMM_OK) return st;
+        if ((st = upload_gathered(x, &rg, &dev, s)) != PAIRHMM_OK) return st;
+    } else {
+        if ((st = ensure_inputs(rg)) != PAIRHMM_OK) return st;
+        // only the byte range the batch references is copied; device base pointers
+        // are shifted so the caller's absolute offsets stay valid
+        const int64_t rlo = rg.read_min, rn = rg.read_end - rg.read_min;
+        const int64_t hlo = rg.hap_min, hn = rg.hap_end - rg.hap_min;
+        std::vector<HostUploader::Copy> inputs = {
+            {in_read_bases_.ptr, b.read_bases + rlo, (size_t)rn},
+            {in_bq_.ptr, b.base_quals + rlo, (size_t)rn},
+            {in_iq_.ptr, b.ins_quals + rlo, (size_t)rn},
+            {in_dq_.ptr, b.del_quals + rlo, (size_t)rn},
+            {in_read_off_.ptr, b.read_offsets, (size_t)(8 * rg.num_reads)},
+            {in_read_len_.ptr, b.read_lengths, (size_t)(4 * rg.num_reads)},
+            {in_hap_bases_.ptr, b.hap_bases + hlo, (size_t)hn},
+            {in_hap_off_.ptr, b.hap_offsets, (size_t)(8 * rg.num_haps)},
+            {in_hap_len_.ptr, b.hap_lengths, (size_t)(4 * rg.num_haps)},
+        };
+        if (opts_.gcp) inputs.push_back({in_gq_.ptr, b.gcp_quals + rlo, (size_t)rn});
+        cudaError_t up = uploader_.start(opts_.device, inputs, s);
+        st = build_index(b, table_->rules, *fp64_, idx_, err);
+        const cudaError_t upf = uploader_.finish();
+        if (up == cudaSuccess) up = upf;
+        if (up != cudaSuccess) return cuda_fail(up, "input upload");
+        if (st != PAIRHMM_OK) return fail(st, err);
+        if ((st = ensure_buffers(x)) != PAIRHMM_OK) return st;
+        if ((st = upload_index(x, s)) != PAIRHMM_OK) return st;
+
+        auto shifted = [](const DevBuf& d, int64_t lo) {
+            return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(d.ptr) - (uintptr_t)lo);
+        };
+        dev.read_bases = shifted(in_read_bases_, rlo);
+        dev.base_quals = shifted(in_bq_, rlo);
+        dev.ins_quals = shifted(in_iq_, rlo);
+        dev.del_quals = shifted(in_dq_, rlo);
+        dev.gcp_quals = opts_.gcp ? shifted(in_gq_, rlo) : nullptr;
+        dev.read_offsets = in_read_off_.as<int64_t>();
+        dev.read_lengths = in_read_len_.as<int32_t>();
+        dev.hap_bases = shifted(in_hap_bases_, hlo);
+        dev.hap_offsets = in_hap_off_.as<int64_t>();
+        dev.hap_lengths = in_hap_len_.as<int32_t>();
+    }
     stats_.pairs = x.num_pairs;
     stats_.cells = x.cells;
     stats_.multi_tile_pairs = x.multi_tile_pairs;
-    if ((st = ensure_buffers(x, false)) != PAIRHMM_OK) return st;
-    if ((st = upload_index(x, s)) != PAIRHMM_OK) return st;
-
-    pairhmm_batch_t dev = b;
-    auto shifted = [](const DevBuf& d, int64_t lo) {
-        return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(d.ptr) - (uintptr_t)lo);
-    };
-    dev.read_bases = shifted(in_read_bases_, rlo);
-    dev.base_quals = shifted(in_bq_, rlo);
-    dev.ins_quals = shifted(in_iq_, rlo);
-    dev.del_quals = shifted(in_dq_, rlo);
-    dev.gcp_quals = opts_.gcp ? shifted(in_gq_, rlo) : nullptr;
-    dev.read_offsets = in_read_off_.as<int64_t>();
-    dev.read_lengths = in_read_len_.as<int32_t>();
-    dev.hap_bases = shifted(in_hap_bases_, hlo);
-    dev.hap_offsets = in_hap_off_.as<int64_t>();
-    dev.hap_lengths = in_hap_len_.as<int32_t>();
 
     PHMM_CUDA(cudaEventRecord(ev0_, s));
     if (mark_start) PHMM_CUDA(cudaEventRecord(mark_start, s));
@@ -1139,7 +1193,7 @@ pairhmm_status_t Engine::host_begin(const pairhmm_batch_t& b, float* scores, cud
         PHMM_CUDA(cudaMemcpyAsync(scores, scores_.ptr, 4 * (size_t)x.num_pairs, cudaMemcpyDeviceToHost, s));
     pend_scores_ = scores;
     pend_pairs_ = x.num_pairs;
-    stats_.h2d_bytes = 4 * rn + hn + 12 * x.num_reads + 12 * x.num_haps + index_bytes(x);
+    stats_.h2d_bytes = (int64_t)input_bytes(rg, opts_.gcp != 0) + index_bytes(x);
     stats_.d2h_bytes = 4 * x.num_pairs + (int64_t)sizeof(unsigned long long) * 2 * kMaxFp64Classes;
     stats_.launches = launches_;
     stats_.fp32_launches = fp32_launches_;
@@ -1331,7 +1385,7 @@ pairhmm_status_t Engine::compute_device(const pairhmm_batch_t& b, int32_t, int32
     stats_.rescued_ext = -1;
     if (x.num_pairs == 0) return PAIRHMM_OK;
     if (!scores) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, "null scores");
-    if ((st = ensure_buffers(x, false)) != PAIRHMM_OK) return st;
+    if ((st = ensure_buffers(x)) != PAIRHMM_OK) return st;
     cudaStream_t s = stream_;
     PHMM_CUDA(cudaEventRecord(ev0_, stream));
     PHMM_CUDA(cudaStreamWaitEvent(s, ev0_, 0));

@@ -156,9 +156,14 @@ private:
     // stage 0: packing + work list, 1: FP32 launches, 2: FP64 pass
     pairhmm_status_t enqueue_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, const Plan& plan,
                                       float* d_scores, cudaStream_t s, int stage);
-    pairhmm_status_t ensure_buffers(const BatchIndex& idx, bool host_inputs);
+    pairhmm_status_t ensure_buffers(const BatchIndex& idx);
     pairhmm_status_t ensure_inputs(const InputRanges& r);
+    // The index (and, gathered, the inputs too: `in` points at the host arrays and comes
+    // back pointing at device copies) onto the device.
     pairhmm_status_t upload_index(const BatchIndex& idx, cudaStream_t s);
+    pairhmm_status_t upload_gathered(const BatchIndex& idx, const InputRanges* r, pairhmm_batch_t* in,
+                                     cudaStream_t s);
+    static size_t input_bytes(const InputRanges& r, bool gcp);
     int persistent_grid(const void* kernel, int threads, size_t smem);
     static int64_t index_bytes(const BatchIndex& x);
     int64_t hbins_of(const BatchIndex& x) const;
@@ -184,7 +189,7 @@ private:
     pairhmm_status_t ensure_side_streams(int n);
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
     int64_t launches_ = 0, fp32_launches_ = 0;
-    cudaGraphExec_t graph_exec_[3] = {nullptr, nullptr, nullptr};  // prep, FP32, FP64
+    cudaGraphExec_t graph_exec_ = nullptr;   // the whole batch: prep, FP32, FP64
     pairhmm_stats_t stats_{};
     std::string last_error_;
 
@@ -195,6 +200,13 @@ private:
     DevBuf in_hap_bases_, in_hap_off_, in_hap_len_;
     DevBuf read_record_, read_local_, rec_haps_, rec_hap_base_, rec_pair_base_, read_start_, hap_start_;
     DevBuf unit_read0_, unit_read1_, unit_bucket_;
+    DevBuf arena_;   // a small batch's inputs and index, uploaded in one copy
+    // the current batch's index on the device
+    struct IndexPtrs {
+        const int32_t *read_record, *read_local, *rec_haps, *unit_read0, *unit_read1, *unit_bucket;
+        const int64_t *rec_hap_base, *rec_pair_base, *read_start, *hap_start;
+        const long long* list_start;
+    } ix_{};
     DevBuf read_pack_, read_meta_, hap_code_, hist_, cursor_, items_, rescue_, counters_, scores_, scratch_;
     DevBuf rescue_off_, rescue_ext_, rsort_;
     // host-to-device uploads (caller inputs, index) and the reused index

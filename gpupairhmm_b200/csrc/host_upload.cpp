@@ -79,6 +79,11 @@ cudaError_t HostUploader::start(int device, const std::vector<Copy>& copies, cud
     pieces_.clear();
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return e;
+    // pieces of about a sixteenth of the job, so that a mid-size job's host copies and
+    // DMAs overlap too, not only those of several slots' worth
+    size_t total = 0;
+    for (const Copy& c : copies) total += c.bytes;
+    const size_t piece = std::min(kSlotBytes, std::max(kPieceBytes, (total / 16 + 4095) & ~size_t(4095)));
     for (const Copy& c : copies) {
         if (c.bytes == 0) continue;
         if (is_page_locked(c.src)) {
@@ -86,9 +91,9 @@ cudaError_t HostUploader::start(int device, const std::vector<Copy>& copies, cud
             direct_ += c.bytes;
             continue;
         }
-        for (size_t off = 0; off < c.bytes; off += kSlotBytes)
+        for (size_t off = 0; off < c.bytes; off += piece)
             pieces_.push_back({static_cast<char*>(c.dst) + off, static_cast<const char*>(c.src) + off,
-                               std::min(kSlotBytes, c.bytes - off)});
+                               std::min(piece, c.bytes - off)});
         staged_ += c.bytes;
     }
     if (pieces_.empty()) return cudaSuccess;
@@ -120,6 +125,20 @@ cudaError_t HostUploader::finish() {
     for (cudaError_t x : err_)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
+}
+
+cudaError_t HostUploader::gather(int device, void* base, size_t total, const std::vector<Part>& parts,
+                                 cudaStream_t s) {
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = ensure_staging();
+    if (e == cudaSuccess) e = cudaEventSynchronize(done_[0]);  // the slot's earlier use is over
+    if (e != cudaSuccess) return e;
+    for (const Part& p : parts)
+        if (p.bytes) std::memcpy(stage_ + p.offset, p.src, p.bytes);
+    staged_ = total;
+    direct_ = 0;
+    e = cudaMemcpyAsync(base, stage_, total, cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? cudaEventRecord(done_[0], s) : e;
 }
 
 cudaError_t HostUploader::download(int device, void* dst, const void* src, size_t bytes, cudaStream_t s) {

@@ -49,6 +49,18 @@ public:
         return e != cudaSuccess ? e : f;
     }
 
+    // A small job: every source is copied to its offset of one staging slot by the
+    // calling thread, and the slot goes to device memory `base` in one DMA.  With a copy
+    // of its own for each array and the copy threads woken twice, the upload was half of
+    // a one-region call.  total <= kGatherBytes.
+    struct Part {
+        size_t offset;
+        const void* src;
+        size_t bytes;
+    };
+    static constexpr size_t kGatherBytes = size_t(384) << 10;
+    cudaError_t gather(int device, void* base, size_t total, const std::vector<Part>& parts, cudaStream_t s);
+
     // Device-to-host copy of `bytes` after the work already on stream s: one
     // DMA into a page-locked `dst`, else chunks through the staging slots,
     // each copied out on the host as soon as its DMA lands.  Returns when dst
@@ -66,6 +78,7 @@ private:
     static constexpr int kThreads = 4;
     static constexpr int kSlotsPerThread = 2;
     static constexpr size_t kSlotBytes = size_t(8) << 20;
+    static constexpr size_t kPieceBytes = size_t(256) << 10;   // smallest piece
     cudaError_t ensure_staging();
     void worker_loop(int t);
     void copy_pieces(int t);
