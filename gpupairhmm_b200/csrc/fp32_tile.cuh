@@ -67,14 +67,14 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
         {
             const Item it = *item;
             const int H = v.hap_len[it.hap];
-            const uint32_t* hw = reinterpret_cast<const uint32_t*>(v.hap_code + v.hap_start[it.hap]);
+            const PackedHap hap(reinterpret_cast<const uint32_t*>(v.hap_code + v.hap_start[it.hap]), H);
             typename T::Reads rd;
             unsigned kmin = kNoKey, kmax = 0;
 #pragma unroll
             for (int s = 0; s < T::NS; ++s) {
                 const int read = s && it.read1 >= 0 ? it.read1 : it.read0;
                 rd.L[s] = v.read_len[read];
-                rd.pack[s] = v.read_pack + v.read_start[read];
+                rd.read[s].p = v.read_pack + v.read_start[read];
                 rd.beta[s] = kBeta;
                 rd.inv_beta[s] = 1.0f / kBeta;
                 if constexpr (GCP) {
@@ -94,7 +94,7 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
             if (SERIAL && v.rescue_enabled)
                 stop = (double)tile_threshold(rd.L[0], H, v.read_meta[item->read0].range);
             rd.ph = ph;
-            T::run(rd, hw, H, K, uni, tab, ring, border, rows, t, T::kBlockGroup ? warp : 0, lane, stop, sum);
+            T::run(rd, hap, H, K, uni, tab, ring, border, rows, t, T::kBlockGroup ? warp : 0, lane, stop, sum);
         }
 
         // a serial pair that stopped has no sum: below any threshold
@@ -133,7 +133,7 @@ template <class V, int G, int R, int W, bool GCP, bool SERIAL = false>
 ConfigInfo make_tile_config() {
     using T = TileWavefront<V, G, R, W, GCP, false, SERIAL>;
     ConfigInfo c{};
-    c.G = T::NL;
+    c.G = T::kLanes;
     c.R = R;
     c.multi_tile = W > 1;
     c.packed = T::NS == 2;

@@ -57,10 +57,10 @@ fp64_tile_kernel(DevView v, const Task* __restrict__ items, const unsigned long 
         {
             const Task it = *item;
             const int H = v.hap_len[it.hap];
-            const uint32_t* hw = reinterpret_cast<const uint32_t*>(v.hap_code + v.hap_start[it.hap]);
+            const PackedHap hap(reinterpret_cast<const uint32_t*>(v.hap_code + v.hap_start[it.hap]), H);
             typename T::Reads rd;
             rd.L[0] = v.read_len[it.read];
-            rd.pack[0] = v.read_pack + v.read_start[it.read];
+            rd.read[0].p = v.read_pack + v.read_start[it.read];
             rd.ph = ph;
             const float eps = GCP ? ph[v.read_gcp[it.read]] : kEps;
             rd.eps[0] = (double)eps;
@@ -69,7 +69,7 @@ fp64_tile_kernel(DevView v, const Task* __restrict__ items, const unsigned long 
             const unsigned kmax = __reduce_max_sync(kFullMask, key);
             const bool uni = __reduce_min_sync(kFullMask, key) == kmax && kmax != kNoKey;
             const int K = T::kBlockGroup ? 0 : (int)((__reduce_max_sync(kFullMask, (unsigned)(H + G)) + 3u) & ~3u);
-            T::run(rd, hw, H, K, uni, tab, ring, nullptr, 0, t, T::kBlockGroup ? warp : 0, lane, 0.0, sum);
+            T::run(rd, hap, H, K, uni, tab, ring, nullptr, 0, t, T::kBlockGroup ? warp : 0, lane, 0.0, sum);
         }
         if (active && t == G - 1 && (!T::kBlockGroup || warp == W - 1)) {
             const volatile Task* vi = item;   // read again rather than kept over the steps
@@ -103,7 +103,7 @@ template <int G, int R, int W, bool GCP, bool EXT>
 Fp64Config make_tile64_config() {
     using T = TileWavefront<double, G, R, W, GCP, EXT>;
     Fp64Config c{};
-    c.G = T::NL;
+    c.G = T::kLanes;
     c.R = R;
     c.ext = EXT;
     c.gcp = GCP;

@@ -9,12 +9,19 @@
 // call allocates nothing: no cudaMalloc, no cudaFree, no allocating library
 // routine, no host heap either.
 //
-// The kernel is a variant of the multi-tile FP32 wavefront (G = 32 lanes,
-// R = 16 positions per lane, tiles of 512 read positions) that reads the
-// caller's bytes directly instead of a packed copy.  Its only scratch, the
-// per-warp border between read tiles, lives in kScratchBytes of statically
-// allocated device memory defined below: every GPU that loads this library
-// holds that much memory until the process exits.  Limits: haplotype length
+// The kernel reads the caller's bytes directly instead of a packed copy.  A warp
+// takes a few consecutive pairs of the list at a time and runs those of one shape
+// together on the exact tiles of wavefront_tile.cuh: 8 lanes a pair up to 160
+// positions, 16 up to 320, then 32 lanes with the read's parts in turn.  Few pairs
+// (reads of at most 8 positions, gap probabilities too small for that kernel's
+// range) take a general form: the whole warp, 16 positions a lane, read tiles of
+// 512.  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
+// the general form for all (one pair on 512 positions a warp, eleven operations a
+// cell); what bounds it is the instruction cache (several shapes in flight) and the
+// last pairs of a short list.
+// The only scratch, the per-warp border between a read's parts, lives in
+// kScratchBytes of statically allocated device memory defined below: every GPU
+// that loads this library holds that much memory until the process exits.  Limits: haplotype length
 // up to kMaxHapLength; any read length.  Results are FP32 only, with no FP64
 // recompute of pairs whose FP32 result underflows (those return what FP32
 // gives, possibly -inf, as the reference does).
@@ -33,6 +40,7 @@
 
 #include "../../include/pairhmm_b200.h"
 #include "device_common.cuh"
+#include "wavefront_tile.cuh"
 
 namespace phmm {
 namespace noalloc {
@@ -61,42 +69,128 @@ __device__ __forceinline__ uint32_t encode(uint8_t c) {
 
 __device__ __forceinline__ float ph_of(const float* ph, uint8_t q) { return ph[q > 127 ? 127 : q]; }
 
-// One pair per warp, read tiles of kT positions, beta absorbed into I and D
-// (M keeps alpha, so no division and no degenerate-alpha case):
+// The work queue: pairs handed out so far and blocks done.  The last block of a call
+// sets both back to zero, so a call needs no other launch before it.
+static __device__ unsigned g_queue[2];
+
+struct Args {
+    const uint8_t *read_bases, *base_quals, *ins_quals, *del_quals, *hap_bases;
+    const pairhmm_pair_t* pairs;
+    int64_t num_pairs;
+    float* scores;
+    float4* scratch;    // per warp 2 * rows
+    int64_t rows;
+    int64_t nwarps;
+    int max_h;
+    int grab;           // pairs a warp takes at a time, at most 32
+};
+
+// A read's positions straight from the caller's arrays, as the packed words hold them.
+struct ByteRead {
+    const uint8_t *b, *bq, *iq, *dq;
+    __device__ __forceinline__ uint32_t word(int c) const {
+        auto q = [&](const uint8_t* a) { const uint32_t v = __ldg(a + c); return v > 127u ? 127u : v; };
+        return encode(__ldg(b + c)) | (q(bq) << 8) | (q(iq) << 16) | (q(dq) << 24);
+    }
+};
+struct ByteHap {
+    const uint8_t* p;
+    int H;
+    __device__ __forceinline__ uint32_t codes(int i) const {
+        uint32_t w = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w |= encode(__ldg(p + min_i(4 * i + j, H - 1))) << (8 * j);
+        return w;
+    }
+};
+
+constexpr int kMaxR = 20;
+// R is a multiple of 4, so a lane holds R .. R-4 positions (the read's length over the
+// lanes, rounded down, may be one below the shape's smallest).  With an R for every 8
+// positions some 15 shapes were in flight and the kernel waited for instructions
+// (no_instruction 4.8 of 7 cycles per issue, 2.1 ms).
+constexpr int kStepR = 4;
+constexpr int span_of(int R) { return R > kStepR ? kStepR + 1 : R; }
+constexpr int kTableBytes = 5 * (kMaxR / 4) * 32 * 16;   // per warp
+constexpr int kRingBytes = 64 * 16;
+constexpr size_t kSmem = (kThreads / 32) * (size_t)(kTableBytes + kRingBytes);
+
+// Pairs `mine` (by lane: the group's pair, or -1) of one shape.  The general form
+// takes what this refuses: returns false (warp-uniform) where some pair's gap
+// probabilities lie too far below 1.
+template <int G, int R>
+__device__ __noinline__ bool run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
+    using T = TileWavefront<float, G, R, G == 32 ? 0 : 1, false, false, G == 32, ByteRead, ByteHap, span_of(R)>;
+    const int lane = threadIdx.x & 31;
+    const int t = lane % G;
+    // groups without a pair repeat the first group's and write nothing
+    const int64_t first = __shfl_sync(kFullMask, mine, 0);
+    const pairhmm_pair_t pr = a.pairs[mine >= 0 ? mine : first];
+    const int L = pr.read_length, H = pr.hap_length;
+    typename T::Reads rd;
+    rd.ph = ph;
+    rd.read[0] = ByteRead{a.read_bases + pr.read_offset, a.base_quals + pr.read_offset, a.ins_quals + pr.read_offset,
+                          a.del_quals + pr.read_offset};
+    rd.L[0] = L;
+    rd.beta[0] = kBeta;
+    rd.inv_beta[0] = 1.0f / kBeta;
+    // what the engine's preparation notes per read
+    const uint32_t w0 = rd.read[0].word(0);
+    bool same = true;
+    float bias = 0.0f, least = 1.0f;
+    for (int c = t; c < L; c += G) {
+        const uint32_t w = rd.read[0].word(c);
+        same = same && (w >> 16) == ((w0 >> 16) & 0xffu) * 0x101u;
+        least = fminf(least, ph[(w >> 16) & 0xffu]);
+        bias += tile_emission_error(1.0f - ph[(w >> 8) & 0xffu], T::link(rd, 0, c + 1));
+    }
+#pragma unroll
+    for (int d = G / 2; d >= 1; d >>= 1) bias += __shfl_xor_sync(kFullMask, bias, d);
+    // N lies 1/delta below M; D enters 2H/beta above the general form's boundary value.
+    // Up to 2^8 of the low end of the range is given up here
+    if (__any_sync(kFullMask, least * (256.0f * 2.0f / kBeta) * (float)H < 1.0f)) return false;
+    const unsigned key = (w0 >> 16) & 0xffu;
+    const bool uni = __all_sync(kFullMask, same) &&
+                     __reduce_min_sync(kFullMask, key) == __reduce_max_sync(kFullMask, key);
+    const int K = (int)((__reduce_max_sync(kFullMask, (unsigned)(H + G)) + 3u) & ~3u);
+    typename T::Sum sum;
+    sum.s[0] = 0.0;
+    auto* tab = reinterpret_cast<typename T::Word*>(smem);
+    static_assert(T::kSmemBytes <= kTableBytes && (G < 32 || T::kRing * sizeof(typename T::RingRow) <= kRingBytes),
+                  "the block's shared memory holds every shape's table and ring");
+    auto* ring = reinterpret_cast<typename T::RingRow*>(smem + kTableBytes);
+    const ByteHap hap{a.hap_bases + pr.hap_offset, H};
+    T::run(rd, hap, H, K, uni, tab, ring, reinterpret_cast<typename T::RingRow*>(wscr), a.rows, t, 0, lane, 0.0, sum,
+           parts);
+    if (mine >= 0 && t == G - 1)
+        a.scores[mine] = (float)(log10(sum.s[0] / (double)H) - log10((double)kTileD0) -
+                                 (double)(bias * 0.43429448f));
+    __syncwarp();
+    return true;
+}
+
+// The general form: one pair on the warp, read tiles of kT positions, beta absorbed
+// into I and D (M keeps alpha, so no division and no degenerate-alpha case):
 //   M(j,c)  = lambda*(alpha_c*M(j-1,c-1) + It(j-1,c-1) + Dt(j-1,c-1))
 //   It(j,c) = eps_c*It(j,c-1) + beta*delta_c*M(j,c-1)
 //   Dt(j,c) = beta*sigma_c*M(j-1,c) + eps*Dt(j-1,c)
-__global__ void __launch_bounds__(kThreads)
-forward_pairs_kernel(const uint8_t* __restrict__ read_bases, const uint8_t* __restrict__ base_quals,
-                     const uint8_t* __restrict__ ins_quals, const uint8_t* __restrict__ del_quals,
-                     const uint8_t* __restrict__ hap_bases, const pairhmm_pair_t* __restrict__ pairs,
-                     int64_t num_pairs, float* __restrict__ scores, float4* scratch, int64_t rows,
-                     int64_t nwarps, int max_h) {
-    __shared__ float ph[128];
-    for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = c_ph2pr[i];
-    __syncthreads();
+__device__ __noinline__ void run_general(const Args& a, const float* ph, float4* wscr, int64_t pi) {
     const int t = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= nwarps) return;  // the scratch holds borders for nwarps warps only
-    float4* const wscr = scratch + warp * 2 * rows;
-
-    for (int64_t pi = warp; pi < num_pairs; pi += nwarps) {  // warp-uniform
-        const pairhmm_pair_t pr = pairs[pi];
+    const int64_t rows = a.rows;
+    float* const scores = a.scores;
+    {
+        const pairhmm_pair_t pr = a.pairs[pi];
         const int L = pr.read_length, H = pr.hap_length;
-        if (L < 1 || H < 1 || H > max_h) {  // H beyond the declared bound would overrun the border rows
-            if (t == 0) scores[pi] = NAN;
-            continue;
-        }
-        const uint8_t* rb = read_bases + pr.read_offset;
-        const uint8_t* bq = base_quals + pr.read_offset;
-        const uint8_t* iq = ins_quals + pr.read_offset;
-        const uint8_t* dq = del_quals + pr.read_offset;
-        const uint8_t* hb = hap_bases + pr.hap_offset;
+        const uint8_t* rb = a.read_bases + pr.read_offset;
+        const uint8_t* bq = a.base_quals + pr.read_offset;
+        const uint8_t* iq = a.ins_quals + pr.read_offset;
+        const uint8_t* dq = a.del_quals + pr.read_offset;
+        const uint8_t* hb = a.hap_bases + pr.hap_offset;
         const int ntiles = (L + kT - 1) / kT;
         const float Dbound = kBeta * (kScale / (float)H);
         double acc = 0.0;  // summed in double: up to 16384 rows of similar size
         int rlane = -1;
-        for (int tile = 0; tile < ntiles; ++tile) {  // (pair loop strides by nwarps)
+        for (int tile = 0; tile < ntiles; ++tile) {
             const bool last = tile == ntiles - 1;
             const int p0 = tile * kT + t * kR;
             float lm[kR], lx[kR], alpha[kR], dlt[kR], sig[kR], eps[kR], M[kR], D[kR];
@@ -192,6 +286,85 @@ forward_pairs_kernel(const uint8_t* __restrict__ read_bases, const uint8_t* __re
     }
 }
 
+// Shape of a pair's tile: 0 general, else lanes << 8 | positions a lane.
+__device__ __forceinline__ int shape_of(int L) {
+    if (L <= 8) return 0;   // 8 lanes of at least one position
+    const int G = L <= 160 ? 8 : L <= 320 ? 16 : 32;
+    const int lanes = G * (G == 32 ? (L + 32 * kMaxR - 1) / (32 * kMaxR) : 1);
+    return (G << 8) | (((L + lanes - 1) / lanes + kStepR - 1) / kStepR * kStepR);
+}
+
+template <int G, int R0, int R1>   // R0, R0 + kStepR, .. R1
+__device__ __forceinline__ bool run_shape(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int R,
+                                          int parts) {
+    if constexpr (R0 < R1) {
+        if (R != R0) return run_shape<G, R0 + kStepR, R1>(a, ph, smem, wscr, mine, R, parts);
+    }
+    return run_tile<G, R0>(a, ph, smem, wscr, mine, parts);
+}
+
+__global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
+    __shared__ float ph[128];
+    extern __shared__ float4 smem_all[];
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = c_ph2pr[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    char* const smem = reinterpret_cast<char*>(smem_all) + (threadIdx.x >> 5) * (kTableBytes + kRingBytes);
+    float4* const wscr = a.scratch + warp * 2 * a.rows;
+    while (warp < a.nwarps) {  // the scratch holds borders for nwarps warps only
+        unsigned x = 0;
+        if (lane == 0) x = atomicAdd(&g_queue[0], 1u);
+        x = __reduce_max_sync(kFullMask, x);
+        const int64_t p0 = (int64_t)x * a.grab;
+        if (p0 >= a.num_pairs) break;
+        const int64_t pi = p0 + lane;
+        int L = 0, H = 0;
+        bool ok = lane < a.grab && pi < a.num_pairs;
+        if (ok) {
+            L = a.pairs[pi].read_length;
+            H = a.pairs[pi].hap_length;
+            if (L < 1 || H < 1 || H > a.max_h) {  // H beyond the declared bound would overrun the border rows
+                a.scores[pi] = NAN;
+                ok = false;
+            }
+        }
+        const int shape = ok ? shape_of(L) : -1;
+        unsigned left = __ballot_sync(kFullMask, ok);
+        while (left) {
+            const int lead = __ffs(left) - 1;
+            const int sh = __shfl_sync(kFullMask, shape, lead);
+            const int G = sh >> 8, R = sh & 0xff;
+            const unsigned alike = __ballot_sync(kFullMask, ok && shape == sh) & left;
+            // group g takes the g-th of the pairs of this shape, up to as many as the warp has groups
+            const int groups = G ? 32 / G : 1;
+            const int g = G ? lane / G : 0;
+            unsigned pick = alike, taken = 0;
+            int64_t mine = -1;
+            for (int i = 0; i < groups && pick; ++i) {
+                const int l = __ffs(pick) - 1;
+                pick &= pick - 1;
+                taken |= 1u << l;
+                if (i == g) mine = p0 + l;
+            }
+            left &= ~taken;
+            const int parts = G == 32 ? (__shfl_sync(kFullMask, L, lead) + 32 * kMaxR - 1) / (32 * kMaxR) : 1;
+            bool done = false;
+            if (G == 8) done = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 16) done = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 32) done = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
+            if (!done)
+                for (unsigned m = taken; m; m &= m - 1) run_general(a, ph, wscr, p0 + __ffs(m) - 1);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&g_queue[1], 1u) == gridDim.x - 1) {
+        g_queue[0] = 0;   // every block has left the queue
+        g_queue[1] = 0;
+    }
+}
+
 // per-device set-up: the scratch array's device address and the grid size
 struct DeviceState {
     std::atomic<int> ready{0};
@@ -214,7 +387,7 @@ pairhmm_status_t setup(int device, DeviceState& st) {
     st.scratch.store(addr);
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return PAIRHMM_ERR_CUDA;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, forward_pairs_kernel, kThreads, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, forward_pairs_kernel, kThreads, kSmem) != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
     st.max_warps = sms * per_sm * (kThreads / 32);
@@ -260,12 +433,15 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
         const int grid = (int)((warps + warps_per_block - 1) / warps_per_block);
         // cudaLaunchKernel returns this launch's own status, so an error the caller
         // left pending is neither reported as ours nor cleared
-        int max_h = max_hap_length;
-        int64_t np = num_pairs;
-        void* args[] = {(void*)&read_bases, (void*)&base_quals, (void*)&ins_quals, (void*)&del_quals,
-                        (void*)&hap_bases, (void*)&pairs, &np, &scores, &scratch, (void*)&rows, &warps, &max_h};
+        // pairs a warp takes at a time: a few, so that those of one read's haplotypes run
+        // together, but at least four times per warp, so that the last ones end together
+        int grab = (int)(num_pairs / (4 * warps));
+        grab = grab < 1 ? 1 : grab > 8 ? 8 : grab;
+        Args ka{read_bases, base_quals, ins_quals, del_quals, hap_bases, pairs, num_pairs, scores,
+                scratch,    rows,       warps,     max_hap_length, grab};
+        void* args[] = {&ka};
         const cudaError_t le = cudaLaunchKernel(reinterpret_cast<const void*>(&forward_pairs_kernel), dim3(grid),
-                                                dim3(kThreads), args, 0, static_cast<cudaStream_t>(stream));
+                                                dim3(kThreads), args, kSmem, static_cast<cudaStream_t>(stream));
         if (le != cudaSuccess) {
             cudaGetLastError();  // the failed launch's own error, recorded by the runtime as well
             status = PAIRHMM_ERR_CUDA;

@@ -208,19 +208,38 @@ constexpr uint32_t kNoKey = 0xffffffffu;
 // EXT (FP64): a lane keeps its values as true * 2^e with its own exponent e, for
 // pairs whose values span more than a double's range; see wavefront_fp64.cuh, whose
 // extended tier works the same way.
-template <class V, int G, int R, int W, bool GCP, bool EXT = false, bool SERIAL = false>
+// Where a group's read positions and haplotype codes come from: the batch's packed
+// layout.  word(c): a position as read_pack holds it; codes(i): the codes of rows
+// 4i .. 4i+3, behind the haplotype's end any codes (those rows are past the result's).
+struct PackedRead {
+    const uint32_t* p;
+    __device__ __forceinline__ uint32_t word(int c) const { return __ldg(p + c); }
+};
+struct PackedHap {
+    const uint32_t* p;
+    int last;
+    __device__ __forceinline__ PackedHap(const uint32_t* codes, int H) : p(codes), last(((H + 15) & ~15) / 4 - 1) {}
+    __device__ __forceinline__ uint32_t codes(int i) const { return __ldg(p + min_i(i, last)); }
+};
+
+// SERIAL with W = 0: the number of parts is given at run time.
+// SPAN: lanes hold R .. R-SPAN+1 positions, so that one kernel takes reads of
+// (NL*(R-SPAN+1), NL*R] positions, at a select more per step and value for each.
+template <class V, int G, int R, int W, bool GCP, bool EXT = false, bool SERIAL = false, class Read = PackedRead,
+          class Hap = PackedHap, int SPAN = 2>
 struct TileWavefront {
     using O = LaneOps<V>;
     using S = typename O::S;
     static constexpr bool kDouble = std::is_same<S, double>::value;
     static_assert(W == 1 || G == 32, "a group of several warps fills them");
-    static_assert(R >= 2, "a lane holds R or R-1 positions, at least one");
+    static constexpr bool kParts = W > 1 || SERIAL;   // a group may have several parts
+    static_assert(SPAN >= 2 && R >= SPAN, "a lane holds at least one position");
     static_assert(!EXT || kDouble, "lane exponents go with doubles");
     static constexpr int NS = O::kSides;
     static constexpr int NG = 32 / G;    // groups per warp
-    static constexpr int NL = G * W;     // lanes per group
+    static constexpr int kLanes = G * W;  // lanes per group (0: given at run time)
     static constexpr bool kBlockGroup = W > 1 && !SERIAL;
-    static_assert(!SERIAL || (W > 1 && NS == 1 && !kDouble), "serial parts: one FP32 read per warp");
+    static_assert(!SERIAL || (W != 1 && NS == 1 && !kDouble), "serial parts: one FP32 read per warp");
     static constexpr int VN = 16 / (int)sizeof(V);     // values per 16-byte table word
     static constexpr int Q = (R + VN - 1) / VN;        // table words per lane and code
     static constexpr int kTableWords = 5 * Q * 32;     // per warp
@@ -237,20 +256,21 @@ struct TileWavefront {
     };
     // steps unrolled.  A batch of long reads has some 14 classes of few pairs, whose kernels
     // run side by side: at 4 steps (11 KB of code each) they thrashed the instruction cache,
-    // 64 long-read regions' FP32 stage 14.6 ms against 7.0 at 2 steps and 7.9 at 1
-    static constexpr int kUnroll = SERIAL ? 2 : 4;
+    // 64 long-read regions' FP32 stage 14.6 ms against 7.0 at 2 steps and 7.9 at 1; the
+    // flat list's kernel has its shapes side by side in one launch
+    static constexpr int kUnroll = SERIAL || !std::is_same<Read, PackedRead>::value ? 2 : 4;
     static constexpr int kMaxShift = 640;   // EXT: largest scale difference a hand-off converts
     static constexpr size_t kSmemBytes = (size_t)kTableWords * sizeof(Word);  // per warp, the table
     static constexpr int kWarps = kBlockGroup ? W : 2;   // per block
     // rings per block; a group's first part reads its (constant) boundary from one too,
     // so that no step branches on which part it runs
-    static constexpr int kRings = W > 1 ? kWarps : 0;
+    static constexpr int kRings = kParts ? kWarps : 0;
     static constexpr int kBorderPad = 32;   // serial: row j sits at entry j + 32 of a buffer
     static constexpr size_t kBlockSmem = 128 * sizeof(float) + kWarps * kSmemBytes + kRings * kRing * sizeof(RingRow);
 
     struct Reads {
         const float* ph;            // the probabilities (shared memory)
-        const uint32_t* pack[NS];   // packed words of the read's positions
+        Read read[NS];
         int L[NS];
         S eps[NS];                  // GCP only
         S beta[NS];
@@ -267,7 +287,7 @@ struct TileWavefront {
         float d, s;
     };
     __device__ __forceinline__ static Gap gap(const Reads& rd, int s, int c) {
-        const uint32_t w = __ldg(rd.pack[s] + c);
+        const uint32_t w = rd.read[s].word(c);
         return Gap{rd.ph[(w >> 16) & 0x7fu], rd.ph[(w >> 24) & 0x7fu]};
     }
     // the boundary before position c, c = L being the read's end
@@ -281,11 +301,12 @@ struct TileWavefront {
     // border: serial, the warp's column buffer of `rows` rows.
     // UNI: one gap quality at all positions of all the warp's reads
     template <bool UNI>
-    __device__ __forceinline__ static void loop(const Reads& rd, const uint32_t* hw, int H, int K, Word* tab,
+    __device__ __forceinline__ static void loop(const Reads& rd, const Hap& hap, int H, int K, Word* tab,
                                                 RingRow* ring, RingRow* border, int64_t rows, int t, int warp,
-                                                int lane, Sum& sum) {
+                                                int parts, int lane, Sum& sum) {
+        const int NL = G * parts;      // lanes of the group
         const int u = warp * 32 + t;   // lane of the group
-        bool full[NS];
+        bool holds[SPAN - 1][NS];   // [j]: the lane holds at least R - j positions
         V wv[UNI ? 1 : R], xv[UNI ? 1 : R], N[R], D[R];
         {
             S w[NS][UNI ? 1 : R], x[NS][UNI ? 1 : R];
@@ -294,9 +315,17 @@ struct TileWavefront {
             int p0[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                const int m = rd.L[s] - NL * (R - 1);
-                full[s] = u < m;
-                p0[s] = u * (R - 1) + min_i(u, m);
+                int m, base;   // m lanes hold base + 1 positions, the others base
+                if constexpr (SPAN == 2) {
+                    base = R - 1;
+                    m = rd.L[s] - NL * base;
+                } else {
+                    base = rd.L[s] / NL;
+                    m = rd.L[s] - NL * base;
+                }
+#pragma unroll
+                for (int j = 0; j < SPAN - 1; ++j) holds[j][s] = base + (u < m ? 1 : 0) >= R - j;
+                p0[s] = u * base + min_i(u, m);
                 if constexpr (UNI) {
                     if constexpr (kDouble) {
                         const Gap g = gap(rd, s, 0);
@@ -380,7 +409,7 @@ struct TileWavefront {
                         uint32_t code = 0;
                         const int c = p0[s] + r;
                         if (r < R && c < rd.L[s]) {
-                            const uint32_t word = __ldg(rd.pack[s] + c);
+                            const uint32_t word = rd.read[s].word(c);
                             code = word & 0xffu;
                             const float p = rd.ph[(word >> 8) & 0x7fu];
                             const float pm = 1.0f - p;    // pairhmm_kernels.cuh:1244
@@ -438,15 +467,12 @@ struct TileWavefront {
         bool empty = !first;
         sum.e = 0;
         int h = 4;
-        // code words of this group's haplotype; behind its end the last word is re-read
-        // (those rows are past the result's last one)
-        const int wlast = ((H + 15) & ~15) / 4 - 1;
-        uint32_t wcur = __ldg(hw);
-        uint32_t wnext = __ldg(hw + 1);
+        uint32_t wcur = hap.codes(0);
+        uint32_t wnext = hap.codes(1);
         RingRow fetched{};   // serial: row 32*b + t of the block of 32 rows after the next
         const RingRow* left = ring;      // rows of the column before this part
         RingRow* right = border;         // rows of its last column, one per step
-        const bool writer = W > 1 && warp + 1 < W && t == 31;
+        const bool writer = kParts && warp + 1 < parts && t == 31;
         if constexpr (SERIAL) {
             __syncwarp();
             if (warp > 0) {
@@ -465,7 +491,7 @@ struct TileWavefront {
             __syncwarp();
         }
         auto four_steps = [&](int k0) {
-            const uint32_t wpref = __ldg(hw + min_i((k0 >> 2) + 2, wlast));
+            const uint32_t wpref = hap.codes((k0 >> 2) + 2);
             if constexpr (SERIAL) {
                 if (warp > 0 && (k0 & 31) == 0) {
                     __syncwarp();
@@ -514,7 +540,8 @@ struct TileWavefront {
                 // a position first forms what the next one takes from its old N, so that N is
                 // replaced in place (with the old N carried along instead, the compiler moves
                 // the lane's N by one register a step, on the FMA pipe)
-                V P = O::fma(Mul, wv[0], Xul), I = O::fma(Iul, eps, Mul), X = zero, Ip = zero, Xp = zero, Ilast = zero;
+                V P = O::fma(Mul, wv[0], Xul), I = O::fma(Iul, eps, Mul), X = zero, Ilast = zero;
+                V Ic[SPAN], Xc[SPAN];   // I and X after position R-1-j
 #pragma unroll
                 for (int q = 0; q < Q; ++q) {
                     const Word lw = row[q * 32];
@@ -522,10 +549,6 @@ struct TileWavefront {
                     for (int i = 0; i < VN; ++i) {
                         const int r = q * VN + i;
                         if (r < R) {
-                            if (r == R - 1) {
-                                Ip = Ilast;
-                                Xp = X;
-                            }
                             if constexpr (UNI) X = O::add(D[r], I);
                             else X = O::fma(D[r], xv[r], I);
                             D[r] = O::fma(D[r], eps, N[r]);
@@ -536,20 +559,28 @@ struct TileWavefront {
                                 I = O::fma(I, eps, N[r]);
                             }
                             N[r] = Nnew;
+                            if (r >= R - SPAN) {
+                                Ic[R - 1 - r] = Ilast;
+                                Xc[R - 1 - r] = X;
+                            }
                         }
                     }
                 }
-                V Id = Ilast, Xd = X;
-                Id = O::sel(full, Id, Ip);
-                Xd = O::sel(full, Xd, Xp);
+                V Id = Ic[SPAN - 1], Xd = Xc[SPAN - 1], Ne = N[R - SPAN];
+#pragma unroll
+                for (int j = SPAN - 2; j >= 0; --j) {
+                    Id = O::sel(holds[j], Ic[j], Id);
+                    Xd = O::sel(holds[j], Xc[j], Xd);
+                    Ne = O::sel(holds[j], N[R - 1 - j], Ne);
+                }
                 const V T = O::fma(Nl, wend, Id);
                 if constexpr (kDouble) {
                     if (k <= kres) sum.s[0] += T;
                 } else {
                     if (k <= kres) a4 = O::add(a4, T);
                 }
-                Nl = O::sel(full, N[R - 1], N[R - 2]);
-                if constexpr (W > 1) {
+                Nl = Ne;
+                if constexpr (kParts) {
                     // the last lane is at row k - 31; rows before the first land in the padding
                     // (serial) or in slots the next part has not reached yet.  serial: the row
                     // was fetched by this warp 64 steps ago or more
@@ -564,7 +595,7 @@ struct TileWavefront {
                     eMl = __shfl_up_sync(kFullMask, e, 1, G);
                     eIul = eMl;
                 }
-                if constexpr (W > 1) {
+                if constexpr (kParts) {
                     const RingRow b = left[(k + 1) & (kRing - 1)];  // broadcast
                     if (t == 0) {
                         Ml = b.n;
@@ -647,20 +678,20 @@ struct TileWavefront {
 
     // All parts of a warp's task.  threshold: below half of it on a part's last column
     // a serial pair stops (0: never).  Returns false if it stopped.
-    __device__ __forceinline__ static bool run(const Reads& rd, const uint32_t* hw, int H, int K, bool uni, Word* tab,
+    __device__ __forceinline__ static bool run(const Reads& rd, const Hap& hap, int H, int K, bool uni, Word* tab,
                                                RingRow* ring, RingRow* border, int64_t rows, int t, int warp, int lane,
-                                               double threshold, Sum& sum) {
+                                               double threshold, Sum& sum, int parts = W) {
         if constexpr (!SERIAL) {
-            if (uni) loop<true>(rd, hw, H, K, tab, ring, border, rows, t, warp, lane, sum);
-            else loop<false>(rd, hw, H, K, tab, ring, border, rows, t, warp, lane, sum);
+            if (uni) loop<true>(rd, hap, H, K, tab, ring, border, rows, t, warp, parts, lane, sum);
+            else loop<false>(rd, hap, H, K, tab, ring, border, rows, t, warp, parts, lane, sum);
         } else {
-            for (int part = 0; part < W; ++part) {
-                if (uni) loop<true>(rd, hw, H, K, tab, ring, border, rows, t, part, lane, sum);
-                else loop<false>(rd, hw, H, K, tab, ring, border, rows, t, part, lane, sum);
+            for (int part = 0; part < parts; ++part) {
+                if (uni) loop<true>(rd, hap, H, K, tab, ring, border, rows, t, part, parts, lane, sum);
+                else loop<false>(rd, hap, H, K, tab, ring, border, rows, t, part, parts, lane, sum);
                 __syncwarp();   // the part's rows are written
-                if (threshold > 0.0 && part + 1 < W) {
+                if (SPAN == 2 && threshold > 0.0 && part + 1 < parts) {
                     // M = N/n, I + D one row up = X on the part's last column
-                    const int c = (part + 1) * 32 * (R - 1) + min_i((part + 1) * 32, rd.L[0] - NL * (R - 1));
+                    const int c = (part + 1) * 32 * (R - 1) + min_i((part + 1) * 32, rd.L[0] - G * parts * (R - 1));
                     const double inv_n = 1.0 / (double)gap(rd, 0, c).d;
                     double mass = 0.0;
                     for (int j = t; j <= H; j += 32) mass += (double)border[kBorderPad + j].n * inv_n + (double)border[kBorderPad + j].x;

@@ -132,3 +132,47 @@ def test_fp64_tiles_match_oracle(gaps, gcp):
     assert want.min() < -650 and st.rescued > 0.9 * (want < -70).sum() and st.rescued_ext > 0
     assert_log10_close(few, want, what="FP64 tiles")
     np.testing.assert_array_equal(few, many)
+
+
+@pytest.mark.parametrize("gaps", ["one", "each", "high"])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_flat_list_shapes_match_oracle(gaps, shuffled):
+    """The allocation-free entry point at the edges of its shapes (8, 16 and 32 lanes,
+    one to five parts; the general form for the shortest reads and for gap qualities
+    beyond its exact tiles' range), in list order and with every warp's pairs mixed;
+    twice, since a call leaves its queue empty for the next."""
+    import torch
+    rng = np.random.default_rng(8)
+    b = _Builder()
+    for L in (1, 2, 8, 9, 16, 17, 152, 153, 160, 161, 176, 177, 320, 321, 352, 640, 641, 704, 1280, 1281, 1344, 1921,
+              2600):
+        H = np.array([L + 30, L + 1, max(1, L - 3), L + 200])
+        base = ACGT[rng.integers(0, 4, size=int(H.max()))]
+        reads = [base[:L].copy() for _ in range(3)]
+        for r in reads:
+            m = rng.random(L) < 0.003
+            r[m] = ACGT[rng.integers(0, 4, size=int(m.sum()))]
+        n = 3 * L
+        q = {"one": np.full(n, 40), "each": rng.integers(20, 46, size=n), "high": rng.integers(55, 94, size=n)}[gaps]
+        b.add_concat(np.full(3, L), np.concatenate(reads), rng.integers(20, 41, size=n).astype(np.uint8),
+                     q.astype(np.uint8), q.astype(np.uint8), H, np.concatenate([base[:h] for h in H]))
+    batch = b.build()
+    want = oracle.batch_log10(batch)
+    pairs, r0, h0 = [], 0, 0
+    for nr, nh in zip(batch.reads_per_record, batch.haps_per_record):
+        pairs += [(batch.read_offsets[i], batch.hap_offsets[j], batch.read_lengths[i], batch.hap_lengths[j])
+                  for i in range(r0, r0 + nr) for j in range(h0, h0 + nh)]
+        r0, h0 = r0 + nr, h0 + nh
+    order = rng.permutation(len(pairs)) if shuffled else np.arange(len(pairs))
+    pairs = np.array(pairs, dtype=g.PAIR_DTYPE)[order]
+    dev = torch.device("cuda:0")
+    d = [torch.from_numpy(np.ascontiguousarray(getattr(batch, k))).to(dev)
+         for k in ("read_bases", "base_quals", "ins_quals", "del_quals", "hap_bases")]
+    dpairs = torch.from_numpy(pairs.view(np.uint8)).to(dev)
+    ok = want[order] > -60.0
+    assert ok.mean() > 0.9
+    for _ in range(2):
+        scores = torch.full((len(pairs),), 7.0, dtype=torch.float32, device=dev)
+        g.forward_pairs_noalloc(0, *d, dpairs, len(pairs), int(batch.hap_lengths.max()), scores)
+        torch.cuda.synchronize(dev)
+        assert_log10_close(scores.cpu().numpy()[ok], want[order][ok], what=f"flat list, {gaps}")
