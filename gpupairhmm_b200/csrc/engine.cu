@@ -1392,7 +1392,9 @@ pairhmm_status_t Engine::compute_device(const pairhmm_batch_t& b, int32_t, int32
     if ((st = upload_index(x, s)) != PAIRHMM_OK) return st;
     PHMM_CUDA(cudaEventRecord(ev0_, s));
     if ((st = run_pipeline(b, x, scores, s)) != PAIRHMM_OK) return st;
-    PHMM_CUDA(cudaStreamWaitEvent(stream, ev1_, 0));
+    // an ordinary record behind the graph: the marks are recorded by the graph's nodes
+    PHMM_CUDA(cudaEventRecord(fork_, s));
+    PHMM_CUDA(cudaStreamWaitEvent(stream, fork_, 0));
     stats_.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     stats_.device_ms = -1.0;
     return PAIRHMM_OK;

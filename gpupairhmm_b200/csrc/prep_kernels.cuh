@@ -80,7 +80,7 @@ __device__ __forceinline__ uint32_t pack_position(uint32_t base, uint32_t bq, ui
 // Also notes per read what the exact-tile kernels ask of all its positions.  Forming
 // their coefficients here too, 16 bytes a position, was measured: 2.3 times the
 // stage's time (0.11 -> 0.25 ms for 2,000 uneven regions) for 1% of the FP32 stage's.
-__device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int64_t nblocks) {
+__device__ __forceinline__ void pack_reads(const PrepArgs& a, const float* ph, int64_t block, int64_t nblocks) {
     const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (nblocks * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -107,7 +107,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
             if (a.gcp_quals) {
                 const uint32_t g = min((uint32_t)a.gcp_quals[src], 127u);
                 key |= g << 8;
-                beta = (float)(1.0 - (double)a.ph2pr[g]);  // gpuworker.cuh:1049
+                beta = (float)(1.0 - (double)ph[g]);  // gpuworker.cuh:1049
                 if (!(beta >= kMinAlpha)) flags = 1u;      // gcp quality 0: nothing to rescale by
             }
         }
@@ -130,7 +130,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
             }
             dst[c >> 2] = make_uint4(w[0], w[1], w[2], w[3]);
             {
-                float d = a.ph2pr[(w[0] >> 16) & 0x7fu], sg = a.ph2pr[(w[0] >> 24) & 0x7fu];
+                float d = ph[(w[0] >> 16) & 0x7fu], sg = ph[(w[0] >> 24) & 0x7fu];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (c + j >= L) break;
@@ -139,12 +139,12 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, int64_t block, int
                     if (c + j + 1 < L) {
                         const uint32_t in = j < 3 ? (w[j < 3 ? j + 1 : 3] >> 16) & 0x7fu : min((uint32_t)iq[c + 4], 127u);
                         const uint32_t sd = j < 3 ? (w[j < 3 ? j + 1 : 3] >> 24) & 0x7fu : min((uint32_t)dq[c + 4], 127u);
-                        dn = a.ph2pr[in];
-                        sn = a.ph2pr[sd];
+                        dn = ph[in];
+                        sn = ph[sd];
                     }
                     const TileLink k = tile_link(c + j + 1 < L ? 1.0f - (dn + sn) : beta, dn, beta, inv_beta);
                     range = fmaxf(range, k.id + 2.0f * (1.0f + sg * k.id));
-                    bias += tile_emission_error(1.0f - a.ph2pr[(w[j] >> 8) & 0x7fu], k);
+                    bias += tile_emission_error(1.0f - ph[(w[j] >> 8) & 0x7fu], k);
                     if (!(fabsf(1.0f - (d + sg)) >= kMinAlpha)) flags |= 1u;
                     d = dn;
                     sg = sn;
@@ -210,6 +210,7 @@ __device__ __forceinline__ void pack_haps(const PrepArgs& a, int64_t block, int6
 
 __global__ void __launch_bounds__(256)
 pack_kernel(PrepArgs a, FillArgs f, int fill_blocks, int read_blocks) {
+    __shared__ float ph[128];
     const int b = blockIdx.x;
     if (b < fill_blocks) {
         for (int k = 0; k < kFillRanges; ++k)
@@ -217,7 +218,9 @@ pack_kernel(PrepArgs a, FillArgs f, int fill_blocks, int read_blocks) {
                  i += (long long)fill_blocks * blockDim.x)
                 f.ptr[k][i] = f.value[k];
     } else if (b < fill_blocks + read_blocks) {
-        pack_reads(a, b - fill_blocks, read_blocks);
+        if (threadIdx.x < 128) ph[threadIdx.x] = a.ph2pr[threadIdx.x];
+        __syncthreads();
+        pack_reads(a, ph, b - fill_blocks, read_blocks);
     } else {
         pack_haps(a, b - fill_blocks - read_blocks, gridDim.x - fill_blocks - read_blocks);
     }

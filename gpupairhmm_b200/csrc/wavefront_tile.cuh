@@ -10,8 +10,8 @@
 // 6.5 cycles, and ran at 0.60-0.63 of the pipe, scalar or packed.  So the
 // recurrence is scaled here for few register operands, not few instructions:
 //   I unscaled (true I times the pair's scale), eps an immediate
-//   N = n_c*M with n_c = beta*delta_{c+1}/beta, so that what N feeds into the next
-//       column's I has weight 1
+//   N = n_c*M with n_c = delta_{c+1}, so that what N feeds into the next column's I
+//       has weight 1 (in FP32 the n that the rounded w below stands for)
 //   D^ = D/d_c with d_c = sigma_c/n_c, so that what N feeds into D has weight 1
 //     P(j,c)  = w_c*N(j-1,c-1) + X(j,c-1)      w_c = alpha_c/(beta*delta_c)
 //     N(j,c)  = l_c(h_j)*P(j,c)                l_c = beta*n_c*lambda
@@ -191,7 +191,7 @@ __device__ __forceinline__ float tile_emission(float pm, const TileLink& next) {
 // log10 on average); their sum is taken off the score.
 __device__ __forceinline__ float tile_emission_error(float pm, const TileLink& next) {
     const float l = tile_emission(pm, next);
-    return l != 0.0f ? -(fmaf(pm, next.g, -l) + pm * next.e) / l : 0.0f;
+    return l != 0.0f ? -__fdividef(fmaf(pm, next.g, -l) + pm * next.e, l) : 0.0f;
 }
 
 // What the preparation notes per read.
@@ -205,9 +205,6 @@ struct ReadMeta {
 static_assert(sizeof(ReadMeta) == 16, "ReadMeta is one 16-byte word");
 constexpr uint32_t kNoKey = 0xffffffffu;
 
-// EXT (FP64): a lane keeps its values as true * 2^e with its own exponent e, for
-// pairs whose values span more than a double's range; see wavefront_fp64.cuh, whose
-// extended tier works the same way.
 // Where a group's read positions and haplotype codes come from: the batch's packed
 // layout.  word(c): a position as read_pack holds it; codes(i): the codes of rows
 // 4i .. 4i+3, behind the haplotype's end any codes (those rows are past the result's).
@@ -222,6 +219,9 @@ struct PackedHap {
     __device__ __forceinline__ uint32_t codes(int i) const { return __ldg(p + min_i(i, last)); }
 };
 
+// EXT (FP64): a lane keeps its values as true * 2^e with its own exponent e, for
+// pairs whose values span more than a double's range; see wavefront_fp64.cuh, whose
+// extended tier works the same way.
 // SERIAL with W = 0: the number of parts is given at run time.
 // SPAN: lanes hold R .. R-SPAN+1 positions, so that one kernel takes reads of
 // (NL*(R-SPAN+1), NL*R] positions, at a select more per step and value for each.
