@@ -40,6 +40,10 @@ constexpr int kCtrTotal = kMaxBuckets + 4 * kMaxFp64Classes;
 // rounds of resident warps, so the order decides little and the three launches of the
 // sort are a third of the stage of a small batch
 constexpr int64_t kNoSortPairs = 4096;
+// Batches of more pairs than this, or whose launches have not been the same for a while,
+// are launched kernel by kernel (see run_pipeline).
+constexpr int64_t kGraphMaxPairs = 4096;
+constexpr int64_t kGraphAfter = 8;
 // multi-tile FP64 pairs up to which the two tiers run fused (about one round of
 // resident warps of that class's kernel on 148 SMs)
 constexpr int64_t kFuseMaxPairs = 2048;
@@ -365,6 +369,8 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
     if (wrong) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, wrong);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     graph_exec_ = nullptr;
+    last_shape_.clear();
+    shape_repeats_ = 0;
     if (ready_) return build_tables(rules);
     tables_[0].rules = rules;
     return PAIRHMM_OK;
@@ -1059,6 +1065,16 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
     return p;
 }
 
+// What decides a batch's launches and their dependencies (not their arguments).
+std::vector<uint8_t> Engine::launch_shape(const BatchIndex& x, const Plan& plan) const {
+    std::vector<uint8_t> shape = {(uint8_t)(table_ == &tables_[1]), (uint8_t)(x.num_pairs > kNoSortPairs),
+                                  (uint8_t)plan.side[1], (uint8_t)plan.side[2]};
+    for (const int64_t n : x.bucket_items) shape.push_back(n != 0);
+    for (const int64_t n : x.class_pairs) shape.push_back(n != 0);
+    shape.push_back(x.class_pairs[fp64_->classes.size() - 1] <= kFuseMaxPairs);
+    return shape;
+}
+
 pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchIndex& x, float* d_scores,
                                       cudaStream_t s) {
     if (x.num_pairs == 0) return PAIRHMM_OK;
@@ -1068,7 +1084,20 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     const pairhmm_status_t side = ensure_side_streams(std::max(plan.side[1], plan.side[2]));
     if (side != PAIRHMM_OK) return side;
     const cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
-    if (!opts_.use_graphs) {
+    // A graph only for small batches that launch the same kernels as the kept graph, or as
+    // the eight batches before: instantiating one costs more than its 7-37 launches, and
+    // mixed small batches rarely have the same length classes.  Measured per call, graph /
+    // launches, changing batches of uneven regions: 4 regions 0.65 / 0.30 ms, 24 regions
+    // 1.57 / 0.67, 80 regions 1.38 / 1.29; the same batch again with a kept graph: 1 region
+    // 0.186 / 0.192, 4 regions 0.256 / 0.268, 12 regions 0.585 / 0.564, 300 regions 3.67 / 3.51.
+    bool use_graph = false;
+    if (opts_.use_graphs && x.num_pairs <= kGraphMaxPairs) {
+        std::vector<uint8_t> shape = launch_shape(x, plan);
+        shape_repeats_ = shape == last_shape_ ? shape_repeats_ + 1 : 0;
+        use_graph = shape_repeats_ >= kGraphAfter || (graph_exec_ && shape == graph_shape_);
+        last_shape_ = std::move(shape);
+    }
+    if (!use_graph) {
         for (int stage = 0; stage < 3; ++stage) {
             const pairhmm_status_t st = enqueue_pipeline(in, x, plan, d_scores, s, stage);
             if (st != PAIRHMM_OK) return st;
@@ -1106,6 +1135,7 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     }
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaGraphInstantiate");
+    graph_shape_ = last_shape_;
     PHMM_CUDA(cudaGraphLaunch(graph_exec_, s));
     return PAIRHMM_OK;
 }

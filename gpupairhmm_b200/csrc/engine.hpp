@@ -153,6 +153,7 @@ private:
         size_t scratch_bytes = 0;
     };
     Plan make_plan(const BatchIndex& idx);
+    std::vector<uint8_t> launch_shape(const BatchIndex& x, const Plan& plan) const;
     // stage 0: packing + work list, 1: FP32 launches, 2: FP64 pass
     pairhmm_status_t enqueue_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, const Plan& plan,
                                       float* d_scores, cudaStream_t s, int stage);
@@ -190,6 +191,8 @@ private:
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
     int64_t launches_ = 0, fp32_launches_ = 0;
     cudaGraphExec_t graph_exec_ = nullptr;   // the whole batch: prep, FP32, FP64
+    std::vector<uint8_t> graph_shape_, last_shape_;  // launch_shape of the kept graph and of the last batch
+    int64_t shape_repeats_ = 0;               // batches before the last one with its shape, in a row
     pairhmm_stats_t stats_{};
     std::string last_error_;
 
