@@ -13,9 +13,10 @@
 // takes a few consecutive pairs of the list at a time and runs those of one shape
 // together on the exact tiles of wavefront_tile.cuh: 8 lanes a pair up to 160
 // positions, 16 up to 320, then 32 lanes with the read's parts in turn.  Few pairs
-// (reads of at most 8 positions, gap probabilities too small for that kernel's
-// range) take a general form: the whole warp, 16 positions a lane, read tiles of
-// 512.  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
+// take a general form, the whole warp, 16 positions a lane, read tiles of 512: reads of
+// at most 8 positions, gap probabilities too small for the tiles' range, and, once
+// more, pairs whose sum on the tiles is too small for it (there is no FP64 pass behind
+// this entry point, and the general form's range reaches further down).  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
 // the general form for all (one pair on 512 positions a warp, eleven operations a
 // cell); what bounds it is the instruction cache (several shapes in flight) and the
 // last pairs of a short list.
@@ -115,11 +116,13 @@ constexpr int kTableBytes = 5 * (kMaxR / 4) * 32 * 16;   // per warp
 constexpr int kRingBytes = 64 * 16;
 constexpr size_t kSmem = (kThreads / 32) * (size_t)(kTableBytes + kRingBytes);
 
-// Pairs `mine` (by lane: the group's pair, or -1) of one shape.  The general form
-// takes what this refuses: returns false (warp-uniform) where some pair's gap
-// probabilities lie too far below 1.
+// Pairs `mine` (by lane: the group's pair, or -1) of one shape.  Returns (warp-uniform)
+// the lanes whose pair the general form computes instead: no score is written for it.
+// These are pairs whose sum lies so low that the tiles' rounding in the denormal range,
+// which sets in earlier than the general form's (N lies 1/delta below M), could be more
+// than 2^-23 of it; and all of them where some pair's gap probabilities lie too far below 1.
 template <int G, int R>
-__device__ __noinline__ bool run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
+__device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
     using T = TileWavefront<float, G, R, G == 32 ? 0 : 1, false, false, G == 32, ByteRead, ByteHap, span_of(R)>;
     const int lane = threadIdx.x & 31;
     const int t = lane % G;
@@ -137,18 +140,23 @@ __device__ __noinline__ bool run_tile(const Args& a, const float* ph, char* smem
     // what the engine's preparation notes per read
     const uint32_t w0 = rd.read[0].word(0);
     bool same = true;
-    float bias = 0.0f, least = 1.0f;
+    float bias = 0.0f, least = 1.0f, range = 0.0f;
     for (int c = t; c < L; c += G) {
         const uint32_t w = rd.read[0].word(c);
         same = same && (w >> 16) == ((w0 >> 16) & 0xffu) * 0x101u;
         least = fminf(least, ph[(w >> 16) & 0xffu]);
-        bias += tile_emission_error(1.0f - ph[(w >> 8) & 0xffu], T::link(rd, 0, c + 1));
+        const TileLink k = T::link(rd, 0, c + 1);
+        range = fmaxf(range, tile_range(k, ph[(w >> 24) & 0xffu]));
+        bias += tile_emission_error(1.0f - ph[(w >> 8) & 0xffu], k);
     }
 #pragma unroll
-    for (int d = G / 2; d >= 1; d >>= 1) bias += __shfl_xor_sync(kFullMask, bias, d);
-    // N lies 1/delta below M; D enters 2H/beta above the general form's boundary value.
-    // Up to 2^8 of the low end of the range is given up here
-    if (__any_sync(kFullMask, least * (256.0f * 2.0f / kBeta) * (float)H < 1.0f)) return false;
+    for (int d = G / 2; d >= 1; d >>= 1) {
+        bias += __shfl_xor_sync(kFullMask, bias, d);
+        range = fmaxf(range, __shfl_xor_sync(kFullMask, range, d));
+    }
+    const bool result = mine >= 0 && t == G - 1;
+    if (__any_sync(kFullMask, least * (256.0f * 2.0f / kBeta) * (float)H < 1.0f))
+        return __ballot_sync(kFullMask, result);
     const unsigned key = (w0 >> 16) & 0xffu;
     const bool uni = __all_sync(kFullMask, same) &&
                      __reduce_min_sync(kFullMask, key) == __reduce_max_sync(kFullMask, key);
@@ -162,11 +170,11 @@ __device__ __noinline__ bool run_tile(const Args& a, const float* ph, char* smem
     const ByteHap hap{a.hap_bases + pr.hap_offset, H};
     T::run(rd, hap, H, K, uni, tab, ring, reinterpret_cast<typename T::RingRow*>(wscr), a.rows, t, 0, lane, 0.0, sum,
            parts);
-    if (mine >= 0 && t == G - 1)
+    const bool kept = sum.s[0] >= (double)tile_rounding(L, H, range) && sum.s[0] <= (double)FLT_MAX;
+    if (result && kept)
         a.scores[mine] = (float)(log10(sum.s[0] / (double)H) - log10((double)kTileD0) -
                                  (double)(bias * 0.43429448f));
-    __syncwarp();
-    return true;
+    return __ballot_sync(kFullMask, result && !kept);
 }
 
 // The general form: one pair on the warp, read tiles of kT positions, beta absorbed
@@ -295,7 +303,7 @@ __device__ __forceinline__ int shape_of(int L) {
 }
 
 template <int G, int R0, int R1>   // R0, R0 + kStepR, .. R1
-__device__ __forceinline__ bool run_shape(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int R,
+__device__ __forceinline__ unsigned run_shape(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int R,
                                           int parts) {
     if constexpr (R0 < R1) {
         if (R != R0) return run_shape<G, R0 + kStepR, R1>(a, ph, smem, wscr, mine, R, parts);
@@ -349,12 +357,12 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
             }
             left &= ~taken;
             const int parts = G == 32 ? (__shfl_sync(kFullMask, L, lead) + 32 * kMaxR - 1) / (32 * kMaxR) : 1;
-            bool done = false;
-            if (G == 8) done = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 16) done = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 32) done = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
-            if (!done)
-                for (unsigned m = taken; m; m &= m - 1) run_general(a, ph, wscr, p0 + __ffs(m) - 1);
+            unsigned general = 1u;   // lanes whose `mine` the general form computes
+            if (G == 8) general = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 16) general = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 32) general = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
+            for (; general; general &= general - 1)
+                run_general(a, ph, wscr, __shfl_sync(kFullMask, mine, __ffs(general) - 1));
             __syncwarp();
         }
     }

@@ -143,7 +143,7 @@ __device__ __forceinline__ void pack_reads(const PrepArgs& a, const float* ph, i
                         sn = ph[sd];
                     }
                     const TileLink k = tile_link(c + j + 1 < L ? 1.0f - (dn + sn) : beta, dn, beta, inv_beta);
-                    range = fmaxf(range, k.id + 2.0f * (1.0f + sg * k.id));
+                    range = fmaxf(range, tile_range(k, sg));
                     bias += tile_emission_error(1.0f - ph[(w[j] >> 8) & 0x7fu], k);
                     if (!(fabsf(1.0f - (d + sg)) >= kMinAlpha)) flags |= 1u;
                     d = dn;

@@ -143,15 +143,20 @@ constexpr float kTileD0 = FLT_MAX / 8.0f;
 constexpr int kScaledExp = 836;
 constexpr double kScaled = 0x1p836;
 
-// Smallest sum of T the FP32 pass keeps.  N, I and D^ each round by at most 2^-150
-// in the denormal range; as terms of T they weigh at most 1/n, 1 and d, range being
-// the read's largest 1/n + 2*(1 + d), and every path reaches the last position at
-// most once, so S >= L*H*2^-127*range keeps the error below 2^-23 of S.  The second
-// term is rescue_threshold in this scale (the sum there is beta*T over
-// (FLT_MAX/16)/H): no pair that wavefront_fp32.cuh would pass on is kept here.
+// Smallest sum of T that rounding in the denormal range leaves good to 2^-23: N, I and
+// D^ each round by at most 2^-150 there; as terms of T they weigh at most 1/n, 1 and d,
+// range being the read's largest 1/n + 2*(1 + d) (tile_range of its positions), and every
+// path reaches the last position at most once.
+__device__ __forceinline__ float tile_rounding(int L, int H, float range) {
+    return (float)L * (float)H * 0x1p-127f * range;
+}
+
+// Smallest sum of T the FP32 pass keeps.  The second term is rescue_threshold in this
+// scale (the sum there is beta*T over (FLT_MAX/16)/H): no pair that wavefront_fp32.cuh
+// would pass on is kept here.
 __device__ __forceinline__ float tile_threshold(int L, int H, float range) {
     const float cells = (float)L * (float)H * 0x1p-127f;
-    return fmaxf(cells * range, 3.0f * cells * (float)H * (2.0f / kBeta));
+    return fmaxf(tile_rounding(L, H, range), 3.0f * cells * (float)H * (2.0f / kBeta));
 }
 
 // Smallest sum the FP64 pass's scaled tier keeps: the same terms each round by at most
@@ -180,6 +185,12 @@ __device__ __forceinline__ TileLink tile_link(float a, float d, float beta, floa
         k.e = fmaf(-k.g, k.w, a) * rw;
     }
     return k;
+}
+
+// A position's share of a read's range: k the boundary behind it, sg its deletion
+// gap-open probability.
+__device__ __forceinline__ float tile_range(const TileLink& k, float sg) {
+    return k.id + 2.0f * (1.0f + sg * k.id);
 }
 
 // l of a match (pm = 1 - p) or mismatch (pm = p/3), rounded once.
