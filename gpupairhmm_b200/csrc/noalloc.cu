@@ -13,10 +13,10 @@
 // takes a few consecutive pairs of the list at a time and runs those of one shape
 // together on the exact tiles of wavefront_tile.cuh: 8 lanes a pair up to 160
 // positions, 16 up to 320, then 32 lanes with the read's parts in turn.  Few pairs
-// take a general form, the whole warp, 16 positions a lane, read tiles of 512: reads of
-// at most 8 positions, gap probabilities too small for the tiles' range, and, once
-// more, pairs whose sum on the tiles is too small for it (there is no FP64 pass behind
-// this entry point, and the general form's range reaches further down).  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
+// take a general form, the whole warp, 4 to 16 positions a lane by the read's length,
+// longer reads in tiles of 512: reads of at most 8 positions, and, once more, pairs whose sum on the tiles is too small for
+// their range (there is no FP64 pass behind this entry point, and the general form's
+// range reaches further down).  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
 // the general form for all (one pair on 512 positions a warp, eleven operations a
 // cell); what bounds it is the instruction cache (several shapes in flight) and the
 // last pairs of a short list.
@@ -46,9 +46,6 @@
 namespace phmm {
 namespace noalloc {
 
-constexpr int kG = 32;
-constexpr int kR = 16;
-constexpr int kT = kG * kR;
 constexpr int kMaxHapLength = 16384;
 constexpr size_t kScratchBytes = size_t(64) << 20;  // 64 MiB
 constexpr int kThreads = 64;                        // 2 warps per block
@@ -120,7 +117,8 @@ constexpr size_t kSmem = (kThreads / 32) * (size_t)(kTableBytes + kRingBytes);
 // the lanes whose pair the general form computes instead: no score is written for it.
 // These are pairs whose sum lies so low that the tiles' rounding in the denormal range,
 // which sets in earlier than the general form's (N lies 1/delta below M), could be more
-// than 2^-23 of it; and all of them where some pair's gap probabilities lie too far below 1.
+// than 2^-23 of it.  That is the pair's own sum, so its form, and with it its score,
+// depends on no other pair of the list.
 template <int G, int R>
 __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
     using T = TileWavefront<float, G, R, G == 32 ? 0 : 1, false, false, G == 32, ByteRead, ByteHap, span_of(R)>;
@@ -140,11 +138,10 @@ __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* 
     // what the engine's preparation notes per read
     const uint32_t w0 = rd.read[0].word(0);
     bool same = true;
-    float bias = 0.0f, least = 1.0f, range = 0.0f;
+    float bias = 0.0f, range = 0.0f;
     for (int c = t; c < L; c += G) {
         const uint32_t w = rd.read[0].word(c);
         same = same && (w >> 16) == ((w0 >> 16) & 0xffu) * 0x101u;
-        least = fminf(least, ph[(w >> 16) & 0xffu]);
         const TileLink k = T::link(rd, 0, c + 1);
         range = fmaxf(range, tile_range(k, ph[(w >> 24) & 0xffu]));
         bias += tile_emission_error(1.0f - ph[(w >> 8) & 0xffu], k);
@@ -154,9 +151,6 @@ __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* 
         bias += __shfl_xor_sync(kFullMask, bias, d);
         range = fmaxf(range, __shfl_xor_sync(kFullMask, range, d));
     }
-    const bool result = mine >= 0 && t == G - 1;
-    if (__any_sync(kFullMask, least * (256.0f * 2.0f / kBeta) * (float)H < 1.0f))
-        return __ballot_sync(kFullMask, result);
     const unsigned key = (w0 >> 16) & 0xffu;
     const bool uni = __all_sync(kFullMask, same) &&
                      __reduce_min_sync(kFullMask, key) == __reduce_max_sync(kFullMask, key);
@@ -170,6 +164,7 @@ __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* 
     const ByteHap hap{a.hap_bases + pr.hap_offset, H};
     T::run(rd, hap, H, K, uni, tab, ring, reinterpret_cast<typename T::RingRow*>(wscr), a.rows, t, 0, lane, 0.0, sum,
            parts);
+    const bool result = mine >= 0 && t == G - 1;
     const bool kept = sum.s[0] >= (double)tile_rounding(L, H, range) && sum.s[0] <= (double)FLT_MAX;
     if (result && kept)
         a.scores[mine] = (float)(log10(sum.s[0] / (double)H) - log10((double)kTileD0) -
@@ -177,12 +172,14 @@ __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* 
     return __ballot_sync(kFullMask, result && !kept);
 }
 
-// The general form: one pair on the warp, read tiles of kT positions, beta absorbed
-// into I and D (M keeps alpha, so no division and no degenerate-alpha case):
+// The general form: one pair on the warp, R positions a lane, read tiles of 32 * R, beta
+// absorbed into I and D (M keeps alpha, so no division and no degenerate-alpha case):
 //   M(j,c)  = lambda*(alpha_c*M(j-1,c-1) + It(j-1,c-1) + Dt(j-1,c-1))
 //   It(j,c) = eps_c*It(j,c-1) + beta*delta_c*M(j,c-1)
 //   Dt(j,c) = beta*sigma_c*M(j-1,c) + eps*Dt(j-1,c)
+template <int R>
 __device__ __noinline__ void run_general(const Args& a, const float* ph, float4* wscr, int64_t pi) {
+    constexpr int T = 32 * R;
     const int t = threadIdx.x & 31;
     const int64_t rows = a.rows;
     float* const scores = a.scores;
@@ -194,17 +191,17 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
         const uint8_t* iq = a.ins_quals + pr.read_offset;
         const uint8_t* dq = a.del_quals + pr.read_offset;
         const uint8_t* hb = a.hap_bases + pr.hap_offset;
-        const int ntiles = (L + kT - 1) / kT;
+        const int ntiles = (L + T - 1) / T;
         const float Dbound = kBeta * (kScale / (float)H);
         double acc = 0.0;  // summed in double: up to 16384 rows of similar size
         int rlane = -1;
         for (int tile = 0; tile < ntiles; ++tile) {
             const bool last = tile == ntiles - 1;
-            const int p0 = tile * kT + t * kR;
-            float lm[kR], lx[kR], alpha[kR], dlt[kR], sig[kR], eps[kR], M[kR], D[kR];
-            uint32_t xc[kR];
+            const int p0 = tile * T + t * R;
+            float lm[R], lx[R], alpha[R], dlt[R], sig[R], eps[R], M[R], D[R];
+            uint32_t xc[R];
 #pragma unroll
-            for (int r = 0; r < kR; ++r) {
+            for (int r = 0; r < R; ++r) {
                 const int c = p0 + r;
                 const bool in = c < L;
                 const float p = in ? ph_of(ph, bq[c]) : 1.0f;
@@ -222,17 +219,17 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
             }
             int t_res = 0, r_res = 0;
             if (last) {
-                const int rel = L - 1 - tile * kT;
-                t_res = rel / kR;
-                r_res = rel - t_res * kR;
+                const int rel = L - 1 - tile * T;
+                t_res = rel / R;
+                r_res = rel - t_res * R;
             }
-            const int kg = last ? H + t_res : H + kG - 1;
+            const int kg = last ? H + t_res : H + 32 - 1;
             const bool res_lane = last && t == t_res;
-            const bool addM = r_res == kR - 1;
+            const bool addM = r_res == R - 1;
             if (res_lane) rlane = t;
             float4* ein = wscr + ((tile - 1) & 1) * rows;
             float4* eout = wscr + (tile & 1) * rows;
-            const bool writer = !last && t == kG - 1;
+            const bool writer = !last && t == 32 - 1;
             float Ml = 0.f, Dl = 0.f, Mul = 0.f, Dul = 0.f, Iul = 0.f;
             if (t == 0 && tile == 0) { Dl = Dbound; Dul = Dbound; }
             uint32_t h = 4u;
@@ -242,7 +239,7 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
                 h = hn;
                 float Mdiag = Mul, Idiag = Iul, Xdiag = Iul + Dul;
 #pragma unroll
-                for (int r = 0; r < kR; ++r) {
+                for (int r = 0; r < R; ++r) {
                     const float lam = (xc[r] == 4u || h == 4u || xc[r] == h) ? lm[r] : lx[r];
                     const float Mold = M[r];
                     const float Dold = D[r];
@@ -255,18 +252,18 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
                 }
                 if (res_lane) {
                     float a = Idiag;
-                    if (addM && k < kg) a = fmaf(kBeta, M[kR - 1], a);
+                    if (addM && k < kg) a = fmaf(kBeta, M[R - 1], a);
                     acc += (double)a;
                 }
                 if (writer) {
-                    const int j = k - (kG - 1);
-                    if (j >= 0 && j < H) *reinterpret_cast<float2*>(eout + j) = make_float2(M[kR - 1], D[kR - 1]);
+                    const int j = k - (32 - 1);
+                    if (j >= 0 && j < H) *reinterpret_cast<float2*>(eout + j) = make_float2(M[R - 1], D[R - 1]);
                     if (j >= 1 && j - 1 < H) reinterpret_cast<float*>(eout + (j - 1))[2] = Idiag;
                 }
                 Mul = Ml;
                 Dul = Dl;
-                Ml = __shfl_up_sync(kFullMask, M[kR - 1], 1);
-                Dl = __shfl_up_sync(kFullMask, D[kR - 1], 1);
+                Ml = __shfl_up_sync(kFullMask, M[R - 1], 1);
+                Dl = __shfl_up_sync(kFullMask, D[R - 1], 1);
                 Iul = __shfl_up_sync(kFullMask, Idiag, 1);
                 if (t == 0) {
                     if (tile > 0) {
@@ -292,6 +289,18 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
         }
         if (t == rlane) scores[pi] = (float)(log10(acc) - (log10((double)kScale) + log10((double)kBeta)));
     }
+}
+
+// Positions a lane by read length: with 16 for every read (tiles of 512), a list of 46,336
+// pairs of 70-250 positions that all score too low for the tiles took 7.8 ms, with the
+// lengths' own 4-8 it takes 5.2 ms (5.0 ms with one form of 16 for every list).
+__device__ __forceinline__ void general(const Args& a, const float* ph, float4* wscr, int64_t pi) {
+    const int L = a.pairs[pi].read_length;   // warp-uniform
+    if (L <= 128) run_general<4>(a, ph, wscr, pi);
+    else if (L <= 192) run_general<6>(a, ph, wscr, pi);
+    else if (L <= 256) run_general<8>(a, ph, wscr, pi);
+    else if (L <= 384) run_general<12>(a, ph, wscr, pi);
+    else run_general<16>(a, ph, wscr, pi);
 }
 
 // Shape of a pair's tile: 0 general, else lanes << 8 | positions a lane.
@@ -357,12 +366,11 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
             }
             left &= ~taken;
             const int parts = G == 32 ? (__shfl_sync(kFullMask, L, lead) + 32 * kMaxR - 1) / (32 * kMaxR) : 1;
-            unsigned general = 1u;   // lanes whose `mine` the general form computes
-            if (G == 8) general = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 16) general = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 32) general = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
-            for (; general; general &= general - 1)
-                run_general(a, ph, wscr, __shfl_sync(kFullMask, mine, __ffs(general) - 1));
+            unsigned redo = 1u;   // lanes whose `mine` the general form computes
+            if (G == 8) redo = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 16) redo = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 32) redo = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
+            for (; redo; redo &= redo - 1) general(a, ph, wscr, __shfl_sync(kFullMask, mine, __ffs(redo) - 1));
             __syncwarp();
         }
     }
@@ -432,7 +440,7 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
     if (status == PAIRHMM_OK && scratch != st.scratch.load()) st.scratch.store(scratch);
     if (status == PAIRHMM_OK) {
         // border rows per buffer for this call, and how many warps the scratch holds
-        const int64_t rows = ((int64_t)max_hap_length + 2 * kG + 8 + 63) / 64 * 64;
+        const int64_t rows = ((int64_t)max_hap_length + 2 * 32 + 8 + 63) / 64 * 64;
         const int64_t per_warp = 2 * rows * (int64_t)sizeof(float4);
         int64_t warps = (int64_t)(kScratchBytes / (size_t)per_warp);
         if (warps > st.max_warps) warps = st.max_warps;

@@ -76,3 +76,24 @@ def test_low_end_of_the_range_is_kept(gaps, plain_engine):
     assert np.isfinite(got[low]).all()
     rms = lambda x: float(np.sqrt(np.mean((x[low] - want[low]) ** 2)))
     assert rms(got) <= 3.0 * rms(plain), (rms(got), rms(plain))
+
+
+def test_score_does_not_depend_on_the_list():
+    """Pairs of the same shapes with ordinary and with very high gap qualities, scores from
+    near zero to below the range: in list order, many times over and shuffled (a warp then
+    takes several pairs at a time and mixes the two), and in short lists (one pair a warp
+    at a time), bitwise the same pair by pair."""
+    lengths = [30, 101, 103, 150, 152, 200, 250, 330, 650, 700]
+    from gpupairhmm_b200 import synth
+    batch = synth.concat([ladder(5, lengths, 40, haps=3), ladder(6, lengths, (80, 127), haps=3),
+                          ladder(7, lengths, (30, 93), haps=3)])
+    pairs = pair_list(batch)
+    call = flat_call(batch)
+    want = call(pairs)
+    assert np.isfinite(want).mean() > 0.3 and (want == -np.inf).any()
+    rng = np.random.default_rng(9)
+    many = np.tile(np.arange(len(pairs)), 50)   # 72,000 pairs: 8 at a time
+    for order in (many, rng.permutation(many), rng.permutation(many)):
+        np.testing.assert_array_equal(call(pairs[order]), want[order])
+    for part in np.array_split(rng.permutation(len(pairs))[:600], 40):
+        np.testing.assert_array_equal(call(pairs[part]), want[part])
