@@ -31,7 +31,8 @@
 // contents.  Nothing in it has to start at zero: within a pair each border row
 // is written by one tile before the next tile reads it.  Calls whose work
 // overlaps on the GPU (two streams, or two host threads) race on the scratch
-// and must be serialised by the caller.
+// and must be serialised by the caller; an overlap can spoil the scores of the
+// calls that overlap (reads of several parts or tiles), never a later call's.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -67,9 +68,14 @@ __device__ __forceinline__ uint32_t encode(uint8_t c) {
 
 __device__ __forceinline__ float ph_of(const float* ph, uint8_t q) { return ph[q > 127 ? 127 : q]; }
 
-// The work queue: pairs handed out so far and blocks done.  The last block of a call
-// sets both back to zero, so a call needs no other launch before it.
-static __device__ unsigned g_queue[2];
+// The work queues: list positions handed out so far.  A call takes the next word in turn
+// and clears it in a launch of its own ahead of its kernel, so it relies on nothing that
+// an earlier call left, and calls that overlap hand out their own pairs each (a captured
+// call keeps its word: its replays clear it too).
+constexpr unsigned kQueues = 1024;
+static __device__ unsigned g_queue[kQueues];
+
+__global__ void clear_queue_kernel(unsigned queue) { g_queue[queue] = 0; }
 
 struct Args {
     const uint8_t *read_bases, *base_quals, *ins_quals, *del_quals, *hap_bases;
@@ -81,6 +87,7 @@ struct Args {
     int64_t nwarps;
     int max_h;
     int grab;           // pairs a warp takes at a time, at most 32
+    unsigned queue;     // the call's word of g_queue
 };
 
 // A read's positions straight from the caller's arrays, as the packed words hold them.
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
     float4* const wscr = a.scratch + warp * 2 * a.rows;
     while (warp < a.nwarps) {  // the scratch holds borders for nwarps warps only
         unsigned x = 0;
-        if (lane == 0) x = atomicAdd(&g_queue[0], 1u);
+        if (lane == 0) x = atomicAdd(&g_queue[a.queue], 1u);
         x = __reduce_max_sync(kFullMask, x);
         const int64_t p0 = (int64_t)x * a.grab;
         if (p0 >= a.num_pairs) break;
@@ -374,17 +381,13 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
             __syncwarp();
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&g_queue[1], 1u) == gridDim.x - 1) {
-        g_queue[0] = 0;   // every block has left the queue
-        g_queue[1] = 0;
-    }
 }
 
 // per-device set-up: the scratch array's device address and the grid size
 struct DeviceState {
     std::atomic<int> ready{0};
     std::atomic<float4*> scratch{nullptr};
+    std::atomic<unsigned> calls{0};   // queue words given out
     int max_warps = 0;
 };
 DeviceState g_state[kMaxDevices];
@@ -454,10 +457,13 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
         int grab = (int)(num_pairs / (4 * warps));
         grab = grab < 1 ? 1 : grab > 8 ? 8 : grab;
         Args ka{read_bases, base_quals, ins_quals, del_quals, hap_bases, pairs, num_pairs, scores,
-                scratch,    rows,       warps,     max_hap_length, grab};
-        void* args[] = {&ka};
-        const cudaError_t le = cudaLaunchKernel(reinterpret_cast<const void*>(&forward_pairs_kernel), dim3(grid),
-                                                dim3(kThreads), args, kSmem, static_cast<cudaStream_t>(stream));
+                scratch,    rows,       warps,     max_hap_length, grab,    st.calls.fetch_add(1) % kQueues};
+        void *args[] = {&ka}, *queue[] = {&ka.queue};
+        cudaError_t le = cudaLaunchKernel(reinterpret_cast<const void*>(&clear_queue_kernel), dim3(1), dim3(1), queue,
+                                          0, static_cast<cudaStream_t>(stream));
+        if (le == cudaSuccess)
+            le = cudaLaunchKernel(reinterpret_cast<const void*>(&forward_pairs_kernel), dim3(grid), dim3(kThreads),
+                                  args, kSmem, static_cast<cudaStream_t>(stream));
         if (le != cudaSuccess) {
             cudaGetLastError();  // the failed launch's own error, recorded by the runtime as well
             status = PAIRHMM_ERR_CUDA;

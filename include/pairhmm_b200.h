@@ -280,7 +280,8 @@ void pairhmm_set_host_threads(int32_t threads);
  * compiled into the module and needs no upload.  Launch errors are this
  * call's own: an error the caller left pending is neither returned nor
  * cleared.  All calls share the scratch: calls that overlap on the GPU race
- * and must be serialised by the caller.
+ * and must be serialised by the caller (an overlap can spoil those calls'
+ * scores, not a later call's: each clears its own work queue).
  */
 typedef struct pairhmm_pair {
     int64_t read_offset;

@@ -97,3 +97,34 @@ def test_score_does_not_depend_on_the_list():
         np.testing.assert_array_equal(call(pairs[order]), want[order])
     for part in np.array_split(rng.permutation(len(pairs))[:600], 40):
         np.testing.assert_array_equal(call(pairs[part]), want[part])
+
+
+def test_calls_of_different_sizes_follow_one_another():
+    """Every call starts from its own empty queue: lists from one pair to some 70,000, one
+    after another on one stream, each scored whole; and a call captured in a graph, whose
+    replays come between other calls."""
+    import torch
+    batch = ladder(3, [9, 40, 100, 151, 250, 700], (30, 45), reads=8, haps=3)
+    pairs = pair_list(batch)
+    call = flat_call(batch)
+    want = call(pairs)
+    assert not np.any(want == np.float32(7.0))
+    rng = np.random.default_rng(4)
+    dev = torch.device("cuda:0")
+    d = [torch.from_numpy(np.ascontiguousarray(getattr(batch, k))).to(dev)
+         for k in ("read_bases", "base_quals", "ins_quals", "del_quals", "hap_bases")]
+    order = rng.integers(0, len(pairs), size=5000)
+    dpairs = torch.from_numpy(pairs[order].view(np.uint8)).to(dev)
+    scores = torch.empty(len(order), dtype=torch.float32, device=dev)
+    side = torch.cuda.Stream(dev)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        g.forward_pairs_noalloc(0, *d, dpairs, len(order), int(batch.hap_lengths.max()), scores, side)
+    for n in (70000, 1, 3, 20000, 64, 2, 40000, 500):
+        pick = rng.integers(0, len(pairs), size=n)
+        np.testing.assert_array_equal(call(pairs[pick]), want[pick])
+        scores.fill_(7.0)
+        torch.cuda.synchronize(dev)
+        graph.replay()
+        torch.cuda.synchronize(dev)
+        np.testing.assert_array_equal(scores.cpu().numpy(), want[order])
