@@ -35,6 +35,7 @@
 // calls that overlap (reads of several parts or tiles), never a later call's.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cfloat>
 #include <cstdint>
@@ -68,14 +69,17 @@ __device__ __forceinline__ uint32_t encode(uint8_t c) {
 
 __device__ __forceinline__ float ph_of(const float* ph, uint8_t q) { return ph[q > 127 ? 127 : q]; }
 
-// The work queues: list positions handed out so far.  A call takes the next word in turn
-// and clears it in a launch of its own ahead of its kernel, so it relies on nothing that
+// The work queues: list positions handed out so far.  A call takes the next words in turn
+// and clears them in a launch of its own ahead of its kernel, so it relies on nothing that
 // an earlier call left, and calls that overlap hand out their own pairs each (a captured
-// call keeps its word: its replays clear it too).
+// call keeps its words: its replays clear them too).
 constexpr unsigned kQueues = 1024;
-static __device__ unsigned g_queue[kQueues];
+static __device__ unsigned g_queue[kQueues][2];   // the tiles' and the general form's
 
-__global__ void clear_queue_kernel(unsigned queue) { g_queue[queue] = 0; }
+__global__ void clear_queue_kernel(unsigned queue) { g_queue[queue][0] = g_queue[queue][1] = 0; }
+
+// Marks a pair's score between the call's two kernels: a NaN that no score is.
+constexpr uint32_t kToGeneral = 0x7fa50a51u;
 
 struct Args {
     const uint8_t *read_bases, *base_quals, *ins_quals, *del_quals, *hap_bases;
@@ -87,7 +91,8 @@ struct Args {
     int64_t nwarps;
     int max_h;
     int grab;           // pairs a warp takes at a time, at most 32
-    unsigned queue;     // the call's word of g_queue
+    int look;           // pairs a warp of the general form looks through at a time, at most 32
+    unsigned queue;     // the call's words of g_queue
 };
 
 // A read's positions straight from the caller's arrays, as the packed words hold them.
@@ -120,14 +125,13 @@ constexpr int kTableBytes = 5 * (kMaxR / 4) * 32 * 16;   // per warp
 constexpr int kRingBytes = 64 * 16;
 constexpr size_t kSmem = (kThreads / 32) * (size_t)(kTableBytes + kRingBytes);
 
-// Pairs `mine` (by lane: the group's pair, or -1) of one shape.  Returns (warp-uniform)
-// the lanes whose pair the general form computes instead: no score is written for it.
-// These are pairs whose sum lies so low that the tiles' rounding in the denormal range,
+// Pairs `mine` (by lane: the group's pair, or -1) of one shape.  Marked for the general
+// form are pairs whose sum lies so low that the tiles' rounding in the denormal range,
 // which sets in earlier than the general form's (N lies 1/delta below M), could be more
 // than 2^-23 of it.  That is the pair's own sum, so its form, and with it its score,
 // depends on no other pair of the list.
 template <int G, int R>
-__device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
+__device__ __noinline__ void run_tile(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int parts) {
     using T = TileWavefront<float, G, R, G == 32 ? 0 : 1, false, false, G == 32, ByteRead, ByteHap, span_of(R)>;
     const int lane = threadIdx.x & 31;
     const int t = lane % G;
@@ -171,12 +175,13 @@ __device__ __noinline__ unsigned run_tile(const Args& a, const float* ph, char* 
     const ByteHap hap{a.hap_bases + pr.hap_offset, H};
     T::run(rd, hap, H, K, uni, tab, ring, reinterpret_cast<typename T::RingRow*>(wscr), a.rows, t, 0, lane, 0.0, sum,
            parts);
-    const bool result = mine >= 0 && t == G - 1;
-    const bool kept = sum.s[0] >= (double)tile_rounding(L, H, range) && sum.s[0] <= (double)FLT_MAX;
-    if (result && kept)
-        a.scores[mine] = (float)(log10(sum.s[0] / (double)H) - log10((double)kTileD0) -
-                                 (double)(bias * 0.43429448f));
-    return __ballot_sync(kFullMask, result && !kept);
+    if (mine >= 0 && t == G - 1) {
+        const bool kept = sum.s[0] >= (double)tile_rounding(L, H, range) && sum.s[0] <= (double)FLT_MAX;
+        a.scores[mine] = kept ? (float)(log10(sum.s[0] / (double)H) - log10((double)kTileD0) -
+                                        (double)(bias * 0.43429448f))
+                              : __uint_as_float(kToGeneral);
+    }
+    __syncwarp();
 }
 
 // The general form: one pair on the warp, R positions a lane, read tiles of 32 * R, beta
@@ -240,10 +245,12 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
             float Ml = 0.f, Dl = 0.f, Mul = 0.f, Dul = 0.f, Iul = 0.f;
             if (t == 0 && tile == 0) { Dl = Dbound; Dul = Dbound; }
             uint32_t h = 4u;
+            uint8_t base = t == 0 ? hb[0] : 0;   // of the next step, a step ahead of its use
             for (int k = 0; k <= kg; ++k) {
                 uint32_t hn = __shfl_up_sync(kFullMask, h, 1);
-                if (t == 0) hn = k < H ? encode(hb[k]) : 4u;
+                if (t == 0) hn = k < H ? encode(base) : 4u;
                 h = hn;
+                if (t == 0 && k + 1 < H) base = __ldg(hb + k + 1);
                 float Mdiag = Mul, Idiag = Iul, Xdiag = Iul + Dul;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -257,11 +264,9 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
                     Idiag = In;
                     Xdiag = In + Dold;
                 }
-                if (res_lane) {
-                    float a = Idiag;
-                    if (addM && k < kg) a = fmaf(kBeta, M[R - 1], a);
-                    acc += (double)a;
-                }
+                float a = Idiag;
+                if (addM && k < kg) a = fmaf(kBeta, M[R - 1], a);
+                acc += (double)(res_lane ? a : 0.f);
                 if (writer) {
                     const int j = k - (32 - 1);
                     if (j >= 0 && j < H) *reinterpret_cast<float2*>(eout + j) = make_float2(M[R - 1], D[R - 1]);
@@ -298,18 +303,6 @@ __device__ __noinline__ void run_general(const Args& a, const float* ph, float4*
     }
 }
 
-// Positions a lane by read length: with 16 for every read (tiles of 512), a list of 46,336
-// pairs of 70-250 positions that all score too low for the tiles took 7.8 ms, with the
-// lengths' own 4-8 it takes 5.2 ms (5.0 ms with one form of 16 for every list).
-__device__ __forceinline__ void general(const Args& a, const float* ph, float4* wscr, int64_t pi) {
-    const int L = a.pairs[pi].read_length;   // warp-uniform
-    if (L <= 128) run_general<4>(a, ph, wscr, pi);
-    else if (L <= 192) run_general<6>(a, ph, wscr, pi);
-    else if (L <= 256) run_general<8>(a, ph, wscr, pi);
-    else if (L <= 384) run_general<12>(a, ph, wscr, pi);
-    else run_general<16>(a, ph, wscr, pi);
-}
-
 // Shape of a pair's tile: 0 general, else lanes << 8 | positions a lane.
 __device__ __forceinline__ int shape_of(int L) {
     if (L <= 8) return 0;   // 8 lanes of at least one position
@@ -319,12 +312,12 @@ __device__ __forceinline__ int shape_of(int L) {
 }
 
 template <int G, int R0, int R1>   // R0, R0 + kStepR, .. R1
-__device__ __forceinline__ unsigned run_shape(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int R,
+__device__ __forceinline__ void run_shape(const Args& a, const float* ph, char* smem, float4* wscr, int64_t mine, int R,
                                           int parts) {
     if constexpr (R0 < R1) {
         if (R != R0) return run_shape<G, R0 + kStepR, R1>(a, ph, smem, wscr, mine, R, parts);
     }
-    return run_tile<G, R0>(a, ph, smem, wscr, mine, parts);
+    run_tile<G, R0>(a, ph, smem, wscr, mine, parts);
 }
 
 __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
@@ -338,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
     float4* const wscr = a.scratch + warp * 2 * a.rows;
     while (warp < a.nwarps) {  // the scratch holds borders for nwarps warps only
         unsigned x = 0;
-        if (lane == 0) x = atomicAdd(&g_queue[a.queue], 1u);
+        if (lane == 0) x = atomicAdd(&g_queue[a.queue][0], 1u);
         x = __reduce_max_sync(kFullMask, x);
         const int64_t p0 = (int64_t)x * a.grab;
         if (p0 >= a.num_pairs) break;
@@ -373,11 +366,45 @@ __global__ void __launch_bounds__(kThreads, 6) forward_pairs_kernel(Args a) {
             }
             left &= ~taken;
             const int parts = G == 32 ? (__shfl_sync(kFullMask, L, lead) + 32 * kMaxR - 1) / (32 * kMaxR) : 1;
-            unsigned redo = 1u;   // lanes whose `mine` the general form computes
-            if (G == 8) redo = run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 16) redo = run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
-            else if (G == 32) redo = run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
-            for (; redo; redo &= redo - 1) general(a, ph, wscr, __shfl_sync(kFullMask, mine, __ffs(redo) - 1));
+            if (G == 8) run_shape<8, 4, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 16) run_shape<16, 12, 20>(a, ph, smem, wscr, mine, R, 1);
+            else if (G == 32) run_shape<32, 12, 20>(a, ph, smem, wscr, mine, R, parts);
+            else if (lane == 0) a.scores[mine] = __uint_as_float(kToGeneral);
+            __syncwarp();
+        }
+    }
+}
+
+// The pairs the tiles left: a warp looks through up to 32 of the list at a time.  A launch
+// of its own, not the tiles' kernel: side by side the two thrashed the instruction cache,
+// and a warp's low pairs ran one after the other while other warps had none.  46,336 pairs
+// of 70-250 positions, 59% of them low: 4.8 -> 3.7 ms; all low 5.2 -> 4.6 (7.8 with 16
+// positions a lane for every read, instead of 4-16 by its length; 5.0 without tiles, on
+// the general form alone); none low 1.71 -> 1.71.  What bounds it: a step's serial chain,
+// some 430 cycles for 4 positions a lane when the warp is alone (16 short pairs, 12 of them
+// low: 131 us, 97 on the general form alone).
+__global__ void __launch_bounds__(kThreads, 6) general_pairs_kernel(Args a) {
+    __shared__ float ph[128];
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) ph[i] = c_ph2pr[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    float4* const wscr = a.scratch + warp * 2 * a.rows;
+    while (warp < a.nwarps) {
+        unsigned x = 0;
+        if (lane == 0) x = atomicAdd(&g_queue[a.queue][1], 1u);
+        const int64_t p0 = (int64_t)__shfl_sync(kFullMask, x, 0) * a.look;
+        if (p0 >= a.num_pairs) break;
+        const bool mine = lane < a.look && p0 + lane < a.num_pairs &&
+                          __float_as_uint(a.scores[p0 + lane]) == kToGeneral;
+        for (unsigned m = __ballot_sync(kFullMask, mine); m; m &= m - 1) {
+            const int64_t pi = p0 + __ffs(m) - 1;
+            const int L = a.pairs[pi].read_length;   // warp-uniform
+            if (L <= 128) run_general<4>(a, ph, wscr, pi);
+            else if (L <= 192) run_general<6>(a, ph, wscr, pi);
+            else if (L <= 256) run_general<8>(a, ph, wscr, pi);
+            else if (L <= 384) run_general<12>(a, ph, wscr, pi);
+            else run_general<16>(a, ph, wscr, pi);
             __syncwarp();
         }
     }
@@ -456,14 +483,19 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
         // together, but at least four times per warp, so that the last ones end together
         int grab = (int)(num_pairs / (4 * warps));
         grab = grab < 1 ? 1 : grab > 8 ? 8 : grab;
+        // the general form's: one pair each for a short list, since any may be low
+        const int look = (int)std::min<int64_t>(32, std::max<int64_t>(1, num_pairs / (8 * warps)));
         Args ka{read_bases, base_quals, ins_quals, del_quals, hap_bases, pairs, num_pairs, scores,
-                scratch,    rows,       warps,     max_hap_length, grab,    st.calls.fetch_add(1) % kQueues};
+                scratch,    rows,       warps,     max_hap_length, grab, look, st.calls.fetch_add(1) % kQueues};
         void *args[] = {&ka}, *queue[] = {&ka.queue};
         cudaError_t le = cudaLaunchKernel(reinterpret_cast<const void*>(&clear_queue_kernel), dim3(1), dim3(1), queue,
                                           0, static_cast<cudaStream_t>(stream));
         if (le == cudaSuccess)
             le = cudaLaunchKernel(reinterpret_cast<const void*>(&forward_pairs_kernel), dim3(grid), dim3(kThreads),
                                   args, kSmem, static_cast<cudaStream_t>(stream));
+        if (le == cudaSuccess)
+            le = cudaLaunchKernel(reinterpret_cast<const void*>(&general_pairs_kernel), dim3(grid), dim3(kThreads),
+                                  args, 0, static_cast<cudaStream_t>(stream));
         if (le != cudaSuccess) {
             cudaGetLastError();  // the failed launch's own error, recorded by the runtime as well
             status = PAIRHMM_ERR_CUDA;
