@@ -270,6 +270,10 @@ struct TileWavefront {
     // 64 long-read regions' FP32 stage 14.6 ms against 7.0 at 2 steps and 7.9 at 1; the
     // flat list's kernel has its shapes side by side in one launch
     static constexpr int kUnroll = SERIAL || !std::is_same<Read, PackedRead>::value ? 2 : 4;
+    // rows of the result summed in double one by one; else a step block's four rows in FP32
+    // first (the flat list's general form sums row by row, and so do its tiles; the engine's
+    // FP32 kernels sum by fours)
+    static constexpr bool kRowSums = kDouble || !std::is_same<Read, PackedRead>::value;
     static constexpr int kMaxShift = 640;   // EXT: largest scale difference a hand-off converts
     static constexpr size_t kSmemBytes = (size_t)kTableWords * sizeof(Word);  // per warp, the table
     static constexpr int kWarps = kBlockGroup ? W : 2;   // per block
@@ -585,8 +589,8 @@ struct TileWavefront {
                     Ne = O::sel(holds[j], N[R - 1 - j], Ne);
                 }
                 const V T = O::fma(Nl, wend, Id);
-                if constexpr (kDouble) {
-                    if (k <= kres) sum.s[0] += T;
+                if constexpr (kRowSums) {
+                    if (k <= kres) sum.s[0] += (double)O::side(T, 0);
                 } else {
                     if (k <= kres) a4 = O::add(a4, T);
                 }
@@ -645,7 +649,7 @@ struct TileWavefront {
                     if (k <= kres) sum.e = e;
                 }
             }
-            if constexpr (!kDouble) {
+            if constexpr (!kRowSums) {
                 if (kres >= 0) {
 #pragma unroll
                     for (int s = 0; s < NS; ++s) sum.s[s] += (double)O::side(a4, s);
