@@ -103,6 +103,28 @@ std::vector<TileRule> gcp_rules() {
     return rules;
 }
 
+// Tables of an engine without the FP64 pass: padded tiles (autotune.py's picks; in gcp
+// mode the kernels compiled with that option).  A score then is what single precision
+// gives, down to the end of its range, and values on exact tiles lie up to 1/delta lower:
+// between 1e-72 and 1e-76 scores of reads with gap qualities 60-93 were off by 0.07 (rms
+// of log10) or -inf there, and are good to 2e-6 on these.
+std::vector<TileRule> padded_rules(bool gcp) {
+    if (gcp)
+        return {
+            {64, 4, 16, false},   {128, 8, 16, false},   {160, 8, 20, false},    {256, 16, 16, false},
+            {512, 32, 16, false}, {1024, 32, 32, false}, {1 << 30, 32, 32, true},
+        };
+    return {
+        {16, 4, 4, false},         {32, 4, 8, false, true},    {48, 4, 12, false, true},  {64, 4, 16, false},
+        {80, 4, 20, false},        {96, 8, 12, false, true},   {112, 4, 28, false},       {128, 8, 16, false, true},
+        {144, 8, 18, false},       {160, 8, 20, false},        {176, 8, 22, false},       {192, 16, 12, false, true},
+        {224, 8, 28, false},       {256, 16, 16, false, true}, {288, 16, 18, false},      {320, 16, 20, false},
+        {384, 32, 12, false, true}, {448, 16, 28, false},      {512, 32, 16, false, true}, {640, 32, 20, false},
+        {768, 32, 24, false},      {896, 32, 28, false},       {1024, 32, 32, false},     {1280, 32, 20, true},
+        {1536, 32, 24, true},      {1792, 32, 28, true},       {1 << 30, 32, 32, true},
+    };
+}
+
 // The table of a batch of few pairs: the same, with 32 lanes a group wherever an
 // exact tile has fewer, and blocks of 8 warps (256 lanes) from 641 positions on.  Results do not change: the exact tiles' do not depend on the
 // shape, and the other classes stay.
@@ -238,7 +260,9 @@ const char* check_rules(const std::vector<TileRule>& rules, bool gcp) {
 }
 
 std::vector<TileRule> default_rules(const pairhmm_options_t& o) {
-    return o.mode == PAIRHMM_MODE_PLAIN ? plain_rules() : o.gcp ? gcp_rules() : engine_default_rules();
+    if (o.mode == PAIRHMM_MODE_PLAIN) return plain_rules();
+    if (!o.fp64_rescue) return padded_rules(o.gcp != 0);
+    return o.gcp ? gcp_rules() : engine_default_rules();
 }
 }  // namespace
 
@@ -376,10 +400,14 @@ pairhmm_status_t Engine::set_tile_table(const std::vector<TileRule>& rules) {
     return PAIRHMM_OK;
 }
 
+bool Engine::has_default_table(const std::vector<TileRule>& rules) const {
+    return opts_.mode != PAIRHMM_MODE_PLAIN && rules == default_rules(opts_);
+}
+
 pairhmm_status_t Engine::build_tables(const std::vector<TileRule>& rules) {
     TileTable built[2];
     built[0].rules = rules;
-    if (rules == default_rules(opts_) && opts_.mode != PAIRHMM_MODE_PLAIN) built[1].rules = small_rules(rules);
+    if (has_default_table(rules) && opts_.fp64_rescue) built[1].rules = small_rules(rules);
     for (TileTable& t : built) {
         const char* wrong = t.rules.empty() ? nullptr : check_rules(t.rules, opts_.gcp != 0);
         if (wrong) return fail(PAIRHMM_ERR_INVALID_ARGUMENT, wrong);

@@ -119,6 +119,8 @@ public:
     // Replace the tile table of the current mode (autotuner).
     pairhmm_status_t set_tile_table(const std::vector<TileRule>& rules);
     const std::vector<TileRule>& tile_table() const { return tables_[0].rules; }
+    // engine form with the table it was made with
+    bool has_default_table() const { return has_default_table(tables_[0].rules); }
     int device() const { return opts_.device; }
     bool gcp() const { return opts_.gcp != 0; }
     int64_t budget_bytes() const { return opts_.device_budget_bytes; }
@@ -134,6 +136,7 @@ private:
     pairhmm_status_t host_begin(const pairhmm_batch_t& b, float* scores, cudaEvent_t mark_start,
                                 cudaEvent_t mark_end);
     pairhmm_status_t host_end();
+    bool has_default_table(const std::vector<TileRule>& rules) const;
     pairhmm_status_t build_tables(const std::vector<TileRule>& rules);
     // the table for a batch of these records becomes the current one
     void choose_table(int64_t num_records, const int32_t* reads_per_record, const int32_t* haps_per_record,

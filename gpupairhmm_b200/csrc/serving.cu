@@ -134,7 +134,7 @@ pairhmm_status_t ServingQueue::enqueue(const std::vector<std::shared_ptr<Region>
                 o.gcp = parent_.gcp() ? 1 : 0;
                 auto e = std::make_unique<Engine>(o);
                 pairhmm_status_t is = e->init();
-                if (is == PAIRHMM_OK) is = e->set_tile_table(parent_.tile_table());
+                if (is == PAIRHMM_OK && !parent_.has_default_table()) is = e->set_tile_table(parent_.tile_table());
                 // device memory for the slot's batches up front (its budget, at most
                 // kReservePerSlot): a batch larger than any before then grows its buffers
                 // inside the pool instead of mapping memory while the other slots run

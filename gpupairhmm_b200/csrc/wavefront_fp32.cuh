@@ -411,8 +411,10 @@ struct Fp32Wavefront {
         if (valid && !handed_off && t == rlane) {
             const float res = (float)(log10(accd) - (log10((double)kScale) + log10((double)beta)));
             v.scores[task.out] = res;
-            if (degenerate ||
-                (v.rescue_enabled && !(accd >= (double)rescue_threshold(L, H) && accd <= (double)FLT_MAX))) {
+            // an overflow (gap qualities beyond 60 that differ from position to position can reach
+            // it at any score) is no result of single precision: with or without the rescue
+            if (degenerate || !(accd <= (double)FLT_MAX) ||
+                (v.rescue_enabled && !(accd >= (double)rescue_threshold(L, H)))) {
                 append_rescue(v, L, task);
             }
         }

@@ -243,13 +243,15 @@ struct Fp32x2Wavefront {
         const double off = log10((double)kScale) + log10((double)kBeta);
         if (resA) {
             v.scores[it.out0] = (float)(log10(accdA) - off);
-            if (degA || (v.rescue_enabled && !(accdA >= (double)rescue_threshold(LA, H) && accdA <= (double)FLT_MAX))) {
+            if (degA || !(accdA <= (double)FLT_MAX) ||
+                (v.rescue_enabled && !(accdA >= (double)rescue_threshold(LA, H)))) {
                 append_rescue(v, LA, Task{ra, it.hap, it.out0});
             }
         }
         if (resB) {
             v.scores[it.out1] = (float)(log10(accdB) - off);
-            if (degB || (v.rescue_enabled && !(accdB >= (double)rescue_threshold(LB, H) && accdB <= (double)FLT_MAX))) {
+            if (degB || !(accdB <= (double)FLT_MAX) ||
+                (v.rescue_enabled && !(accdB >= (double)rescue_threshold(LB, H)))) {
                 append_rescue(v, LB, Task{rb, it.hap, it.out1});
             }
         }
