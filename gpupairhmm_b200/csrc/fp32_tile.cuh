@@ -92,7 +92,7 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
             const int K = T::kBlockGroup ? 0 : (int)((__reduce_max_sync(kFullMask, (unsigned)(H + G)) + 3u) & ~3u);
             double stop = 0.0;
             if (SERIAL && v.rescue_enabled)
-                stop = (double)tile_threshold(rd.L[0], H, v.read_meta[item->read0].range);
+                stop = (double)tile_threshold(rd.L[0], H, v.read_meta[item->read0].range, rd.beta[0]);
             rd.ph = ph;
             T::run(rd, hap, H, K, uni, tab, ring, border, rows, t, T::kBlockGroup ? warp : 0, lane, stop, sum);
         }
@@ -111,8 +111,9 @@ fp32_tile_kernel(DevView v, const Item* __restrict__ items, long long num_items,
                 const int L = v.read_len[read];
                 const ReadMeta meta = v.read_meta[read];
                 v.scores[out] = (float)(log10(sum.s[s] / (double)H) - log10((double)kTileD0) - (double)meta.bias);
+                const float beta = GCP ? (float)(1.0 - (double)ph[v.read_gcp[read]]) : kBeta;
                 if ((meta.flags & 1u) ||
-                    (v.rescue_enabled && !(sum.s[s] >= (double)tile_threshold(L, H, meta.range) &&
+                    (v.rescue_enabled && !(sum.s[s] >= (double)tile_threshold(L, H, meta.range, beta) &&
                                            sum.s[s] <= (double)FLT_MAX)))
                     append_rescue(v, L, Task{read, hap, out});
             }

@@ -152,11 +152,11 @@ __device__ __forceinline__ float tile_rounding(int L, int H, float range) {
 }
 
 // Smallest sum of T the FP32 pass keeps.  The second term is rescue_threshold in this
-// scale (the sum there is beta*T over (FLT_MAX/16)/H): no pair that wavefront_fp32.cuh
-// would pass on is kept here.
-__device__ __forceinline__ float tile_threshold(int L, int H, float range) {
+// scale (the sum there is beta*T, beta the read's own in gcp mode, over (FLT_MAX/16)/H): no
+// pair that wavefront_fp32.cuh would pass on is kept here.
+__device__ __forceinline__ float tile_threshold(int L, int H, float range, float beta) {
     const float cells = (float)L * (float)H * 0x1p-127f;
-    return fmaxf(tile_rounding(L, H, range), 3.0f * cells * (float)H * (2.0f / kBeta));
+    return fmaxf(tile_rounding(L, H, range), 3.0f * cells * (float)H * (2.0f / beta));
 }
 
 // Smallest sum the FP64 pass's scaled tier keeps: the same terms each round by at most

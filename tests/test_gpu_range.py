@@ -10,6 +10,15 @@ from test_gpu_flat import ladder
 
 pytestmark = pytest.mark.gpu
 
+
+def pair_lengths(batch):
+    """Read and haplotype length of every score."""
+    R, H = batch.reads_per_record, batch.haps_per_record
+    first = np.cumsum(H) - H
+    return (np.repeat(batch.read_lengths, np.repeat(H, R)).astype(np.float64),
+            np.concatenate([np.tile(batch.hap_lengths[f:f + n], r) for f, n, r in zip(first, H, R)]).astype(np.float64))
+
+
 LENGTHS = [20, 40, 70, 101, 120, 150, 151, 200, 250, 300, 330, 500, 700]
 
 
@@ -36,3 +45,24 @@ def test_engine_without_fp64_keeps_the_range(gaps, gcp, plain_engine):
     assert rms(got) <= 3.0 * rms(plain), (rms(got), rms(plain))
     kept = want > -72.0
     assert_log10_close(got[kept], want[kept], what=f"gaps {gaps} gcp {gcp}")
+
+
+@pytest.mark.parametrize("quality", [1, 2, 4])
+def test_gcp_threshold_counts_the_reads_own_beta(quality):
+    """Single precision keeps a pair down to 3*L*H*2^-127 of a sum that carries the read's
+    beta = 1 - p(gcp) (FLT_MAX/16 = 2^124 the boundary's scale): every pair below that is
+    recomputed in double, also where low gcp qualities make beta small."""
+    # lengths at which unrelated reads score about there
+    lengths = {1: range(640, 800, 8), 2: range(300, 380, 4), 4: range(150, 230, 4)}[quality]
+    batch = ladder(3, lengths, 20, rates=(0.1, 0.75))
+    batch.gcp_quals[:] = quality
+    want = oracle.batch_log10(batch, gcp=True)
+    L, H = pair_lengths(batch)
+    beta = 1.0 - 10.0 ** (-quality / 10.0)
+    below = want < np.log10(3.0 * L * H / beta) - (127 + 124) * np.log10(2.0) - 1e-3
+    default = want < np.log10(3.0 * L * H / 0.9) - (127 + 124) * np.log10(2.0) - 1e-3
+    assert below.sum() > default.sum()
+    with g.Engine(gcp=True) as e:
+        got = e.compute(batch)
+        assert e.stats().rescued >= below.sum()
+    assert_log10_close(got, want)
