@@ -325,10 +325,10 @@ pairhmm_status_t Engine::reserve_pool(size_t bytes) {
     return PAIRHMM_OK;
 }
 
-pairhmm_status_t Engine::ensure_side_streams(int n) {
-    for (int i = 0; i < n; ++i) {
-        if (!side_[i]) PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
-        if (!join_[i]) PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
+pairhmm_status_t Engine::make_side_streams() {
+    for (int i = 0; i < kSideStreams; ++i) {
+        PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
+        PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
     }
     return PAIRHMM_OK;
 }
@@ -379,6 +379,10 @@ pairhmm_status_t Engine::init() {
             return fail(PAIRHMM_ERR_UNSUPPORTED, "FP64 class without compiled kernel");
         PHMM_CUDA(fp64_lut_[w].ensure(kFp64LutSize));
         PHMM_CUDA(cudaMemcpy(fp64_lut_[w].ptr, fp64_tables_[w].lut.data(), kFp64LutSize, cudaMemcpyHostToDevice));
+    }
+    if (opts_.mode != PAIRHMM_MODE_PLAIN) {   // the plain form launches on one stream
+        const pairhmm_status_t st = make_side_streams();
+        if (st != PAIRHMM_OK) return st;
     }
     ready_ = true;
     return build_tables(default_rules(opts_));
@@ -793,19 +797,47 @@ int64_t Engine::index_bytes(const BatchIndex& x) {
            8 * (int64_t)(x.rec_hap_base.size() + x.rec_pair_base.size() + x.read_start.size() + x.hap_start.size());
 }
 
-// The grid of a persistent launch: every block that fits at once.  A kernel's shared
-// memory opt-in and occupancy are asked for on its first use (each loads the kernel's
-// code, so an engine pays for the few tiles its batches need, not for all).
-int Engine::persistent_grid(const void* kernel, int threads, size_t smem) {
-    const auto it = blocks_per_sm_.find(kernel);
-    if (it != blocks_per_sm_.end()) return it->second * num_sms_;
+// A kernel's shared memory opt-in and occupancy, which load its code (about 0.4 ms in a
+// process that has not used it).
+pairhmm_status_t Engine::load_kernel(const void* kernel, int threads, size_t smem) {
+    if (blocks_per_sm_.count(kernel)) return PAIRHMM_OK;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    blocks_per_sm_.emplace(kernel, per_sm);
-    return per_sm * num_sms_;
+    PHMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PHMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    blocks_per_sm_.emplace(kernel, std::max(per_sm, 1));
+    return PAIRHMM_OK;
 }
+
+// The kernels a batch on these tables launches, or (x null) could launch.  A batch's own
+// are loaded ahead of its plan: creating an engine with all 200 of both tables takes 90 ms
+// in a fresh process, 14 ms without.
+pairhmm_status_t Engine::load_kernels(const TileTable& table, const Fp64Table& fp64, const BatchIndex* x) {
+    pairhmm_status_t st = PAIRHMM_OK;
+    auto load = [&](const auto* c) {
+        if (st == PAIRHMM_OK) st = load_kernel(c->kernel, c->block_threads, c->smem_bytes);
+    };
+    for (size_t b = 0; b < table.cfg.size(); ++b)
+        if (!x || x->bucket_items[b] != 0) load(table.cfg[b]);
+    for (size_t c = 0; c < fp64.classes.size(); ++c) {
+        if (x && x->class_pairs[c] == 0) continue;
+        load(fp64.classes[c].scaled);
+        load(fp64.exts[fp64.classes[c].ext].cfg);
+        if (c + 1 == fp64.classes.size()) load(fp64.fused);
+    }
+    return st;
+}
+
+pairhmm_status_t Engine::load_all_kernels() {
+    PHMM_CUDA(cudaSetDevice(opts_.device));
+    for (int i = 0; i < 2; ++i) {
+        const pairhmm_status_t st = load_kernels(tables_[i], fp64_tables_[i], nullptr);
+        if (st != PAIRHMM_OK) return st;
+    }
+    return PAIRHMM_OK;
+}
+
+// The grid of a persistent launch: every block that fits at once.
+int Engine::persistent_grid(const void* kernel) const { return blocks_per_sm_.at(kernel) * num_sms_; }
 
 pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const BatchIndex& x, const Plan& plan,
                                           float* d_scores, cudaStream_t s, int stage) {
@@ -1011,7 +1043,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     return join();
 }
 
-Engine::Plan Engine::make_plan(const BatchIndex& x) {
+Engine::Plan Engine::make_plan(const BatchIndex& x) const {
     const int nb = (int)table_->rules.size();
     const bool plain = opts_.mode == PAIRHMM_MODE_PLAIN;
     Plan p;
@@ -1031,7 +1063,7 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
         const ConfigInfo* c = table_->cfg[b];
         const int64_t tasks = (x.bucket_items[b] + c->per_task - 1) / c->per_task;
         const int64_t need_blocks = (tasks + c->tasks_per_block - 1) / c->tasks_per_block;
-        const int64_t resident = persistent_grid(c->kernel, c->block_threads, c->smem_bytes);
+        const int64_t resident = persistent_grid(c->kernel);
         int64_t grid = plain ? need_blocks : std::min(resident, need_blocks);
         if (c->scratch_bytes_per_row) {
             const int64_t per_warp = (int64_t)c->scratch_bytes_per_row * p.rows;
@@ -1055,7 +1087,7 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
     for (const Fp64Table::Ext& e : fp64_->exts) n_scratch += e.cfg->scratch_bytes_per_row > 0 && !e.own_stream;
     auto fp64_grid = [&](const Fp64Config* c, int64_t pairs, int64_t& bytes) {
         const int64_t tasks = (pairs + c->per_task - 1) / c->per_task;
-        int64_t grid = std::min<int64_t>(persistent_grid(c->kernel, c->block_threads, c->smem_bytes),
+        int64_t grid = std::min<int64_t>(persistent_grid(c->kernel),
                                          (tasks + c->tasks_per_block - 1) / c->tasks_per_block);
         grid = std::max<int64_t>(grid, 1);
         bytes = 0;
@@ -1077,8 +1109,6 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) {
             p.fp64_grid[c] = fp64_grid(scaled, x.class_pairs[c], bytes);
             if (e.own_stream) slice = bytes;
             else scratch += bytes;
-            if (c + 1 == (int)fp64_->classes.size())   // the fused form has the scaled form's grid
-                persistent_grid(fp64_->fused->kernel, fp64_->fused->block_threads, fp64_->fused->smem_bytes);
         }
         if (pairs == 0) continue;
         p.fp64_ext_scratch[i] = scratch;
@@ -1107,10 +1137,10 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
                                       cudaStream_t s) {
     if (x.num_pairs == 0) return PAIRHMM_OK;
     // every buffer the launches reference exists before capture starts
+    const pairhmm_status_t loaded = load_kernels(*table_, *fp64_, &x);
+    if (loaded != PAIRHMM_OK) return loaded;
     const Plan plan = make_plan(x);
     PHMM_CUDA(scratch_.ensure(plan.scratch_bytes));
-    const pairhmm_status_t side = ensure_side_streams(std::max(plan.side[1], plan.side[2]));
-    if (side != PAIRHMM_OK) return side;
     const cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
     // A graph only for small batches that launch the same kernels as the kept graph, or as
     // the eight batches before: instantiating one costs more than its 7-37 launches, and

@@ -108,6 +108,8 @@ public:
     // keeps `bytes` of device memory in the engine's pool (allocated once and freed), so
     // that buffer growth up to that size maps no new memory while other work runs
     pairhmm_status_t reserve_pool(size_t bytes);
+    // loads every kernel of the engine's tables, so that no batch's first use of a class does
+    pairhmm_status_t load_all_kernels();
     pairhmm_status_t compute_host(const pairhmm_batch_t& b, float* scores);
     pairhmm_status_t compute_device(const pairhmm_batch_t& b, int32_t max_read_len, int32_t max_hap_len,
                                     float* scores, cudaStream_t stream);
@@ -155,7 +157,7 @@ private:
         std::vector<int64_t> scratch_off;   // by bucket: multi-tile kernels run side by side
         size_t scratch_bytes = 0;
     };
-    Plan make_plan(const BatchIndex& idx);
+    Plan make_plan(const BatchIndex& idx) const;
     std::vector<uint8_t> launch_shape(const BatchIndex& x, const Plan& plan) const;
     // stage 0: packing + work list, 1: FP32 launches, 2: FP64 pass
     pairhmm_status_t enqueue_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, const Plan& plan,
@@ -168,7 +170,9 @@ private:
     pairhmm_status_t upload_gathered(const BatchIndex& idx, const InputRanges* r, pairhmm_batch_t* in,
                                      cudaStream_t s);
     static size_t input_bytes(const InputRanges& r, bool gcp);
-    int persistent_grid(const void* kernel, int threads, size_t smem);
+    pairhmm_status_t load_kernels(const TileTable& table, const Fp64Table& fp64, const BatchIndex* x);
+    pairhmm_status_t load_kernel(const void* kernel, int threads, size_t smem);
+    int persistent_grid(const void* kernel) const;
     static int64_t index_bytes(const BatchIndex& x);
     int64_t hbins_of(const BatchIndex& x) const;
 
@@ -181,16 +185,16 @@ private:
     const Fp64Table* fp64_ = &fp64_tables_[0];
     DevBuf fp64_lut_[2];
     int num_sms_ = 0;
-    std::unordered_map<const void*, int> blocks_per_sm_;  // kernels used so far
+    std::unordered_map<const void*, int> blocks_per_sm_;  // kernels loaded so far
     bool ready_ = false;
     cudaStream_t stream_ = nullptr;
     // the launches of one stage (bucket kernels, FP64 classes) fork onto side
     // streams so that their tails overlap and a small batch's buckets run side
     // by side; they join back into stream_ before the stage ends
     static constexpr int kSideStreams = 16;
-    cudaStream_t side_[kSideStreams] = {};   // created as batches need them
+    cudaStream_t side_[kSideStreams] = {};
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
-    pairhmm_status_t ensure_side_streams(int n);
+    pairhmm_status_t make_side_streams();
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
     int64_t launches_ = 0, fp32_launches_ = 0;
     cudaGraphExec_t graph_exec_ = nullptr;   // the whole batch: prep, FP32, FP64
