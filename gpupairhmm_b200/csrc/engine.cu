@@ -958,13 +958,20 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     const int nside = plan.side[stage];
     int nlaunch = 0;
     auto next_stream = [&]() { return nside ? side_[nlaunch++ % nside] : s; };
+    // staged_: the host waits in the streams' place
     auto fork = [&]() {
-        if (nside) PHMM_CUDA(cudaEventRecord(fork_, s));
+        if (nside && staged_) PHMM_CUDA(cudaStreamSynchronize(s));
+        if (!nside || staged_) return PAIRHMM_OK;
+        PHMM_CUDA(cudaEventRecord(fork_, s));
         for (int i = 0; i < nside; ++i) PHMM_CUDA(cudaStreamWaitEvent(side_[i], fork_, 0));
         return PAIRHMM_OK;
     };
     auto join = [&]() {
         for (int i = 0; i < nside; ++i) {
+            if (staged_) {
+                PHMM_CUDA(cudaStreamSynchronize(side_[i]));
+                continue;
+            }
             PHMM_CUDA(cudaEventRecord(join_[i], side_[i]));
             PHMM_CUDA(cudaStreamWaitEvent(s, join_[i], 0));
         }
@@ -1017,6 +1024,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
         };
         const int last = (int)fp64_->classes.size() - 1;
         bool shared_ext[kMaxFp64Classes] = {};
+        std::vector<std::pair<cudaStream_t, int>> behind;
         for (int c = last; c >= 0; --c) {
             if (x.class_pairs[c] == 0) continue;
             const Fp64Table::Class& k = fp64_->classes[c];
@@ -1027,8 +1035,26 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
             PHMM_CUDA(launch(fuse ? fp64_->fused : k.scaled, false, c, plan.fp64_grid[c], plan.fp64_scratch[c], k.ext,
                              on));
             if (!e.own_stream) shared_ext[k.ext] = true;
+            else if (!fuse && staged_ && nside) behind.push_back({on, k.ext});
             else if (!fuse)
                 PHMM_CUDA(launch(e.cfg, true, k.ext, plan.fp64_ext_grid[k.ext], plan.fp64_ext_scratch[k.ext], 0, on));
+        }
+        while (!behind.empty()) {   // staged_: an extended class once its stream's scaled class is done
+            const size_t waiting = behind.size();
+            for (size_t i = 0; i < behind.size();) {
+                const cudaError_t q = cudaStreamQuery(behind[i].first);
+                if (q == cudaErrorNotReady) {
+                    cudaGetLastError();
+                    ++i;
+                    continue;
+                }
+                PHMM_CUDA(q);
+                const int e = behind[i].second;
+                PHMM_CUDA(launch(fp64_->exts[e].cfg, true, e, plan.fp64_ext_grid[e], plan.fp64_ext_scratch[e], 0,
+                                 behind[i].first));
+                behind.erase(behind.begin() + i);
+            }
+            if (behind.size() == waiting) std::this_thread::yield();
         }
         bool any = false;
         for (bool b : shared_ext) any = any || b;
@@ -1149,7 +1175,7 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     // 1.57 / 0.67, 80 regions 1.38 / 1.29; the same batch again with a kept graph: 1 region
     // 0.186 / 0.192, 4 regions 0.256 / 0.268, 12 regions 0.585 / 0.564, 300 regions 3.67 / 3.51.
     bool use_graph = false;
-    if (opts_.use_graphs && x.num_pairs <= kGraphMaxPairs) {
+    if (opts_.use_graphs && !staged_ && x.num_pairs <= kGraphMaxPairs) {
         std::vector<uint8_t> shape = launch_shape(x, plan);
         shape_repeats_ = shape == last_shape_ ? shape_repeats_ + 1 : 0;
         use_graph = shape_repeats_ >= kGraphAfter || (graph_exec_ && shape == graph_shape_);

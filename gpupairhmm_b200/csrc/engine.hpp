@@ -104,6 +104,11 @@ public:
     Engine(const Engine&) = delete;
     Engine& operator=(const Engine&) = delete;
 
+    // The host thread waits for what a launch depends on, instead of enqueueing the launch
+    // with a wait ahead of it.  A device has 8 launch queues (by default), which all streams
+    // share in turn, and a wait in one holds up every later launch in it, whichever stream
+    // that is of: for engines with long kernels beside ones with short batches (serving.cu).
+    void set_staged(bool on) { staged_ = on; }
     pairhmm_status_t init();
     // keeps `bytes` of device memory in the engine's pool (allocated once and freed), so
     // that buffer growth up to that size maps no new memory while other work runs
@@ -192,6 +197,7 @@ private:
     // streams so that their tails overlap and a small batch's buckets run side
     // by side; they join back into stream_ before the stage ends
     static constexpr int kSideStreams = 16;
+    bool staged_ = false;
     cudaStream_t side_[kSideStreams] = {};
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
     pairhmm_status_t make_side_streams();

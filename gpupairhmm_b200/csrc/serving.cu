@@ -133,6 +133,14 @@ pairhmm_status_t ServingQueue::enqueue(const std::vector<std::shared_ptr<Region>
                 o.pipeline_chunks = 1;  // merged batches stay small: one pass
                 o.gcp = parent_.gcp() ? 1 : 0;
                 auto e = std::make_unique<Engine>(o);
+                // long batches' waits must not sit in the launch queues that short ones share.
+                // Short regions' p50 at 8,000 / 20,000 / 40,000 regions/s, 5% long: 2.9 / 8.7 /
+                // 62 -> 0.23 / 0.56 / 10.6 ms (long ones 4.5 / 9.5 / 55 -> 3.4 / 6.4 / 31).
+                // Fewer side streams (2 for the heavy slots, none for the light: 8 streams in
+                // all) gave 0.34 / 1.4 / 18, but 4.4 against 0.94 ms for short regions alone at
+                // 40,000; a share of the SMs, narrower tiles for long reads or priorities for
+                // the light slots' streams gave nothing.
+                e->set_staged(s >= kLightSlots);
                 pairhmm_status_t is = e->init();
                 if (is == PAIRHMM_OK && !parent_.has_default_table()) is = e->set_tile_table(parent_.tile_table());
                 // code loading, too, would stall the other slots' launches if a length class
