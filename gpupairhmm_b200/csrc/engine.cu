@@ -40,9 +40,10 @@ constexpr int kCtrTotal = kMaxBuckets + 4 * kMaxFp64Classes;
 // rounds of resident warps, so the order decides little and the three launches of the
 // sort are a third of the stage of a small batch
 constexpr int64_t kNoSortPairs = 4096;
-// Batches of more pairs than this, or whose launches have not been the same for a while,
-// are launched kernel by kernel (see run_pipeline).
+// Batches of more pairs or length classes than this, or whose launches have not been the
+// same for a while, are launched kernel by kernel (see run_pipeline).
 constexpr int64_t kGraphMaxPairs = 4096;
+constexpr int kGraphMaxClasses = 6;
 constexpr int64_t kGraphAfter = 8;
 // multi-tile FP64 pairs up to which the two tiers run fused (about one round of
 // resident warps of that class's kernel on 148 SMs)
@@ -1170,12 +1171,13 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     const cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
     // A graph only for small batches that launch the same kernels as the kept graph, or as
     // the eight batches before: instantiating one costs more than its 7-37 launches, and
-    // mixed small batches rarely have the same length classes.  Measured per call, graph /
-    // launches, changing batches of uneven regions: 4 regions 0.65 / 0.30 ms, 24 regions
-    // 1.57 / 0.67, 80 regions 1.38 / 1.29; the same batch again with a kept graph: 1 region
-    // 0.186 / 0.192, 4 regions 0.256 / 0.268, 12 regions 0.585 / 0.564, 300 regions 3.67 / 3.51.
+    // mixed small batches rarely have the same length classes (changing batches of uneven
+    // regions, graph / launches a call: 4 regions 0.65 / 0.30 ms, 24 regions 1.57 / 0.67).
+    // And only for few classes: the same batch again, classes of 96-4,000 pairs in all,
+    // graph over launches: 1-3 classes 0.91-1.0, 4-6 0.92-1.03, 8 0.96-1.2, 10 1.05-1.18,
+    // 12 1.0-1.13.
     bool use_graph = false;
-    if (opts_.use_graphs && !staged_ && x.num_pairs <= kGraphMaxPairs) {
+    if (opts_.use_graphs && !staged_ && x.num_pairs <= kGraphMaxPairs && plan.side[1] <= kGraphMaxClasses) {
         std::vector<uint8_t> shape = launch_shape(x, plan);
         shape_repeats_ = shape == last_shape_ ? shape_repeats_ + 1 : 0;
         use_graph = shape_repeats_ >= kGraphAfter || (graph_exec_ && shape == graph_shape_);
