@@ -326,10 +326,10 @@ pairhmm_status_t Engine::reserve_pool(size_t bytes) {
     return PAIRHMM_OK;
 }
 
-pairhmm_status_t Engine::make_side_streams() {
-    for (int i = 0; i < kSideStreams; ++i) {
-        PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
-        PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
+pairhmm_status_t Engine::ensure_side_streams(int n) {
+    for (int i = 0; i < n; ++i) {
+        if (!side_[i]) PHMM_CUDA(cudaStreamCreateWithFlags(&side_[i], cudaStreamNonBlocking));
+        if (!join_[i]) PHMM_CUDA(cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming));
     }
     return PAIRHMM_OK;
 }
@@ -380,10 +380,6 @@ pairhmm_status_t Engine::init() {
             return fail(PAIRHMM_ERR_UNSUPPORTED, "FP64 class without compiled kernel");
         PHMM_CUDA(fp64_lut_[w].ensure(kFp64LutSize));
         PHMM_CUDA(cudaMemcpy(fp64_lut_[w].ptr, fp64_tables_[w].lut.data(), kFp64LutSize, cudaMemcpyHostToDevice));
-    }
-    if (opts_.mode != PAIRHMM_MODE_PLAIN) {   // the plain form launches on one stream
-        const pairhmm_status_t st = make_side_streams();
-        if (st != PAIRHMM_OK) return st;
     }
     ready_ = true;
     return build_tables(default_rules(opts_));
@@ -828,13 +824,13 @@ pairhmm_status_t Engine::load_kernels(const TileTable& table, const Fp64Table& f
     return st;
 }
 
-pairhmm_status_t Engine::load_all_kernels() {
+pairhmm_status_t Engine::load_all() {
     PHMM_CUDA(cudaSetDevice(opts_.device));
     for (int i = 0; i < 2; ++i) {
         const pairhmm_status_t st = load_kernels(tables_[i], fp64_tables_[i], nullptr);
         if (st != PAIRHMM_OK) return st;
     }
-    return PAIRHMM_OK;
+    return ensure_side_streams(kSideStreams);
 }
 
 // The grid of a persistent launch: every block that fits at once.
@@ -1167,6 +1163,8 @@ pairhmm_status_t Engine::run_pipeline(const pairhmm_batch_t& in, const BatchInde
     const pairhmm_status_t loaded = load_kernels(*table_, *fp64_, &x);
     if (loaded != PAIRHMM_OK) return loaded;
     const Plan plan = make_plan(x);
+    const pairhmm_status_t side = ensure_side_streams(std::max(plan.side[1], plan.side[2]));
+    if (side != PAIRHMM_OK) return side;
     PHMM_CUDA(scratch_.ensure(plan.scratch_bytes));
     const cudaEvent_t marks[3] = {ev_prep_, ev_fp32_, ev1_};
     // A graph only for small batches that launch the same kernels as the kept graph, or as

@@ -113,8 +113,9 @@ public:
     // keeps `bytes` of device memory in the engine's pool (allocated once and freed), so
     // that buffer growth up to that size maps no new memory while other work runs
     pairhmm_status_t reserve_pool(size_t bytes);
-    // loads every kernel of the engine's tables, so that no batch's first use of a class does
-    pairhmm_status_t load_all_kernels();
+    // loads every kernel of the engine's tables and makes its side streams, so that no batch's
+    // first use of a class does
+    pairhmm_status_t load_all();
     pairhmm_status_t compute_host(const pairhmm_batch_t& b, float* scores);
     pairhmm_status_t compute_device(const pairhmm_batch_t& b, int32_t max_read_len, int32_t max_hap_len,
                                     float* scores, cudaStream_t stream);
@@ -198,9 +199,9 @@ private:
     // by side; they join back into stream_ before the stage ends
     static constexpr int kSideStreams = 16;
     bool staged_ = false;
-    cudaStream_t side_[kSideStreams] = {};
+    cudaStream_t side_[kSideStreams] = {};   // created as batches need them
     cudaEvent_t fork_ = nullptr, join_[kSideStreams] = {};
-    pairhmm_status_t make_side_streams();
+    pairhmm_status_t ensure_side_streams(int n);
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_prep_ = nullptr, ev_fp32_ = nullptr;
     int64_t launches_ = 0, fp32_launches_ = 0;
     cudaGraphExec_t graph_exec_ = nullptr;   // the whole batch: prep, FP32, FP64

@@ -145,7 +145,7 @@ pairhmm_status_t ServingQueue::enqueue(const std::vector<std::shared_ptr<Region>
                 if (is == PAIRHMM_OK && !parent_.has_default_table()) is = e->set_tile_table(parent_.tile_table());
                 // code loading, too, would stall the other slots' launches if a length class
                 // first came up while they run
-                if (is == PAIRHMM_OK) is = e->load_all_kernels();
+                if (is == PAIRHMM_OK) is = e->load_all();
                 // device memory for the slot's batches up front (its budget, at most
                 // kReservePerSlot): a batch larger than any before then grows its buffers
                 // inside the pool instead of mapping memory while the other slots run
