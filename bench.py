@@ -407,9 +407,8 @@ def run_serving(args, local_rank):
            "latency": "arrival to scores on the host (submission delay + submit-to-done)"}
 
     eng = g.Engine(device=local_rank)
-    # regions with a read beyond the longest single tile run on the multi-tile slots
-    single_max = max(m for m, _, _, kind in eng.tile_table() if kind not in (1, 4))
-    heavy = [int(np.max(r.read_lengths)) > single_max for r in pool.regions]
+    # regions with a read beyond this run on the multi-tile slots
+    heavy = [int(np.max(r.read_lengths)) > g.LONG_READ for r in pool.regions]
     warm = eng.submit_many(pool, range(300))  # warm the queue's engines (a burst of both kinds)
     for i, tk in enumerate(warm):
         eng.drain(tk, pool.num_pairs[i])
@@ -652,7 +651,7 @@ def run_ours(args, cfg, rank, world, local_rank):
                          "flop_per_cell": FLOPS_PER_CELL,
                          # 11 algorithmic FLOP per cell in 5 FMA-pipe instructions (4 FFMA + 1 FMUL)
                          "instruction_mix_ceiling": round(FLOPS_PER_CELL / 10, 4),
-                         "kernel": "fp32_bucket_kernel (all length buckets)",
+                         "kernel": "fp32_tile_kernel (exact tiles; all length buckets)",
                          "stage_ms_per_step": {"prep": round(prep_ms / args.steps, 3),
                                                "fp32": round(fp32_ms / args.steps, 3),
                                                "fp64": round(fp64_ms / args.steps, 3)}},

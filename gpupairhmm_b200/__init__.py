@@ -31,6 +31,9 @@ CLI_PATH = HERE / "pairhmm_b200"
 
 MODE_ENGINE = 0
 MODE_PLAIN = 1
+# Reads beyond this count as multi-tile (Stats.multi_tile_pairs), and a region with one goes to
+# the serving queue's slots for long reads (kLongRead in engine.cu, default tile tables).
+LONG_READ = 1024
 
 STATUS = {
     0: "ok", 1: "invalid argument", 2: "CUDA error", 3: "out of memory", 4: "region exceeds the device budget",
@@ -413,7 +416,8 @@ class Engine:
     def tile_table(self) -> list[tuple[int, int, int, int]]:
         """(max read length, G, R, kind) with kind 0 = one tile, 1 = multi-tile,
         2 = one tile, two reads per group in packed FP32, 3 = the same with exact
-        tiles, 4 = exact tiles over a block of G/32 warps."""
+        tiles, 4 = exact tiles of more than 32 lanes (64, 96: one warp with its parts in
+        turn; 256: a block of 8 warps)."""
         n = ctypes.c_int32()
         _check(lib().pairhmm_get_tile_table(self._h, None, None, None, None, 0, ctypes.byref(n)), self._h)
         arrs = [np.zeros(n.value, dtype=np.int32) for _ in range(4)]

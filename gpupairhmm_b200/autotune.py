@@ -7,7 +7,7 @@ length uniform in the class, haplotype length = read length + U{50..400},
 base quality U{10..40}, ins/del 40 -- and keeps the fastest.  Classes beyond
 the largest single tile are timed with the multi-tile configurations.
 Adjacent classes with the same winner merge into one rule.  The engine's own
-table takes padded tiles only outside 33-640 positions, where it has exact tiles
+table takes padded tiles only outside 33-4,096 positions, where it has exact tiles
 (engine.cu); ``Engine.set_tile_table`` takes any table.
 
 Output:

@@ -1,13 +1,19 @@
-// Host-side engine: batch validation and indexing, device buffers, the
-// per-batch launch sequence and its CUDA-graph replay.
+// Host-side engine: batch validation and indexing, device buffers and the
+// per-batch launch sequence.
 //
-// Launch sequence of one batch (all on one stream, replayed as one graph):
+// Launch sequence of one batch:
 //   pack                        caller SoA -> packed HBM layout; the batch's fills
 //   bin_count, hist_scan,
 //   bin_scatter                 sorted work list
-//   fp32_bucket_kernel<G,R,MT>  one launch per non-empty length bucket
-//   fp64_rescue_kernel<scaled>  pairs flagged by the FP32 pass, in doubles
-//   fp64_rescue_kernel<ext>     the few beyond the scaled doubles' range
+//   fp32_tile_kernel,
+//   fp32_bucket_kernel          one launch per non-empty length bucket: exact tiles for reads
+//                               of 33-4,096 positions, else (user tables, the plain form, engines
+//                               without the FP64 pass) padded ones
+//   fp64_tile_kernel,
+//   fp64_rescue_kernel          per length class, pairs flagged by the FP32 pass in doubles,
+//                               then the few beyond the scaled doubles' range
+// A stage's launches fork onto side streams and join back.  Small batches that repeat are
+// launched as one graph (run_pipeline).
 // Compared with the reference executor (gpuworker.cuh:559-973) there is no
 // device-to-host synchronisation inside a batch: the host derives bucket sizes
 // and every bucket's range of work items from the record structure it already
@@ -36,10 +42,12 @@ constexpr int kCtrExt = kMaxBuckets + kMaxFp64Classes;
 constexpr int kCtrTaskScaled = kMaxBuckets + 2 * kMaxFp64Classes;
 constexpr int kCtrTaskExt = kMaxBuckets + 3 * kMaxFp64Classes;
 constexpr int kCtrTotal = kMaxBuckets + 4 * kMaxFp64Classes;
-// pairs up to which the FP64 lists are not sorted by haplotype length: at most two
-// rounds of resident warps, so the order decides little and the three launches of the
-// sort are a third of the stage of a small batch
-constexpr int64_t kNoSortPairs = 4096;
+// FP64 groups, in warps, up to which the lists are not sorted by haplotype length: at most
+// a few rounds of resident warps, so the order decides little and the three launches of
+// the sort are a third of the stage of a small batch.  Unsorted / sorted: one uneven region
+// 175 / 189 us, one long-read region (64 pairs on 8 warps each) 2.49 / 2.52 ms, 64 long-read
+// regions (4,096 pairs on 4 warps each) 21.3 / 20.5 ms.
+constexpr int64_t kNoSortWarps = 4096;
 // Batches of more pairs or length classes than this, or whose launches have not been the
 // same for a while, are launched kernel by kernel (see run_pipeline).
 constexpr int64_t kGraphMaxPairs = 4096;
@@ -933,7 +941,7 @@ pairhmm_status_t Engine::enqueue_pipeline(const pairhmm_batch_t& in, const Batch
     // FP64 pass: first sort each class's list by haplotype length into the
     // work-item buffer (free once the FP32 stage is done), same class offsets
     const int64_t upper = x.num_pairs;  // pairs the FP64 lists could hold
-    const bool sorted = upper > kNoSortPairs;
+    const bool sorted = fp64_warps(x) > kNoSortWarps;
     Task* const fp64_lists = sorted ? items_.as<Task>() : rescue_.as<Task>();
     if (stage == 2 && sorted) {
         RescueSortArgs ra{};
@@ -1146,9 +1154,17 @@ Engine::Plan Engine::make_plan(const BatchIndex& x) const {
     return p;
 }
 
+// Warps of the FP64 groups that the batch's pairs could take, a narrower group counting as one.
+int64_t Engine::fp64_warps(const BatchIndex& x) const {
+    int64_t warps = 0;
+    for (size_t c = 0; c < fp64_->classes.size(); ++c)
+        warps += x.class_pairs[c] * std::max(fp64_->classes[c].scaled->G / 32, 1);
+    return warps;
+}
+
 // What decides a batch's launches and their dependencies (not their arguments).
 std::vector<uint8_t> Engine::launch_shape(const BatchIndex& x, const Plan& plan) const {
-    std::vector<uint8_t> shape = {(uint8_t)(table_ == &tables_[1]), (uint8_t)(x.num_pairs > kNoSortPairs),
+    std::vector<uint8_t> shape = {(uint8_t)(table_ == &tables_[1]), (uint8_t)(fp64_warps(x) > kNoSortWarps),
                                   (uint8_t)plan.side[1], (uint8_t)plan.side[2]};
     for (const int64_t n : x.bucket_items) shape.push_back(n != 0);
     for (const int64_t n : x.class_pairs) shape.push_back(n != 0);

@@ -164,6 +164,7 @@ private:
         size_t scratch_bytes = 0;
     };
     Plan make_plan(const BatchIndex& idx) const;
+    int64_t fp64_warps(const BatchIndex& x) const;
     std::vector<uint8_t> launch_shape(const BatchIndex& x, const Plan& plan) const;
     // stage 0: packing + work list, 1: FP32 launches, 2: FP64 pass
     pairhmm_status_t enqueue_pipeline(const pairhmm_batch_t& dev_in, const BatchIndex& idx, const Plan& plan,

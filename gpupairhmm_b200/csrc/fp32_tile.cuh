@@ -10,7 +10,10 @@ namespace phmm {
 // Resident blocks per SM asked of the register allocator.  One-warp groups run in
 // 64-thread blocks: the paths with per-position w and x hold 8R + ~50 registers a
 // lane (packed), so up to R = 10 six blocks fit 168 registers and beyond that four
-// blocks; the shared tables (2.5 KB a warp and position pair) allow as many.
+// blocks (182-255 registers allocated at R = 11-20, the one-gap-quality path's too: both
+// paths are one kernel).  The shared tables, 2.5 KB a warp and position pair, are 51 KB a
+// block at R = 19-20, where four blocks fit whatever the registers are.  Blocks of 8 warps
+// spill 4-60 bytes at R = 8-16.
 // Scalar groups hold 4R + ~60: serial parts take eight blocks up to R = 14 and six up
 // to R = 24 (168 registers), block groups 16 warps.
 template <class V, int R, int W, bool SERIAL>

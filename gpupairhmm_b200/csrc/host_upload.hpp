@@ -1,7 +1,8 @@
 // Host-to-device upload of caller buffers for one batch.
 //
 // Page-locked sources (cudaMallocHost / cudaHostAlloc / cudaHostRegister) are
-// copied by DMA straight from the caller's memory.  Pageable sources go
+// copied by DMA straight from the caller's memory, but for jobs small enough to be
+// gathered (gather, below), whose sources the calling thread copies whatever they are.  Pageable sources go
 // through a ring of page-locked staging slots: several host threads each copy
 // a slot's worth out of the caller's memory and enqueue that slot's DMA, then
 // reuse the slot once its DMA has completed, so the host copies run in

@@ -54,7 +54,9 @@ void ServingQueue::stats(pairhmm_serving_stats_t* out) {
 
 int64_t ServingQueue::estimate_device_bytes(const Region& r) {
     // inputs (4 byte arrays + haplotypes), packed copies, work items, rescue
-    // list and scores, plus the per-read/per-haplotype index arrays
+    // list and scores, plus the per-read/per-haplotype index arrays.  Not the border
+    // scratch of long reads, which the resident warps set, not the regions: up to 0.2 GB
+    // a length class at haplotypes of 5,000, 4 GiB in all
     int64_t pos = 0, hb = 0;
     for (int64_t i = 0; i < r.reads; ++i) pos += (r.read_len()[i] + 3) & ~3;
     for (int64_t h = 0; h < r.haps; ++h) hb += (r.hap_len()[h] + 15) & ~15;

@@ -9,10 +9,10 @@
 // is already admitting, uploading and launching, so the work of regions that
 // arrive while others are on the device overlaps with them.
 //
-// Regions with reads longer than the largest single tile (multi-tile work,
-// whose pairs each take a long serial wavefront) queue separately and run on
-// their own two slots, so that a batch of short regions never waits behind
-// them and a long region waits for at most one batch of long ones.
+// Regions with reads of more than 1,024 positions (multi-tile work, whose pairs each take
+// a long serial wavefront) queue separately and run on their own two slots, so
+// that a batch of short regions is not merged or queued behind them (it still shares the
+// SMs with them) and a long region waits for at most one batch of long ones.
 #pragma once
 
 #include <algorithm>

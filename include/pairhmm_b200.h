@@ -91,7 +91,7 @@ typedef struct pairhmm_batch {
 /* Execution forms. */
 enum {
     /* Persistent, length-bucketed, H-sorted work queue; tuned tile per bucket;
-     * CUDA-graph launched; FP64 rescue of FP32 underflows. */
+     * FP64 rescue of FP32 underflows. */
     PAIRHMM_MODE_ENGINE = 0,
     /* One launch per read-length partition with the reference's generic tile
      * table (tuningconfigs.hpp:33-57), no sorting, FP32 only.  Kept as the
@@ -102,8 +102,12 @@ enum {
 typedef struct pairhmm_options {
     int32_t device;       /* CUDA ordinal, default 0 */
     int32_t mode;         /* PAIRHMM_MODE_* */
-    int32_t fp64_rescue;  /* 1 (default): recompute FP32 underflows in FP64 */
-    int32_t use_graphs;   /* 1 (default): replay the per-batch launch sequence as a CUDA graph */
+    int32_t fp64_rescue;  /* 1 (default): recompute FP32 underflows in FP64; 0: scores are what
+                             single precision gives (pairs that it cannot compute at all, for
+                             ins+del qualities of about 3 or an overflow, still go to FP64) */
+    int32_t use_graphs;   /* 1 (default): batches of up to 4,096 pairs and 6 length classes whose
+                             launches have been the same for eight batches go as one CUDA graph;
+                             0: always launch kernel by kernel */
     int64_t device_budget_bytes; /* serving admission budget; 0 = 40 GiB */
     int32_t pipeline_chunks; /* compute_host: 0 (default) = batches of 2M+ pairs run as up to
                                 8 chunks of at least 1M pairs whose uploads overlap the previous
@@ -200,13 +204,16 @@ pairhmm_status_t pairhmm_serving_stats(pairhmm_engine_t* engine, pairhmm_serving
  * kind[i] (the `multi_tile` argument): 0 = one tile, 1 = several tiles
  * (reads longer than the tile), 2 = one tile with two reads of a record per
  * group in packed FP32 arithmetic, 3 = the same with exact tiles (the class must
- * lie within (group*(regs-1), group*regs]), 4 = exact tiles over a block of
- * group/32 warps, one read per group.  This is the run-time form of the
+ * lie within (group*(regs-1), group*regs]), 4 = exact tiles of more than 32 lanes,
+ * one read per group: 64 or 96 lanes are one warp with two or three parts in turn,
+ * 256 a block of 8 warps.  This is the run-time form of the
  * reference's compile-time tuning tables (tuningconfigs.hpp:33-269) and of its
  * partition rule "first tile size >= read length" (utility_kernels.cuh:45-57).
  * Only compiled (group, regs, kind) triples are accepted; the last entry must
  * be of kind 1.  The default table has a twin for batches of few pairs, which
- * pairhmm_get_tile_table does not list; results are the same with either.
+ * pairhmm_get_tile_table does not list; results are the same with either.  Engines
+ * with fp64_rescue = 0 have a default table of padded tiles, whose range in single
+ * precision reaches further down.
  */
 pairhmm_status_t pairhmm_set_tile_table(pairhmm_engine_t* engine, const int32_t* max_len, const int32_t* group,
                                         const int32_t* regs, const int32_t* multi_tile, int32_t n);
@@ -266,13 +273,15 @@ void pairhmm_set_host_threads(int32_t threads);
  * with the same meaning as in pairhmm_batch_t, `pairs` a flat list (offsets
  * into those arrays and lengths), `scores` one float per pair.  Work is
  * ordered on `stream` (a cudaStream_t, NULL = legacy default); the call does
- * not wait for it.  Nothing is allocated: the kernel's only scratch (borders
- * between 512-position read tiles) is a 64 MiB statically allocated device
+ * not wait for it.  Nothing is allocated: the kernels' only scratch (borders
+ * between the parts of a long read) is a 64 MiB statically allocated device
  * array that every GPU loading the library keeps until exit.  Limits:
  * max_hap_length in [1, 16384] (above: PAIRHMM_ERR_LIMIT, nothing launched)
  * and every pair's hap_length <= max_hap_length (a longer pair, or an empty
  * read or haplotype, gets NaN); any read length.  FP32 only: pairs whose FP32
- * result underflows are not recomputed in FP64.  The first call on a device
+ * result underflows are not recomputed in FP64 (a pair near the end of the range is
+ * computed once more in a form whose range reaches further down; a list of mostly such
+ * pairs takes both).  The first call on a device
  * sets it up (the scratch array's device address, the grid size); make that
  * first call before any stream capture.  Every call checks the address
  * against a fresh symbol lookup, so the entry point stays valid after the

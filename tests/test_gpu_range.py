@@ -66,3 +66,15 @@ def test_gcp_threshold_counts_the_reads_own_beta(quality):
         got = e.compute(batch)
         assert e.stats().rescued >= below.sum()
     assert_log10_close(got, want)
+
+
+@pytest.mark.parametrize("few", [True, False])
+def test_long_reads_are_counted_beyond_the_same_length(few):
+    """LONG_READ is where the engine's tables begin to count pairs as multi-tile, on the table
+    for few pairs and on the one for many."""
+    batch = ladder(4, [640, 641, g.LONG_READ - 1, g.LONG_READ, g.LONG_READ + 1, 1500], 40,
+                   rates=(0.0, 0.02), reads=4 if few else 1200, haps=1 if few else 2)
+    L, _ = pair_lengths(batch)
+    with g.Engine() as e:
+        e.compute(batch)
+        assert e.stats().multi_tile_pairs == (L > g.LONG_READ).sum()
