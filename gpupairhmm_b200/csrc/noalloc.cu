@@ -13,19 +13,20 @@
 // takes a few consecutive pairs of the list at a time and runs those of one shape
 // together on the exact tiles of wavefront_tile.cuh: 8 lanes a pair up to 160
 // positions, 16 up to 320, then 32 lanes with the read's parts in turn.  Few pairs
-// take a general form, the whole warp, 4 to 16 positions a lane by the read's length,
-// longer reads in tiles of 512: reads of at most 8 positions, and, once more, pairs whose sum on the tiles is too small for
-// their range (there is no FP64 pass behind this entry point, and the general form's
-// range reaches further down).  24,600 pairs of 70-250 x 120-650 positions take 1.16 ms, against 4.0 ms with
+// take a general form in a second launch, the whole warp, 4 to 16 positions a lane by
+// the read's length, longer reads in tiles of 512: reads of at most 8 positions, and,
+// once more, pairs whose sum on the tiles is too small for their range (there is no
+// FP64 pass behind this entry point, and the general form's range reaches further
+// down).  24,600 pairs of 70-250 x 120-650 positions take 1.09 ms, against 4.0 ms with
 // the general form for all (one pair on 512 positions a warp, eleven operations a
 // cell); what bounds it is the instruction cache (several shapes in flight) and the
 // last pairs of a short list.
 // The only scratch, the per-warp border between a read's parts, lives in
 // kScratchBytes of statically allocated device memory defined below: every GPU
-// that loads this library holds that much memory until the process exits.  Limits: haplotype length
-// up to kMaxHapLength; any read length.  Results are FP32 only, with no FP64
-// recompute of pairs whose FP32 result underflows (those return what FP32
-// gives, possibly -inf, as the reference does).
+// that loads this library holds that much memory until the process exits (the work
+// queues take 8 KB more).  Limits: haplotype length up to kMaxHapLength; any read
+// length.  Results are FP32 only, with no FP64 recompute of pairs whose FP32 result
+// underflows (those return what FP32 gives, possibly -inf, as the reference does).
 //
 // Every call shares the one scratch array and it keeps the last call's
 // contents.  Nothing in it has to start at zero: within a pair each border row
@@ -477,8 +478,6 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
         if (warps > num_pairs) warps = num_pairs;
         const int64_t warps_per_block = kThreads / 32;
         const int grid = (int)((warps + warps_per_block - 1) / warps_per_block);
-        // cudaLaunchKernel returns this launch's own status, so an error the caller
-        // left pending is neither reported as ours nor cleared
         // pairs a warp takes at a time: a few, so that those of one read's haplotypes run
         // together, but at least four times per warp, so that the last ones end together
         int grab = (int)(num_pairs / (4 * warps));
@@ -488,6 +487,8 @@ extern "C" pairhmm_status_t pairhmm_forward_pairs_noalloc(
         Args ka{read_bases, base_quals, ins_quals, del_quals, hap_bases, pairs, num_pairs, scores,
                 scratch,    rows,       warps,     max_hap_length, grab, look, st.calls.fetch_add(1) % kQueues};
         void *args[] = {&ka}, *queue[] = {&ka.queue};
+        // cudaLaunchKernel returns this launch's own status, so an error the caller
+        // left pending is neither reported as ours nor cleared
         cudaError_t le = cudaLaunchKernel(reinterpret_cast<const void*>(&clear_queue_kernel), dim3(1), dim3(1), queue,
                                           0, static_cast<cudaStream_t>(stream));
         if (le == cudaSuccess)
